@@ -524,14 +524,8 @@ static jsm_status linear(jsm_decoder* m, const Proj& p, const void* X, long long
         r.chained = true;
         return linear_bf16_launch(r, st);
     }
-    for (int t0 = 0; t0 < T; t0 += 256) {
-        a.T = std::min(256, T - t0);
-        a.X = static_cast<const __nv_bfloat16*>(X) + (long long)t0 * x_stride;
-        a.Y = out_f32 ? static_cast<void*>(static_cast<float*>(Y) + (long long)t0 * p.N)
-                      : static_cast<void*>(static_cast<__nv_bfloat16*>(Y) + (long long)t0 * p.N);
-        DEC_TRY(linear_packed_launch(a, st));
-    }
-    return JSM_OK;
+    a.T = T; a.X = X; a.Y = Y;
+    return linear_packed_tokens(a, st);
 }
 
 // ---- one pass -----------------------------------------------------------------------------------------------------

@@ -35,7 +35,7 @@ struct PackedArgs {
     const void* R;            // [T, N] bf16 residual or null
     void* Y;                  // [T, N] bf16 or f32
     bool out_f32 = false;
-    int T = 0, N = 0, K = 0;  // T <= 256 per launch
+    int T = 0, N = 0, K = 0;
     long long x_row_stride = 0;
     float* ws = nullptr;      // fp32 partials of the tiles shared between CTAs (linear_packed_ws_floats)
     size_t ws_floats = 0;
@@ -105,7 +105,10 @@ size_t linear_packed_bytes(int N, int K, int paired);
 size_t linear_packed_ws_floats(int T, int N, int K, int paired);
 // packs (or, with unpack, rebuilds) a row-major [N, K] matrix ([2N, K] gate rows then up rows when paired)
 jsm_status linear_pack_launch(const void* W, int N, int K, int paired, void* packed, bool unpack, cudaStream_t st);
-jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st);
+jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st);  // T <= 256
+// any T; the launches of a call that is split share R, Y and the row statistics of the whole call
+jsm_status linear_packed_tokens(const PackedArgs& a, cudaStream_t st);
+jsm_status linear_tiled_launch(const PackedArgs& a, cudaStream_t st);
 // exchange regions (tp_comm.cu): [flags | buffer A | buffer B | push buffer 0 | push buffer 1]
 size_t tp_region_bytes(int max_tokens, int d);
 size_t tp_buffer_offset(int which, int max_tokens, int d);

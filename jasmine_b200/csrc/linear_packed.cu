@@ -24,6 +24,7 @@
 // requested (and more is prefetched into L2) before griddepcontrol.wait; X, R, Y and the workspace come after it.
 #include "tc_utils.cuh"
 #include "linear_bf16.cuh"
+#include "linear_epilogue.cuh"
 #include <math.h>
 #include <mutex>
 #include <algorithm>
@@ -36,21 +37,6 @@ using namespace tc;
 constexpr int PK_TILE_BYTES = 128 * 64 * 2;  // one packed unit: 128 rows x 64 k, bf16
 constexpr int PK_THREADS = 224;
 constexpr int PK_MAX_STAGES = 12;
-
-__device__ __noinline__ float pk_gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752440f)); }
-__device__ __forceinline__ float pk_silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }  // 2 ulp division: short code
-// gate/up pair with clamps: min(g, limit) * sigmoid(alpha * min(g, limit)) * (clamp(u, -limit, limit) + 1)
-__device__ __forceinline__ float pk_clamped_glu(float g, float u, float alpha, float limit) {
-    g = fminf(g, limit);
-    u = fminf(fmaxf(u, -limit), limit);
-    return __fdividef(g, 1.0f + __expf(-alpha * g)) * (u + 1.0f);
-}
-
-// gate/up pair with the tanh form of GELU: z (1 + tanh(y)) / 2 = z / (1 + e^(-2y)), y = sqrt(2/pi) (z + 0.044715 z^3)
-__device__ __forceinline__ float pk_gelu_glu(float z, float u) {
-    const float y2 = 1.5957691216057308f * fmaf(0.044715f * z * z, z, z);
-    return __fdividef(z, 1.0f + __expf(-y2)) * u;
-}
 
 __device__ __forceinline__ void bulk_prefetch_l2(const void* gsrc, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes) : "memory");
@@ -1128,21 +1114,81 @@ static jsm_status launch_packed(const CUtensorMap& mx, const CUtensorMap& mx2, P
     return JSM_OK;
 }
 
-jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st) {
-    if (a.T <= 0 || a.N <= 0) return JSM_OK;
-    const bool tp_push = a.tp && a.tp->push, tp_reduce = a.tp && a.tp->reduce;
+// What a launch takes, whichever kernel runs it.  The workspace is asked for by the streaming kernel only, but a call is accepted
+// or refused by its shape alone, not by the kernel that its token count selects (T: tokens of one launch of that kernel).
+static jsm_status packed_check(const PackedArgs& a, int T, int paired) {
+    const bool tp_push = a.tp && a.tp->push;
     if (!a.X || !a.Wp || (!a.Y && !tp_push)) JSM_FAIL(JSM_INVALID_ARG, "linear_packed: null pointer");
     if (a.K <= 0 || a.K % 8) JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: K (%d) must be a positive multiple of 8", a.K);
     if (a.N % 4) JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: N (%d) must be a multiple of 4", a.N);
-    if (a.T > 256) JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: at most 256 tokens per launch (%d)", a.T);
     if (a.epilogue < LIN_NONE || a.epilogue > LIN_GELU_GLU) JSM_FAIL(JSM_INVALID_ARG, "linear_packed: epilogue %d", a.epilogue);
     const bool glu = a.epilogue == LIN_CLAMPED_GLU || a.epilogue == LIN_GELU_GLU;
-    const int paired = a.epilogue == LIN_SILU_MUL || glu ? 1 : 0;
     if (glu && (a.out_f32 || a.ssq_in || a.tp))
         JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: the clamped and GELU gate/up projections write bf16, without a fused norm or exchange");
     if (paired && a.bias) JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: the gate/up projection takes no bias");
     if (a.epilogue == LIN_RESIDUAL && !a.R) JSM_FAIL(JSM_INVALID_ARG, "linear_packed: residual epilogue without R");
     if (a.bias && (reinterpret_cast<uintptr_t>(a.bias) & 15)) JSM_FAIL(JSM_INVALID_ARG, "linear_packed: bias must be 16-byte aligned");
+    int nt, kbt;
+    pk_dims(a.N, a.K, paired, &nt, &kbt);
+    const int grid = linear_packed_grid(a.N, a.K, paired, T);
+    const long long U = (long long)nt * kbt;
+    if ((U + 1) * ((long long)grid + 1) >= (1ll << 31))  // the kernel partitions the units in 32-bit arithmetic
+        JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: %lld units of work on %d CTAs exceed one launch (a packed matrix of tens of gigabytes)", U, grid);
+    const bool shared_tiles = (U % grid) != 0 || ((U / grid) % kbt) != 0;
+    if (shared_tiles) {
+        if (!a.ws || !a.counters)
+            JSM_FAIL(JSM_INVALID_ARG, "linear_packed: no workspace on this device (jsm_linear_pack / jsm_linear_packed_reserve size it at set-up time)");
+        if ((size_t)nt * linear_packed_slots(a.N, a.K, paired, T) * (size_t)T * 128 > a.ws_floats)
+            JSM_FAIL(JSM_INVALID_ARG, "linear_packed: workspace of %zu floats, %zu needed", a.ws_floats, linear_packed_ws_floats(T, a.N, a.K, paired));
+        if (nt > a.n_counters) JSM_FAIL(JSM_INVALID_ARG, "linear_packed: %d tile counters, %d needed", a.n_counters, nt);
+    }
+    if (a.ssq_out && (paired || a.out_f32)) JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: row statistics are written for plain bf16 outputs only");
+    if (a.ssq_in && a.ssq_in_tiles <= 0) JSM_FAIL(JSM_INVALID_ARG, "linear_packed: row statistics without their tile count");
+    return JSM_OK;
+}
+
+static int packed_paired(const PackedArgs& a) {
+    return a.epilogue == LIN_SILU_MUL || a.epilogue == LIN_CLAMPED_GLU || a.epilogue == LIN_GELU_GLU ? 1 : 0;
+}
+
+// Which kernel takes a call of T tokens over a depth of K.  Measured (us, streaming / tiled): T = 256: 28 / 17 at 4096 x 4096, 43 / 37 at
+// 4096 x 11008, 41 / 9 at 2048 x 2048 (f32 out).  T = 100: 24 / 9 at 2048 x 2048 and 12 / 7 at 4096 x 576, but 16 / 17 at 4096 x 4096
+// and 26 / 36 at 4096 x 11008: up to 128 tokens a deep matrix gains more from the streaming kernel's split along K.
+static bool use_tiled(int T, int K) { return T > 128 || (T > 64 && K < 4096); }
+
+// Any number of tokens, in one launch of the tiled kernel (linear_tiled.cu) or launches of at most 256 tokens.
+jsm_status linear_packed_tokens(const PackedArgs& a, cudaStream_t st) {
+    if (a.T <= 0 || a.N <= 0) return JSM_OK;
+    if (use_tiled(a.T, a.K) && !a.tp) {
+        jsm_status s = packed_check(a, std::min(a.T, 256), packed_paired(a));
+        return s != JSM_OK ? s : linear_tiled_launch(a, st);
+    }
+    PackedArgs c = a;
+    const long long xs = a.x_row_stride > 0 ? a.x_row_stride : a.K;
+    if (a.ssq_stride <= 0) c.ssq_stride = a.T;
+    for (int t0 = 0; t0 < a.T; t0 += 256) {
+        c.T = std::min(256, a.T - t0);
+        c.X = static_cast<const __nv_bfloat16*>(a.X) + t0 * xs;
+        c.R = a.R ? static_cast<const __nv_bfloat16*>(a.R) + (size_t)t0 * a.N : nullptr;
+        if (a.Y)
+            c.Y = a.out_f32 ? static_cast<void*>(static_cast<float*>(a.Y) + (size_t)t0 * a.N)
+                            : static_cast<void*>(static_cast<__nv_bfloat16*>(a.Y) + (size_t)t0 * a.N);
+        c.ssq_in = a.ssq_in ? a.ssq_in + t0 : nullptr;
+        c.ssq_out = a.ssq_out ? a.ssq_out + t0 : nullptr;
+        jsm_status s = linear_packed_launch(c, st);
+        if (s != JSM_OK) return s;
+    }
+    return JSM_OK;
+}
+
+jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st) {
+    if (a.T <= 0 || a.N <= 0) return JSM_OK;
+    const bool tp_push = a.tp && a.tp->push, tp_reduce = a.tp && a.tp->reduce;
+    if (a.T > 256) JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: at most 256 tokens per launch (%d)", a.T);
+    const bool glu = a.epilogue == LIN_CLAMPED_GLU || a.epilogue == LIN_GELU_GLU;
+    const int paired = packed_paired(a);
+    jsm_status s = packed_check(a, a.T, paired);
+    if (s != JSM_OK) return s;
     PkParams P;
     P.T = a.T; P.N = a.N; P.K = a.K;
     pk_dims(a.N, a.K, paired, &P.n_tiles, &P.kbt);
@@ -1152,27 +1198,13 @@ jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st) {
     P.bias = a.bias; P.R = (const __nv_bfloat16*)a.R; P.Y = a.Y; P.Wp = (const uint8_t*)a.Wp;
     const int grid = linear_packed_grid(a.N, a.K, paired, a.T);
     P.max_slots = linear_packed_slots(a.N, a.K, paired, a.T);
-    const long long U = (long long)P.n_tiles * P.kbt;
-    if ((U + 1) * ((long long)grid + 1) >= (1ll << 31))  // the kernel partitions the units in 32-bit arithmetic
-        JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: %lld units of work on %d CTAs exceed one launch (a packed matrix of tens of gigabytes)", U, grid);
-    const bool shared_tiles = (U % grid) != 0 || ((U / grid) % P.kbt) != 0;
-    if (shared_tiles) {
-        if (!a.ws || !a.counters)
-            JSM_FAIL(JSM_INVALID_ARG, "linear_packed: no workspace on this device (jsm_linear_pack / jsm_linear_packed_reserve size it at set-up time)");
-        if ((size_t)P.n_tiles * P.max_slots * (size_t)a.T * 128 > a.ws_floats)
-            JSM_FAIL(JSM_INVALID_ARG, "linear_packed: workspace of %zu floats, %zu needed", a.ws_floats,
-                     linear_packed_ws_floats(a.T, a.N, a.K, paired));
-        if (P.n_tiles > a.n_counters) JSM_FAIL(JSM_INVALID_ARG, "linear_packed: %d tile counters, %d needed", a.n_counters, P.n_tiles);
-    }
     P.ws = a.ws; P.counters = a.counters;
     P.err = tc_error_word();
-    if (a.ssq_out && (paired || a.out_f32)) JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: row statistics are written for plain bf16 outputs only");
-    if (a.ssq_in && (a.ssq_in_tiles <= 0 || a.K <= 0)) JSM_FAIL(JSM_INVALID_ARG, "linear_packed: row statistics without their tile count");
     P.ssq_in = a.ssq_in; P.ssq_in_tiles = a.ssq_in_tiles; P.ssq_stride = a.ssq_stride > 0 ? a.ssq_stride : a.T;
     P.inv_d = 1.0f / (float)a.K; P.eps = a.eps; P.ssq_out = a.ssq_out;
     const int bn = a.T <= 16 ? 16 : a.T <= 32 ? 32 : a.T <= 64 ? 64 : a.T <= 128 ? 128 : 256;
     CUtensorMap mx;
-    jsm_status s = make_tmap_bf16_2d(&mx, a.X, (uint64_t)a.T, (uint64_t)a.K, (uint64_t)(a.x_row_stride > 0 ? a.x_row_stride : a.K), bn, 64);
+    s = make_tmap_bf16_2d(&mx, a.X, (uint64_t)a.T, (uint64_t)a.K, (uint64_t)(a.x_row_stride > 0 ? a.x_row_stride : a.K), bn, 64);
     if (s != JSM_OK) return s;
     // the same matrix as [k-block][row][64]: a box two k-blocks deep lands as two consecutive swizzled X blocks
     const long long xs = a.x_row_stride > 0 ? a.x_row_stride : a.K;
@@ -1432,18 +1464,8 @@ static jsm_status linear_bf16_packed_entry(const void* d_X, const void* d_packed
         const PkWorkspace& w = g_pk_ws[dev];
         a.ws = w.ws; a.ws_floats = w.ws_floats; a.counters = w.counters; a.n_counters = w.n_counters;
     }
-    // more than 256 tokens: token chunks, each streaming the weights once
-    for (int t0 = 0; t0 < T; t0 += 256) {
-        const int tc = T - t0 < 256 ? T - t0 : 256;
-        a.T = tc;
-        a.X = reinterpret_cast<const __nv_bfloat16*>(d_X) + (size_t)t0 * K;
-        a.R = d_R ? reinterpret_cast<const __nv_bfloat16*>(d_R) + (size_t)t0 * N : nullptr;
-        a.Y = a.out_f32 ? static_cast<void*>(reinterpret_cast<float*>(d_Y) + (size_t)t0 * N)
-                        : static_cast<void*>(reinterpret_cast<__nv_bfloat16*>(d_Y) + (size_t)t0 * N);
-        jsm_status s = linear_packed_launch(a, st);
-        if (s != JSM_OK) return s;
-    }
-    return JSM_OK;
+    a.T = T; a.X = d_X; a.R = d_R; a.Y = d_Y;
+    return linear_packed_tokens(a, st);
 }
 
 extern "C" jsm_status jsm_linear_bf16_packed(const void* d_X, const void* d_packed, const float* d_bias, int epilogue, const void* d_R,

@@ -466,7 +466,7 @@ struct RowStats {
     float* out = nullptr;       // [ceil(N/128)][T] sums of squares of the outputs
 };
 
-// One projection over packed weights for any number of tokens: chunks of 256 tokens, each streaming the weights once.
+// One projection over packed weights for any number of tokens.
 static jsm_status run_linear(jsm_model* m, const __nv_bfloat16* X, long long x_stride, const uint8_t* Wp, int N, int K, int epilogue,
                              const __nv_bfloat16* R, void* Y, bool out_f32, int T, cudaStream_t st, RowStats rs = RowStats(),
                              int stats_stride = 0, const TpFuse* tp = nullptr) {
@@ -478,18 +478,9 @@ static jsm_status run_linear(jsm_model* m, const __nv_bfloat16* X, long long x_s
     a.ssq_in_tiles = rs.in_tiles;
     a.ssq_stride = stats_stride > 0 ? stats_stride : T;
     a.tp = tp;  // fused exchanges come with at most TP_PUSH_MAX_T tokens: one chunk
-    for (int t0 = 0; t0 < T; t0 += 256) {
-        a.T = T - t0 < 256 ? T - t0 : 256;
-        a.X = X + (long long)t0 * x_stride;
-        a.R = R ? R + (long long)t0 * N : nullptr;
-        a.Y = out_f32 ? static_cast<void*>(reinterpret_cast<float*>(Y) + (long long)t0 * N)
-                      : static_cast<void*>(reinterpret_cast<__nv_bfloat16*>(Y) + (long long)t0 * N);
-        a.ssq_in = rs.in ? rs.in + t0 : nullptr;
-        a.ssq_out = rs.out ? rs.out + t0 : nullptr;
-        jsm_status s = linear_packed_launch(a, st);
-        if (s != JSM_OK) return s;
-    }
-    return JSM_OK;
+    a.T = T; a.X = X; a.R = R; a.Y = Y;
+    a.ssq_in = rs.in; a.ssq_out = rs.out;
+    return linear_packed_tokens(a, st);
 }
 
 // h += X . W^T (the residual stream).  One GPU: the projection adds into h in its epilogue and leaves the row

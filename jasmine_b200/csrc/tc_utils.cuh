@@ -57,6 +57,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
 }
 
+// One lane of a converged warp, chosen so that the compiler knows that it is one.  The tensor-core and copy instructions take their
+// operands from uniform registers: issued under `if (lane == 0)` every one of them costs about 185 cycles (a loop over the lanes
+// that might be active), under elect_one() in warp-uniform code a handful.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred P;\nelect.sync _|P, 0xffffffff;\nselp.u32 %0, 1, 0, P;\n}\n" : "=r"(p));
+    return p != 0;
+}
+// mbar_wait of a whole converged warp: the same answer in every lane
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* err_word, int code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, err_word, code));
+}
+
 // 1-D bulk copy global -> shared (this CTA), completion counted in bytes on `bar`; both addresses 16-byte aligned
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem_dst)),
