@@ -166,13 +166,19 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
     const uint32_t tmem_base = tmem_base_smem;
     const uint32_t S_COL[2] = {0, 128}, O_COL[2] = {256, 256 + VD};
 
+    // (warps 0 and 1 run converged, one elected lane issues: see elect_one)
     if (warp == 0) {
-        if (lane == 0) {
+        {
             // Q: both tiles, in slabs of 64 columns
-            mbar_expect_tx(&q_full, 2 * QK_BYTES);
-            for (int t = 0; t < 2; ++t)
-                for (int c = 0; c < QKD / 64; ++c)
-                    tma_load_2d(q_smem + t * QK_BYTES + c * FA_SLAB, &tmap_q, h * P.q_hs + c * 64, b * P.Tq + q0 + t * FA_BM, &q_full);
+            if (elect_one()) {
+                mbar_expect_tx(&q_full, 2 * QK_BYTES);
+#pragma unroll
+                for (int t = 0; t < 2; ++t)
+#pragma unroll
+                    for (int c = 0; c < QKD / 64; ++c)
+                        tma_load_2d(q_smem + t * QK_BYTES + c * FA_SLAB, &tmap_q, h * P.q_hs + c * 64, b * P.Tq + q0 + t * FA_BM, &q_full);
+            }
+            __syncwarp();
             int k_issued = 0, v_issued = 0;
             // paged: 64 columns of a key tile are a slab of two pages (a tile's second half behind the last page repeats it: masked)
             auto slab = [&](uint8_t* dst, int j, int c, uint64_t* bar) {
@@ -184,17 +190,25 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
             };
             for (int j = j_lo; j < n_max; ++j) {
                 const int i = j - j_lo, ks = i % KST, vs = i % VST;
-                if (i >= KST && !mbar_wait(&k_empty[ks], ((i / KST) & 1) ^ 1, &abort_flag, P.err, TC_TIMEOUT_EMPTY)) break;
-                mbar_expect_tx(&k_full[ks], QK_BYTES);
-                for (int c = 0; c < QKD / 64; ++c)
-                    if (PAGED) slab(k_smem + ks * QK_BYTES + c * FA_SLAB, j, c, &k_full[ks]);
-                    else tma_load_2d(k_smem + ks * QK_BYTES + c * FA_SLAB, &tmap_k, hk * QKD + c * 64, b * P.Tk + j * FA_BN, &k_full[ks]);
+                if (i >= KST && !mbar_wait_warp(&k_empty[ks], ((i / KST) & 1) ^ 1, &abort_flag, P.err, TC_TIMEOUT_EMPTY)) break;
+                if (elect_one()) {
+                    mbar_expect_tx(&k_full[ks], QK_BYTES);
+#pragma unroll
+                    for (int c = 0; c < QKD / 64; ++c)
+                        if (PAGED) slab(k_smem + ks * QK_BYTES + c * FA_SLAB, j, c, &k_full[ks]);
+                        else tma_load_2d(k_smem + ks * QK_BYTES + c * FA_SLAB, &tmap_k, hk * QKD + c * 64, b * P.Tk + j * FA_BN, &k_full[ks]);
+                }
+                __syncwarp();
                 k_issued = i + 1;
-                if (i >= VST && !mbar_wait(&v_empty[vs], ((i / VST) & 1) ^ 1, &abort_flag, P.err, TC_TIMEOUT_EMPTY)) break;
-                mbar_expect_tx(&v_full[vs], V_BYTES);
-                for (int c = 0; c < VD / 64; ++c)
-                    if (PAGED) slab(v_smem + vs * V_BYTES + c * FA_SLAB, j, QKD / 64 + c, &v_full[vs]);
-                    else tma_load_2d(v_smem + vs * V_BYTES + c * FA_SLAB, &tmap_v, hk * VD + c * 64, b * P.Tk + j * FA_BN, &v_full[vs]);
+                if (i >= VST && !mbar_wait_warp(&v_empty[vs], ((i / VST) & 1) ^ 1, &abort_flag, P.err, TC_TIMEOUT_EMPTY)) break;
+                if (elect_one()) {
+                    mbar_expect_tx(&v_full[vs], V_BYTES);
+#pragma unroll
+                    for (int c = 0; c < VD / 64; ++c)
+                        if (PAGED) slab(v_smem + vs * V_BYTES + c * FA_SLAB, j, QKD / 64 + c, &v_full[vs]);
+                        else tma_load_2d(v_smem + vs * V_BYTES + c * FA_SLAB, &tmap_v, hk * VD + c * 64, b * P.Tk + j * FA_BN, &v_full[vs]);
+                }
+                __syncwarp();
                 v_issued = i + 1;
             }
             if (abort_flag) {  // let the copies in flight land before the CTA exits (bounded)
@@ -207,66 +221,77 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc_qk = instr_desc_bf16(FA_BM, FA_BN, 0, 0);  // both operands K-major (head_dim contiguous)
             constexpr uint32_t idesc_pv = instr_desc_bf16(FA_BM, VD, 0, 1);   // V is N-contiguous: MN-major B
-            bool ok = mbar_wait(&q_full, 0, &abort_flag, P.err, TC_TIMEOUT_FULL);
+            bool ok = mbar_wait_warp(&q_full, 0, &abort_flag, P.err, TC_TIMEOUT_FULL);
             // S_t(j) = Q_t . K(j)^T into the S columns of tile t (overwrites P_t(j-1): the tensor pipe runs the MMAs of
             // this thread in issue order, so the P.V product issued before it has read P by then)
             auto issue_s = [&](int t, uint32_t k_addr) {
                 const uint32_t q_addr = smem_u32(q_smem + t * QK_BYTES);
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < QKD / 16; ++kk) {
-                    const uint32_t off = (kk / 4) * FA_SLAB;
-                    mma_ss(tmem_base + S_COL[t], smem_desc_sw128(q_addr + off) + (uint64_t)((kk % 4) * 2),
-                           smem_desc_sw128(k_addr + off) + (uint64_t)((kk % 4) * 2), idesc_qk, kk > 0 ? 1u : 0u);
+                    for (int kk = 0; kk < QKD / 16; ++kk) {
+                        const uint32_t off = (kk / 4) * FA_SLAB;
+                        mma_ss(tmem_base + S_COL[t], smem_desc_sw128(q_addr + off) + (uint64_t)((kk % 4) * 2),
+                               smem_desc_sw128(k_addr + off) + (uint64_t)((kk % 4) * 2), idesc_qk, kk > 0 ? 1u : 0u);
+                    }
+                    mma_commit(&s_full[t]);
                 }
-                mma_commit(&s_full[t]);
+                __syncwarp();
             };
             // The scores run one key tile ahead of the P.V products: S_t(j+1) is issued right after O_t += P_t(j).V(j),
             // so the softmax of one query tile overlaps the softmax of the other instead of alternating with it.
             auto active = [&](int t, int j) { return j >= lo[t] && j < n_tiles[t]; };
             if (ok && n_max > j_lo) {
-                ok = mbar_wait(&k_full[0], 0, &abort_flag, P.err, TC_TIMEOUT_FULL);
+                ok = mbar_wait_warp(&k_full[0], 0, &abort_flag, P.err, TC_TIMEOUT_FULL);
                 tc_fence_after();
                 if (ok) {
                     const uint32_t k_addr = smem_u32(k_smem);
 #pragma unroll
                     for (int t = 0; t < 2; ++t)
                         if (active(t, j_lo)) issue_s(t, k_addr);
-                    mma_commit(&k_empty[0]);
+                    if (elect_one()) mma_commit(&k_empty[0]);
+                    __syncwarp();
                 }
             }
             for (int j = j_lo; j < n_max && ok; ++j) {
                 const int i = j - j_lo, vs = i % VST, s1 = (i + 1) % KST;
                 const bool more = j + 1 < n_max;
-                if (!mbar_wait(&v_full[vs], (i / VST) & 1, &abort_flag, P.err, TC_TIMEOUT_FULL)) { ok = false; break; }
+                if (!mbar_wait_warp(&v_full[vs], (i / VST) & 1, &abort_flag, P.err, TC_TIMEOUT_FULL)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t v_addr = smem_u32(v_smem + vs * V_BYTES);
                 const uint32_t k_addr = smem_u32(k_smem + s1 * QK_BYTES);
 #pragma unroll
                 for (int t = 0; t < 2; ++t) {
                     if (active(t, j)) {
-                        if (!mbar_wait(&p_ready[t], (j - lo[t]) & 1, &abort_flag, P.err, TC_TIMEOUT_MISC)) { ok = false; break; }
+                        if (!mbar_wait_warp(&p_ready[t], (j - lo[t]) & 1, &abort_flag, P.err, TC_TIMEOUT_MISC)) { ok = false; break; }
                         tc_fence_after();
+                        if (elect_one()) {
 #pragma unroll
-                        for (int kk = 0; kk < FA_BN / 16; ++kk) {
-                            // 16 keys = two 8-row groups of 1024 bytes; the 64-column slabs of V are 16 KB apart
-                            const uint64_t v_desc = smem_desc_sw128_mn(v_addr + kk * 2048, FA_SLAB);
-                            mma_ts(tmem_base + O_COL[t], tmem_base + S_COL[t] + kk * 8, v_desc, idesc_pv, (j > lo[t] || kk > 0) ? 1u : 0u);
+                            for (int kk = 0; kk < FA_BN / 16; ++kk) {
+                                // 16 keys = two 8-row groups of 1024 bytes; the 64-column slabs of V are 16 KB apart
+                                const uint64_t v_desc = smem_desc_sw128_mn(v_addr + kk * 2048, FA_SLAB);
+                                mma_ts(tmem_base + O_COL[t], tmem_base + S_COL[t] + kk * 8, v_desc, idesc_pv, (j > lo[t] || kk > 0) ? 1u : 0u);
+                            }
                         }
+                        __syncwarp();
                     }
                     if (t == 0 && more) {
-                        if (!mbar_wait(&k_full[s1], ((i + 1) / KST) & 1, &abort_flag, P.err, TC_TIMEOUT_FULL)) { ok = false; break; }
+                        if (!mbar_wait_warp(&k_full[s1], ((i + 1) / KST) & 1, &abort_flag, P.err, TC_TIMEOUT_FULL)) { ok = false; break; }
                         tc_fence_after();
                     }
                     if (active(t, j + 1)) issue_s(t, k_addr);
                 }
                 if (!ok) break;
-                mma_commit(&v_empty[vs]);
-                if (more) mma_commit(&k_empty[s1]);
+                if (elect_one()) {
+                    mma_commit(&v_empty[vs]);
+                    if (more) mma_commit(&k_empty[s1]);
+                }
+                __syncwarp();
             }
-            if (ok) mma_commit(&o_done);
+            if (ok && elect_one()) mma_commit(&o_done);
+            __syncwarp();
         }
     } else {
         // ---- softmax / correction / epilogue: one thread per query row

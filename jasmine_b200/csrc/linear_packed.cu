@@ -257,31 +257,30 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
     const uint32_t tmem_base = tmem_base_smem;
 
     if (warp == 0) {
-        // ---- producer ------------------------------------------------------------------------------------
-        if (lane == 0) {
-            const uint8_t* wsrc = P.Wp + (size_t)u_begin * PK_TILE_BYTES;
+        // ---- producer (the warp walks the stages together, one elected lane issues) -------------------------------
+        {
             // weights first: the ring is filled with W before the predecessor kernel has finished (constant weights);
             // the X blocks of the same stages follow once it has
             // loop state kept incrementally (k-block within the tile, stage, phase): no division per request
             int rem = u_end - u_begin, kb = u_begin % P.kbt;
             int i = 0, s = 0;
             uint32_t ph = 0;
-            const uint8_t* src = wsrc;
-            auto issue = [&]() {
+            const uint8_t* src = P.Wp + (size_t)u_begin * PK_TILE_BYTES;
+            while (rem > 0) {  // the first ring goes out at once: before the predecessor kernel has finished
+                if (i >= stages && !mbar_wait_warp(&empty_bar[s], ph ^ 1, &abort_flag, P.err, TC_TIMEOUT_EMPTY)) break;
                 const int n = pk_chunk(P.pair_ok, min(P.kbt - kb, rem));
-                mbar_expect_tx(&full_bar[s], (uint32_t)n * PK_TILE_BYTES);
-                bulk_load(tiles + (size_t)s * STAGE_BYTES, src, (uint32_t)n * PK_TILE_BYTES, &full_bar[s]);
+                if (elect_one()) {
+                    mbar_expect_tx(&full_bar[s], (uint32_t)n * PK_TILE_BYTES);
+                    bulk_load(tiles + (size_t)s * STAGE_BYTES, src, (uint32_t)n * PK_TILE_BYTES, &full_bar[s]);
+                }
+                __syncwarp();
                 src += (size_t)n * PK_TILE_BYTES;
                 rem -= n;
                 kb += n;
                 if (kb == P.kbt) kb = 0;
                 ++i;
                 if (++s == stages) { s = 0; ph ^= 1; }
-            };
-            while (rem > 0) {  // the first ring goes out at once: before the predecessor kernel has finished
-                if (i >= stages && !mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, P.err, TC_TIMEOUT_EMPTY)) break;
-                issue();
-                if (i == stages) PK_TRACE(1);  // first ring of W requested
+                if (i == stages && lane == 0) PK_TRACE(1);  // first ring of W requested
             }
             const int issued = i;
             if (abort_flag) {  // let the copies in flight land before the CTA exits (bounded)
@@ -297,27 +296,32 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
         }
     } else if (warp == 6) {
         // ---- X producer: the token blocks of every stage, once the predecessor kernel has written them --------------
-        if (lane == 0) {
+        {
             if (tp_reduce) {
                 // X is the residual stream that the first CTAs of this launch are completing (h += the ranks' slots).  Its
                 // readiness is announced through an epoch word, not by the end of the predecessor kernel; then the generic
                 // writes of the reducing CTAs are ordered before the copy engine's reads.  Nothing else the X producer
-                // touches belongs to another kernel, so it does not wait for the predecessor.
+                // touches belongs to another kernel, so it does not wait for the predecessor.  (Every lane waits and fences:
+                // any of them may be the one that issues.)
                 const int E = *reinterpret_cast<const volatile int*>(P.tp_pass) * P.tp_n_sites + P.tp_site + 1;
                 pk_wait_epoch(P.tp_state + 2, E, P.tp_wait, P.err);
                 pk_fence_proxy_async();
+                __syncwarp();
             } else chain_wait();
-            PK_TRACE(2);  // predecessor complete (fused exchange: h complete)
+            if (lane == 0) PK_TRACE(2);  // predecessor complete (fused exchange: h complete)
             int rem = u_end - u_begin, kb = u_begin % P.kbt;
             int i = 0, s = 0;
             uint32_t ph = 0;
             while (rem > 0) {
-                if (i >= stages && !mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, P.err, TC_TIMEOUT_EMPTY)) break;
+                if (i >= stages && !mbar_wait_warp(&empty_bar[s], ph ^ 1, &abort_flag, P.err, TC_TIMEOUT_EMPTY)) break;
                 const int n = pk_chunk(P.pair_ok, min(P.kbt - kb, rem));
-                uint8_t* xs = tiles + (size_t)s * STAGE_BYTES + X_OFF;
-                mbar_expect_tx(&full_bar[s], (uint32_t)n * B_BYTES);
-                if (n == 2) tma_load_3d(xs, &tmap_x2, 0, 0, kb, &full_bar[s]);
-                else tma_load_2d(xs, &tmap_x, kb * 64, 0, &full_bar[s]);
+                if (elect_one()) {
+                    uint8_t* xs = tiles + (size_t)s * STAGE_BYTES + X_OFF;
+                    mbar_expect_tx(&full_bar[s], (uint32_t)n * B_BYTES);
+                    if (n == 2) tma_load_3d(xs, &tmap_x2, 0, 0, kb, &full_bar[s]);
+                    else tma_load_2d(xs, &tmap_x, kb * 64, 0, &full_bar[s]);
+                }
+                __syncwarp();
                 rem -= n;
                 kb += n;
                 if (kb == P.kbt) kb = 0;
@@ -332,7 +336,7 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
         }
     } else if (warp == 1) {
         // ---- MMA issuer ------------------------------------------------------------------------------------
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc = instr_desc_bf16(128, BN);
             bool ok = true;
             int it = 0, seg = 0, s = 0;
@@ -343,34 +347,38 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
                 const int buf = seg & 1;
                 if (seg >= 2) {
                     // the epilogue must have drained this buffer's previous segment
-                    if (!mbar_wait(&acc_empty[buf], ((seg >> 1) - 1) & 1, &abort_flag, P.err, TC_TIMEOUT_MISC)) { ok = false; break; }
+                    if (!mbar_wait_warp(&acc_empty[buf], ((seg >> 1) - 1) & 1, &abort_flag, P.err, TC_TIMEOUT_MISC)) { ok = false; break; }
                     tc_fence_after();
                 }
                 const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);
                 for (int j = 0; j < len; ++it) {
                     const int n = pk_chunk(P.pair_ok, len - j);
-                    if (!mbar_wait(&full_bar[s], ph, &abort_flag, P.err, TC_TIMEOUT_FULL)) { ok = false; break; }
-                    if (it == 0) PK_TRACE(3);  // first stage landed
+                    if (!mbar_wait_warp(&full_bar[s], ph, &abort_flag, P.err, TC_TIMEOUT_FULL)) { ok = false; break; }
+                    if (it == 0 && lane == 0) PK_TRACE(3);  // first stage landed
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(tiles + (size_t)s * STAGE_BYTES);
-                    for (int q = 0; q < n; ++q) {
-                        const uint64_t a_desc = smem_desc_sw128(a_addr + q * PK_TILE_BYTES);
-                        const uint64_t b_desc = smem_desc_sw128(a_addr + X_OFF + q * B_BYTES);
+                    if (elect_one()) {
+                        for (int q = 0; q < n; ++q) {
+                            const uint64_t a_desc = smem_desc_sw128(a_addr + q * PK_TILE_BYTES);
+                            const uint64_t b_desc = smem_desc_sw128(a_addr + X_OFF + q * B_BYTES);
 #pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            mma_ss(d_tmem, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (j > 0 || q > 0 || k > 0) ? 1u : 0u);
+                            for (int k = 0; k < 4; ++k)
+                                mma_ss(d_tmem, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (j > 0 || q > 0 || k > 0) ? 1u : 0u);
+                        }
+                        mma_commit(&empty_bar[s]);
                     }
-                    mma_commit(&empty_bar[s]);
+                    __syncwarp();
                     j += n;
                     if (++s == stages) { s = 0; ph ^= 1; }
                 }
                 if (!ok) break;
-                mma_commit(&acc_full[buf]);
+                if (elect_one()) mma_commit(&acc_full[buf]);
+                __syncwarp();
                 rem -= len;
                 kb0 = 0;  // every segment after the first starts a tile
                 ++seg;
             }
-            PK_TRACE(4);  // last MMA issued
+            if (lane == 0) PK_TRACE(4);  // last MMA issued
         }
         if (CL && P.cluster_s > 1) {
             __syncwarp();
