@@ -4,8 +4,12 @@
 // reference-exact fp32 paths (small models, parity tests); the bf16 projections of
 // the large model go through the tcgen05 kernel instead.
 #include "common.cuh"
+#include "mma_utils.cuh"
+#include "tc_utils.cuh"
 
 namespace jsm {
+
+using tc::smem_u32;
 
 struct MatD {
     const float* p;
@@ -13,84 +17,175 @@ struct MatD {
     long long rs, cs;
 };
 
-constexpr int TM = 64, TN = 64, TK = 16;
-
 __device__ __forceinline__ float gelu_f(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752440f)); }
 
-// ORDERED: the reference's summation order (see above).  Otherwise every block of TK products is summed with fused
-// multiply-adds before it joins the total: shorter chains of roundings, for fp32 models that have no order to match.
-template <bool ORDERED>
-__global__ void __launch_bounds__(256) dot_f32_kernel(MatD A, MatD B, MatD bias, int has_bias, int epilogue, MatD R,
-                                                      float* Cp, long long crs, long long ccs, int M, int N, int K) {
-    __shared__ float As[TK][TM + 1];
-    __shared__ float Bs[TK][TN + 1];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+// Tile.  128 threads own TMM * 8 rows x TNN * 16 columns, TMM x TNN outputs each (rows ty + 8 i, columns tx + 16 j).  Blocks of
+// 32 products are staged [row or column][k] by asynchronous copies, so that a thread reads four of them with one load and the
+// four rows or eight columns of a quarter warp lie in different banks (pitch 36).
+constexpr int DOT_THREADS = 128, DOT_KB = 32, DOT_PITCH = DOT_KB + 4;
+constexpr int dot_stages(int tnn) { return tnn == 1 ? 8 : 4; }
+constexpr int dot_smem(int tmm, int tnn) { return dot_stages(tnn) * (8 * tmm + 16 * tnn) * DOT_PITCH * 4; }
 
-    for (int k0 = 0; k0 < K; k0 += TK) {
-        // A tile: TM x TK, B tile: TK x TN (1024 elements each, 4 per thread)
+// 32 products' worth of ROWS rows of an operand (row stride rs, stride ks along the products), zeros where there is nothing.
+// vec: contiguous products, 16-byte aligned rows.
+template <int ROWS>
+__device__ __forceinline__ void dot_stage(uint32_t dst, const float* p, int row0, int rows, long long rs, long long ks, int k0, int K, bool vec) {
+    if (vec) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            int idx = threadIdx.x + e * 256;
-            // choose the faster-varying index along the contiguous axis of each operand
-            int am, ak;
-            if (A.cs == 1) { ak = idx % TK; am = idx / TK; } else { am = idx % TM; ak = idx / TM; }
-            int gm = m0 + am, gk = k0 + ak;
-            As[ak][am] = (gm < M && gk < K) ? A.p[gm * A.rs + gk * A.cs] : 0.0f;
-            int bk, bn;
-            if (B.cs == 1) { bn = idx % TN; bk = idx / TN; } else { bk = idx % TK; bn = idx / TK; }
-            int gn = n0 + bn;
-            gk = k0 + bk;
-            Bs[bk][bn] = (gn < N && gk < K) ? B.p[gk * B.rs + gn * B.cs] : 0.0f;
+        for (int e = threadIdx.x; e < ROWS * (DOT_KB / 4); e += DOT_THREADS) {
+            const int r = e / (DOT_KB / 4), c = e % (DOT_KB / 4) * 4;
+            const int left = row0 + r < rows ? min(max(K - k0 - c, 0), 4) : 0;
+            const float* src = left ? p + (row0 + r) * rs + k0 + c : p;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (r * DOT_PITCH + c) * 4), "l"(reinterpret_cast<uint64_t>(src)), "r"(left * 4)
+                         : "memory");
         }
-        __syncthreads();
-        const int kmax = (K - k0) < TK ? (K - k0) : TK;  // never add the zero padding: -0.0 + 0.0 would flip a sign
-        float part[4][4];
-        if (!ORDERED)
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) part[i][j] = 0.0f;
-        for (int k = 0; k < kmax; ++k) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[k][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[k][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (ORDERED) acc[i][j] = __fadd_rn(acc[i][j], __fmul_rn(a[i], b[j]));
-                    else part[i][j] = fmaf(a[i], b[j], part[i][j]);
-                }
+    } else {
+        const bool along_k = rs != 1;  // the threads walk the contiguous direction
+        for (int e = threadIdx.x; e < ROWS * DOT_KB; e += DOT_THREADS) {
+            const int r = along_k ? e / DOT_KB : e % ROWS, c = along_k ? e % DOT_KB : e / ROWS;
+            const bool on = row0 + r < rows && k0 + c < K;
+            cp_async4(dst + (r * DOT_PITCH + c) * 4, on ? p + (row0 + r) * rs + (k0 + c) * ks : p, on);
         }
-        if (!ORDERED)
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
-        __syncthreads();
     }
+}
+
+// Before, one 64 x 64 tile per CTA staged element by element: 64 x 128 x 128 took 27 us, 300 x 1024 x 2752 (f32 model) 182 us.
+// What bounds it: with few outputs the chain of K dependent additions and the launch, with many the fp32 pipe (two instructions
+// per product in the reference's order, one per two products otherwise).
+// ORDERED: the reference's summation order (see above).  The zeros behind the last product change nothing: a sum that starts
+// at +0 never becomes -0.
+// Otherwise: even and odd products of a block of 32 form two chains of fused multiply-adds (packed pairs), which join the total
+// once per block; a cluster of CTAs shares the products of a tile (whole blocks each) and adds its totals in rank order.
+template <bool ORDERED, int TMM, int TNN>
+__global__ void __launch_bounds__(DOT_THREADS) dot_f32_kernel(MatD A, MatD B, MatD bias, int has_bias, int epilogue, MatD R,
+                                                              float* Cp, long long crs, long long ccs, int M, int N, int K, int vec_a, int vec_b) {
+    constexpr int BM = 8 * TMM, BN = 16 * TNN, STAGES = dot_stages(TNN), STAGE = (BM + BN) * DOT_PITCH;
+    static_assert(STAGES * STAGE >= BM * BN, "the totals of a tile are exchanged through the ring");
+    extern __shared__ __align__(16) float dot_ring[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ty = (warp >> 1) * 4 + (lane >> 3), tx = (warp & 1) * 8 + (lane & 7);
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int splits = ORDERED ? 1 : gridDim.z, rank = ORDERED ? 0 : blockIdx.z;
+    const int blocks = (K + DOT_KB - 1) / DOT_KB, b0 = (int)((long long)blocks * rank / splits), mine = (int)((long long)blocks * (rank + 1) / splits) - b0;
+    const uint32_t ring = smem_u32(dot_ring);
+    auto stage_a = [&](int i) { dot_stage<BM>(ring + (i % STAGES) * STAGE * 4, A.p, m0, M, A.rs, A.cs, (b0 + i) * DOT_KB, K, vec_a); };
+    auto stage_b = [&](int i) { dot_stage<BN>(ring + ((i % STAGES) * STAGE + BM * DOT_PITCH) * 4, B.p, n0, N, B.cs, B.rs, (b0 + i) * DOT_KB, K, vec_b); };
+    if (!ORDERED) {  // B holds weights: they may be requested before the predecessor kernel has ended
+        chain_trigger();
+        for (int i = 0; i < STAGES - 1 && i < mine; ++i) stage_b(i);
+        chain_wait();
+    }
+#pragma unroll 1
+    for (int i = 0; i < STAGES - 1; ++i) {
+        if (i < mine) {
+            stage_a(i);
+            if (ORDERED) stage_b(i);
+        }
+        cp_async_commit();
+    }
+    float acc[TMM][TNN];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < TMM; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-            if (m < M && n < N) {
-                float v = acc[i][j];
-                if (has_bias) v = __fadd_rn(v, bias.p[(m % bias.rows) * bias.rs + (n % bias.cols) * bias.cs]);
-                if (epilogue == 1) v = v > 0.0f ? v : 0.0f * v;
-                else if (epilogue == 2) v = gelu_f(v);
-                else if (epilogue == 3) v = __fadd_rn(v, R.p[(m % R.rows) * R.rs + (n % R.cols) * R.cs]);
-                Cp[m * crs + n * ccs] = v;
+        for (int j = 0; j < TNN; ++j) acc[i][j] = 0.0f;
+#pragma unroll 1
+    for (int b = 0; b < mine; ++b) {
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();  // block b is here, and everybody is done with block b - 1, whose place is filled again
+        if (b + STAGES - 1 < mine) {
+            stage_a(b + STAGES - 1);
+            stage_b(b + STAGES - 1);
+        }
+        cp_async_commit();
+        const float *as = dot_ring + (b % STAGES) * STAGE + ty * DOT_PITCH, *bs = dot_ring + (b % STAGES) * STAGE + (BM + tx) * DOT_PITCH;
+        uint64_t part[TMM][TNN];
+        if (!ORDERED)
+#pragma unroll
+            for (int i = 0; i < TMM; ++i)
+#pragma unroll
+                for (int j = 0; j < TNN; ++j) part[i][j] = 0;
+#pragma unroll 2
+        for (int k = 0; k < DOT_KB; k += 4) {
+            if constexpr (ORDERED) {
+                float4 x[TMM], y[TNN];
+#pragma unroll
+                for (int i = 0; i < TMM; ++i) x[i] = *reinterpret_cast<const float4*>(as + i * 8 * DOT_PITCH + k);
+#pragma unroll
+                for (int j = 0; j < TNN; ++j) y[j] = *reinterpret_cast<const float4*>(bs + j * 16 * DOT_PITCH + k);
+#pragma unroll
+                for (int i = 0; i < TMM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TNN; ++j) {
+                        float s = acc[i][j];
+                        s = __fadd_rn(s, __fmul_rn(x[i].x, y[j].x));
+                        s = __fadd_rn(s, __fmul_rn(x[i].y, y[j].y));
+                        s = __fadd_rn(s, __fmul_rn(x[i].z, y[j].z));
+                        acc[i][j] = __fadd_rn(s, __fmul_rn(x[i].w, y[j].w));
+                    }
+            } else {
+                ulonglong2 x[TMM], y[TNN];
+#pragma unroll
+                for (int i = 0; i < TMM; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(as + i * 8 * DOT_PITCH + k);
+#pragma unroll
+                for (int j = 0; j < TNN; ++j) y[j] = *reinterpret_cast<const ulonglong2*>(bs + j * 16 * DOT_PITCH + k);
+#pragma unroll
+                for (int i = 0; i < TMM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TNN; ++j) part[i][j] = f2_fma(x[i].y, y[j].y, f2_fma(x[i].x, y[j].x, part[i][j]));
             }
         }
+        if (!ORDERED)
+#pragma unroll
+            for (int i = 0; i < TMM; ++i)
+#pragma unroll
+                for (int j = 0; j < TNN; ++j) {
+                    float even, odd;
+                    f2_unpack(part[i][j], even, odd);
+                    acc[i][j] += even + odd;
+                }
+    }
+    if constexpr (ORDERED) {
+#pragma unroll
+        for (int i = 0; i < TMM; ++i)
+#pragma unroll
+            for (int j = 0; j < TNN; ++j) {
+                const int m = m0 + ty + 8 * i, n = n0 + tx + 16 * j;
+                if (m < M && n < N) {
+                    float v = acc[i][j];
+                    if (has_bias) v = __fadd_rn(v, bias.p[(m < bias.rows ? m : m % bias.rows) * bias.rs + (n < bias.cols ? n : n % bias.cols) * bias.cs]);
+                    if (epilogue == 1) v = v > 0.0f ? v : 0.0f * v;
+                    else if (epilogue == 2) v = gelu_f(v);
+                    else if (epilogue == 3) v = __fadd_rn(v, R.p[(m < R.rows ? m : m % R.rows) * R.rs + (n < R.cols ? n : n % R.cols) * R.cs]);
+                    Cp[m * crs + n * ccs] = v;
+                }
+            }
+    } else {
+        cp_async_wait<0>();
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < TMM; ++i)
+#pragma unroll
+            for (int j = 0; j < TNN; ++j) dot_ring[(ty + 8 * i) * BN + tx + 16 * j] = acc[i][j];
+        if (splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        else __syncthreads();
+        // this CTA's share of the rows (8 TMM >= splits, both powers of two)
+        const int rows = BM / splits;
+        for (int e = threadIdx.x; e < rows * BN; e += DOT_THREADS) {
+            const int r = rank * rows + e / BN, c = e % BN;
+            float v = 0.0f;
+            if (splits == 1) v = dot_ring[r * BN + c];
+            else
+                for (int s = 0; s < splits; ++s) {
+                    uint32_t addr;
+                    float t;
+                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(ring + (r * BN + c) * 4), "r"(s));
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(t) : "r"(addr) : "memory");
+                    v += t;
+                }
+            if (m0 + r < M && n0 + c < N) Cp[(m0 + r) * crs + (n0 + c) * ccs] = v;
+        }
+        if (splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
 }
 
 static MatD to_d(const jsm_mat& m) {
@@ -100,14 +195,53 @@ static MatD to_d(const jsm_mat& m) {
     return d;
 }
 
-// C = A . B in fp32 without the reference's order (operands as in jsm_dot_f32, checked by the caller)
-jsm_status dot_f32_launch(const jsm_mat& A, const jsm_mat& B, const jsm_mat& Cm, cudaStream_t st) {
-    const dim3 grid((Cm.cols + TN - 1) / TN, (Cm.rows + TM - 1) / TM);
+// contiguous products in 16-byte aligned rows
+static int dot_vec(const float* p, long long rs, long long ks) { return ks == 1 && rs % 4 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+
+template <bool ORDERED, int TMM, int TNN>
+static jsm_status dot_launch(const MatD& A, const MatD& B, const MatD* bias, int epilogue, const MatD* R, float* C, long long crs, long long ccs, int splits,
+                             cudaStream_t st) {
+    constexpr int smem = dot_smem(TMM, TNN);
+    static bool attr_done = false;  // per instantiation
+    if (!attr_done) {
+        JSM_CUDA_CHECK(cudaFuncSetAttribute(dot_f32_kernel<ORDERED, TMM, TNN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        attr_done = true;
+    }
     const MatD none{nullptr, 1, 1, 0, 0};
-    dot_f32_kernel<false><<<grid, 256, 0, st>>>(to_d(A), to_d(B), none, 0, 0, none, reinterpret_cast<float*>(Cm.data), Cm.row_stride, Cm.col_stride,
-                                                A.rows, B.cols, A.cols);
-    JSM_LAUNCH_CHECK();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((B.cols + 16 * TNN - 1) / (16 * TNN), (A.rows + 8 * TMM - 1) / (8 * TMM), splits);
+    cfg.blockDim = dim3(DOT_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = splits;
+    cfg.attrs = ORDERED || !chained_launch_enabled() ? attr + 1 : attr;
+    cfg.numAttrs = (cfg.attrs == attr ? 1 : 0) + (splits > 1 ? 1 : 0);
+    JSM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, dot_f32_kernel<ORDERED, TMM, TNN>, A, B, bias ? *bias : none, bias ? 1 : 0, epilogue, R ? *R : none, C, crs, ccs, A.rows,
+                                      B.cols, A.cols, dot_vec(A.p, A.rs, A.cs), dot_vec(B.p, B.cs, B.rs)));
+    g_launches.fetch_add(1);
     return JSM_OK;
+}
+
+// C = A . B in fp32 without the reference's order (operands as in jsm_dot_f32, checked by the caller; B holds weights, constant
+// while the stream runs).  Few rows take 16 x 64 tiles.  The products of a tile are shared by as many CTAs as even out the
+// multiprocessors' loads: rounds of CTAs times blocks of products each, and about four blocks' time for a CTA's start and end.
+jsm_status dot_f32_launch(const jsm_mat& A, const jsm_mat& B, const jsm_mat& Cm, cudaStream_t st) {
+    const bool few = A.rows <= 32;
+    const int tiles = (B.cols + 63) / 64 * (few ? (A.rows + 15) / 16 : (A.rows + 63) / 64), blocks = (A.cols + DOT_KB - 1) / DOT_KB;
+    int splits = 1;
+    long long best = -1;
+    for (int s = 1; s <= 8 && s <= blocks; s *= 2) {
+        const long long cost = (long long)((tiles * s + sm_count() - 1) / sm_count()) * ((blocks + s - 1) / s + 4);
+        if (best < 0 || cost < best) { best = cost; splits = s; }
+    }
+    float* C = reinterpret_cast<float*>(Cm.data);
+    return few ? dot_launch<false, 2, 4>(to_d(A), to_d(B), nullptr, 0, nullptr, C, Cm.row_stride, Cm.col_stride, splits, st)
+               : dot_launch<false, 8, 4>(to_d(A), to_d(B), nullptr, 0, nullptr, C, Cm.row_stride, Cm.col_stride, splits, st);
 }
 
 }  // namespace jsm
@@ -128,12 +262,13 @@ extern "C" jsm_status jsm_dot_f32(jsm_mat A, jsm_mat B, const jsm_mat* bias, int
     if ((bias && (bias->dtype != JSM_F32 || !bias->data || bias->rows <= 0 || bias->cols <= 0)) ||
         (R && (R->dtype != JSM_F32 || !R->data || R->rows <= 0 || R->cols <= 0)))
         JSM_FAIL(JSM_INVALID_ARG, "jsm_dot_f32: bad bias / residual operand");
-    MatD bd = bias ? to_d(*bias) : MatD{nullptr, 1, 1, 0, 0};
-    MatD rd = R ? to_d(*R) : MatD{nullptr, 1, 1, 0, 0};
-    dim3 grid((Cm.cols + TN - 1) / TN, (Cm.rows + TM - 1) / TM);
-    dot_f32_kernel<true><<<grid, 256, 0, as_stream(stream)>>>(to_d(A), to_d(B), bd, bias ? 1 : 0, epilogue, rd,
-                                                        reinterpret_cast<float*>(Cm.data), Cm.row_stride, Cm.col_stride,
-                                                        A.rows, B.cols, A.cols);
-    JSM_LAUNCH_CHECK();
-    return JSM_OK;
+    MatD bd, rd;
+    if (bias) bd = to_d(*bias);
+    if (R) rd = to_d(*R);
+    const MatD *pb = bias ? &bd : nullptr, *pr = R ? &rd : nullptr;
+    float* C = reinterpret_cast<float*>(Cm.data);
+    // 64 x 64 tiles once they occupy half of the multiprocessors, 16 x 16 tiles (one output pair per thread) below
+    if ((long long)((Cm.cols + 63) / 64) * ((Cm.rows + 63) / 64) * 2 > sm_count())
+        return dot_launch<true, 8, 4>(to_d(A), to_d(B), pb, epilogue, pr, C, Cm.row_stride, Cm.col_stride, 1, as_stream(stream));
+    return dot_launch<true, 2, 1>(to_d(A), to_d(B), pb, epilogue, pr, C, Cm.row_stride, Cm.col_stride, 1, as_stream(stream));
 }
