@@ -44,82 +44,142 @@ __device__ __forceinline__ float rec_sigmoid(float x) { return 1.0f / (1.0f + ex
 __device__ __forceinline__ float rec_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 
 // ---- prompts, any sizes up to 256 key components, f32 arithmetic throughout ---------------------------------------
-// A CTA owns 16 columns of one head's state; eight threads share a column (rows sub, sub + 8, ...).
-constexpr int RS_COLS = 16, RS_SUB = 8, RS_THREADS = RS_COLS * RS_SUB, RS_TT = 16;
+// A chain of tokens: what bounds a token is the latency of S^T k (products, a reduction over the threads of a column) before
+// its update may start, with the state's columns as the only parallelism.  A CTA owns 8 columns of one head's state, sixteen
+// threads a column (vectors of V rows sub V, (sub + 16) V, ...: one or two wide loads of k and q per token), and four more
+// warps than it needs for that bring and normalise the next tokens meanwhile, two per warp.  The outputs of four tokens are
+// reduced together, off the chain.
+constexpr int RS_COLS = 8, RS_SUB = 16, RS_WALK = RS_COLS * RS_SUB, RS_LOAD = 256, RS_THREADS = RS_WALK + RS_LOAD;
+constexpr int rs_tokens(int kw) { return kw > 128 ? 8 : 16; }  // tokens staged at a time
 
-template <typename T, int NS, bool DELTA>
+template <typename T, int NR, bool DELTA>
 __global__ void __launch_bounds__(RS_THREADS) rec_scan_kernel(RecArgs a, RecDims d) {
-    constexpr int KW = 8 * NS;  // rows of the state, rounded up
-    __shared__ float ks[RS_TT][KW], qs[RS_TT][KW], vs[RS_TT][RS_COLS], gs[RS_TT], bs[RS_TT];
+    constexpr int KW = RS_SUB * NR, V = NR < 4 ? NR : 4, TT = rs_tokens(KW), PER_LANE = (KW + 31) / 32;  // KW: rows of the state, rounded up
+    __shared__ __align__(16) float ks[2][TT][KW], qs[2][TT][KW];
+    __shared__ float vs[2][TT][RS_COLS], gs[2][TT], bs[2][TT];
     chain_trigger();
     chain_wait();
-    const int tid = threadIdx.x, col = tid / RS_SUB, sub = tid % RS_SUB, warp = tid >> 5, lane = tid & 31;
-    const int h = blockIdx.y, g = h / (d.H / d.G), seg = blockIdx.z, kp = d.kp(), vp = d.vp(), cc = d.conv_cols();
-    const int c = blockIdx.x * RS_COLS + col;
-    const bool live = c < vp;
-    const int start = a.seg_start[seg], len = a.seg_len[seg];
-    float* state = a.S + ((long long)a.seg_slot[seg] * d.H + h) * kp * vp + c;
-    const bool fresh = a.seg_pos0[seg] == 0;
-    float S[NS];
+    const int tid = threadIdx.x, lane = tid & 31, h = blockIdx.y, g = h / (d.H / d.G), seg = blockIdx.z, kp = d.kp(), vp = d.vp(), cc = d.conv_cols();
+    const int start = a.seg_start[seg], len = a.seg_len[seg], c0 = blockIdx.x * RS_COLS;
+    const T* qkv = static_cast<const T*>(a.qkv) + (long long)start * cc;
+    auto stage = [&](int t0) {  // warps behind the walking ones: tokens t0 .. t0 + TT - 1 into the buffer of their turn
+        const int n = min(TT, len - t0), buf = t0 / TT & 1, lw = (tid - RS_WALK) >> 5;
+        float q[TT * 32 / RS_LOAD][PER_LANE], k[TT * 32 / RS_LOAD][PER_LANE];
 #pragma unroll
-    for (int i = 0; i < NS; ++i) {
-        const int r = sub + 8 * i;
-        S[i] = live && r < kp && !fresh ? state[(long long)r * vp] : 0.0f;
-    }
-    const T* qkv = static_cast<const T*>(a.qkv);
-    const float decay = DELTA ? 0.0f : a.decay[h];
-    for (int t0 = 0; t0 < len; t0 += RS_TT) {
-        const int n = min(RS_TT, len - t0);
-        __syncthreads();
-        for (int t = warp; t < n; t += RS_THREADS / 32) {
-            const T* row = qkv + (long long)(start + t0 + t) * cc;
-            float sq = 0.0f, sk = 0.0f;
-            for (int i = lane; i < KW; i += 32) {
-                const float q = i < kp ? to_f32(row[g * kp + i]) : 0.0f, k = i < kp ? to_f32(row[(d.G + g) * kp + i]) : 0.0f;
-                qs[t][i] = q; ks[t][i] = k;
-                sq = fmaf(q, q, sq); sk = fmaf(k, k, sk);
+        for (int x = 0; x < TT * 32 / RS_LOAD; ++x) {
+            const int t = lw + x * (RS_LOAD / 32);
+            const T* row = qkv + (long long)(t0 + t) * cc;
+#pragma unroll
+            for (int e = 0; e < PER_LANE; ++e) {
+                const int i = lane + 32 * e;
+                const bool on = t < n && i < kp;
+                q[x][e] = on ? to_f32(row[g * kp + i]) : 0.0f;
+                k[x][e] = on ? to_f32(row[(d.G + g) * kp + i]) : 0.0f;
             }
+            if (t < n && lane < RS_COLS) vs[buf][t][lane] = c0 + lane < vp ? to_f32(row[2 * d.G * kp + h * vp + c0 + lane]) : 0.0f;
+            if (DELTA && t < n && lane == 31) {
+                const float* ba = a.ba + (long long)(start + t0 + t) * d.ba_cols();
+                bs[buf][t] = rec_sigmoid(ba[h]);
+                gs[buf][t] = expf(a.A[h] * rec_softplus(ba[d.ba_cols() / 2 + h] + a.dt_bias[h]));
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < TT * 32 / RS_LOAD; ++x) {
+            const int t = lw + x * (RS_LOAD / 32);
+            float sq = 0.0f, sk = 0.0f;
             if (DELTA) {
+#pragma unroll
+                for (int e = 0; e < PER_LANE; ++e) {
+                    sq = fmaf(q[x][e], q[x][e], sq);
+                    sk = fmaf(k[x][e], k[x][e], sk);
+                }
                 sq = sqrtf(warp_sum(sq) + UNIT_EPS);
                 sk = sqrtf(warp_sum(sk) + UNIT_EPS);
-                for (int i = lane; i < KW; i += 32) { qs[t][i] = qs[t][i] / sq * a.q_scale; ks[t][i] /= sk; }
             }
-            const int vc = blockIdx.x * RS_COLS + lane;
-            if (lane < RS_COLS) vs[t][lane] = vc < vp ? to_f32(row[2 * d.G * kp + h * vp + vc]) : 0.0f;
-            if (DELTA && lane == 0) {
-                const float* ba = a.ba + (long long)(start + t0 + t) * d.ba_cols();
-                bs[t] = rec_sigmoid(ba[h]);
-                gs[t] = expf(a.A[h] * rec_softplus(ba[d.ba_cols() / 2 + h] + a.dt_bias[h]));
+#pragma unroll
+            for (int e = 0; e < PER_LANE; ++e) {
+                const int i = lane + 32 * e;
+                if (t < n && i < KW) {
+                    qs[buf][t][i] = DELTA ? q[x][e] / sq * a.q_scale : q[x][e];
+                    ks[buf][t][i] = DELTA ? k[x][e] / sk : k[x][e];
+                }
             }
+        }
+    };
+    if (tid >= RS_WALK) {
+        stage(0);
+        __syncthreads();
+        for (int t0 = 0; t0 < len; t0 += TT) {
+            if (t0 + TT < len) stage(t0 + TT);
+            __syncthreads();
+        }
+        return;
+    }
+    const int col = tid / RS_SUB, sub = tid % RS_SUB, c = c0 + col;
+    const bool live = c < vp, fresh = a.seg_pos0[seg] == 0;
+    float* state = a.S + ((long long)a.seg_slot[seg] * d.H + h) * kp * vp + c;
+    auto row_of = [&](int i) { return ((i / V) * RS_SUB + sub) * V + i % V; };
+    float S[NR];
+#pragma unroll
+    for (int i = 0; i < NR; ++i) S[i] = live && row_of(i) < kp && !fresh ? state[(long long)row_of(i) * vp] : 0.0f;
+    const float decay = DELTA ? 0.0f : a.decay[h];
+    auto rows = [&](const float* p, float (&x)[NR]) {  // this thread's rows of a staged vector
+#pragma unroll
+        for (int i = 0; i < NR; i += V) {
+            if constexpr (V == 4) {
+                const float4 w = *reinterpret_cast<const float4*>(p + (i / V * RS_SUB + sub) * V);
+                x[i] = w.x; x[i + 1] = w.y; x[i + 2] = w.z; x[i + 3] = w.w;
+            } else {
+                const float2 w = *reinterpret_cast<const float2*>(p + (i / V * RS_SUB + sub) * V);
+                x[i] = w.x; x[i + 1] = w.y;
+            }
+        }
+    };
+    __syncthreads();
+    for (int t0 = 0; t0 < len; t0 += TT) {
+        const int n = min(TT, len - t0), buf = t0 / TT & 1;
+        for (int t4 = 0; t4 < n; t4 += 4) {
+            float o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int t = t4 + x;
+                if (t >= n) break;
+                float k[NR], q[NR];
+                rows(ks[buf][t], k);
+                rows(qs[buf][t], q);
+                const float gt = DELTA ? gs[buf][t] : decay;
+                float u = vs[buf][t][col];
+                if (DELTA) {
+                    float p[2] = {0.0f, 0.0f};
+#pragma unroll
+                    for (int i = 0; i < NR; ++i) p[i & 1] = fmaf(S[i], k[i], p[i & 1]);
+                    p[0] += p[1];
+#pragma unroll
+                    for (int y = 1; y < RS_SUB; y <<= 1) p[0] += __shfl_xor_sync(0xffffffffu, p[0], y);
+                    u = bs[buf][t] * fmaf(-gt, p[0], u);
+                }
+#pragma unroll
+                for (int i = 0; i < NR; ++i) {
+                    S[i] = fmaf(k[i], u, S[i] * gt);
+                    o[x] = fmaf(S[i], q[i], o[x]);
+                }
+            }
+            // four sums over the sixteen threads of a column: thread sub ends with token (sub & 3)
+            const bool odd = sub & 1, high = sub & 2;
+            float r0 = (odd ? o[1] : o[0]) + __shfl_xor_sync(0xffffffffu, odd ? o[0] : o[1], 1);
+            const float r1 = (odd ? o[3] : o[2]) + __shfl_xor_sync(0xffffffffu, odd ? o[2] : o[3], 1);
+            r0 = (high ? r1 : r0) + __shfl_xor_sync(0xffffffffu, high ? r0 : r1, 2);
+            r0 += __shfl_xor_sync(0xffffffffu, r0, 4);
+            r0 += __shfl_xor_sync(0xffffffffu, r0, 8);
+            const int t = t4 + sub;
+            if (live && sub < 4 && t < n) static_cast<T*>(a.out)[(long long)(start + t0 + t) * d.H * vp + h * vp + c] = from_f32<T>(r0);
         }
         __syncthreads();
-        for (int t = 0; t < n; ++t) {
-            const float gt = DELTA ? gs[t] : decay;
-            float u = vs[t][col], k[NS], o = 0.0f;
-#pragma unroll
-            for (int i = 0; i < NS; ++i) { k[i] = ks[t][sub + 8 * i]; S[i] *= gt; }
-            if (DELTA) {
-                float p = 0.0f;
-#pragma unroll
-                for (int i = 0; i < NS; ++i) p = fmaf(S[i], k[i], p);
-#pragma unroll
-                for (int x = 1; x < RS_SUB; x <<= 1) p += __shfl_xor_sync(0xffffffffu, p, x);
-                u = bs[t] * (u - p);
-            }
-#pragma unroll
-            for (int i = 0; i < NS; ++i) {
-                S[i] = fmaf(k[i], u, S[i]);
-                o = fmaf(S[i], qs[t][sub + 8 * i], o);
-            }
-#pragma unroll
-            for (int x = 1; x < RS_SUB; x <<= 1) o += __shfl_xor_sync(0xffffffffu, o, x);
-            if (live && sub == 0) static_cast<T*>(a.out)[(long long)(start + t0 + t) * d.H * vp + h * vp + c] = from_f32<T>(o);
-        }
     }
     if (live)
 #pragma unroll
-        for (int i = 0; i < NS; ++i)
-            if (sub + 8 * i < kp) state[(long long)(sub + 8 * i) * vp] = S[i];
+        for (int i = 0; i < NR; ++i)
+            if (row_of(i) < kp) state[(long long)row_of(i) * vp] = S[i];
 }
 
 // ---- prompts on the tensor cores ----------------------------------------------------------------------------------
@@ -883,17 +943,17 @@ static RecArgs rec_args(bool f32, const RecDims& d, const RecWeights& w, const R
     return a;
 }
 
-template <typename T, int NS, bool DELTA>
+template <typename T, int NR, bool DELTA>
 static jsm_status scan_go(const RecArgs& a, const RecDims& d, int n_segs, cudaStream_t st) {
-    JSM_CUDA_CHECK(launch_chained(rec_scan_kernel<T, NS, DELTA>, dim3((d.vp() + RS_COLS - 1) / RS_COLS, d.H, n_segs), dim3(RS_THREADS), 0, st, a, d));
+    JSM_CUDA_CHECK(launch_chained(rec_scan_kernel<T, NR, DELTA>, dim3((d.vp() + RS_COLS - 1) / RS_COLS, d.H, n_segs), dim3(RS_THREADS), 0, st, a, d));
     JSM_LAUNCH_CHECK();
     return JSM_OK;
 }
 template <typename T, bool DELTA>
 static jsm_status scan_sized(const RecArgs& a, const RecDims& d, int n_segs, cudaStream_t st) {
     const int kp = d.kp();
-    return kp <= 32 ? scan_go<T, 4, DELTA>(a, d, n_segs, st) : kp <= 64 ? scan_go<T, 8, DELTA>(a, d, n_segs, st)
-         : kp <= 128 ? scan_go<T, 16, DELTA>(a, d, n_segs, st) : scan_go<T, 32, DELTA>(a, d, n_segs, st);
+    return kp <= 32 ? scan_go<T, 2, DELTA>(a, d, n_segs, st) : kp <= 64 ? scan_go<T, 4, DELTA>(a, d, n_segs, st)
+         : kp <= 128 ? scan_go<T, 8, DELTA>(a, d, n_segs, st) : scan_go<T, 16, DELTA>(a, d, n_segs, st);
 }
 
 template <typename T>

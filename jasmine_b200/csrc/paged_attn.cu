@@ -197,6 +197,106 @@ __global__ void __launch_bounds__(128) attn_paged_simt_kernel(const T* __restric
     for (int i = threadIdx.x; i < d.vdim; i += 128) out[(long long)t * d.out_cols() + h * d.vdim + i] = from_f32<T>(o[i] * f);
 }
 
+// The same for portions of prompts: a warp per (token, head of the group) row, eight rows of one kv head per CTA, which share
+// tiles of 32 keys and values in shared memory - the kernel above reads every key once per token and head and waits for it, 32
+// lanes a key.  Here a lane owns a key of the tile (vector loads, an odd number of 16-byte pieces per row: no bank conflicts)
+// and then columns lane, lane + 32, ... of the output.
+constexpr int AR_ROWS = 8, AR_KEYS = 32, AR_MAX_SMEM = 160 * 1024;
+__host__ __device__ constexpr int ar_pitch(int n) { return ((n + 3) / 4 | 1) * 4; }
+static size_t ar_smem(const AttnDims& d) { return sizeof(float) * ((size_t)(AR_KEYS + AR_ROWS) * ar_pitch(d.dim) + AR_KEYS * ar_pitch(d.vdim)); }
+
+template <typename T, int VR>  // VR: output columns per lane
+__global__ void __launch_bounds__(AR_ROWS * 32) attn_paged_rows_kernel(const T* __restrict__ q, AttnDims d, const float* __restrict__ sink, const T* __restrict__ pool,
+                                                                       const int32_t* __restrict__ block_table, int max_pages, StepTokens tk,
+                                                                       const int32_t* __restrict__ tile_seg, const int32_t* __restrict__ tile_r0, int rows,
+                                                                       const float* __restrict__ gate, T* __restrict__ out) {
+    extern __shared__ __align__(16) float ar_sm[];
+    const int kpitch = ar_pitch(d.dim), vpitch = ar_pitch(d.vdim), dim4 = (d.dim + 3) / 4, vdim4 = (d.vdim + 3) / 4;
+    float *Ks = ar_sm, *Vs = Ks + AR_KEYS * kpitch, *Qs = Vs + AR_KEYS * vpitch;
+    chain_trigger();
+    chain_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = blockIdx.y, gs = d.H / d.G;
+    const int seg = tile_seg[blockIdx.x], rb = tile_r0[blockIdx.x] + blockIdx.z * AR_ROWS;
+    const int n_rows = min(min(AR_ROWS, rows - (int)blockIdx.z * AR_ROWS), tk.seg_len[seg] * gs - rb);
+    if (n_rows <= 0) return;
+    const int pos0 = tk.seg_pos0[seg], r = rb + min(warp, n_rows - 1), h = g * gs + r % gs, pos = pos0 + r / gs;  // (a warp without a row repeats the last one)
+    const long long t = tk.seg_start[seg] + r / gs;
+    const int32_t* bt = block_table + (long long)tk.seg_row[seg] * max_pages;
+    float* qrow = Qs + warp * kpitch;
+    for (int i = lane; i < dim4 * 4; i += 32) qrow[i] = i < d.dim ? to_f32(q[t * d.q_cols() + h * d.qh() + i]) : 0.0f;
+    const int first = d.mask.first(pos), lo = d.mask.first(pos0 + rb / gs), hi = pos0 + (rb + n_rows - 1) / gs;
+    float m = sink ? sink[h] : -INFINITY, l = sink ? 1.0f : 0.0f, o[VR];
+#pragma unroll
+    for (int i = 0; i < VR; ++i) o[i] = 0.0f;
+    for (int c0 = lo; c0 <= hi; c0 += AR_KEYS) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < AR_KEYS * (dim4 + vdim4); e += AR_ROWS * 32) {
+            const int j = e / (dim4 + vdim4), x = e % (dim4 + vdim4), key = c0 + j;
+            const bool value = x >= dim4;
+            const int c = (value ? x - dim4 : x) * 4;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (key <= hi) {
+                const T* src = cache_at(const_cast<T*>(pool), d, bt[key / PAGE], g, value ? 1 : 0, key % PAGE, c);
+                if constexpr (sizeof(T) == 4) {
+                    v = *reinterpret_cast<const float4*>(src);
+                } else {
+                    const uint2 w = *reinterpret_cast<const uint2*>(src);
+                    v = make_float4(bf16lo(w.x), bf16hi(w.x), bf16lo(w.y), bf16hi(w.y));
+                }
+            }
+            *reinterpret_cast<float4*>((value ? Vs + j * vpitch : Ks + j * kpitch) + c) = v;
+        }
+        __syncthreads();
+        float a0 = 0.0f, a1 = 0.0f;
+        for (int i = 0; i < dim4; ++i) {
+            const float4 x = *reinterpret_cast<const float4*>(qrow + 4 * i), y = *reinterpret_cast<const float4*>(Ks + lane * kpitch + 4 * i);
+            a0 = fmaf(x.x, y.x, a0); a1 = fmaf(x.y, y.y, a1);
+            a0 = fmaf(x.z, y.z, a0); a1 = fmaf(x.w, y.w, a1);
+        }
+        const int key = c0 + lane;
+        const float s = key >= first && key <= pos ? (a0 + a1) * d.scale : -INFINITY;
+        const float m_new = fmaxf(m, warp_max(s));
+        if (m_new == -INFINITY) continue;  // (no key of this row yet: the whole warp agrees)
+        const float p = expf(s - m_new), alpha = expf(m - m_new);
+        l = l * alpha + warp_sum(p);
+        m = m_new;
+#pragma unroll
+        for (int i = 0; i < VR; ++i) o[i] *= alpha;
+        const int j_end = min(AR_KEYS, pos + 1 - c0);  // (a value that the row does not see may be anything)
+#pragma unroll 4
+        for (int j = max(0, first - c0); j < j_end; ++j) {
+            const float pj = __shfl_sync(0xffffffffu, p, j);
+#pragma unroll
+            for (int i = 0; i < VR; ++i)
+                if (lane + 32 * i < d.vdim) o[i] = fmaf(pj, Vs[j * vpitch + lane + 32 * i], o[i]);
+        }
+    }
+    if (warp >= n_rows) return;
+    const float f = (gate ? gate[t * d.H + h] : 1.0f) / l;
+#pragma unroll
+    for (int i = 0; i < VR; ++i)
+        if (lane + 32 * i < d.vdim) out[t * d.out_cols() + h * d.vdim + lane + 32 * i] = from_f32<T>(o[i] * f);
+}
+
+template <typename T, int VR>
+static jsm_status rows_go(const AttnDims& d, const AttnWeights& w, const AttnCache& cache, const StepTokens& tk, const AttnTiles& tl, const void* q,
+                          const float* gates, void* out, cudaStream_t st) {
+    static bool attr_done = false;
+    if (!attr_done) {
+        JSM_CUDA_CHECK(cudaFuncSetAttribute(attn_paged_rows_kernel<T, VR>, cudaFuncAttributeMaxDynamicSharedMemorySize, AR_MAX_SMEM));
+        attr_done = true;
+    }
+    JSM_CUDA_CHECK(launch_chained(attn_paged_rows_kernel<T, VR>, dim3(tl.n_tiles, d.G, (tl.rows + AR_ROWS - 1) / AR_ROWS), dim3(AR_ROWS * 32), ar_smem(d), st,
+                                  (const T*)q, d, w.sink, (const T*)cache.pool, cache.block_table, cache.max_pages, tk, tl.tile_seg, tl.tile_r0, tl.rows, gates, (T*)out));
+    JSM_LAUNCH_CHECK();
+    return JSM_OK;
+}
+template <typename T>
+static jsm_status rows_sized(const AttnDims& d, const AttnWeights& w, const AttnCache& cache, const StepTokens& tk, const AttnTiles& tl, const void* q,
+                             const float* gates, void* out, cudaStream_t st) {
+    return d.vdim <= 128 ? rows_go<T, 4>(d, w, cache, tk, tl, q, gates, out, st) : rows_go<T, 8>(d, w, cache, tk, tl, q, gates, out, st);
+}
+
 // ---- bf16 on the tensor cores -------------------------------------------------------------------------------------
 // A CTA owns 8 NB (token, head of the group) rows of one segment and kv head, and a run of pages.  A producer thread fetches
 // one block - the keys and values of the kv head in a page - per stage of a three-stage ring.  Each of four warps takes 16
@@ -533,6 +633,9 @@ jsm_status attn_paged_launch(bool f32, const AttnDims& d, const AttnWeights& w, 
     if (tl.n_tiles <= 0 || tl.t_count <= 0) return JSM_OK;
     const float* gates = d.gated ? gate : nullptr;
     if (f32 || !attn_mma_usable(d)) {
+        // rows in groups of eight once they make a CTA for every multiprocessor; a few rows keep a CTA each
+        if (tk.max_len > 1 && d.vdim <= 256 && ar_smem(d) <= AR_MAX_SMEM && (long long)tl.t_count * d.H >= (long long)AR_ROWS * sm_count())
+            return f32 ? rows_sized<float>(d, w, cache, tk, tl, q, gates, out, st) : rows_sized<__nv_bfloat16>(d, w, cache, tk, tl, q, gates, out, st);
         const size_t smem = sizeof(float) * (pad8(d.dim) + pad8(d.vdim) + 128 + 8);
         if (smem > 48 * 1024) JSM_FAIL(JSM_UNSUPPORTED, "attention: heads of %d / %d components", d.dim, d.vdim);
         if (f32)
