@@ -9,6 +9,7 @@ is missing, `lib()` raises.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 from pathlib import Path
 
@@ -200,43 +201,62 @@ def host_ptr(a):
 
 
 # ---- torch plumbing ------------------------------------------------------------
+_torch_module, _dtypes = None, {}
+
+
 def _torch():
-    import torch
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        _dtypes.update({torch.float32: F32, torch.bfloat16: BF16, torch.int32: I32})
+        _torch_module = torch
+    return _torch_module
 
 
 def stream_ptr() -> int:
-    return _torch().cuda.current_stream().cuda_stream
+    """Address of torch's current stream (the raw query: no Stream object is made for it)."""
+    torch = _torch()
+    if torch.cuda.is_initialized():
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    return torch.cuda.current_stream().cuda_stream
 
 
 def dtype_of(t) -> int:
-    torch = _torch()
-    return {torch.float32: F32, torch.bfloat16: BF16, torch.int32: I32}[t.dtype]
+    _torch()
+    return _dtypes[t.dtype]
 
 
 def mat(t, rows: int | None = None, cols: int | None = None) -> Mat:
     """A 2-D torch tensor (any strides, i.e. views and transposes) as a jsm_mat."""
     if t.dim() == 1:
         t = t.unsqueeze(0)
-    assert t.dim() == 2
-    return Mat(t.data_ptr(), t.shape[0], t.shape[1], t.stride(0), t.stride(1), dtype_of(t))
+    shape, stride = t.shape, t.stride()  # (each attribute of a tensor costs a call into torch: asked once)
+    assert len(shape) == 2
+    return Mat(t.data_ptr(), shape[0], shape[1], stride[0], stride[1], _dtypes[t.dtype] if _dtypes else dtype_of(t))
+
+
+@functools.lru_cache(maxsize=64)
+def _array(kind, n):
+    """The ctypes array type of n structs: making a type takes longer than filling it."""
+    return kind * n
 
 
 def program(instrs):
     """[(op, arg_or_imm), ...] -> (Instr array, n).  LEAF takes a leaf index, IMM/POW a float."""
-    arr = (Instr * len(instrs))()
+    n = len(instrs)
+    arr = _array(Instr, n)()
     for k, ins in enumerate(instrs):
         op = ins[0]
         a = ins[1] if len(ins) > 1 else 0
         if op in (OP_IMM, OP_POW):
-            arr[k] = Instr(op, 0, float(a))
+            arr[k] = (op, 0, float(a))
         else:
-            arr[k] = Instr(op, int(a), 0.0)
-    return arr, len(instrs)
+            arr[k] = (op, int(a), 0.0)
+    return arr, n
 
 
 def _leaves(ts):
-    arr = (Mat * max(1, len(ts)))()
+    arr = _array(Mat, max(1, len(ts)))()
     for k, t in enumerate(ts):
         arr[k] = mat(t)
     return arr, len(ts)
