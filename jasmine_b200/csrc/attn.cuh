@@ -13,6 +13,9 @@ jsm_status flash_prefill_launch(const void* q, const void* k, const void* v, voi
 
 jsm_status rope_apply_strided(const void* d_x, void* d_out, jsm_dtype dtype, const float* d_table, int d, int n_heads,
                               const int32_t* d_positions, int T, long long row_stride, void* stream);
+// fused rows [q | k | v] of a prompt (heads of 128): q and k rotated in place, rotated k and v also into the pages of the token's sequence
+jsm_status rope_append_launch(void* x, long long row_stride, int Hq, int Hkv, const float* table, void* pool, const int32_t* block_table, int max_pages,
+                              const int32_t* seq_ids, const int32_t* positions, int T, cudaStream_t st);
 
 // decode attention of grouped-query models on the tensor cores (attn_decode_mma.cu)
 bool attn_decode_mma_usable(int G, int chunk, const void* pool);

@@ -606,10 +606,8 @@ static jsm_status forward_tokens(jsm_model* m, const int32_t* d_ids, int T, bool
                                            m->attn_counters, m->attn, st);
         } else {
             // prompt of one sequence starting at position 0: rotate q and k in place (the first Hq + Hkv heads of every
-            // fused row), cache K and V, then causal attention over the fresh q, k, v
-            s = rope_apply_strided(m->qkv, m->qkv, JSM_BF16, m->rope, D, m->Hq_l + m->Hkv_l, m->pos, T, m->qkv_dim, st);
-            if (s != JSM_OK) return s;
-            s = jsm_kv_append(L.pool, m->block_table, m->pages_per_seq, kk, vv, m->qkv_dim, m->seq_ids, m->pos, T, m->Hkv_l, D, nullptr, st);
+            // fused row) and cache K and V, then causal attention over the fresh q, k, v
+            s = rope_append_launch(m->qkv, m->qkv_dim, m->Hq_l, m->Hkv_l, m->rope, L.pool, m->block_table, m->pages_per_seq, m->seq_ids, m->pos, T, st);
             if (s != JSM_OK) return s;
             if (T >= 128)
                 s = flash_prefill_launch(m->qkv, kk, vv, m->attn, 1, T, T, m->Hq_l, m->Hkv_l, 1, scale, nullptr, st, m->qkv_dim,

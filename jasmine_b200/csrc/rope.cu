@@ -113,6 +113,50 @@ __global__ void __launch_bounds__(256) rope_apply_bf16_heads_kernel(const __nv_b
     }
 }
 
+// A prompt's fused rows [q heads | k heads | v heads] of 128 columns: queries and keys are rotated in place, rotated keys and
+// values also go to their cache pages.  One pass over the rows, 16 bytes per thread and head, in place of a rotation and an append
+// that read the keys again in 4-byte pieces with a block per token and head: 5.8 + 19.2 -> 6 us for 512 tokens of 32 + 32 + 32
+// heads.  Block and table as above.
+__global__ void __launch_bounds__(256) rope_append_kernel(__nv_bfloat16* __restrict__ x, long long row_stride, int Hq, int Hkv,
+                                                          const float4* __restrict__ table, __nv_bfloat16* __restrict__ pool,
+                                                          const int32_t* __restrict__ block_table, int max_pages,
+                                                          const int32_t* __restrict__ seq_ids, const int32_t* __restrict__ positions) {
+    constexpr int D = 128;
+    chain_trigger();
+    chain_wait();
+    const int qd = threadIdx.x & 15, hl = threadIdx.x >> 4, t = blockIdx.x, n_heads = Hq + 2 * Hkv;
+    const int pos = positions[t], seq = seq_ids[t];
+    __nv_bfloat16* row = x + (long long)t * row_stride + 8 * qd;
+    const float4* e = table + (long long)pos * (D / 2) + qd * 4;
+    const float4 c[4] = {e[0], e[1], e[2], e[3]};
+    const long long page = block_table[(long long)seq * max_pages + pos / JSM_PAGE_SIZE];
+    __nv_bfloat16* entry = pool + page * (2ll * Hkv * JSM_PAGE_SIZE * D) + (pos % JSM_PAGE_SIZE) * D + 8 * qd;  // key of kv head 0; values follow the keys
+    for (int h0 = hl; h0 < n_heads; h0 += 64) {
+        uint4 w[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (h0 + 16 * u < n_heads) w[u] = *reinterpret_cast<const uint4*>(row + (long long)(h0 + 16 * u) * D);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int h = h0 + 16 * u;
+            if (h >= n_heads) break;
+            if (h < Hq + Hkv) {
+                const uint32_t in[4] = {w[u].x, w[u].y, w[u].z, w[u].w};
+                uint32_t o[4];
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    const float x0 = bf16lo(in[p]), x1 = bf16hi(in[p]);
+                    o[p] = pack_bf16x2(__fadd_rn(__fmul_rn(c[p].x, x0), __fmul_rn(-c[p].w, x1)),
+                                       __fadd_rn(__fmul_rn(c[p].y, x0), __fmul_rn(c[p].z, x1)));
+                }
+                w[u] = make_uint4(o[0], o[1], o[2], o[3]);
+                *reinterpret_cast<uint4*>(row + (long long)h * D) = w[u];
+            }
+            if (h >= Hq) *reinterpret_cast<uint4*>(entry + (long long)(h - Hq) * JSM_PAGE_SIZE * D) = w[u];
+        }
+    }
+}
+
 // Queries and keys of a prefill in ONE launch (two tensors, the same positions): a thread issues the loads of all its
 // heads of both tensors before the first rotation (four 16-byte loads in flight per thread at 32 + 32 heads instead of
 // two), and the table entries of the next token are requested before the current token is rotated.
@@ -219,6 +263,14 @@ extern "C" jsm_status jsm_rope_table(float* d_table, int mode, int d, float thet
 extern "C" jsm_status jsm_rope_apply(const void* d_x, void* d_out, jsm_dtype dtype, const float* d_table, int d, int n_heads,
                                      const int32_t* d_positions, int T, void* stream) {
     return jsm::rope_apply_strided(d_x, d_out, dtype, d_table, d, n_heads, d_positions, T, (long long)n_heads * d, stream);
+}
+
+jsm_status jsm::rope_append_launch(void* x, long long row_stride, int Hq, int Hkv, const float* table, void* pool, const int32_t* block_table, int max_pages,
+                                   const int32_t* seq_ids, const int32_t* positions, int T, cudaStream_t st) {
+    JSM_CUDA_CHECK(launch_chained(rope_append_kernel, dim3(T), dim3(256), 0, st, (__nv_bfloat16*)x, row_stride, Hq, Hkv, (const float4*)table,
+                                  (__nv_bfloat16*)pool, block_table, max_pages, seq_ids, positions));
+    JSM_LAUNCH_CHECK();
+    return JSM_OK;
 }
 
 // rows of `row_stride` elements whose first n_heads * d entries are rotated (in place when d_out == d_x)
