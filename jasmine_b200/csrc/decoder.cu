@@ -34,7 +34,6 @@ struct Proj {  // one projection: N outputs, K inputs, both rounded up to multip
     int N = 0, K = 0, paired = 0;
     uint8_t* packed = nullptr;  // bf16 models
     float* w32 = nullptr;       // f32 models, [N][K]
-    void* rows = nullptr;       // bf16 models, projections with few outputs or few inputs: also row-major, for many tokens
 };
 
 struct DecLayer {
@@ -295,14 +294,14 @@ static jsm_status build_scan(jsm_decoder* m, DecLayer& L, const std::string& pre
             h.put_row(d.rp() + d.np() + j, *xp, d.dt_rank + d.state + j);
         }
         DEC_TRY(upload_proj(m, h, &L.xp));
-        if (!m->f32) DEC_TRY(upload_plain(m, h, &L.xp.rows));
     }
     {
         HostMatrix h(m->f32, ip, d.rp());
         for (int j = 0; j < d.inner; ++j) h.put_row(j, *dt, j);
         DEC_TRY(upload_proj(m, h, &L.dt));
-        if (!m->f32) DEC_TRY(upload_plain(m, h, &L.dt.rows));
-        L.sw.dt = m->f32 ? (void*)L.dt.w32 : L.dt.rows;
+        void* rows = L.dt.w32;  // (the decode step takes them row-major)
+        if (!m->f32) DEC_TRY(upload_plain(m, h, &rows));
+        L.sw.dt = rows;
     }
     {
         HostMatrix h(m->f32, wp, ip);
@@ -459,8 +458,9 @@ static jsm_status build_recurrence(jsm_decoder* m, DecLayer& L, const std::strin
         h.put_row(d.ba_cols() / 2 + i, *a, i);
     }
     DEC_TRY(upload_proj(m, h, &L.xp));
-    if (!m->f32) DEC_TRY(upload_plain(m, h, &L.xp.rows));
-    L.rw.ba = m->f32 ? (void*)L.xp.w32 : L.xp.rows;
+    void* rows = L.xp.w32;  // (the decode step takes them row-major)
+    if (!m->f32) DEC_TRY(upload_plain(m, h, &rows));
+    L.rw.ba = rows;
     return JSM_OK;
 }
 
@@ -510,20 +510,6 @@ static jsm_status linear(jsm_decoder* m, const Proj& p, const void* X, long long
     a.N = p.N; a.K = p.K; a.x_row_stride = x_stride;
     a.ws = m->ws; a.ws_floats = m->ws_floats; a.counters = m->counters; a.n_counters = m->n_counters;
     a.chained = true;  // the weights are constant while the model's stream runs
-    if (p.rows && T > 64 && x_stride == p.K) {
-        // the packed kernel streams the weights once per 256 tokens over all SMs, which suits wide and deep matrices; here one
-        // launch tiles outputs x tokens, split along K while that leaves SMs idle
-        const int tiles = ((p.N + 127) / 128) * ((T + 127) / 128);
-        LinearArgs r;
-        r.X = X; r.W = p.rows; r.bias = nullptr; r.epilogue = LIN_NONE; r.R = nullptr; r.Y = Y;
-        r.out_mode = out_f32 ? 1 : 0;
-        r.T = T; r.N = p.N; r.K = p.K; r.impl = 2;
-        r.splits = std::max(1, std::min(sm_count() / tiles, p.K / 512));
-        r.ws = r.splits > 1 ? m->ws : nullptr;
-        r.counters = m->counters;
-        r.chained = true;
-        return linear_bf16_launch(r, st);
-    }
     a.T = T; a.X = X; a.Y = Y;
     return linear_packed_tokens(a, st);
 }
