@@ -26,28 +26,50 @@ constexpr int DOT_THREADS = 128, DOT_KB = 32, DOT_PITCH = DOT_KB + 4;
 constexpr int dot_stages(int tnn) { return tnn == 1 ? 8 : 4; }
 constexpr int dot_smem(int tmm, int tnn) { return dot_stages(tnn) * (8 * tmm + 16 * tnn) * DOT_PITCH * 4; }
 
-// 32 products' worth of ROWS rows of an operand (row stride rs, stride ks along the products), zeros where there is nothing.
-// vec: contiguous products, 16-byte aligned rows.
+// One thread's part in staging 32 products' worth of ROWS rows of an operand (row stride rs, stride ks along the products), zeros where
+// there is nothing.  vec: contiguous products, 16-byte aligned rows; a thread has the same four products of every 16th row, so
+// its addresses and bounds are worked out once.
 template <int ROWS>
-__device__ __forceinline__ void dot_stage(uint32_t dst, const float* p, int row0, int rows, long long rs, long long ks, int k0, int K, bool vec) {
-    if (vec) {
-#pragma unroll
-        for (int e = threadIdx.x; e < ROWS * (DOT_KB / 4); e += DOT_THREADS) {
-            const int r = e / (DOT_KB / 4), c = e % (DOT_KB / 4) * 4;
-            const int left = row0 + r < rows ? min(max(K - k0 - c, 0), 4) : 0;
-            const float* src = left ? p + (row0 + r) * rs + k0 + c : p;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (r * DOT_PITCH + c) * 4), "l"(reinterpret_cast<uint64_t>(src)), "r"(left * 4)
-                         : "memory");
-        }
-    } else {
-        const bool along_k = rs != 1;  // the threads walk the contiguous direction
-        for (int e = threadIdx.x; e < ROWS * DOT_KB; e += DOT_THREADS) {
-            const int r = along_k ? e / DOT_KB : e % ROWS, c = along_k ? e % DOT_KB : e / ROWS;
-            const bool on = row0 + r < rows && k0 + c < K;
-            cp_async4(dst + (r * DOT_PITCH + c) * 4, on ? p + (row0 + r) * rs + (k0 + c) * ks : p, on);
+struct DotLoader {
+    static constexpr int STEP = DOT_THREADS / (DOT_KB / 4), N = ROWS / STEP;  // rows per pass, passes
+    static_assert(ROWS % STEP == 0, "whole passes");
+    const float *base, *p;  // the operand; vec: first piece of the thread
+    long long rs, ks;
+    int row0, rows, K, c;
+    bool vec;
+    uint32_t dst;     // offset of the thread's first piece in a stage
+    __device__ __forceinline__ DotLoader(const float* base, int row0, int rows, long long rs, long long ks, int K, bool vec)
+        : base(base), p(base), rs(rs), ks(ks), row0(row0), rows(rows), K(K), vec(vec) {
+        const int r = threadIdx.x / (DOT_KB / 4);
+        c = threadIdx.x % (DOT_KB / 4) * 4;
+        dst = (r * DOT_PITCH + c) * 4;
+        if (vec) {
+            p = base + (long long)(row0 + r) * rs + c;
+            this->rows = rows - row0 - r;  // pass i has a row if i STEP < rows
         }
     }
-}
+    __device__ __forceinline__ void operator()(uint32_t stage, int k0) const {
+        if (vec) {
+            const int left = min(max(K - k0 - c, 0), 4) * 4;
+            const float* src = p + k0;
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const int bytes = i * STEP < rows ? left : 0;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(stage + dst + i * STEP * DOT_PITCH * 4),
+                             "l"(reinterpret_cast<uint64_t>(bytes ? src : base)), "r"(bytes)
+                             : "memory");
+                src += STEP * rs;
+            }
+        } else {
+            const bool along_k = rs != 1;  // the threads walk the contiguous direction
+            for (int e = threadIdx.x; e < ROWS * DOT_KB; e += DOT_THREADS) {
+                const int r = along_k ? e / DOT_KB : e % ROWS, x = along_k ? e % DOT_KB : e / ROWS;
+                const bool on = row0 + r < rows && k0 + x < K;
+                cp_async4(stage + (r * DOT_PITCH + x) * 4, on ? base + (row0 + r) * rs + (k0 + x) * ks : base, on);
+            }
+        }
+    }
+};
 
 // Before, one 64 x 64 tile per CTA staged element by element: 64 x 128 x 128 took 27 us, 300 x 1024 x 2752 (f32 model) 182 us.
 // What bounds it: with few outputs the chain of K dependent additions and the launch, with many the fp32 pipe (two instructions
@@ -57,7 +79,7 @@ __device__ __forceinline__ void dot_stage(uint32_t dst, const float* p, int row0
 // Otherwise: even and odd products of a block of 32 form two chains of fused multiply-adds (packed pairs), which join the total
 // once per block; a cluster of CTAs shares the products of a tile (whole blocks each) and adds its totals in rank order.
 template <bool ORDERED, int TMM, int TNN>
-__global__ void __launch_bounds__(DOT_THREADS) dot_f32_kernel(MatD A, MatD B, MatD bias, int has_bias, int epilogue, MatD R,
+__global__ void __launch_bounds__(DOT_THREADS, TMM == 8 ? 3 : 4) dot_f32_kernel(MatD A, MatD B, MatD bias, int has_bias, int epilogue, MatD R,
                                                               float* Cp, long long crs, long long ccs, int M, int N, int K, int vec_a, int vec_b) {
     constexpr int BM = 8 * TMM, BN = 16 * TNN, STAGES = dot_stages(TNN), STAGE = (BM + BN) * DOT_PITCH;
     static_assert(STAGES * STAGE >= BM * BN, "the totals of a tile are exchanged through the ring");
@@ -68,8 +90,10 @@ __global__ void __launch_bounds__(DOT_THREADS) dot_f32_kernel(MatD A, MatD B, Ma
     const int splits = ORDERED ? 1 : gridDim.z, rank = ORDERED ? 0 : blockIdx.z;
     const int blocks = (K + DOT_KB - 1) / DOT_KB, b0 = (int)((long long)blocks * rank / splits), mine = (int)((long long)blocks * (rank + 1) / splits) - b0;
     const uint32_t ring = smem_u32(dot_ring);
-    auto stage_a = [&](int i) { dot_stage<BM>(ring + (i % STAGES) * STAGE * 4, A.p, m0, M, A.rs, A.cs, (b0 + i) * DOT_KB, K, vec_a); };
-    auto stage_b = [&](int i) { dot_stage<BN>(ring + ((i % STAGES) * STAGE + BM * DOT_PITCH) * 4, B.p, n0, N, B.cs, B.rs, (b0 + i) * DOT_KB, K, vec_b); };
+    const DotLoader<BM> load_a(A.p, m0, M, A.rs, A.cs, K, vec_a);
+    const DotLoader<BN> load_b(B.p, n0, N, B.cs, B.rs, K, vec_b);
+    auto stage_a = [&](int i) { load_a(ring + (i % STAGES) * STAGE * 4, (b0 + i) * DOT_KB); };
+    auto stage_b = [&](int i) { load_b(ring + ((i % STAGES) * STAGE + BM * DOT_PITCH) * 4, (b0 + i) * DOT_KB); };
     if (!ORDERED) {  // B holds weights: they may be requested before the predecessor kernel has ended
         chain_trigger();
         for (int i = 0; i < STAGES - 1 && i < mine; ++i) stage_b(i);
@@ -98,15 +122,9 @@ __global__ void __launch_bounds__(DOT_THREADS) dot_f32_kernel(MatD A, MatD B, Ma
         }
         cp_async_commit();
         const float *as = dot_ring + (b % STAGES) * STAGE + ty * DOT_PITCH, *bs = dot_ring + (b % STAGES) * STAGE + (BM + tx) * DOT_PITCH;
-        uint64_t part[TMM][TNN];
-        if (!ORDERED)
-#pragma unroll
-            for (int i = 0; i < TMM; ++i)
-#pragma unroll
-                for (int j = 0; j < TNN; ++j) part[i][j] = 0;
+        if constexpr (ORDERED) {
 #pragma unroll 2
-        for (int k = 0; k < DOT_KB; k += 4) {
-            if constexpr (ORDERED) {
+            for (int k = 0; k < DOT_KB; k += 4) {
                 float4 x[TMM], y[TNN];
 #pragma unroll
                 for (int i = 0; i < TMM; ++i) x[i] = *reinterpret_cast<const float4*>(as + i * 8 * DOT_PITCH + k);
@@ -122,7 +140,11 @@ __global__ void __launch_bounds__(DOT_THREADS) dot_f32_kernel(MatD A, MatD B, Ma
                         s = __fadd_rn(s, __fmul_rn(x[i].z, y[j].z));
                         acc[i][j] = __fadd_rn(s, __fmul_rn(x[i].w, y[j].w));
                     }
-            } else {
+            }
+        } else {
+            uint64_t part[TMM][TNN];  // (a product's operands are a pass over all outputs apart: no instruction waits for the one before it)
+#pragma unroll
+            for (int k = 0; k < DOT_KB; k += 4) {
                 ulonglong2 x[TMM], y[TNN];
 #pragma unroll
                 for (int i = 0; i < TMM; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(as + i * 8 * DOT_PITCH + k);
@@ -131,10 +153,12 @@ __global__ void __launch_bounds__(DOT_THREADS) dot_f32_kernel(MatD A, MatD B, Ma
 #pragma unroll
                 for (int i = 0; i < TMM; ++i)
 #pragma unroll
-                    for (int j = 0; j < TNN; ++j) part[i][j] = f2_fma(x[i].y, y[j].y, f2_fma(x[i].x, y[j].x, part[i][j]));
+                    for (int j = 0; j < TNN; ++j) part[i][j] = k == 0 ? f2_mul(x[i].x, y[j].x) : f2_fma(x[i].x, y[j].x, part[i][j]);
+#pragma unroll
+                for (int i = 0; i < TMM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TNN; ++j) part[i][j] = f2_fma(x[i].y, y[j].y, part[i][j]);
             }
-        }
-        if (!ORDERED)
 #pragma unroll
             for (int i = 0; i < TMM; ++i)
 #pragma unroll
@@ -143,6 +167,7 @@ __global__ void __launch_bounds__(DOT_THREADS) dot_f32_kernel(MatD A, MatD B, Ma
                     f2_unpack(part[i][j], even, odd);
                     acc[i][j] += even + odd;
                 }
+        }
     }
     if constexpr (ORDERED) {
 #pragma unroll
