@@ -109,6 +109,7 @@ jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st);  // T <= 
 // any T; the launches of a call that is split share R, Y and the row statistics of the whole call
 jsm_status linear_packed_tokens(const PackedArgs& a, cudaStream_t st);
 jsm_status linear_tiled_launch(const PackedArgs& a, cudaStream_t st);
+jsm_status linear_mid_launch(const PackedArgs& a, cudaStream_t st);  // T <= 128, without an exchange
 // exchange regions (tp_comm.cu): [flags | buffer A | buffer B | push buffer 0 | push buffer 1]
 size_t tp_region_bytes(int max_tokens, int d);
 size_t tp_buffer_offset(int which, int max_tokens, int d);

@@ -1167,9 +1167,9 @@ static bool use_tiled(int T, int K) { return T > 128 || (T > 64 && K < 4096); }
 // Any number of tokens, in one launch of the tiled kernel (linear_tiled.cu) or launches of at most 256 tokens.
 jsm_status linear_packed_tokens(const PackedArgs& a, cudaStream_t st) {
     if (a.T <= 0 || a.N <= 0) return JSM_OK;
-    if (use_tiled(a.T, a.K) && !a.tp) {
+    if (!a.tp && a.T > 16) {
         jsm_status s = packed_check(a, std::min(a.T, 256), packed_paired(a));
-        return s != JSM_OK ? s : linear_tiled_launch(a, st);
+        return s != JSM_OK ? s : use_tiled(a.T, a.K) ? linear_tiled_launch(a, st) : linear_mid_launch(a, st);
     }
     PackedArgs c = a;
     const long long xs = a.x_row_stride > 0 ? a.x_row_stride : a.K;
