@@ -94,16 +94,12 @@ __global__ void __launch_bounds__(DOT_THREADS, TMM == 8 ? 3 : 4) dot_f32_kernel(
     const DotLoader<BN> load_b(B.p, n0, N, B.cs, B.rs, K, vec_b);
     auto stage_a = [&](int i) { load_a(ring + (i % STAGES) * STAGE * 4, (b0 + i) * DOT_KB); };
     auto stage_b = [&](int i) { load_b(ring + ((i % STAGES) * STAGE + BM * DOT_PITCH) * 4, (b0 + i) * DOT_KB); };
-    if (!ORDERED) {  // B holds weights: they may be requested before the predecessor kernel has ended
-        chain_trigger();
-        for (int i = 0; i < STAGES - 1 && i < mine; ++i) stage_b(i);
-        chain_wait();
-    }
+    if (!ORDERED) chain_trigger();
 #pragma unroll 1
     for (int i = 0; i < STAGES - 1; ++i) {
         if (i < mine) {
             stage_a(i);
-            if (ORDERED) stage_b(i);
+            stage_b(i);
         }
         cp_async_commit();
     }
@@ -238,22 +234,19 @@ static jsm_status dot_launch(const MatD& A, const MatD& B, const MatD* bias, int
     cfg.blockDim = dim3(DOT_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = splits;
-    cfg.attrs = ORDERED || !chained_launch_enabled() ? attr + 1 : attr;
-    cfg.numAttrs = (cfg.attrs == attr ? 1 : 0) + (splits > 1 ? 1 : 0);
+    cudaLaunchAttribute attr[1];  // (plain stream order: see launch_spread)
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = splits;
+    cfg.attrs = attr;
+    cfg.numAttrs = splits > 1 ? 1 : 0;
     JSM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, dot_f32_kernel<ORDERED, TMM, TNN>, A, B, bias ? *bias : none, bias ? 1 : 0, epilogue, R ? *R : none, C, crs, ccs, A.rows,
                                       B.cols, A.cols, dot_vec(A.p, A.rs, A.cs), dot_vec(B.p, B.cs, B.rs)));
     g_launches.fetch_add(1);
     return JSM_OK;
 }
 
-// C = A . B in fp32 without the reference's order (operands as in jsm_dot_f32, checked by the caller; B holds weights, constant
-// while the stream runs).  Few rows take 16 x 64 tiles.  The products of a tile are shared by as many CTAs as even out the
+// C = A . B in fp32 without the reference's order (operands as in jsm_dot_f32, checked by the caller).  Few rows take 16 x 64 tiles.  The products of a tile are shared by as many CTAs as even out the
 // multiprocessors' loads: rounds of CTAs times blocks of products each, and about four blocks' time for a CTA's start and end.
 jsm_status dot_f32_launch(const jsm_mat& A, const jsm_mat& B, const jsm_mat& Cm, cudaStream_t st) {
     const bool few = A.rows <= 32;

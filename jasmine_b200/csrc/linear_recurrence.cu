@@ -945,7 +945,7 @@ static RecArgs rec_args(bool f32, const RecDims& d, const RecWeights& w, const R
 
 template <typename T, int NR, bool DELTA>
 static jsm_status scan_go(const RecArgs& a, const RecDims& d, int n_segs, cudaStream_t st) {
-    JSM_CUDA_CHECK(launch_chained(rec_scan_kernel<T, NR, DELTA>, dim3((d.vp() + RS_COLS - 1) / RS_COLS, d.H, n_segs), dim3(RS_THREADS), 0, st, a, d));
+    JSM_CUDA_CHECK(launch_spread(rec_scan_kernel<T, NR, DELTA>, dim3((d.vp() + RS_COLS - 1) / RS_COLS, d.H, n_segs), dim3(RS_THREADS), 0, st, a, d));
     JSM_LAUNCH_CHECK();
     return JSM_OK;
 }
@@ -998,7 +998,7 @@ static jsm_status chunk_go(const RecArgs& a, const RecDims& d, const RecChunks& 
     if (s != JSM_OK) return s;
     s = make_tmap_bf16_2d(&map_v, a.qkv, (uint64_t)n_tok, (uint64_t)d.conv_cols(), (uint64_t)d.conv_cols(), RC_C, cols, false);
     if (s != JSM_OK) return s;
-    JSM_CUDA_CHECK(launch_chained(rec_chunk_kernel<KT, DELTA>, dim3((d.vp() + cols - 1) / cols, d.H, n_segs), dim3(cols * 8 + 32), smem, st, map_qk, map_v, a, d, ch.seg_chunk0,
+    JSM_CUDA_CHECK(launch_spread(rec_chunk_kernel<KT, DELTA>, dim3((d.vp() + cols - 1) / cols, d.H, n_segs), dim3(cols * 8 + 32), smem, st, map_qk, map_v, a, d, ch.seg_chunk0,
                                   static_cast<const uint8_t*>(ch.ws), tc_error_word()));
     JSM_LAUNCH_CHECK();
     return JSM_OK;

@@ -286,7 +286,7 @@ static jsm_status rows_go(const AttnDims& d, const AttnWeights& w, const AttnCac
         JSM_CUDA_CHECK(cudaFuncSetAttribute(attn_paged_rows_kernel<T, VR>, cudaFuncAttributeMaxDynamicSharedMemorySize, AR_MAX_SMEM));
         attr_done = true;
     }
-    JSM_CUDA_CHECK(launch_chained(attn_paged_rows_kernel<T, VR>, dim3(tl.n_tiles, d.G, (tl.rows + AR_ROWS - 1) / AR_ROWS), dim3(AR_ROWS * 32), ar_smem(d), st,
+    JSM_CUDA_CHECK(launch_spread(attn_paged_rows_kernel<T, VR>, dim3(tl.n_tiles, d.G, (tl.rows + AR_ROWS - 1) / AR_ROWS), dim3(AR_ROWS * 32), ar_smem(d), st,
                                   (const T*)q, d, w.sink, (const T*)cache.pool, cache.block_table, cache.max_pages, tk, tl.tile_seg, tl.tile_r0, tl.rows, gates, (T*)out));
     JSM_LAUNCH_CHECK();
     return JSM_OK;

@@ -588,7 +588,7 @@ static jsm_status scan_go(const ScanArgs& a, cudaStream_t st) {
         JSM_CUDA_CHECK(cudaFuncSetAttribute(scan_kernel<T, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         attr_done = true;
     }
-    JSM_CUDA_CHECK(launch_chained(scan_kernel<T, NS>, dim3((a.ip + SC_CH - 1) / SC_CH, a.n_segs), dim3(SC_THREADS), scan_smem<T>(a.np, NS), st, a));
+    JSM_CUDA_CHECK(launch_spread(scan_kernel<T, NS>, dim3((a.ip + SC_CH - 1) / SC_CH, a.n_segs), dim3(SC_THREADS), scan_smem<T>(a.np, NS), st, a));
     JSM_LAUNCH_CHECK();
     return JSM_OK;
 }
