@@ -193,14 +193,8 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
     __shared__ uint32_t tmem_base_smem;
     __shared__ int abort_flag;
     __shared__ int is_last_smem[2];
-    // ROWS: whole tiles that do not end the CTA's range take the row-per-thread epilogue straight from the accumulator (the
-    // stage ring is busy).  The images of up to 64 tokens have a staging tile of their own instead and send every whole
-    // tile through the vectorised epilogue: one epilogue, a third less code to fetch in the tail that runs once per launch.
-    constexpr bool ROWS = BN >= 128;
-    __shared__ float pair_smem[ROWS ? 64 * 17 : 1];   // paired epilogue: up values of 16 token columns, padded rows
-    __shared__ float row_scale[256];                  // 1 / rms of every token when the RMSNorm is fused into this projection
-    __shared__ float ssq_part[ROWS ? 4 * 256 : 1];    // per-warp sums of squares of a whole tile's outputs
-    __shared__ __align__(16) float stage_small[ROWS ? 4 : BN * 128];  // up to 64 tokens: a whole tile's accumulator
+    __shared__ float row_scale[BN];       // 1 / rms of every token when the RMSNorm is fused into this projection
+    __shared__ __align__(16) float stage_small[BN * 128];  // a whole tile's accumulator: every tile takes the one vectorised epilogue
     __shared__ int tp_ok_smem;            // reduce: every peer's flag arrived in time
 
     // PRM: what the image can do.  -1: everything; 0 / 1: plain tiles only / gate-up pairs only (what the other kind needs is
@@ -587,98 +581,14 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
             tc_fence_after();
             const bool scaled = has_ssq_in;
             const uint32_t acc_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN);
-            // A whole tile that is this CTA's last segment goes through shared memory (the stage ring is free: every MMA
-            // of the CTA has completed) and the vectorised epilogue below, whose stores are 8 or 16 bytes per thread and
-            // contiguous per token; earlier segments overlap the main loop and keep the row-per-thread epilogue.
-            const bool local = whole && (!ROWS || ((u + len == u_end) && P.local_epi));
-            bool rows_done = false;
-            if constexpr (ROWS) {
-            if (whole && !local) {
-                rows_done = true;
-                // ---- the tile is complete in this CTA: epilogue straight from the accumulator
-                if (!paired) {
-                    const int n = tile * 128 + row;
-                    const bool valid = n < P.N;
-                    const float bias = (biasp && valid) ? biasp[n] : 0.0f;
-#pragma unroll 1
-                    for (int c0 = 0; c0 < BN; c0 += 16) {
-                        if (c0 >= P.T) break;
-                        uint32_t r[16];
-                        tmem_ld16(acc_addr + c0, r);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const int t = c0 + j;  // warp-uniform
-                            if (t < P.T) {
-                                float v = __uint_as_float(r[j]);
-                                if (scaled) v *= row_scale[t];
-                                v += bias;
-                                if (epi == LIN_RELU) v = fmaxf(v, 0.0f);
-                                else if (epi == LIN_GELU) v = pk_gelu(v);
-                                else if ((!paired && epi == LIN_RESIDUAL) && valid) v += __bfloat162float(P.R[(size_t)t * P.N + n]);
-                                float stored = v;
-                                if (!f32o) {
-                                    const __nv_bfloat16 hb = __float2bfloat16_rn(v);
-                                    stored = __bfloat162float(hb);
-                                    if (valid) reinterpret_cast<__nv_bfloat16*>(P.Y)[(size_t)t * P.N + n] = hb;
-                                } else if (valid) {
-                                    reinterpret_cast<float*>(P.Y)[(size_t)t * P.N + n] = v;
-                                }
-                                if (want_ssq) {  // sum of squares of what was stored, over the 128 features of the tile
-                                    const float sq = warp_sum(valid ? stored * stored : 0.0f);
-                                    if (lane == 0) ssq_part[quad * 256 + t] = sq;
-                                }
-                            }
-                        }
-                    }
-                    if (want_ssq) {
-                        asm volatile("bar.sync 1, 128;" ::: "memory");
-                        for (int t = etid; t < P.T; t += 128)
-                            P.ssq_out[(size_t)tile * P.ssq_stride + t] = (ssq_part[t] + ssq_part[256 + t]) + (ssq_part[512 + t] + ssq_part[768 + t]);
-                        asm volatile("bar.sync 1, 128;" ::: "memory");
-                    }
-                } else {
-                    // lanes 0..63 hold gate, lanes 64..127 the matching up rows: hand the up values over through shared memory
-                    const int f = row & 63;
-                    const int n = tile * 64 + f;
-#pragma unroll 1
-                    for (int c0 = 0; c0 < BN; c0 += 16) {
-                        if (c0 >= P.T) break;
-                        uint32_t r[16];
-                        tmem_ld16(acc_addr + c0, r);
-                        tmem_ld_wait();
-                        if (row >= 64) {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) pair_smem[f * 17 + j] = __uint_as_float(r[j]);
-                        }
-                        asm volatile("bar.sync 1, 128;" ::: "memory");
-                        if (row < 64 && n < P.N) {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                const int t = c0 + j;
-                                if (t < P.T) {
-                                    const float sc = scaled ? row_scale[t] : 1.0f;
-                                    const float v = gate_up(__uint_as_float(r[j]) * sc, pair_smem[f * 17 + j] * sc);
-                                    if (f32o) reinterpret_cast<float*>(P.Y)[(size_t)t * P.N + n] = v;
-                                    else reinterpret_cast<__nv_bfloat16*>(P.Y)[(size_t)t * P.N + n] = __float2bfloat16_rn(v);
-                                }
-                            }
-                        }
-                        asm volatile("bar.sync 1, 128;" ::: "memory");
-                    }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty[buf]);
-            }
-            }
-            if (!rows_done) {
+            const bool local = whole;  // a whole tile goes through its staging tile, a shared one as described below
+            {
                 // ---- shared tile: store the raw partial in this CTA's slot, the last contributor folds
                 // aligned split: the contributors are the CTAs of this cluster and the partial goes to this CTA's own shared
                 // memory (the stage ring is free: every MMA of the CTA has completed); otherwise to its workspace slot
                 const bool cl = CL && P.cluster_s > 1 && !local;
-                float* part_smem = (!ROWS && local) ? stage_small : reinterpret_cast<float*>(tiles);
-                if (!ROWS && local) asm volatile("bar.sync 1, 128;" ::: "memory");  // the previous tile's fold has read the staging tile
+                float* part_smem = local ? stage_small : reinterpret_cast<float*>(tiles);
+                if (local) asm volatile("bar.sync 1, 128;" ::: "memory");  // the previous tile's fold has read the staging tile
                 const bool to_smem = cl || local || solo;
                 if (BN >= 32 && to_smem) {
                     // 32 columns per round trip to tensor memory
@@ -1159,41 +1069,22 @@ static int packed_paired(const PackedArgs& a) {
     return a.epilogue == LIN_SILU_MUL || a.epilogue == LIN_CLAMPED_GLU || a.epilogue == LIN_GELU_GLU ? 1 : 0;
 }
 
-// Which kernel takes a call of T tokens over a depth of K.  Measured (us, streaming / tiled): T = 256: 28 / 17 at 4096 x 4096, 43 / 37 at
-// 4096 x 11008, 41 / 9 at 2048 x 2048 (f32 out).  T = 100: 24 / 9 at 2048 x 2048 and 12 / 7 at 4096 x 576, but 16 / 17 at 4096 x 4096
-// and 26 / 36 at 4096 x 11008: up to 128 tokens a deep matrix gains more from the streaming kernel's split along K.
+// Which kernel takes a call of 17 tokens or more over a depth of K.  The tiled kernel gains from its whole tiles of 256 tokens, the one for a
+// few dozen tokens from its split along K: T = 100, us: 2048 x 2048 9 tiled; 4096 x 11008 36 tiled, 26 split; 2048 x 5504 15 split.
 static bool use_tiled(int T, int K) { return T > 128 || (T > 64 && K < 4096); }
 
-// Any number of tokens, in one launch of the tiled kernel (linear_tiled.cu) or launches of at most 256 tokens.
+// Any number of tokens: the streaming kernel below up to 16 (and for exchanges), linear_mid.cu, linear_tiled.cu.
 jsm_status linear_packed_tokens(const PackedArgs& a, cudaStream_t st) {
     if (a.T <= 0 || a.N <= 0) return JSM_OK;
-    if (!a.tp && a.T > 16) {
-        jsm_status s = packed_check(a, std::min(a.T, 256), packed_paired(a));
-        return s != JSM_OK ? s : use_tiled(a.T, a.K) ? linear_tiled_launch(a, st) : linear_mid_launch(a, st);
-    }
-    PackedArgs c = a;
-    const long long xs = a.x_row_stride > 0 ? a.x_row_stride : a.K;
-    if (a.ssq_stride <= 0) c.ssq_stride = a.T;
-    for (int t0 = 0; t0 < a.T; t0 += 256) {
-        c.T = std::min(256, a.T - t0);
-        c.X = static_cast<const __nv_bfloat16*>(a.X) + t0 * xs;
-        c.R = a.R ? static_cast<const __nv_bfloat16*>(a.R) + (size_t)t0 * a.N : nullptr;
-        if (a.Y)
-            c.Y = a.out_f32 ? static_cast<void*>(static_cast<float*>(a.Y) + (size_t)t0 * a.N)
-                            : static_cast<void*>(static_cast<__nv_bfloat16*>(a.Y) + (size_t)t0 * a.N);
-        c.ssq_in = a.ssq_in ? a.ssq_in + t0 : nullptr;
-        c.ssq_out = a.ssq_out ? a.ssq_out + t0 : nullptr;
-        jsm_status s = linear_packed_launch(c, st);
-        if (s != JSM_OK) return s;
-    }
-    return JSM_OK;
+    if ((a.tp && (a.tp->push || a.tp->reduce)) || a.T <= 16) return linear_packed_launch(a, st);
+    jsm_status s = packed_check(a, std::min(a.T, 256), packed_paired(a));
+    return s != JSM_OK ? s : use_tiled(a.T, a.K) ? linear_tiled_launch(a, st) : linear_mid_launch(a, st);
 }
 
 jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st) {
     if (a.T <= 0 || a.N <= 0) return JSM_OK;
     const bool tp_push = a.tp && a.tp->push, tp_reduce = a.tp && a.tp->reduce;
-    if (a.T > 256) JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: at most 256 tokens per launch (%d)", a.T);
-    const bool glu = a.epilogue == LIN_CLAMPED_GLU || a.epilogue == LIN_GELU_GLU;
+    if (a.T > (tp_push || tp_reduce ? TP_PUSH_MAX_T : 16)) JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: the fused exchange takes at most %d tokens (%d)", TP_PUSH_MAX_T, a.T);
     const int paired = packed_paired(a);
     jsm_status s = packed_check(a, a.T, paired);
     if (s != JSM_OK) return s;
@@ -1210,7 +1101,7 @@ jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st) {
     P.err = tc_error_word();
     P.ssq_in = a.ssq_in; P.ssq_in_tiles = a.ssq_in_tiles; P.ssq_stride = a.ssq_stride > 0 ? a.ssq_stride : a.T;
     P.inv_d = 1.0f / (float)a.K; P.eps = a.eps; P.ssq_out = a.ssq_out;
-    const int bn = a.T <= 16 ? 16 : a.T <= 32 ? 32 : a.T <= 64 ? 64 : a.T <= 128 ? 128 : 256;
+    const int bn = a.T <= 16 ? 16 : a.T <= 32 ? 32 : 64;
     CUtensorMap mx;
     s = make_tmap_bf16_2d(&mx, a.X, (uint64_t)a.T, (uint64_t)a.K, (uint64_t)(a.x_row_stride > 0 ? a.x_row_stride : a.K), bn, 64);
     if (s != JSM_OK) return s;
@@ -1258,73 +1149,27 @@ jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st) {
             P.tp_mode = 2;
         }
     }
-    // A launch pays for the size of the image it runs.  The common launches of a decoder step (up to 64 tokens) have
-    // lean images of their own, chosen below; what remains runs the general images: with the cluster path from 32 tokens
-    // on (cluster size 1 where no cluster forms), with the exchange code when the launch pushes or reduces.
-    const bool with_cl = cluster > 1 || a.T >= 32;
-    const bool with_tp = P.tp_mode != 0;  // (at most 64 tokens: checked above)
-#define PK_GO(BN_)                                                                                  \
-    return with_cl ? launch_packed<BN_, true, 0>(mx, mx2, P, grid, cluster, a.chained, st)     \
-                   : launch_packed<BN_, false, 0>(mx, mx2, P, grid, cluster, a.chained, st)
-#define PK_GO_TP(BN_)                                                                                        \
-    if (with_tp)                                                                                             \
-        return with_cl ? launch_packed<BN_, true, 3>(mx, mx2, P, grid, cluster, a.chained, st)           \
-                       : launch_packed<BN_, false, 3>(mx, mx2, P, grid, cluster, a.chained, st);        \
-    PK_GO(BN_)
-    if (glu) {
-#define PK_GLU(PRM_)                                                                                                  \
-    switch (bn) {                                                                                                      \
-        case 16: return launch_packed<16, false, 0, PRM_>(mx, mx2, P, grid, cluster, a.chained, st);                   \
-        case 32: return cluster > 1 ? launch_packed<32, true, 0, PRM_>(mx, mx2, P, grid, cluster, a.chained, st)       \
-                                    : launch_packed<32, false, 0, PRM_>(mx, mx2, P, grid, cluster, a.chained, st);     \
-        case 64: return cluster > 1 ? launch_packed<64, true, 0, PRM_>(mx, mx2, P, grid, cluster, a.chained, st)       \
-                                    : launch_packed<64, false, 0, PRM_>(mx, mx2, P, grid, cluster, a.chained, st);     \
-        case 128: return launch_packed<128, true, 0, PRM_>(mx, mx2, P, grid, cluster, a.chained, st);                  \
-        default: return launch_packed<256, true, 0, PRM_>(mx, mx2, P, grid, cluster, a.chained, st);                   \
-    }
-        if (a.epilogue == LIN_GELU_GLU) PK_GLU(9) else PK_GLU(6)
-#undef PK_GLU
-    }
-    // plain projections of up to 64 tokens with nothing fused
-    if (bn <= 64 && !with_tp && !paired && !a.bias && a.epilogue == LIN_NONE && !a.ssq_in && !a.ssq_out) {
-#define PK_PLAIN(BN_, CL_)                                                                             \
-    return a.out_f32 ? launch_packed<BN_, CL_, 0, 7>(mx, mx2, P, grid, cluster, a.chained, st)         \
-                     : launch_packed<BN_, CL_, 0, 8>(mx, mx2, P, grid, cluster, a.chained, st)
-        if (bn == 16) { if (!with_cl) PK_PLAIN(16, false); }
-        else if (bn == 32) { if (cluster > 1) PK_PLAIN(32, true); else PK_PLAIN(32, false); }
-        else { if (cluster > 1) PK_PLAIN(64, true); else PK_PLAIN(64, false); }
-#undef PK_PLAIN
-    }
-    // the few-token launches without an exchange (the decode step of one GPU): an image per kind of tile
-    if (bn == 16 && !with_cl && !with_tp) {
-        const bool lean = !a.bias && !a.out_f32;  // the projections of a LLaMA-style decoder step have images of their own
-        if (lean && paired && a.ssq_in) return launch_packed<16, false, 0, 4>(mx, mx2, P, grid, cluster, a.chained, st);
-        if (lean && !paired && a.epilogue == LIN_NONE && a.ssq_in && !a.ssq_out)
-            return launch_packed<16, false, 0, 2>(mx, mx2, P, grid, cluster, a.chained, st);
-        if (lean && !paired && a.epilogue == LIN_RESIDUAL && !a.ssq_in && a.ssq_out)
-            return launch_packed<16, false, 0, 3>(mx, mx2, P, grid, cluster, a.chained, st);
-        return paired ? launch_packed<16, false, 0, 1>(mx, mx2, P, grid, cluster, a.chained, st)
-                      : launch_packed<16, false, 0, 0>(mx, mx2, P, grid, cluster, a.chained, st);
-    }
-    // 17 to 64 tokens without an exchange: the same three images per token block, with and without the cluster path
-    if ((bn == 32 || bn == 64) && !with_tp && !a.bias && !a.out_f32) {
-#define PK_LEAN(BN_, CL_)                                                                                                    \
-    do {                                                                                                                     \
-        if (paired && a.ssq_in) return launch_packed<BN_, CL_, 0, 4>(mx, mx2, P, grid, cluster, a.chained, st);              \
-        if (!paired && a.epilogue == LIN_NONE && a.ssq_in && !a.ssq_out)                                                     \
-            return launch_packed<BN_, CL_, 0, 2>(mx, mx2, P, grid, cluster, a.chained, st);                                  \
-        if (!paired && a.epilogue == LIN_RESIDUAL && !a.ssq_in && a.ssq_out)                                                 \
-            return launch_packed<BN_, CL_, 0, 3>(mx, mx2, P, grid, cluster, a.chained, st);                                  \
-    } while (0)
-        if (bn == 32) {
-            if (cluster > 1) PK_LEAN(32, true); else PK_LEAN(32, false);
-        } else {
-            if (cluster > 1) PK_LEAN(64, true); else PK_LEAN(64, false);
+    // A launch pays for the size of the image it runs.  The common launches of a decoder step have lean images of their own, chosen
+    // below; what remains runs the general images.
+    if (P.tp_mode == 0) {  // up to 16 tokens, no cluster: an image per kind of tile
+#define PK_IMAGE(PRM_) return launch_packed<16, false, 0, PRM_>(mx, mx2, P, grid, cluster, a.chained, st)
+        if (a.epilogue == LIN_GELU_GLU) PK_IMAGE(9);
+        if (a.epilogue == LIN_CLAMPED_GLU) PK_IMAGE(6);
+        if (!paired && !a.bias && a.epilogue == LIN_NONE && !a.ssq_in && !a.ssq_out) {  // plain projections with nothing fused
+            if (a.out_f32) PK_IMAGE(7);
+            PK_IMAGE(8);
         }
-#undef PK_LEAN
+        const bool lean = !a.bias && !a.out_f32;  // the projections of a LLaMA-style decoder step
+        if (lean && paired && a.ssq_in) PK_IMAGE(4);
+        if (lean && !paired && a.epilogue == LIN_NONE && a.ssq_in && !a.ssq_out) PK_IMAGE(2);
+        if (lean && !paired && a.epilogue == LIN_RESIDUAL && !a.ssq_in && a.ssq_out) PK_IMAGE(3);
+        if (paired) PK_IMAGE(1);
+        PK_IMAGE(0);
+#undef PK_IMAGE
     }
+    const bool with_cl = cluster > 1 || a.T >= 32;
     // 17 to 64 tokens of a tensor-parallel rank (flags): the pushing projection and the two reducing ones
-    if ((bn == 32 || bn == 64) && with_tp && !P.tp_inband && !a.bias && !a.out_f32) {
+    if (bn > 16 && !P.tp_inband && !a.bias && !a.out_f32) {
 #define PK_LEAN_TP(BN_, CL_)                                                                                                 \
     do {                                                                                                                     \
         if (P.tp_mode == 1 && !a.ssq_in) return launch_packed<BN_, CL_, 1, 5>(mx, mx2, P, grid, cluster, a.chained, st);     \
@@ -1339,19 +1184,17 @@ jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st) {
         }
 #undef PK_LEAN_TP
     }
-    if (bn == 16 && !with_cl && with_tp && P.tp_inband && !a.bias && !a.out_f32) {  // the decode step of a tensor-parallel rank
+    if (bn == 16 && !with_cl && P.tp_inband && !a.bias && !a.out_f32) {  // the decode step of a tensor-parallel rank
         if (P.tp_mode == 1 && !a.ssq_in) return launch_packed<16, false, 4, 5>(mx, mx2, P, grid, cluster, a.chained, st);  // (plain, nothing else: checked above)
         if (P.tp_mode == 2 && paired) return launch_packed<16, false, 5, 4>(mx, mx2, P, grid, cluster, a.chained, st);
         if (P.tp_mode == 2 && a.epilogue == LIN_NONE && !a.ssq_out) return launch_packed<16, false, 5, 2>(mx, mx2, P, grid, cluster, a.chained, st);
     }
-    switch (bn) {
-        case 16: PK_GO_TP(16);
-        case 32: PK_GO_TP(32);
-        case 64: PK_GO_TP(64);
-        case 128: PK_GO(128);
-        default: PK_GO(256);
-    }
-#undef PK_GO_TP
+#define PK_GO(BN_)                                                                                  \
+    return with_cl ? launch_packed<BN_, true, 3>(mx, mx2, P, grid, cluster, a.chained, st)         \
+                   : launch_packed<BN_, false, 3>(mx, mx2, P, grid, cluster, a.chained, st)
+    if (bn == 16) return launch_packed<16, false, 3>(mx, mx2, P, grid, cluster, a.chained, st);
+    if (bn == 32) PK_GO(32);
+    PK_GO(64);
 #undef PK_GO
 }
 
@@ -1409,7 +1252,7 @@ extern "C" size_t jsm_linear_packed_bytes(int N, int K, int paired) {
     return linear_packed_bytes(N, K, paired ? 1 : 0);
 }
 
-// Grows the workspace of the current device so that any launch of this shape (up to 256 tokens per launch) finds room.
+// Grows the workspace of the current device so that any launch of this shape (as the kernels were split up to 256 tokens: what a call needs does not depend on the kernel it takes) finds room.
 // Set-up time only: synchronises the device when it has to reallocate.
 extern "C" jsm_status jsm_linear_packed_reserve(int N, int K, int paired) {
     if (N <= 0 || K <= 0) JSM_FAIL(JSM_INVALID_ARG, "jsm_linear_packed_reserve: N %d, K %d", N, K);
