@@ -145,17 +145,39 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
     const int n_max = max(n_tiles[0], n_tiles[1]);
     const int j_lo = n_tiles[1] > 0 ? min(lo[0], lo[1]) : lo[0];
 
-    if (threadIdx.x == 0) {
+    // paged: 64 columns of a key tile are a slab of two pages (a tile's second half behind the last page repeats it: masked)
+    auto slab = [&](uint8_t* dst, int j, int c, uint64_t* bar) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const long long page = P.pages[min(2 * j + half, P.n_pages - 1)];
+            bulk_load(dst + half * (FA_SLAB / 2), P.pool + ((page * P.Hkv + hk) * ((QKD + VD) / 64) + c) * (FA_SLAB / 4), FA_SLAB / 2, bar);
+        }
+    };
+    auto load_k = [&](int j, int ks) {
+        mbar_expect_tx(&k_full[ks], QK_BYTES);
+#pragma unroll
+        for (int c = 0; c < QKD / 64; ++c)
+            if (PAGED) slab(k_smem + ks * QK_BYTES + c * FA_SLAB, j, c, &k_full[ks]);
+            else tma_load_2d(k_smem + ks * QK_BYTES + c * FA_SLAB, &tmap_k, hk * QKD + c * 64, b * P.Tk + j * FA_BN, &k_full[ks]);
+    };
+    // the elected lane that makes the barriers asks for Q and the first keys at once, before the block meets
+    if (warp == 0 && elect_one()) {
         abort_flag = 0;
         mbar_init(&q_full, 1);
         mbar_init(&o_done, 1);
         for (int s = 0; s < KST; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
         for (int s = 0; s < VST; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
-        for (int t = 0; t < 2; ++t) { mbar_init(&s_full[t], 1); mbar_init(&p_ready[t], 128); }
+        for (int t = 0; t < 2; ++t) { mbar_init(&s_full[t], 1); mbar_init(&p_ready[t], 4); }  // (a warp each)
         mbar_fence_init();
-        tma_prefetch_desc(&tmap_q);
-        if (!PAGED) { tma_prefetch_desc(&tmap_k); tma_prefetch_desc(&tmap_v); }
+        mbar_expect_tx(&q_full, 2 * QK_BYTES);  // both tiles, in slabs of 64 columns
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int c = 0; c < QKD / 64; ++c)
+                tma_load_2d(q_smem + t * QK_BYTES + c * FA_SLAB, &tmap_q, h * P.q_hs + c * 64, b * P.Tq + q0 + t * FA_BM, &q_full);
+        if (j_lo < n_max) load_k(j_lo, 0);
     }
+    __syncwarp();
     if (warp == 1) {
         tmem_alloc(&tmem_base_smem, 512);
         tmem_relinquish();
@@ -169,35 +191,11 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
     // (warps 0 and 1 run converged, one elected lane issues: see elect_one)
     if (warp == 0) {
         {
-            // Q: both tiles, in slabs of 64 columns
-            if (elect_one()) {
-                mbar_expect_tx(&q_full, 2 * QK_BYTES);
-#pragma unroll
-                for (int t = 0; t < 2; ++t)
-#pragma unroll
-                    for (int c = 0; c < QKD / 64; ++c)
-                        tma_load_2d(q_smem + t * QK_BYTES + c * FA_SLAB, &tmap_q, h * P.q_hs + c * 64, b * P.Tq + q0 + t * FA_BM, &q_full);
-            }
-            __syncwarp();
-            int k_issued = 0, v_issued = 0;
-            // paged: 64 columns of a key tile are a slab of two pages (a tile's second half behind the last page repeats it: masked)
-            auto slab = [&](uint8_t* dst, int j, int c, uint64_t* bar) {
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const long long page = P.pages[min(2 * j + half, P.n_pages - 1)];
-                    bulk_load(dst + half * (FA_SLAB / 2), P.pool + ((page * P.Hkv + hk) * ((QKD + VD) / 64) + c) * (FA_SLAB / 4), FA_SLAB / 2, bar);
-                }
-            };
+            int k_issued = j_lo < n_max ? 1 : 0, v_issued = 0;
             for (int j = j_lo; j < n_max; ++j) {
                 const int i = j - j_lo, ks = i % KST, vs = i % VST;
                 if (i >= KST && !mbar_wait_warp(&k_empty[ks], ((i / KST) & 1) ^ 1, &abort_flag, P.err, TC_TIMEOUT_EMPTY)) break;
-                if (elect_one()) {
-                    mbar_expect_tx(&k_full[ks], QK_BYTES);
-#pragma unroll
-                    for (int c = 0; c < QKD / 64; ++c)
-                        if (PAGED) slab(k_smem + ks * QK_BYTES + c * FA_SLAB, j, c, &k_full[ks]);
-                        else tma_load_2d(k_smem + ks * QK_BYTES + c * FA_SLAB, &tmap_k, hk * QKD + c * 64, b * P.Tk + j * FA_BN, &k_full[ks]);
-                }
+                if (i > 0 && elect_one()) load_k(j, ks);
                 __syncwarp();
                 k_issued = i + 1;
                 if (i >= VST && !mbar_wait_warp(&v_empty[vs], ((i / VST) & 1) ^ 1, &abort_flag, P.err, TC_TIMEOUT_EMPTY)) break;
@@ -401,7 +399,8 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
             l += lsum;
             tmem_st_wait();
             tc_fence_before();
-            mbar_arrive(&p_ready[t]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&p_ready[t]);
         }
         // epilogue: O / l -> bf16 -> global
         if (ok && j_end > j_begin) ok = mbar_wait(&o_done, 0, &abort_flag, P.err, TC_TIMEOUT_ACC);
@@ -413,12 +412,16 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
             __nv_bfloat16* dst = P.out + (long long)(b * P.Tq + (store ? qi : 0)) * P.out_rs + (long long)h * (WIN ? P.v_dim : VD);
             const int v_dim = WIN ? P.v_dim : VD;
             const bool vec = v_dim % 8 == 0;
+            // A thread has a row, so its stores would touch 32 lines at a time (2.6 us at the end of every CTA): the warp's 32 rows pass
+            // through the queries' place - every product has been taken - and leave whole, 16 bytes per lane (1.5 us).
+            uint8_t* rows = q_smem + t * QK_BYTES + quad * (32 * VD * 2);
+            constexpr bool STAGED = VD <= QKD;  // four warps' rows fit the queries' tile; wider values leave straight from the registers
 #pragma unroll
             for (int c = 0; c < VD; c += 32) {
                 uint32_t r[32];
                 tmem_ld32(o_addr + c, r);
                 tmem_ld_wait();
-                if (store && vec) {
+                if (vec && (STAGED || store)) {
 #pragma unroll
                     for (int i = 0; i < 32; i += 8) {
                         uint4 o;
@@ -426,13 +429,24 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
                         o.y = pack_bf16x2(__uint_as_float(r[i + 2]) * inv, __uint_as_float(r[i + 3]) * inv);
                         o.z = pack_bf16x2(__uint_as_float(r[i + 4]) * inv, __uint_as_float(r[i + 5]) * inv);
                         o.w = pack_bf16x2(__uint_as_float(r[i + 6]) * inv, __uint_as_float(r[i + 7]) * inv);
-                        if (c + i < v_dim) *reinterpret_cast<uint4*>(dst + c + i) = o;
+                        if constexpr (STAGED) *reinterpret_cast<uint4*>(rows + lane * (VD * 2) + ((((c + i) / 8) ^ (lane & 7)) * 16)) = o;
+                        else if (c + i < v_dim) *reinterpret_cast<uint4*>(dst + c + i) = o;
                     }
                 } else if (store) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i)
                         if (c + i < v_dim) dst[c + i] = __float2bfloat16_rn(__uint_as_float(r[i]) * inv);
                 }
+            }
+            if (STAGED && vec) {
+                __syncwarp();
+                constexpr int PIECES = VD / 8, STEP = 32 / PIECES;  // 16-byte pieces of a row, rows per pass
+                const int piece = lane % PIECES, row0 = q0 + t * FA_BM + quad * 32;
+                __nv_bfloat16* base = P.out + (long long)b * P.Tq * P.out_rs + (long long)h * v_dim + piece * 8;
+#pragma unroll 4
+                for (int r = lane / PIECES; r < 32; r += STEP)
+                    if (row0 + r < P.Tq && piece * 8 < v_dim)
+                        *reinterpret_cast<uint4*>(base + (long long)(row0 + r) * P.out_rs) = *reinterpret_cast<const uint4*>(rows + r * (VD * 2) + ((piece ^ (r & 7)) * 16));
             }
         }
     }
