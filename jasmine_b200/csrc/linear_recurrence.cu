@@ -76,11 +76,20 @@ __global__ void __launch_bounds__(RS_THREADS) rec_scan_kernel(RecArgs a, RecDims
                 q[x][e] = on ? to_f32(row[g * kp + i]) : 0.0f;
                 k[x][e] = on ? to_f32(row[(d.G + g) * kp + i]) : 0.0f;
             }
-            if (t < n && lane < RS_COLS) vs[buf][t][lane] = c0 + lane < vp ? to_f32(row[2 * d.G * kp + h * vp + c0 + lane]) : 0.0f;
-            if (DELTA && t < n && lane == 31) {
-                const float* ba = a.ba + (long long)(start + t0 + t) * d.ba_cols();
-                bs[buf][t] = rec_sigmoid(ba[h]);
-                gs[buf][t] = expf(a.A[h] * rec_softplus(ba[d.ba_cols() / 2 + h] + a.dt_bias[h]));
+            if (lane < RS_COLS) vs[buf][t][lane] = t < n && c0 + lane < vp ? to_f32(row[2 * d.G * kp + h * vp + c0 + lane]) : 0.0f;
+            if (lane == 31) {  // (behind the last token: nothing is added and nothing decays)
+                float beta = 0.0f, decay = 1.0f;
+                if (t < n) {
+                    if (DELTA) {
+                        const float* ba = a.ba + (long long)(start + t0 + t) * d.ba_cols();
+                        beta = rec_sigmoid(ba[h]);
+                        decay = expf(a.A[h] * rec_softplus(ba[d.ba_cols() / 2 + h] + a.dt_bias[h]));
+                    } else {
+                        decay = a.decay[h];
+                    }
+                }
+                bs[buf][t] = beta;
+                gs[buf][t] = decay;
             }
         }
 #pragma unroll
@@ -99,7 +108,7 @@ __global__ void __launch_bounds__(RS_THREADS) rec_scan_kernel(RecArgs a, RecDims
 #pragma unroll
             for (int e = 0; e < PER_LANE; ++e) {
                 const int i = lane + 32 * e;
-                if (t < n && i < KW) {
+                if (i < KW) {
                     qs[buf][t][i] = DELTA ? q[x][e] / sq * a.q_scale : q[x][e];
                     ks[buf][t][i] = DELTA ? k[x][e] / sk : k[x][e];
                 }
@@ -122,7 +131,6 @@ __global__ void __launch_bounds__(RS_THREADS) rec_scan_kernel(RecArgs a, RecDims
     float S[NR];
 #pragma unroll
     for (int i = 0; i < NR; ++i) S[i] = live && row_of(i) < kp && !fresh ? state[(long long)row_of(i) * vp] : 0.0f;
-    const float decay = DELTA ? 0.0f : a.decay[h];
     auto rows = [&](const float* p, float (&x)[NR]) {  // this thread's rows of a staged vector
 #pragma unroll
         for (int i = 0; i < NR; i += V) {
@@ -142,12 +150,11 @@ __global__ void __launch_bounds__(RS_THREADS) rec_scan_kernel(RecArgs a, RecDims
             float o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
-                const int t = t4 + x;
-                if (t >= n) break;
+                const int t = t4 + x;  // (no branch on the last token: the next tokens' loads move ahead of the chain)
                 float k[NR], q[NR];
                 rows(ks[buf][t], k);
                 rows(qs[buf][t], q);
-                const float gt = DELTA ? gs[buf][t] : decay;
+                const float gt = gs[buf][t];
                 float u = vs[buf][t][col];
                 if (DELTA) {
                     float p[2] = {0.0f, 0.0f};

@@ -200,10 +200,10 @@ __global__ void __launch_bounds__(128) attn_paged_simt_kernel(const T* __restric
 // The same for portions of prompts: a warp per (token, head of the group) row, eight rows of one kv head per CTA, which share
 // tiles of 32 keys and values in shared memory - the kernel above reads every key once per token and head and waits for it, 32
 // lanes a key.  Here a lane owns a key of the tile (vector loads, an odd number of 16-byte pieces per row: no bank conflicts)
-// and then columns lane, lane + 32, ... of the output.
+// and then columns lane, lane + 32, ... of the output.  The next tile is on its way while one is used.
 constexpr int AR_ROWS = 8, AR_KEYS = 32, AR_MAX_SMEM = 160 * 1024;
 __host__ __device__ constexpr int ar_pitch(int n) { return ((n + 3) / 4 | 1) * 4; }
-static size_t ar_smem(const AttnDims& d) { return sizeof(float) * ((size_t)(AR_KEYS + AR_ROWS) * ar_pitch(d.dim) + AR_KEYS * ar_pitch(d.vdim)); }
+static size_t ar_smem(const AttnDims& d) { return sizeof(float) * ((size_t)(2 * AR_KEYS + AR_ROWS) * ar_pitch(d.dim) + 2 * AR_KEYS * ar_pitch(d.vdim)); }
 
 template <typename T, int VR>  // VR: output columns per lane
 __global__ void __launch_bounds__(AR_ROWS * 32) attn_paged_rows_kernel(const T* __restrict__ q, AttnDims d, const float* __restrict__ sink, const T* __restrict__ pool,
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(AR_ROWS * 32) attn_paged_rows_kernel(const T* 
                                                                        const float* __restrict__ gate, T* __restrict__ out) {
     extern __shared__ __align__(16) float ar_sm[];
     const int kpitch = ar_pitch(d.dim), vpitch = ar_pitch(d.vdim), dim4 = (d.dim + 3) / 4, vdim4 = (d.vdim + 3) / 4;
-    float *Ks = ar_sm, *Vs = Ks + AR_KEYS * kpitch, *Qs = Vs + AR_KEYS * vpitch;
+    float *K2 = ar_sm, *V2 = K2 + 2 * AR_KEYS * kpitch, *Qs = V2 + 2 * AR_KEYS * vpitch;  // two tiles of keys and values
     chain_trigger();
     chain_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = blockIdx.y, gs = d.H / d.G;
@@ -228,25 +228,29 @@ __global__ void __launch_bounds__(AR_ROWS * 32) attn_paged_rows_kernel(const T* 
     float m = sink ? sink[h] : -INFINITY, l = sink ? 1.0f : 0.0f, o[VR];
 #pragma unroll
     for (int i = 0; i < VR; ++i) o[i] = 0.0f;
-    for (int c0 = lo; c0 <= hi; c0 += AR_KEYS) {
-        __syncthreads();
+    auto stage = [&](int c0, int buf) {
         for (int e = threadIdx.x; e < AR_KEYS * (dim4 + vdim4); e += AR_ROWS * 32) {
             const int j = e / (dim4 + vdim4), x = e % (dim4 + vdim4), key = c0 + j;
-            const bool value = x >= dim4;
+            const bool value = x >= dim4, on = key <= hi;
             const int c = (value ? x - dim4 : x) * 4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (key <= hi) {
-                const T* src = cache_at(const_cast<T*>(pool), d, bt[key / PAGE], g, value ? 1 : 0, key % PAGE, c);
-                if constexpr (sizeof(T) == 4) {
-                    v = *reinterpret_cast<const float4*>(src);
-                } else {
-                    const uint2 w = *reinterpret_cast<const uint2*>(src);
-                    v = make_float4(bf16lo(w.x), bf16hi(w.x), bf16lo(w.y), bf16hi(w.y));
-                }
+            const T* src = on ? cache_at(const_cast<T*>(pool), d, bt[key / PAGE], g, value ? 1 : 0, key % PAGE, c) : pool;
+            float* dst = (value ? V2 + (buf * AR_KEYS + j) * vpitch : K2 + (buf * AR_KEYS + j) * kpitch) + c;
+            if constexpr (sizeof(T) == 4) {
+                cp_async16(smem_u32(dst), src, on);
+            } else {
+                const uint2 w = on ? *reinterpret_cast<const uint2*>(src) : make_uint2(0u, 0u);
+                *reinterpret_cast<float4*>(dst) = make_float4(bf16lo(w.x), bf16hi(w.x), bf16lo(w.y), bf16hi(w.y));
             }
-            *reinterpret_cast<float4*>((value ? Vs + j * vpitch : Ks + j * kpitch) + c) = v;
         }
+    };
+    stage(lo, 0);
+    cp_async_commit();
+    for (int c0 = lo, buf = 0; c0 <= hi; c0 += AR_KEYS, buf ^= 1) {
+        if (c0 + AR_KEYS <= hi) stage(c0 + AR_KEYS, buf ^ 1);
+        cp_async_commit();
+        cp_async_wait<1>();
         __syncthreads();
+        const float *Ks = K2 + buf * AR_KEYS * kpitch, *Vs = V2 + buf * AR_KEYS * vpitch;
         float a0 = 0.0f, a1 = 0.0f;
         for (int i = 0; i < dim4; ++i) {
             const float4 x = *reinterpret_cast<const float4*>(qrow + 4 * i), y = *reinterpret_cast<const float4*>(Ks + lane * kpitch + 4 * i);
@@ -256,20 +260,22 @@ __global__ void __launch_bounds__(AR_ROWS * 32) attn_paged_rows_kernel(const T* 
         const int key = c0 + lane;
         const float s = key >= first && key <= pos ? (a0 + a1) * d.scale : -INFINITY;
         const float m_new = fmaxf(m, warp_max(s));
-        if (m_new == -INFINITY) continue;  // (no key of this row yet: the whole warp agrees)
-        const float p = expf(s - m_new), alpha = expf(m - m_new);
-        l = l * alpha + warp_sum(p);
-        m = m_new;
+        if (!(m_new == -INFINITY)) {  // (else no key of this row yet: the whole warp agrees)
+            const float p = expf(s - m_new), alpha = expf(m - m_new);
+            l = l * alpha + warp_sum(p);
+            m = m_new;
 #pragma unroll
-        for (int i = 0; i < VR; ++i) o[i] *= alpha;
-        const int j_end = min(AR_KEYS, pos + 1 - c0);  // (a value that the row does not see may be anything)
+            for (int i = 0; i < VR; ++i) o[i] *= alpha;
+            const int j_end = min(AR_KEYS, pos + 1 - c0);  // (a value that the row does not see may be anything)
 #pragma unroll 4
-        for (int j = max(0, first - c0); j < j_end; ++j) {
-            const float pj = __shfl_sync(0xffffffffu, p, j);
+            for (int j = max(0, first - c0); j < j_end; ++j) {
+                const float pj = __shfl_sync(0xffffffffu, p, j);
 #pragma unroll
-            for (int i = 0; i < VR; ++i)
-                if (lane + 32 * i < d.vdim) o[i] = fmaf(pj, Vs[j * vpitch + lane + 32 * i], o[i]);
+                for (int i = 0; i < VR; ++i)
+                    if (lane + 32 * i < d.vdim) o[i] = fmaf(pj, Vs[j * vpitch + lane + 32 * i], o[i]);
+            }
         }
+        __syncthreads();  // the tile is used up
     }
     if (warp >= n_rows) return;
     const float f = (gate ? gate[t * d.H + h] : 1.0f) / l;
