@@ -1,4 +1,4 @@
-// bf16 projections of a few dozen tokens (17 to 128) over packed weights (the layout of linear_packed.cu): Y[t, n] = sum_k X[t, k] W[n, k],
+// bf16 projections of a few dozen tokens (17 to 128; fewer where a matrix has few tiles) over packed weights (the layout of linear_packed.cu): Y[t, n] = sum_k X[t, k] W[n, k],
 // the batched decode step's and short prompt's form of weight_net_t::forward (mat_net_t.hpp:38-49).
 //
 // What bounds it.  The weights are read once, so the floor is the memory's; but a launch moves only 8 to 50 MB (1.3 to 8 us), and
@@ -91,13 +91,14 @@ __device__ __forceinline__ bool lm_wait_cluster(uint64_t* bar, uint32_t parity, 
 }
 
 // KIND: 0 plain (optionally a fused norm's row factor, row statistics), 1 the same with bias and activations, 2 gate/up pairs, 3 with a residual
-constexpr int lm_stages(int bn) { return bn == 32 ? 4 : bn == 64 ? 3 : 2; }
+constexpr int lm_stages(int bn) { return bn <= 32 ? 4 : bn == 64 ? 3 : 2; }
 constexpr int lm_smem(int bn) { return lm_stages(bn) * 2 * ((int)LM_UNIT + bn * 128) + (bn + 64) * 512 + 1024; }
 
 template <int BN, int KIND>
 __global__ void __launch_bounds__(LM_THREADS, 1) linear_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, LmParams P) {
     constexpr int STAGES = lm_stages(BN);
     constexpr uint32_t X_BYTES = BN * 128, X_OFF = 2 * LM_UNIT, STAGE = 2 * (LM_UNIT + X_BYTES);
+    constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
     constexpr bool PAIRED = KIND == 2;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) linear_mid_kernel(const __grid_
         tma_prefetch_desc(&tmap_x);
     }
     if (warp == 1) {
-        tmem_alloc(&tmem_base_smem, BN);
+        tmem_alloc(&tmem_base_smem, TMEM_COLS);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -335,7 +336,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) linear_mid_kernel(const __grid_
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem, BN);
+        tmem_dealloc(tmem, TMEM_COLS);
     }
     lm_cluster_wait();  // no CTA leaves while a peer may still write into it
 }
@@ -432,6 +433,7 @@ jsm_status linear_mid_launch(const PackedArgs& a, cudaStream_t st) {
 #define LM_GO(BN_) \
     return kind == 3 ? launch_mid<BN_, 3>(a, P, n_tiles, st) : kind == 2 ? launch_mid<BN_, 2>(a, P, n_tiles, st) \
          : kind == 1 ? launch_mid<BN_, 1>(a, P, n_tiles, st) : launch_mid<BN_, 0>(a, P, n_tiles, st)
+    if (a.T <= 16) LM_GO(16);
     if (a.T <= 32) LM_GO(32);
     if (a.T <= 64) LM_GO(64);
     LM_GO(128);

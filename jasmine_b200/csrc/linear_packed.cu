@@ -1073,10 +1073,22 @@ static int packed_paired(const PackedArgs& a) {
 // few dozen tokens from its split along K: T = 100, us: 2048 x 2048 9 tiled; 4096 x 11008 36 tiled, 26 split; 2048 x 5504 15 split.
 static bool use_tiled(int T, int K) { return T > 128 || (T > 64 && K < 4096); }
 
+// Up to 16 tokens, matrices of so few tiles that four CTAs or more share each: linear_mid.cu's clusters fold with one trip, the streaming
+// kernel's CTAs through the workspace.  Back to back, streaming / clusters, us at 8 and at 16 tokens: 160 x 4096 5.6 / 3.8 and 7.1 / 3.9,
+// 1024 x 2752 5.3 / 4.4 and 6.7 / 4.5, 2048 x 2048 5.1 / 4.9 and 6.8 / 4.9, 2048 x 5504 7.4 / 7.5 and 9.2 / 7.6, 3648 x 2048 6.2 / 5.5 and
+// 7.6 / 5.5, 4096 x 4096 9.0 / 8.4 and 9.3 / 8.5, 4096 x 11008 18.3 / 17.3 and 19.1 / 17.4.  Wider matrices: the even split of the stream
+// keeps all SMs at work (8192 x 2048 9.0 / 9.1, gate/up 11008 x 4096 31.7 / 41.0).
+static bool few_tiles(const PackedArgs& a) {
+    int nt, kbt;
+    pk_dims(a.N, a.K, packed_paired(a), &nt, &kbt);
+    return nt * 4 <= sm_count();
+}
+
 // Any number of tokens: the streaming kernel below up to 16 (and for exchanges), linear_mid.cu, linear_tiled.cu.
 jsm_status linear_packed_tokens(const PackedArgs& a, cudaStream_t st) {
     if (a.T <= 0 || a.N <= 0) return JSM_OK;
-    if ((a.tp && (a.tp->push || a.tp->reduce)) || a.T <= 16) return linear_packed_launch(a, st);
+    if (a.tp && (a.tp->push || a.tp->reduce)) return linear_packed_launch(a, st);
+    if (a.T <= 16 && !few_tiles(a)) return linear_packed_launch(a, st);
     jsm_status s = packed_check(a, std::min(a.T, 256), packed_paired(a));
     return s != JSM_OK ? s : use_tiled(a.T, a.K) ? linear_tiled_launch(a, st) : linear_mid_launch(a, st);
 }

@@ -1,5 +1,5 @@
-"""The projection kernel for a few dozen tokens over packed weights against float64 products of the same bf16 inputs: both edges of
-its token blocks of 32 / 64 / 128, tiles and half tiles, one to eight CTAs per tile, k-blocks that do not divide among them, more
+"""The projection kernel for a few dozen tokens (and for few tokens and few tiles) over packed weights against float64 products of the same bf16 inputs: both edges of
+its token blocks of 16 / 32 / 64 / 128, tiles and half tiles, one to eight CTAs per tile, k-blocks that do not divide among them, more
 tiles than the chip holds at once, and the fused norm, residual and row statistics of a decoder step."""
 import pytest
 import torch
@@ -10,7 +10,7 @@ from jasmine_b200.model import Llama
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(17, 64, 64), (17, 132, 72), (31, 12, 2048), (32, 2048, 2048), (33, 388, 648), (40, 200, 4104), (63, 1000, 520), (64, 2048, 5504), (64, 6144, 2048),
+SHAPES = [(1, 64, 64), (5, 160, 4096), (8, 2048, 2048), (9, 4100, 520), (16, 4096, 1032), (16, 2048, 5504), (17, 64, 64), (17, 132, 72), (31, 12, 2048), (32, 2048, 2048), (33, 388, 648), (40, 200, 4104), (63, 1000, 520), (64, 2048, 5504), (64, 6144, 2048),
           (64, 19204, 264), (65, 128, 4096), (100, 300, 4104), (127, 2048, 5504), (128, 4608, 4096)]
 
 
@@ -24,7 +24,7 @@ def test_gate_up_pairs(T, N, K):
     tiled.test_gate_up_pairs(T, N, K)
 
 
-@pytest.mark.parametrize("batch", [17, 33, 64])
+@pytest.mark.parametrize("batch", [9, 17, 33, 64])
 @pytest.mark.parametrize("width,kv", [(512, 4), (1024, 2)])
 def test_decoder_step_rows_agree_with_single_sequences(batch, width, kv):
     """A step of `batch` sequences (fused norms, residual, statistics) gives every row what it gets in a batch of its own."""
