@@ -1076,12 +1076,13 @@ static bool use_tiled(int T, int K) { return T > 128 || (T > 64 && K < 4096); }
 // Up to 16 tokens, matrices of so few tiles that four CTAs or more share each: linear_mid.cu's clusters fold with one trip, the streaming
 // kernel's CTAs through the workspace.  Back to back, streaming / clusters, us at 8 and at 16 tokens: 160 x 4096 5.6 / 3.8 and 7.1 / 3.9,
 // 1024 x 2752 5.3 / 4.4 and 6.7 / 4.5, 2048 x 2048 5.1 / 4.9 and 6.8 / 4.9, 2048 x 5504 7.4 / 7.5 and 9.2 / 7.6, 3648 x 2048 6.2 / 5.5 and
-// 7.6 / 5.5, 4096 x 4096 9.0 / 8.4 and 9.3 / 8.5, 4096 x 11008 18.3 / 17.3 and 19.1 / 17.4.  Wider matrices: the even split of the stream
-// keeps all SMs at work (8192 x 2048 9.0 / 9.1, gate/up 11008 x 4096 31.7 / 41.0).
+// 7.6 / 5.5, 4096 x 4096 9.0 / 8.4 and 9.3 / 8.5, 4096 x 11008 18.3 / 17.3 and 19.1 / 17.4.  And matrices of a tile per CTA on most SMs, where
+// nothing is folded: 12288 x 4096 19.8 / 19.8 and 21.7 / 19.5 (19.9 / 19.1 for one token).  In between and beyond, the even split of
+// the stream keeps all SMs at work (8192 x 2048 9.0 / 9.1, gate/up 11008 x 4096 31.7 / 41.0).
 static bool few_tiles(const PackedArgs& a) {
     int nt, kbt;
     pk_dims(a.N, a.K, packed_paired(a), &nt, &kbt);
-    return nt * 4 <= sm_count();
+    return nt * 4 <= sm_count() || (nt * 10 >= sm_count() * 6 && nt <= sm_count());
 }
 
 // Any number of tokens: the streaming kernel below up to 16 (and for exchanges), linear_mid.cu, linear_tiled.cu.
