@@ -630,8 +630,8 @@ static jsm_status run_mixer(jsm_decoder* m, DecLayer& L, const Pass& P, cudaStre
 // a sublayer's output y joins the residual stream
 static jsm_status join_residual(jsm_decoder* m, const float* gain, int T, cudaStream_t st) {
     const jsm_decoder_config& c = m->c;
-    return c.norm_place == JSM_NORM_SUM ? sum_norm_launch(m->y, m->x, gain, c.norm_eps, c.residual_scale, m->xa, T, c.d_model, m->wp, st)
-                                        : post_norm_add_launch(m->y, m->x, gain, c.norm_eps, m->xa, T, c.d_model, m->wp, st);
+    return c.norm_place == JSM_NORM_SUM ? sum_norm_launch(m->y, m->x, gain, c.norm_eps, c.residual_scale, m->xa, T, c.d_model, m->wp, st, true)
+                                        : post_norm_add_launch(m->y, m->x, gain, c.norm_eps, m->xa, T, c.d_model, m->wp, st, true);
 }
 
 static jsm_status run_layers(jsm_decoder* m, const Pass& P, cudaStream_t st) {

@@ -213,10 +213,10 @@ jsm_status rec_step_launch(bool f32, const RecDims& d, const RecWeights& w, cons
 // ---- token-level (tokens.cu) --------------------------------------------------------------------------------------
 // x[t] = table[ids[t]] * scale in f32, and its bf16 copy xa (or null); table act [vocab][wp]
 jsm_status embed_residual_launch(bool f32, const void* table, const int32_t* ids, float scale, float* x, void* xa, int T, int wp, cudaStream_t st);
-// x += y / rms(y) * gain over the first d of wp columns; xa (bf16 copy, or null)
-jsm_status post_norm_add_launch(const float* y, float* x, const float* gain, float eps, void* xa, int T, int d, int wp, cudaStream_t st);
+// x += y / rms(y) * gain over the first d of wp columns; xa (bf16 copy, or null); fixed_gain: no kernel of the stream writes the gain
+jsm_status post_norm_add_launch(const float* y, float* x, const float* gain, float eps, void* xa, int T, int d, int wp, cudaStream_t st, bool fixed_gain);
 // x <- s / rms(s) * gain, s = alpha x + y
-jsm_status sum_norm_launch(const float* y, float* x, const float* gain, float eps, float alpha, void* xa, int T, int d, int wp, cudaStream_t st);
+jsm_status sum_norm_launch(const float* y, float* x, const float* gain, float eps, float alpha, void* xa, int T, int d, int wp, cudaStream_t st, bool fixed_gain);
 // out[i] = x[rows[i]] / rms * gain, act [n][wp]
 jsm_status final_norm_launch(bool f32, const float* x, const int32_t* rows, const float* gain, float eps, void* out, int n, int d, int wp,
                              cudaStream_t st);

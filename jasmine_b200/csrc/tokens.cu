@@ -165,15 +165,22 @@ __global__ void __launch_bounds__(256) embed_residual_kernel(const T* __restrict
 // SUM false: x <- x + norm(y); true: x <- norm(alpha x + y)
 template <int MAXV, bool SUM>
 __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restrict__ y, float* __restrict__ x, const float* __restrict__ gain,
-                                                            float eps, float alpha, __nv_bfloat16* __restrict__ xa, int d, int wp) {
+                                                            float eps, float alpha, __nv_bfloat16* __restrict__ xa, int d, int wp, int fixed_gain) {
     __shared__ float smem[8];
     chain_trigger();
-    chain_wait();
     const long long base = (long long)blockIdx.x * wp;
     auto load8 = [](const float* p, float (&v)[8]) {
         const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     };
+    // a gain that no kernel of the stream writes arrives while the predecessor ends, not in a round trip of its own behind the sum
+    if (!fixed_gain) chain_wait();
+    float gv[MAXV ? MAXV : 1][8];
+    if constexpr (MAXV > 0)
+#pragma unroll
+        for (int i = 0; i < MAXV; ++i)
+            if ((i * 256 + (int)threadIdx.x) * 8 < wp) load8(gain + (i * 256 + threadIdx.x) * 8, gv[i]);
+    chain_wait();
     float keep[MAXV ? MAXV : 1][8], res[MAXV ? MAXV : 1][8];
     float q = 0.0f;
     if constexpr (MAXV > 0) {
@@ -205,9 +212,7 @@ __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restr
     }
     q = block_sum(q, smem) / (float)d;
     const float rms = sqrtf(q + eps);
-    auto update = [&](int c, const float (&v)[8], float (&r)[8]) {
-        float g[8];
-        load8(gain + c, g);
+    auto update = [&](int c, const float (&v)[8], float (&r)[8], const float (&g)[8]) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) r[e] = SUM ? v[e] / rms * g[e] : r[e] + v[e] / rms * g[e];
         reinterpret_cast<float4*>(x + base + c)[0] = make_float4(r[0], r[1], r[2], r[3]);
@@ -218,7 +223,7 @@ __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restr
 #pragma unroll
         for (int i = 0; i < MAXV; ++i) {
             const int c = (i * 256 + threadIdx.x) * 8;
-            if (c < wp) update(c, keep[i], res[i]);
+            if (c < wp) update(c, keep[i], res[i], gv[i]);
         }
     } else {
         for (int c = threadIdx.x * 8; c < wp; c += 2048) {
@@ -228,7 +233,8 @@ __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restr
             if (SUM)
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[e] = fmaf(alpha, r[e], v[e]);
-            update(c, v, r);
+            load8(gain + c, gv[0]);
+            update(c, v, r, gv[0]);
         }
     }
 }
@@ -324,17 +330,18 @@ jsm_status embed_residual_launch(bool f32, const void* table, const int32_t* ids
 }
 
 template <bool SUM>
-static jsm_status norm_residual(const float* y, float* x, const float* gain, float eps, float alpha, void* xa, int T, int d, int wp, cudaStream_t st) {
-    auto go = [&](auto kernel) { return launch_chained(kernel, dim3(T), dim3(256), 0, st, y, x, gain, eps, alpha, (__nv_bfloat16*)xa, d, wp); };
+static jsm_status norm_residual(const float* y, float* x, const float* gain, float eps, float alpha, void* xa, int T, int d, int wp, cudaStream_t st,
+                                bool fixed_gain) {
+    auto go = [&](auto kernel) { return launch_chained(kernel, dim3(T), dim3(256), 0, st, y, x, gain, eps, alpha, (__nv_bfloat16*)xa, d, wp, fixed_gain ? 1 : 0); };
     JSM_CUDA_CHECK(wp <= 2048 ? go(post_norm_add_kernel<1, SUM>) : wp <= 4096 ? go(post_norm_add_kernel<2, SUM>) : go(post_norm_add_kernel<0, SUM>));
     JSM_LAUNCH_CHECK();
     return JSM_OK;
 }
-jsm_status post_norm_add_launch(const float* y, float* x, const float* gain, float eps, void* xa, int T, int d, int wp, cudaStream_t st) {
-    return norm_residual<false>(y, x, gain, eps, 1.0f, xa, T, d, wp, st);
+jsm_status post_norm_add_launch(const float* y, float* x, const float* gain, float eps, void* xa, int T, int d, int wp, cudaStream_t st, bool fixed_gain) {
+    return norm_residual<false>(y, x, gain, eps, 1.0f, xa, T, d, wp, st, fixed_gain);
 }
-jsm_status sum_norm_launch(const float* y, float* x, const float* gain, float eps, float alpha, void* xa, int T, int d, int wp, cudaStream_t st) {
-    return norm_residual<true>(y, x, gain, eps, alpha, xa, T, d, wp, st);
+jsm_status sum_norm_launch(const float* y, float* x, const float* gain, float eps, float alpha, void* xa, int T, int d, int wp, cudaStream_t st, bool fixed_gain) {
+    return norm_residual<true>(y, x, gain, eps, alpha, xa, T, d, wp, st, fixed_gain);
 }
 
 jsm_status final_norm_launch(bool f32, const float* x, const int32_t* rows, const float* gain, float eps, void* out, int n, int d, int wp,
@@ -428,14 +435,14 @@ extern "C" jsm_status jsm_post_norm_add(const float* d_y, float* d_x, const floa
     if (T <= 0) return JSM_OK;
     if (!d_y || !d_x || !d_gain) JSM_FAIL(JSM_INVALID_ARG, "jsm_post_norm_add: null pointer");
     if (d <= 0 || d % 8) JSM_FAIL(JSM_UNSUPPORTED, "jsm_post_norm_add: d %d (a multiple of 8)", d);
-    return post_norm_add_launch(d_y, d_x, d_gain, eps, d_x_bf16, T, d, d, as_stream(stream));
+    return post_norm_add_launch(d_y, d_x, d_gain, eps, d_x_bf16, T, d, d, as_stream(stream), false);
 }
 
 extern "C" jsm_status jsm_sum_norm(const float* d_y, float* d_x, const float* d_gain, float eps, float alpha, void* d_x_bf16, int T, int d, void* stream) {
     if (T <= 0) return JSM_OK;
     if (!d_y || !d_x || !d_gain) JSM_FAIL(JSM_INVALID_ARG, "jsm_sum_norm: null pointer");
     if (d <= 0 || d % 8) JSM_FAIL(JSM_UNSUPPORTED, "jsm_sum_norm: d %d (a multiple of 8)", d);
-    return sum_norm_launch(d_y, d_x, d_gain, eps, alpha, d_x_bf16, T, d, d, as_stream(stream));
+    return sum_norm_launch(d_y, d_x, d_gain, eps, alpha, d_x_bf16, T, d, d, as_stream(stream), false);
 }
 
 extern "C" jsm_status jsm_logits_finish(float* d_logits, int pitch, int rows, int vocab, float cap, uint64_t* d_keys, int32_t* d_counters,
