@@ -211,10 +211,11 @@ jsm_status jsm_linear_bf16_packed_glu(const void* d_X, const void* d_packed, flo
                                       int K, void* stream);
 
 /* Timeline of the packed projections (profiling aid, off by default; the reference has no tracing).  Between
- * jsm_trace_begin and jsm_trace_end every launch of the packed projection kernel (up to max_launches, eager launches
- * only: not inside a replayed graph) records 8 device time stamps in ns per CTA: resident, first weights requested,
- * predecessor complete, first stage landed, last MMA issued, first / last epilogue done, CTA done.
- * h_stamps: [n_launches][ctas_per_launch][8] uint64, zero where a CTA did not exist. */
+ * jsm_trace_begin and jsm_trace_end every launch of a projection over packed weights, whichever kernel runs it (up to
+ * max_launches, eager launches only: not inside a replayed graph), records 8 device time stamps in ns per CTA (of its
+ * first ctas_per_launch: one per SM): resident, first weights requested, predecessor complete, first stage landed, last
+ * MMA issued, first / last epilogue done, CTA done.
+ * h_stamps: [n_launches][ctas_per_launch][8] uint64, zero where a CTA did not exist or had no such event. */
 jsm_status jsm_trace_begin(int max_launches);
 jsm_status jsm_trace_end(uint64_t* h_stamps, int max_launches, int* n_launches, int* ctas_per_launch);
 

@@ -105,6 +105,17 @@ size_t linear_packed_bytes(int N, int K, int paired);
 size_t linear_packed_ws_floats(int T, int N, int K, int paired);
 // packs (or, with unpack, rebuilds) a row-major [N, K] matrix ([2N, K] gate rows then up rows when paired)
 jsm_status linear_pack_launch(const void* W, int N, int K, int paired, void* packed, bool unpack, cudaStream_t st);
+// place of the next traced launch's stamps ([*ctas][8]; null: no trace runs, or it is full)
+unsigned long long* linear_trace_next(int* ctas);
+// stamp of one CTA, by one thread: 0 resident, 1 first weights requested, 2 predecessor complete, 3 first stage landed, 4 last MMA issued,
+// 5 / 6 first / last epilogue done, 7 CTA done
+__device__ __forceinline__ void lin_stamp(unsigned long long* trace, int ctas, int slot) {
+    if (trace && (int)blockIdx.x < ctas) {
+        unsigned long long t;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+        trace[(size_t)blockIdx.x * 8 + slot] = t;
+    }
+}
 jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st);  // T <= 256
 // any T; the launches of a call that is split share R, Y and the row statistics of the whole call
 jsm_status linear_packed_tokens(const PackedArgs& a, cudaStream_t st);

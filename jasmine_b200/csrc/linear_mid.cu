@@ -46,6 +46,8 @@ struct LmParams {
     float* ssq_out;
     float glu_alpha, glu_limit;
     int* err;
+    unsigned long long* trace;
+    int trace_ctas;
 };
 
 __device__ __forceinline__ uint32_t lm_reg_rank() {
@@ -94,7 +96,9 @@ __device__ __forceinline__ bool lm_wait_cluster(uint64_t* bar, uint32_t parity, 
 constexpr int lm_stages(int bn) { return bn <= 32 ? 4 : bn == 64 ? 3 : 2; }
 constexpr int lm_smem(int bn) { return lm_stages(bn) * 2 * ((int)LM_UNIT + bn * 128) + (bn + 64) * 512 + 1024; }
 
-template <int BN, int KIND>
+// TRACED: an image of its own for launches that record time stamps (tests of a null pointer in every launch cost 0.1 us)
+#define LM_STAMP(slot) do { if constexpr (TRACED) lin_stamp(P.trace, P.trace_ctas, slot); } while (0)
+template <int BN, int KIND, bool TRACED>
 __global__ void __launch_bounds__(LM_THREADS, 1) linear_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, LmParams P) {
     constexpr int STAGES = lm_stages(BN);
     constexpr uint32_t X_BYTES = BN * 128, X_OFF = 2 * LM_UNIT, STAGE = 2 * (LM_UNIT + X_BYTES);
@@ -109,6 +113,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) linear_mid_kernel(const __grid_
     __shared__ float row_scale[BN];
 
     chain_trigger();
+    if (threadIdx.x == 0) LM_STAMP(0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int S = (int)lm_reg_size(), rank = (int)lm_reg_rank(), tile = (int)blockIdx.x / S;
     const int kb0 = P.kbt * rank / S, kb1 = P.kbt * (rank + 1) / S;
@@ -148,6 +153,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) linear_mid_kernel(const __grid_
                 else bulk_load(tiles + s * STAGE, src + (size_t)kb * LM_UNIT, (uint32_t)n * LM_UNIT, &full_bar[s]);
             }
             __syncwarp();
+            if (n_issued == STAGES - 1 && lane == 0) LM_STAMP(1);
             if (++s == STAGES) { s = 0; ph ^= 1; }
         }
         if (abort_flag) {  // let the copies in flight land (bounded)
@@ -158,6 +164,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) linear_mid_kernel(const __grid_
         lm_cluster_arrive();
     } else if (warp == 2) {
         chain_wait();
+        if (lane == 0) LM_STAMP(2);
         int s = 0, i = 0;
         uint32_t ph = 0;
         for (int kb = kb0; kb < kb1; kb += 2, ++i) {
@@ -184,6 +191,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) linear_mid_kernel(const __grid_
         for (int kb = kb0; kb < kb1; kb += 2) {
             ok = mbar_wait_warp(&full_bar[s], ph, &abort_flag, P.err, TC_TIMEOUT_FULL);
             if (!ok) break;
+            if (kb == kb0 && lane == 0) LM_STAMP(3);
             tc_fence_after();
             const uint32_t addr = smem_u32(tiles + s * STAGE);
             const bool both = kb + 1 < kb1;
@@ -202,6 +210,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) linear_mid_kernel(const __grid_
         }
         if (ok && elect_one()) mma_commit(&acc_full);
         __syncwarp();
+        if (lane == 0) LM_STAMP(4);
         lm_cluster_wait();
         lm_cluster_arrive();
     } else if (warp >= 4) {
@@ -327,6 +336,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) linear_mid_kernel(const __grid_
                 for (int lt = etid >> shift; lt < n_own; lt += 256 >> shift) finish(lt, make_uint2(0u, 0u));
             }
         }
+        if (etid == 0) LM_STAMP(5);
     } else {
         lm_cluster_wait();
         lm_cluster_arrive();
@@ -339,10 +349,11 @@ __global__ void __launch_bounds__(LM_THREADS, 1) linear_mid_kernel(const __grid_
         tmem_dealloc(tmem, TMEM_COLS);
     }
     lm_cluster_wait();  // no CTA leaves while a peer may still write into it
+    if (threadIdx.x == 0) LM_STAMP(7);
 }
 
 // clusters of S CTAs that the chip holds at once (15 of eight, 33 of four, 45 of three, although it has 148 multiprocessors)
-template <int BN, int KIND>
+template <int BN, int KIND, bool TRACED>
 static int mid_capacity(int S) {
     static std::mutex mu;
     static int known[9];
@@ -359,7 +370,7 @@ static int mid_capacity(int S) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, linear_mid_kernel<BN, KIND>, &cfg) != cudaSuccess || n <= 0) {
+        if (cudaOccupancyMaxActiveClusters(&n, linear_mid_kernel<BN, KIND, TRACED>, &cfg) != cudaSuccess || n <= 0) {
             cudaGetLastError();
             n = S == 1 ? sm_count() : sm_count() / S * 3 / 4;
         }
@@ -370,28 +381,29 @@ static int mid_capacity(int S) {
 
 // CTAs per tile and the tile's height.  A CTA takes 0.3 us per unit of 16 KB (55 GB/s: the rate of one multiprocessor's copies), or its
 // share of the memory's 6.4 TB/s, and about 4 us around it; clusters that do not fit at once wait for the first ones.
-template <int BN, int KIND>
+template <int BN, int KIND, bool TRACED>
 static void mid_shape(int n_tiles, int kbt, bool may_halve, int* S_out, int* half_out) {
     float best = 0.0f;
     *S_out = 0;
     for (int half = 0; half <= (may_halve ? 1 : 0); ++half)
         for (int S = 1; S <= 8 && S <= kbt; ++S) {
-            const int tiles = n_tiles << half, cap = mid_capacity<BN, KIND>(S), at_once = std::min(tiles, cap) * S;
+            const int tiles = n_tiles << half, cap = mid_capacity<BN, KIND, TRACED>(S), at_once = std::min(tiles, cap) * S;
             const float unit = std::max(half ? 0.17f : 0.3f, (half ? 0.5f : 1.0f) * 16.384e-3f * (float)at_once / 6.4f);
             const float cost = (float)((tiles + cap - 1) / cap) * (4.0f + (S > 1 ? 0.5f : 0.0f) + (float)((kbt + S - 1) / S) * unit);
             if (*S_out == 0 || cost < best) { best = cost; *S_out = S; *half_out = half; }
         }
 }
 
-template <int BN, int KIND>
+template <int BN, int KIND, bool TRACED = false>
 static jsm_status launch_mid(const PackedArgs& a, LmParams& P, int n_tiles, cudaStream_t st) {
+    if (!TRACED && (P.trace = linear_trace_next(&P.trace_ctas))) return launch_mid<BN, KIND, true>(a, P, n_tiles, st);
     static bool attr_done = false;  // per instantiation
     if (!attr_done) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(linear_mid_kernel<BN, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, lm_smem(BN)));
+        JSM_CUDA_CHECK(cudaFuncSetAttribute(linear_mid_kernel<BN, KIND, TRACED>, cudaFuncAttributeMaxDynamicSharedMemorySize, lm_smem(BN)));
         attr_done = true;
     }
     int S, half;
-    mid_shape<BN, KIND>(n_tiles, P.kbt, KIND != 2 && !a.ssq_out, &S, &half);
+    mid_shape<BN, KIND, TRACED>(n_tiles, P.kbt, KIND != 2 && !a.ssq_out, &S, &half);
     P.half = half;
     CUtensorMap mx;
     jsm_status s = make_tmap_bf16_2d(&mx, a.X, (uint64_t)a.T, (uint64_t)a.K, (uint64_t)(a.x_row_stride > 0 ? a.x_row_stride : a.K), BN, 64);
@@ -410,7 +422,7 @@ static jsm_status launch_mid(const PackedArgs& a, LmParams& P, int n_tiles, cuda
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = a.chained && chained_launch_enabled() ? 2 : 1;
-    JSM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, linear_mid_kernel<BN, KIND>, mx, P));
+    JSM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, linear_mid_kernel<BN, KIND, TRACED>, mx, P));
     g_launches.fetch_add(1);
     return JSM_OK;
 }

@@ -66,7 +66,8 @@ struct PkParams {
     int ssq_stride;       // row pitch of ssq_in and ssq_out (tokens of the whole call)
     float inv_d, eps;     // 1 / (features of X), epsilon under the square root
     float* ssq_out;       // [n_tiles][ssq_stride]: sums of squares of this launch's outputs per tile and token, or null
-    unsigned long long* trace;  // optional timeline: 8 time stamps (globaltimer, ns) per CTA of this launch
+    unsigned long long* trace;  // optional timeline: 8 time stamps (globaltimer, ns) for each of the first trace_ctas CTAs of this launch
+    int trace_ctas;
     // tensor-parallel exchange fused into the launch (TpFuse in linear_bf16.cuh; protocol in tp_comm.cu)
     int tp_mode;                // 0 none, 1 push the outputs to every rank's slot, 2 reduce the slots into h before X is read
     int tp_n, tp_rank;
@@ -132,15 +133,7 @@ __device__ __forceinline__ void pk_wait_epoch(const int* p, int E, long long lim
 // local state words of the fused exchange: [0] folding CTAs of a pushing launch done, [1] tiles of h reduced (both
 // self-resetting), [2] epoch up to which h is completely reduced
 
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-#define PK_TRACE(slot)                                                              \
-    do {                                                                            \
-        if (P.trace) P.trace[(size_t)blockIdx.x * 8 + (slot)] = global_ns();        \
-    } while (0)
+#define PK_TRACE(slot) lin_stamp(P.trace, P.trace_ctas, slot)
 
 // unit range of CTA c: [c*U/G, (c+1)*U/G)
 __host__ __device__ inline long long pk_begin(long long c, long long U, long long G) { return c * U / G; }
@@ -980,6 +973,12 @@ size_t linear_packed_ws_floats(int T, int N, int K, int paired) {
 static unsigned long long* g_trace_buf = nullptr;  // [launch][CTA][8]
 static int g_trace_cap = 0, g_trace_n = 0, g_trace_ctas = 0;
 
+unsigned long long* linear_trace_next(int* ctas) {
+    *ctas = g_trace_ctas;
+    if (!g_trace_buf || g_trace_n >= g_trace_cap) return nullptr;
+    return g_trace_buf + (size_t)g_trace_n++ * g_trace_ctas * 8;
+}
+
 template <int BN, bool CL, int TPM, int PRM = -1>
 static jsm_status launch_packed(const CUtensorMap& mx, const CUtensorMap& mx2, PkParams& P, int grid, int cluster, bool chained, cudaStream_t st) {
     constexpr int STAGE_BYTES = 2 * (PK_TILE_BYTES + BN * 128);
@@ -989,11 +988,7 @@ static jsm_status launch_packed(const CUtensorMap& mx, const CUtensorMap& mx2, P
     if (stages > PK_MAX_STAGES) stages = PK_MAX_STAGES;
     if (stages < 2) stages = 2;
     P.stages = stages;
-    P.trace = nullptr;
-    if (g_trace_buf && g_trace_n < g_trace_cap && grid <= g_trace_ctas) {
-        P.trace = g_trace_buf + (size_t)g_trace_n * g_trace_ctas * 8;
-        ++g_trace_n;
-    }
+    P.trace = linear_trace_next(&P.trace_ctas);
     const size_t smem = (size_t)stages * STAGE_BYTES + 1024;
     static bool attr_done = false;  // per instantiation
     if (!attr_done) {

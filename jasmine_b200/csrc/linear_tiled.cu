@@ -48,6 +48,8 @@ struct LtParams {
     float* ssq_out;
     float glu_alpha, glu_limit;
     int* err;
+    unsigned long long* trace;
+    int trace_ctas;
 };
 
 // ---- pairs of CTAs: PTX of cta_group::2 ----------------------------------------------------------------------------------
@@ -97,8 +99,10 @@ __device__ __forceinline__ void lt_arrive_leader(uint32_t leader_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_bar) : "memory");
 }
 
+// TRACED: an image of its own for launches that record time stamps.
+#define LT_STAMP(slot) do { if constexpr (TRACED) lin_stamp(P.trace, P.trace_ctas, slot); } while (0)
 // BN: features (packed rows) per tile.  PAIRED: packed tiles of 64 gate and 64 up rows, BN / 2 outputs per token and tile.
-template <int BN, bool PAIRED>
+template <int BN, bool PAIRED, bool TRACED>
 __global__ void __launch_bounds__(LT_THREADS, 1)
     linear_tiled_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, LtParams P) {
     constexpr int W_ROWS = BN / 2;                 // weight rows per CTA and k-block
@@ -114,6 +118,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1)
     uint8_t* stage_out = tiles + P.stages * STAGE;  // 4 KB per epilogue warp
 
     chain_trigger();
+    if (threadIdx.x == 0) LT_STAMP(0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const int cluster = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
@@ -179,7 +184,9 @@ __global__ void __launch_bounds__(LT_THREADS, 1)
             if (elect_one()) load_w(filled, p);
             __syncwarp();
         }
+        if (lane == 0) LT_STAMP(1);
         chain_wait();
+        if (lane == 0) LT_STAMP(2);
         for (int s = 0; s < filled; ++s, next(px)) {
             if (elect_one()) load_x(s, px);
             __syncwarp();
@@ -216,6 +223,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1)
                 for (int kb = 0; kb < P.kbt; kb += LT_KB) {
                     ok = mbar_wait_warp(&full_bar[s], ph, &abort_flag, P.err, TC_TIMEOUT_FULL);
                     if (!ok) break;
+                    if (it == 0 && kb == 0 && lane == 0) LT_STAMP(3);
                     tc_fence_after();
                     const uint32_t addr = smem_u32(tiles + s * STAGE);
                     const uint64_t a_desc = smem_desc_sw128(addr), b_desc = smem_desc_sw128(addr + LT_KB * X_BYTES);
@@ -236,6 +244,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1)
                 if (ok && elect_one()) lt_commit(&acc_full[buf]);
                 __syncwarp();
             }
+            if (lane == 0) LT_STAMP(4);
         }
     } else {
         const int quad = warp & 3;  // TMEM lanes this warp reads
@@ -364,6 +373,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1)
                     for (int k = 0; k < 8; ++k)
                         if (t0 + 4 * k + r4 < P.T) P.ssq_out[(size_t)tile128 * P.ssq_stride + t0 + 4 * k + r4] = ssq[k];
             }
+            if (warp == 2 && lane == 0) LT_STAMP(it == 0 ? 5 : 6);
         }
     }
     tc_fence_before();
@@ -374,10 +384,12 @@ __global__ void __launch_bounds__(LT_THREADS, 1)
         tc_fence_after();
         lt_tmem_dealloc(tmem_base, TMEM_COLS);
     }
+    if (threadIdx.x == 0) LT_STAMP(7);
 }
 
-template <int BN, bool PAIRED>
+template <int BN, bool PAIRED, bool TRACED = false>
 static jsm_status launch_tiled(const PackedArgs& a, LtParams& P, int n_tiles, cudaStream_t st) {
+    if (!TRACED && (P.trace = linear_trace_next(&P.trace_ctas))) return launch_tiled<BN, PAIRED, true>(a, P, n_tiles, st);
     constexpr int STAGE = LT_KB * (128 * 128 + BN / 2 * 128);
     P.stages = std::min(LT_MAX_STAGES, 192 * 1024 / STAGE);
     const size_t smem = (size_t)P.stages * STAGE + LT_EPI * 4096 + 1024;
@@ -391,7 +403,7 @@ static jsm_status launch_tiled(const PackedArgs& a, LtParams& P, int n_tiles, cu
     if (s != JSM_OK) return s;
     static bool attr_done = false;  // per instantiation
     if (!attr_done) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(linear_tiled_kernel<BN, PAIRED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        JSM_CUDA_CHECK(cudaFuncSetAttribute(linear_tiled_kernel<BN, PAIRED, TRACED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_done = true;
     }
     cudaLaunchConfig_t cfg = {};
@@ -408,7 +420,7 @@ static jsm_status launch_tiled(const PackedArgs& a, LtParams& P, int n_tiles, cu
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = a.chained && chained_launch_enabled() ? 2 : 1;
-    JSM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, linear_tiled_kernel<BN, PAIRED>, mx, mw, P));
+    JSM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, linear_tiled_kernel<BN, PAIRED, TRACED>, mx, mw, P));
     g_launches.fetch_add(1);
     return JSM_OK;
 }
