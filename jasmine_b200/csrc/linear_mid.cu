@@ -379,17 +379,22 @@ static int mid_capacity(int S) {
     return known[S];
 }
 
-// CTAs per tile and the tile's height.  A CTA takes 0.3 us per unit of 16 KB (55 GB/s: the rate of one multiprocessor's copies), or its
-// share of the memory's 6.4 TB/s, and about 4 us around it; clusters that do not fit at once wait for the first ones.
+// CTAs per tile and the tile's height.  A CTA takes 0.3 us per unit of 64 k of a whole tile (the rate of one multiprocessor's copies; beyond 64
+// tokens their bytes show: 0.36), or its share of the memory's 6.4 TB/s, and about 4 us around it; clusters that do not fit at once
+// wait for the first ones.  A unit of a half tile brings the same bytes of tokens: 0.17 us up to 16 of them, 0.19 up to 32, 0.24 up to 64, 0.355
+// up to 128.  8192 x 4096 over 32, 64 and 100 tokens: 128 half tiles 15.1, 18.2 and 27.0 us, 64 clusters of two 12.9, 14.3 and 18.4 us;
+// 2048 x 1024 over 64: half tiles 4.9 us, whole ones 5.4.
 template <int BN, int KIND, bool TRACED>
 static void mid_shape(int n_tiles, int kbt, bool may_halve, int* S_out, int* half_out) {
+    constexpr float whole_us = BN <= 64 ? 0.3f : 0.36f, half_us = BN == 16 ? 0.17f : BN == 32 ? 0.19f : BN == 64 ? 0.24f : 0.355f;
+    constexpr float half_around = BN == 16 ? 4.0f : 3.5f;
     float best = 0.0f;
     *S_out = 0;
     for (int half = 0; half <= (may_halve ? 1 : 0); ++half)
         for (int S = 1; S <= 8 && S <= kbt; ++S) {
             const int tiles = n_tiles << half, cap = mid_capacity<BN, KIND, TRACED>(S), at_once = std::min(tiles, cap) * S;
-            const float unit = std::max(half ? 0.17f : 0.3f, (half ? 0.5f : 1.0f) * 16.384e-3f * (float)at_once / 6.4f);
-            const float cost = (float)((tiles + cap - 1) / cap) * (4.0f + (S > 1 ? 0.5f : 0.0f) + (float)((kbt + S - 1) / S) * unit);
+            const float unit = std::max(half ? half_us : whole_us, (half ? 0.5f : 1.0f) * 16.384e-3f * (float)at_once / 6.4f);
+            const float cost = (float)((tiles + cap - 1) / cap) * ((half ? half_around : 4.0f) + (S > 1 ? 0.5f : 0.0f) + (float)((kbt + S - 1) / S) * unit);
             if (*S_out == 0 || cost < best) { best = cost; *S_out = S; *half_out = half; }
         }
 }

@@ -45,7 +45,6 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* gsrc, uint32_t byte
 struct PkParams {
     int T, N, K;          // tokens (<= BN), output features (paired: gate features), reduction length
     int n_tiles, kbt;     // tiles of 128 packed rows, k-blocks of 64 per tile
-    int local_epi;        // whole tiles that end a CTA's range use the vectorised epilogue through shared memory
     int paired;           // epilogue silu(gate) * up over a paired tile
     int epilogue;         // LIN_* (LIN_SILU_MUL exactly when paired)
     int out_f32;
@@ -186,8 +185,14 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
     __shared__ uint32_t tmem_base_smem;
     __shared__ int abort_flag;
     __shared__ int is_last_smem[2];
-    __shared__ float row_scale[BN];       // 1 / rms of every token when the RMSNorm is fused into this projection
-    __shared__ __align__(16) float stage_small[BN * 128];  // a whole tile's accumulator: every tile takes the one vectorised epilogue
+    // ROWS: whole tiles that do not end the CTA's range take the row-per-thread epilogue straight from the accumulator (the
+    // stage ring is busy).  The images of up to 64 tokens have a staging tile of their own instead and send every whole
+    // tile through the vectorised epilogue: one epilogue, a third less code to fetch in the tail that runs once per launch.
+    constexpr bool ROWS = BN >= 128;
+    __shared__ float pair_smem[ROWS ? 64 * 17 : 1];   // paired epilogue: up values of 16 token columns, padded rows
+    __shared__ float row_scale[256];                  // 1 / rms of every token when the RMSNorm is fused into this projection
+    __shared__ float ssq_part[ROWS ? 4 * 256 : 1];    // per-warp sums of squares of a whole tile's outputs
+    __shared__ __align__(16) float stage_small[ROWS ? 4 : BN * 128];  // up to 64 tokens: a whole tile's accumulator
     __shared__ int tp_ok_smem;            // reduce: every peer's flag arrived in time
 
     // PRM: what the image can do.  -1: everything; 0 / 1: plain tiles only / gate-up pairs only (what the other kind needs is
@@ -560,7 +565,7 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
             const float* tbase = P.ws + (size_t)tile * P.max_slots * slot_stride;
             float* wbase = P.ws + ((size_t)tile * P.max_slots + slot) * slot_stride;
             bool solo = false;
-            if (!whole && u + len == u_end && !(CL && P.cluster_s > 1) && P.local_epi) {
+            if (!whole && u + len == u_end && !(CL && P.cluster_s > 1)) {
                 if (etid == 0) {
                     const int nc = n_contrib;
                     int c;
@@ -574,14 +579,98 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
             tc_fence_after();
             const bool scaled = has_ssq_in;
             const uint32_t acc_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN);
-            const bool local = whole;  // a whole tile goes through its staging tile, a shared one as described below
-            {
+            // A whole tile that is this CTA's last segment goes through shared memory (the stage ring is free: every MMA
+            // of the CTA has completed) and the vectorised epilogue below, whose stores are 8 or 16 bytes per thread and
+            // contiguous per token; earlier segments overlap the main loop and keep the row-per-thread epilogue.
+            const bool local = whole && (!ROWS || u + len == u_end);
+            bool rows_done = false;
+            if constexpr (ROWS) {
+            if (whole && !local) {
+                rows_done = true;
+                // ---- the tile is complete in this CTA: epilogue straight from the accumulator
+                if (!paired) {
+                    const int n = tile * 128 + row;
+                    const bool valid = n < P.N;
+                    const float bias = (biasp && valid) ? biasp[n] : 0.0f;
+#pragma unroll 1
+                    for (int c0 = 0; c0 < BN; c0 += 16) {
+                        if (c0 >= P.T) break;
+                        uint32_t r[16];
+                        tmem_ld16(acc_addr + c0, r);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const int t = c0 + j;  // warp-uniform
+                            if (t < P.T) {
+                                float v = __uint_as_float(r[j]);
+                                if (scaled) v *= row_scale[t];
+                                v += bias;
+                                if (epi == LIN_RELU) v = fmaxf(v, 0.0f);
+                                else if (epi == LIN_GELU) v = pk_gelu(v);
+                                else if ((!paired && epi == LIN_RESIDUAL) && valid) v += __bfloat162float(P.R[(size_t)t * P.N + n]);
+                                float stored = v;
+                                if (!f32o) {
+                                    const __nv_bfloat16 hb = __float2bfloat16_rn(v);
+                                    stored = __bfloat162float(hb);
+                                    if (valid) reinterpret_cast<__nv_bfloat16*>(P.Y)[(size_t)t * P.N + n] = hb;
+                                } else if (valid) {
+                                    reinterpret_cast<float*>(P.Y)[(size_t)t * P.N + n] = v;
+                                }
+                                if (want_ssq) {  // sum of squares of what was stored, over the 128 features of the tile
+                                    const float sq = warp_sum(valid ? stored * stored : 0.0f);
+                                    if (lane == 0) ssq_part[quad * 256 + t] = sq;
+                                }
+                            }
+                        }
+                    }
+                    if (want_ssq) {
+                        asm volatile("bar.sync 1, 128;" ::: "memory");
+                        for (int t = etid; t < P.T; t += 128)
+                            P.ssq_out[(size_t)tile * P.ssq_stride + t] = (ssq_part[t] + ssq_part[256 + t]) + (ssq_part[512 + t] + ssq_part[768 + t]);
+                        asm volatile("bar.sync 1, 128;" ::: "memory");
+                    }
+                } else {
+                    // lanes 0..63 hold gate, lanes 64..127 the matching up rows: hand the up values over through shared memory
+                    const int f = row & 63;
+                    const int n = tile * 64 + f;
+#pragma unroll 1
+                    for (int c0 = 0; c0 < BN; c0 += 16) {
+                        if (c0 >= P.T) break;
+                        uint32_t r[16];
+                        tmem_ld16(acc_addr + c0, r);
+                        tmem_ld_wait();
+                        if (row >= 64) {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) pair_smem[f * 17 + j] = __uint_as_float(r[j]);
+                        }
+                        asm volatile("bar.sync 1, 128;" ::: "memory");
+                        if (row < 64 && n < P.N) {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                const int t = c0 + j;
+                                if (t < P.T) {
+                                    const float sc = scaled ? row_scale[t] : 1.0f;
+                                    const float v = gate_up(__uint_as_float(r[j]) * sc, pair_smem[f * 17 + j] * sc);
+                                    if (f32o) reinterpret_cast<float*>(P.Y)[(size_t)t * P.N + n] = v;
+                                    else reinterpret_cast<__nv_bfloat16*>(P.Y)[(size_t)t * P.N + n] = __float2bfloat16_rn(v);
+                                }
+                            }
+                        }
+                        asm volatile("bar.sync 1, 128;" ::: "memory");
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[buf]);
+            }
+            }
+            if (!rows_done) {
                 // ---- shared tile: store the raw partial in this CTA's slot, the last contributor folds
                 // aligned split: the contributors are the CTAs of this cluster and the partial goes to this CTA's own shared
                 // memory (the stage ring is free: every MMA of the CTA has completed); otherwise to its workspace slot
                 const bool cl = CL && P.cluster_s > 1 && !local;
-                float* part_smem = local ? stage_small : reinterpret_cast<float*>(tiles);
-                if (local) asm volatile("bar.sync 1, 128;" ::: "memory");  // the previous tile's fold has read the staging tile
+                float* part_smem = (!ROWS && local) ? stage_small : reinterpret_cast<float*>(tiles);
+                if (!ROWS && local) asm volatile("bar.sync 1, 128;" ::: "memory");  // the previous tile's fold has read the staging tile
                 const bool to_smem = cl || local || solo;
                 if (BN >= 32 && to_smem) {
                     // 32 columns per round trip to tensor memory
@@ -1064,42 +1153,60 @@ static int packed_paired(const PackedArgs& a) {
     return a.epilogue == LIN_SILU_MUL || a.epilogue == LIN_CLAMPED_GLU || a.epilogue == LIN_GELU_GLU ? 1 : 0;
 }
 
-// Which kernel takes a call of 17 tokens or more over a depth of K.  The tiled kernel gains from its whole tiles of 256 tokens, the one for a
-// few dozen tokens from its split along K: T = 100, us: 2048 x 2048 9 tiled; 4096 x 11008 36 tiled, 26 split; 2048 x 5504 15 split.
-static bool use_tiled(int T, int K) { return T > 128 || (T > 64 && K < 4096); }
-
-// Up to 16 tokens, matrices of so few tiles that four CTAs or more share each: linear_mid.cu's clusters fold with one trip, the streaming
-// kernel's CTAs through the workspace.  Back to back, streaming / clusters, us at 8 and at 16 tokens: 160 x 4096 5.6 / 3.8 and 7.1 / 3.9,
-// 1024 x 2752 5.3 / 4.4 and 6.7 / 4.5, 2048 x 2048 5.1 / 4.9 and 6.8 / 4.9, 2048 x 5504 7.4 / 7.5 and 9.2 / 7.6, 3648 x 2048 6.2 / 5.5 and
-// 7.6 / 5.5, 4096 x 4096 9.0 / 8.4 and 9.3 / 8.5, 4096 x 11008 18.3 / 17.3 and 19.1 / 17.4.  And matrices of a tile per CTA on most SMs, where
-// nothing is folded: 12288 x 4096 19.8 / 19.8 and 21.7 / 19.5 (19.9 / 19.1 for one token).  In between and beyond, the even split of
-// the stream keeps all SMs at work (8192 x 2048 9.0 / 9.1, gate/up 11008 x 4096 31.7 / 41.0).
-static bool few_tiles(const PackedArgs& a) {
+// Which kernel takes a call without an exchange, by tokens, packed tiles of 128 rows and depth.  The streaming kernel splits the stream evenly over
+// all SMs whatever the number of tiles; linear_mid.cu launches a cluster per tile, which folds in one trip but leaves a wave that is
+// nearly empty where there are more tiles than SMs; linear_tiled.cu reads weights once for 256 tokens, without a split along K.
+// Back to back over weights that do not fit L2, us (streaming / clusters / tiled):
+// Up to 16 tokens, clusters where four CTAs or more share a tile (at 8 tokens 160 x 4096 6.0 / 3.9, 2048 x 2048 5.3 / 5.0, 2048 x 5504 8.0 / 7.7,
+// 4096 x 4096 9.1 / 8.2, 4096 x 11008 17.4 / 16.3) and where most SMs have a tile of their own, so that nothing is folded (9600 x 4096 15.5 / 15.0,
+// 12288 x 4096 18.5 / 17.5, at 4 tokens 16384 x 4096 22.3 / 21.6); in between the even split (8192 x 2048 9.0 / 9.1).
+// Up to 64, clusters up to a tile per SM; beyond, at 17 and 64 tokens: gate/up 11008 x 4096 33 / 41 and 39 / 46, 24000 x 2048 20 / 29 and 24 / 34,
+// 32000 x 4096 43 / 44 and 48 / 50.  Three or four blocks of depth and 16 tiles or more have nothing to split: 8192 x 256 at 17 3.4 / 4.1,
+// gate/up 2048 x 256 at 8 3.1 / 4.2 (at 32 6.2 / 4.6).
+// Up to 128, of matrices less than 4096 deep: clusters up to a tile per SM (1024 x 2752 at 65 - / 9.2 / 11.2; gate/up pairs keep the tiled kernel:
+// 3072 x 1024 at 128 - / 9.0 / 8.2), else tiled (22016 x 2048 at 65 34 / 33 / 26).  Deeper: the tokens' bytes pass through every CTA of a
+// tile once more per unit, which the even split spreads best over most of the SMs' number of tiles of 8192 (12288 x 8192 at 128 52 / 54 / 53; up to
+// 80 tokens from a third on: 6144 x 8192 at 65 28 / 29 / 32) and up to 96 tokens from half of the SMs on (12288 x 4096 at 65 27 / 29 / 30); more
+// tiles than SMs: gate/up 11008 x 4096 at 65 41 / 55 / 44, at 128 49 / 60 / 45, but gate/up 28672 x 4096 (three waves) 96 / 130 / 107.
+// More: tiled; a very deep matrix of a few tiles is split (288 x 8192 at 129 21 / - / 26, 1024 x 11008 at 256 29 / - / 34).
+enum PackedRoute { ROUTE_STREAM, ROUTE_CLUSTERS, ROUTE_TILED };
+static PackedRoute packed_route(const PackedArgs& a) {
+    const int sms = sm_count(), T = a.T, K = a.K;
+    const bool paired = packed_paired(a);
     int nt, kbt;
-    pk_dims(a.N, a.K, packed_paired(a), &nt, &kbt);
-    return nt * 4 <= sm_count() || (nt * 10 >= sm_count() * 6 && nt <= sm_count());
+    pk_dims(a.N, K, paired, &nt, &kbt);
+    if (K > 128 && K <= 256 && nt >= 16 && nt <= sms && T <= (paired ? 16 : 24)) return ROUTE_STREAM;
+    if (T <= 16) return nt * 4 <= sms || (nt * 10 >= sms * 6 && nt <= sms) ? ROUTE_CLUSTERS : ROUTE_STREAM;
+    if (T <= 64) return nt > sms && (K >= 512 || !paired) ? ROUTE_STREAM : ROUTE_CLUSTERS;
+    if (T <= 128) {
+        if (K < 4096) return nt <= sms && !paired && K >= 512 ? ROUTE_CLUSTERS : ROUTE_TILED;
+        if ((K >= 8192 && (nt * 10 >= sms * 6 || (T <= 80 && nt * 10 >= sms * 3))) || nt >= 2 * sms) return ROUTE_STREAM;
+        if (nt <= sms) return T <= 96 && nt * 2 > sms ? ROUTE_STREAM : ROUTE_CLUSTERS;
+        return T <= 80 ? ROUTE_STREAM : ROUTE_TILED;
+    }
+    return T <= 256 && K >= 8192 && nt <= 8 && a.epilogue != LIN_CLAMPED_GLU && a.epilogue != LIN_GELU_GLU ? ROUTE_STREAM : ROUTE_TILED;
 }
 
-// Any number of tokens: the streaming kernel below up to 16 (and for exchanges), linear_mid.cu, linear_tiled.cu.
+// Any number of tokens.
 jsm_status linear_packed_tokens(const PackedArgs& a, cudaStream_t st) {
     if (a.T <= 0 || a.N <= 0) return JSM_OK;
     if (a.tp && (a.tp->push || a.tp->reduce)) return linear_packed_launch(a, st);
-    if (a.T <= 16 && !few_tiles(a)) return linear_packed_launch(a, st);
+    const PackedRoute route = packed_route(a);
+    if (route == ROUTE_STREAM) return linear_packed_launch(a, st);
     jsm_status s = packed_check(a, std::min(a.T, 256), packed_paired(a));
-    return s != JSM_OK ? s : use_tiled(a.T, a.K) ? linear_tiled_launch(a, st) : linear_mid_launch(a, st);
+    return s != JSM_OK ? s : route == ROUTE_TILED ? linear_tiled_launch(a, st) : linear_mid_launch(a, st);
 }
 
 jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st) {
     if (a.T <= 0 || a.N <= 0) return JSM_OK;
     const bool tp_push = a.tp && a.tp->push, tp_reduce = a.tp && a.tp->reduce;
-    if (a.T > (tp_push || tp_reduce ? TP_PUSH_MAX_T : 16)) JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: the fused exchange takes at most %d tokens (%d)", TP_PUSH_MAX_T, a.T);
+    if (a.T > 256) JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: at most 256 tokens per launch (%d)", a.T);
     const int paired = packed_paired(a);
     jsm_status s = packed_check(a, a.T, paired);
     if (s != JSM_OK) return s;
     PkParams P;
     P.T = a.T; P.N = a.N; P.K = a.K;
     pk_dims(a.N, a.K, paired, &P.n_tiles, &P.kbt);
-    P.local_epi = 1;
     P.paired = paired; P.epilogue = a.epilogue; P.out_f32 = a.out_f32 ? 1 : 0;
     P.glu_alpha = a.glu_alpha; P.glu_limit = a.glu_limit;
     P.bias = a.bias; P.R = (const __nv_bfloat16*)a.R; P.Y = a.Y; P.Wp = (const uint8_t*)a.Wp;
@@ -1109,7 +1216,7 @@ jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st) {
     P.err = tc_error_word();
     P.ssq_in = a.ssq_in; P.ssq_in_tiles = a.ssq_in_tiles; P.ssq_stride = a.ssq_stride > 0 ? a.ssq_stride : a.T;
     P.inv_d = 1.0f / (float)a.K; P.eps = a.eps; P.ssq_out = a.ssq_out;
-    const int bn = a.T <= 16 ? 16 : a.T <= 32 ? 32 : 64;
+    const int bn = a.T <= 16 ? 16 : a.T <= 32 ? 32 : a.T <= 64 ? 64 : a.T <= 128 ? 128 : 256;
     CUtensorMap mx;
     s = make_tmap_bf16_2d(&mx, a.X, (uint64_t)a.T, (uint64_t)a.K, (uint64_t)(a.x_row_stride > 0 ? a.x_row_stride : a.K), bn, 64);
     if (s != JSM_OK) return s;
@@ -1157,25 +1264,39 @@ jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st) {
             P.tp_mode = 2;
         }
     }
-    // A launch pays for the size of the image it runs.  The common launches of a decoder step have lean images of their own, chosen
+    // A launch pays for the size of the image it runs.  The common launches of up to 64 tokens have lean images of their own, chosen
     // below; what remains runs the general images.
-    if (P.tp_mode == 0) {  // up to 16 tokens, no cluster: an image per kind of tile
-#define PK_IMAGE(PRM_) return launch_packed<16, false, 0, PRM_>(mx, mx2, P, grid, cluster, a.chained, st)
-        if (a.epilogue == LIN_GELU_GLU) PK_IMAGE(9);
-        if (a.epilogue == LIN_CLAMPED_GLU) PK_IMAGE(6);
-        if (!paired && !a.bias && a.epilogue == LIN_NONE && !a.ssq_in && !a.ssq_out) {  // plain projections with nothing fused
-            if (a.out_f32) PK_IMAGE(7);
-            PK_IMAGE(8);
-        }
-        const bool lean = !a.bias && !a.out_f32;  // the projections of a LLaMA-style decoder step
-        if (lean && paired && a.ssq_in) PK_IMAGE(4);
-        if (lean && !paired && a.epilogue == LIN_NONE && a.ssq_in && !a.ssq_out) PK_IMAGE(2);
-        if (lean && !paired && a.epilogue == LIN_RESIDUAL && !a.ssq_in && a.ssq_out) PK_IMAGE(3);
-        if (paired) PK_IMAGE(1);
-        PK_IMAGE(0);
+    const bool with_cl = cluster > 1 || a.T >= 32;
+    if (P.tp_mode == 0) {  // (no cluster forms up to 64 tokens: more tiles than SMs, or fewer than 32 tokens)
+#define PK_IMAGE(BN_, PRM_) return launch_packed<BN_, false, 0, PRM_>(mx, mx2, P, grid, cluster, a.chained, st)
+#define PK_IMAGES(BN_, QKV_, RES_)                                                                                                         \
+    do {                                                                                                                                  \
+        if (a.epilogue == LIN_GELU_GLU) PK_IMAGE(BN_, 9);                                                                                 \
+        if (a.epilogue == LIN_CLAMPED_GLU) PK_IMAGE(BN_, 6);                                                                              \
+        if (!paired && !a.bias && a.epilogue == LIN_NONE && !a.ssq_in && !a.ssq_out) { /* plain projections with nothing fused */         \
+            if (a.out_f32) PK_IMAGE(BN_, 7);                                                                                              \
+            PK_IMAGE(BN_, 8);                                                                                                             \
+        }                                                                                                                                 \
+        const bool lean = !a.bias && !a.out_f32; /* the projections of a LLaMA-style decoder step */                                      \
+        if (lean && paired && a.ssq_in) PK_IMAGE(BN_, 4);                                                                                 \
+        if (lean && !paired && a.epilogue == LIN_NONE && a.ssq_in && !a.ssq_out) PK_IMAGE(BN_, QKV_);                                     \
+        if (lean && !paired && a.epilogue == LIN_RESIDUAL && !a.ssq_in && a.ssq_out) PK_IMAGE(BN_, RES_);                                 \
+        if (paired) PK_IMAGE(BN_, 1);                                                                                                     \
+        PK_IMAGE(BN_, 0);                                                                                                                 \
+    } while (0)
+        if (cluster > 1 && bn <= 64) JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: %d tokens over %d tiles have a kernel of their own", a.T, P.n_tiles);
+        if (bn == 16) PK_IMAGES(16, 2, 3);
+        if (bn == 32) PK_IMAGES(32, 0, 0);  // (more outputs than a model's qkv or width has: no image of their own)
+        if (bn == 64) PK_IMAGES(64, 0, 0);
+#undef PK_IMAGES
+#undef PK_IMAGE
+#define PK_IMAGE(BN_, PRM_) return launch_packed<BN_, true, 0, PRM_>(mx, mx2, P, grid, cluster, a.chained, st)
+        if (bn == 256) PK_IMAGE(256, -1);
+        if (a.epilogue == LIN_GELU_GLU) PK_IMAGE(128, 9);
+        if (a.epilogue == LIN_CLAMPED_GLU) PK_IMAGE(128, 6);
+        PK_IMAGE(128, -1);
 #undef PK_IMAGE
     }
-    const bool with_cl = cluster > 1 || a.T >= 32;
     // 17 to 64 tokens of a tensor-parallel rank (flags): the pushing projection and the two reducing ones
     if (bn > 16 && !P.tp_inband && !a.bias && !a.out_f32) {
 #define PK_LEAN_TP(BN_, CL_)                                                                                                 \
@@ -1260,7 +1381,7 @@ extern "C" size_t jsm_linear_packed_bytes(int N, int K, int paired) {
     return linear_packed_bytes(N, K, paired ? 1 : 0);
 }
 
-// Grows the workspace of the current device so that any launch of this shape (as the kernels were split up to 256 tokens: what a call needs does not depend on the kernel it takes) finds room.
+// Grows the workspace of the current device so that any launch of this shape (up to 256 tokens per launch) finds room.
 // Set-up time only: synchronises the device when it has to reallocate.
 extern "C" jsm_status jsm_linear_packed_reserve(int N, int K, int paired) {
     if (N <= 0 || K <= 0) JSM_FAIL(JSM_INVALID_ARG, "jsm_linear_packed_reserve: N %d, K %d", N, K);
