@@ -260,7 +260,8 @@ __global__ void __launch_bounds__(AR_ROWS * 32) attn_paged_rows_kernel(const T* 
         const int key = c0 + lane;
         const float s = key >= first && key <= pos ? (a0 + a1) * d.scale : -INFINITY;
         const float m_new = fmaxf(m, warp_max(s));
-        if (!(m_new == -INFINITY)) {  // (else no key of this row yet: the whole warp agrees)
+        // (else no key of this row has weight yet: the whole warp agrees; the maximum passes over NaN, which has to reach the sums)
+        if (!(m_new == -INFINITY) || __any_sync(0xffffffffu, s != s)) {
             const float p = expf(s - m_new), alpha = expf(m - m_new);
             l = l * alpha + warp_sum(p);
             m = m_new;
