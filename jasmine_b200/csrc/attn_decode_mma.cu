@@ -295,13 +295,8 @@ __global__ void __launch_bounds__(DM_THREADS) attn_decode_mma_kernel(
 
 template <int G, bool FUSED>
 static jsm_status dm_launch(const CUtensorMap& map, dim3 grid, cudaStream_t st, const DecodeMmaArgs& a) {
-    static bool configured[64] = {false};
-    int dev = 0;
-    JSM_CUDA_CHECK(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64 && !configured[dev]) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(attn_decode_mma_kernel<G, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, DM_SMEM));
-        configured[dev] = true;
-    }
+    static DeviceOnce once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once, attn_decode_mma_kernel<G, FUSED>, DM_SMEM));
     JSM_CUDA_CHECK(launch_chained(attn_decode_mma_kernel<G, FUSED>, grid, dim3(DM_THREADS), (size_t)DM_SMEM, st, map,
                                   (const __nv_bfloat16*)a.q, a.q_stride, (__nv_bfloat16*)a.pool, a.block_table, a.max_pages,
                                   a.context_lens, a.Hq, a.Hkv, a.scale_log2, (const float4*)a.rope, a.n_chunks, a.chunk, a.scratch,

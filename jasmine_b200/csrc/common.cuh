@@ -8,6 +8,7 @@
 #include <stdarg.h>
 #include <atomic>
 #include "../../include/jasmine_b200.h"
+#include "device_once.h"
 
 namespace jsm {
 
@@ -37,6 +38,25 @@ extern std::atomic<uint64_t> g_launches;
         ::jsm::g_launches.fetch_add(1);             \
         JSM_CUDA_CHECK(cudaGetLastError());         \
     } while (0)
+
+// Lets launches of `kernel` on the current device ask for up to `bytes` of dynamic shared memory (0: all that its static arrays leave of 227 KB).
+// `once`: one per kernel.
+template <typename... KArgs>
+inline cudaError_t allow_shared(DeviceOnce& once, void (*kernel)(KArgs...), int bytes) {
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return (cudaError_t)once.run(dev, [&] {
+        int n = bytes;
+        if (n == 0) {
+            cudaFuncAttributes fa;
+            const cudaError_t err = cudaFuncGetAttributes(&fa, kernel);
+            if (err != cudaSuccess) return (int)err;
+            n = 227 * 1024 - (int)fa.sharedSizeBytes;
+        }
+        return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, n);
+    });
+}
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 int sm_count();

@@ -223,11 +223,8 @@ template <bool ORDERED, int TMM, int TNN>
 static jsm_status dot_launch(const MatD& A, const MatD& B, const MatD* bias, int epilogue, const MatD* R, float* C, long long crs, long long ccs, int splits,
                              cudaStream_t st) {
     constexpr int smem = dot_smem(TMM, TNN);
-    static bool attr_done = false;  // per instantiation
-    if (!attr_done) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(dot_f32_kernel<ORDERED, TMM, TNN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        attr_done = true;
-    }
+    static DeviceOnce once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once, dot_f32_kernel<ORDERED, TMM, TNN>, smem));
     const MatD none{nullptr, 1, 1, 0, 0};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((B.cols + 16 * TNN - 1) / (16 * TNN), (A.rows + 8 * TMM - 1) / (8 * TMM), splits);

@@ -940,14 +940,9 @@ template <int VPT, int KIND>
 static cudaError_t launch_staged_pro(int pro, const StagedArgs& S, unsigned grid, size_t smem, cudaStream_t st) {
 #define JSM_RS(PRO_)                                                                                                      \
     {                                                                                                                     \
-        static bool configured[64] = {false};                                                                             \
-        int dev = 0;                                                                                                      \
-        cudaGetDevice(&dev);                                                                                              \
-        if (dev >= 0 && dev < 64 && !configured[dev]) {                                                                   \
-            cudaError_t e = cudaFuncSetAttribute(rows_staged_kernel<VPT, KIND, PRO_>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
-            if (e != cudaSuccess) return e;                                                                               \
-            configured[dev] = true;                                                                                       \
-        }                                                                                                                 \
+        static DeviceOnce once;                                                                                           \
+        const cudaError_t e = allow_shared(once, rows_staged_kernel<VPT, KIND, PRO_>, 200 * 1024);                        \
+        if (e != cudaSuccess) return e;                                                                                   \
         rows_staged_kernel<VPT, KIND, PRO_><<<grid, RS_THREADS, smem, st>>>(S);                                           \
         return cudaGetLastError();                                                                                        \
     }

@@ -463,11 +463,8 @@ static jsm_status flash_go(const CUtensorMap& mq, const CUtensorMap& mk, const C
     constexpr size_t smem = (size_t)(4 * (QKD / 64) + VST * (VD / 64)) * FA_SLAB + 1024;
     static_assert(smem <= 226 * 1024, "query tiles and rings fit the shared memory");
     // a quarter of the exponentials on the FMA pipe: the measured optimum (none: MUFU-bound, half: issue-bound)
-    static bool attr_done = false;
-    if (!attr_done) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(flash_prefill_kernel<1, QKD, VD, VST, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_done = true;
-    }
+    static DeviceOnce once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once, flash_prefill_kernel<1, QKD, VD, VST, MODE>, (int)smem));
     flash_prefill_kernel<1, QKD, VD, VST, MODE><<<grid, FA_THREADS, smem, st>>>(mq, mk, mv, P);
     JSM_LAUNCH_CHECK();
     return JSM_OK;

@@ -664,11 +664,8 @@ size_t latent_part_floats(const LatentDims& d) { return (size_t)sm_count() * LA_
 template <int NT>
 static jsm_status launch_mma(const LatentDims& d, const LatentCache& cache, const StepTokens& tk, const LatentTiles& tl, const LatentScratch& sc,
                              int splits, cudaStream_t st) {
-    static bool attr_done = false;
-    if (!attr_done) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(latent_attn_mma_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        attr_done = true;
-    }
+    static DeviceOnce once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once, latent_attn_mma_kernel<NT>, 226 * 1024));
     JSM_CUDA_CHECK(launch_chained(latent_attn_mma_kernel<NT>, dim3(tl.n_tiles, splits), dim3(256), la_smem(d), st, (const __nv_bfloat16*)sc.q_lat, d,
                                   (const __nv_bfloat16*)cache.pool, cache.block_table, cache.max_pages, tk.seg_start, tk.seg_len, tk.seg_pos0,
                                   tk.seg_row, tl.tile_seg, tl.tile_r0, (__nv_bfloat16*)sc.o_lat, sc.part, splits, la_pitch(d), tc_error_word()));

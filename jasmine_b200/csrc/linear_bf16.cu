@@ -483,11 +483,8 @@ static jsm_status launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const 
     if (stages > 8) stages = 8;
     if (stages < 2) stages = 2;
     const size_t smem = (size_t)stages * STAGE_BYTES + 1024;
-    static bool attr_done = false;  // per instantiation
-    if (!attr_done) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(linear_tc_kernel<BN, GATEUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-        attr_done = true;
-    }
+    static DeviceOnce once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once, linear_tc_kernel<BN, GATEUP>, 220 * 1024));
     dim3 grid((P.N + BM - 1) / BM, (P.T + BN - 1) / BN, splits);
     TcParams Q = P;
     if (Q.w_early) {

@@ -356,9 +356,11 @@ __global__ void __launch_bounds__(LM_THREADS, 1) linear_mid_kernel(const __grid_
 template <int BN, int KIND, bool TRACED>
 static int mid_capacity(int S) {
     static std::mutex mu;
-    static int known[9];
+    static int known[64][9];  // per device
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return S == 1 ? sm_count() : sm_count() / S * 3 / 4;
     std::lock_guard<std::mutex> lock(mu);
-    if (known[S] == 0) {
+    if (known[dev][S] == 0) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(S * 256);
         cfg.blockDim = dim3(LM_THREADS);
@@ -374,9 +376,9 @@ static int mid_capacity(int S) {
             cudaGetLastError();
             n = S == 1 ? sm_count() : sm_count() / S * 3 / 4;
         }
-        known[S] = n;
+        known[dev][S] = n;
     }
-    return known[S];
+    return known[dev][S];
 }
 
 // CTAs per tile and the tile's height.  A CTA takes 0.3 us per unit of 64 k of a whole tile (the rate of one multiprocessor's copies; beyond 64
@@ -402,11 +404,8 @@ static void mid_shape(int n_tiles, int kbt, bool may_halve, int* S_out, int* hal
 template <int BN, int KIND, bool TRACED = false>
 static jsm_status launch_mid(const PackedArgs& a, LmParams& P, int n_tiles, cudaStream_t st) {
     if (!TRACED && (P.trace = linear_trace_next(&P.trace_ctas))) return launch_mid<BN, KIND, true>(a, P, n_tiles, st);
-    static bool attr_done = false;  // per instantiation
-    if (!attr_done) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(linear_mid_kernel<BN, KIND, TRACED>, cudaFuncAttributeMaxDynamicSharedMemorySize, lm_smem(BN)));
-        attr_done = true;
-    }
+    static DeviceOnce once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once, linear_mid_kernel<BN, KIND, TRACED>, lm_smem(BN)));
     int S, half;
     mid_shape<BN, KIND, TRACED>(n_tiles, P.kbt, KIND != 2 && !a.ssq_out, &S, &half);
     P.half = half;

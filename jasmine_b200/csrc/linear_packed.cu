@@ -1079,15 +1079,8 @@ static jsm_status launch_packed(const CUtensorMap& mx, const CUtensorMap& mx2, P
     P.stages = stages;
     P.trace = linear_trace_next(&P.trace_ctas);
     const size_t smem = (size_t)stages * STAGE_BYTES + 1024;
-    static bool attr_done = false;  // per instantiation
-    if (!attr_done) {
-        cudaFuncAttributes fa;
-        JSM_CUDA_CHECK(cudaFuncGetAttributes(&fa, linear_packed_kernel<BN, CL, TPM, PRM>));
-        // 227 KB per CTA in all: what the kernel's static arrays leave is open to the stage ring
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(linear_packed_kernel<BN, CL, TPM, PRM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            227 * 1024 - (int)fa.sharedSizeBytes));
-        attr_done = true;
-    }
+    static DeviceOnce once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once, linear_packed_kernel<BN, CL, TPM, PRM>, 0));  // what the static arrays leave is open to the stage ring
     P.pf_units = 0;
     P.cluster_s = cluster > 1 ? cluster : 0;
     cudaLaunchConfig_t cfg = {};

@@ -987,12 +987,9 @@ size_t rec_chunk_bytes(const RecDims& d) { return (size_t)d.H * rc_block(d.delta
 
 template <int KT, bool DELTA>
 static jsm_status chunk_go(const RecArgs& a, const RecDims& d, const RecChunks& ch, int n_segs, int n_tok, cudaStream_t st) {
-    static bool attr_done = false;
-    if (!attr_done) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(rec_chunk_prep_kernel<DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024));
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(rec_chunk_kernel<KT, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        attr_done = true;
-    }
+    static DeviceOnce once_prep, once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once_prep, rec_chunk_prep_kernel<DELTA>, 80 * 1024));
+    JSM_CUDA_CHECK(allow_shared(once, rec_chunk_kernel<KT, DELTA>, 200 * 1024));
     const int kw = KT * 16;
     JSM_CUDA_CHECK(launch_chained(rec_chunk_prep_kernel<DELTA>, dim3(ch.n_chunks, d.H), dim3(256), (size_t)rc_prep_tiles(kw, DELTA) + (DELTA ? RC_C * 68 * 4 : 0), st, a, d,
                                   ch.chunk_seg, ch.chunk_t0, static_cast<uint8_t*>(ch.ws), kw));
@@ -1034,11 +1031,8 @@ jsm_status rec_scan_launch(bool f32, const RecDims& d, const RecWeights& w, cons
 
 template <typename T, bool IN_SMEM, bool DELTA>
 static jsm_status step_go(const RecArgs& a, const RecDims& d, int lpr, size_t smem, int n_segs, cudaStream_t st) {
-    static bool attr_done = false;
-    if (!attr_done) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(rec_step_kernel<T, IN_SMEM, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_MAX_SMEM));
-        attr_done = true;
-    }
+    static DeviceOnce once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once, rec_step_kernel<T, IN_SMEM, DELTA>, RT_MAX_SMEM));
     JSM_CUDA_CHECK(launch_chained(rec_step_kernel<T, IN_SMEM, DELTA>, dim3(d.H, n_segs), dim3(RT_THREADS), smem, st, a, d, lpr, tc_error_word()));
     JSM_LAUNCH_CHECK();
     return JSM_OK;

@@ -401,11 +401,8 @@ static jsm_status launch_tiled(const PackedArgs& a, LtParams& P, int n_tiles, cu
     // the packed image as rows of 64 elements; it already has the shared-memory order
     s = make_tmap_bf16_2d(&mw, a.Wp, (uint64_t)n_tiles * P.kbt * 128, 64, 64, BN / 2, 64, false);
     if (s != JSM_OK) return s;
-    static bool attr_done = false;  // per instantiation
-    if (!attr_done) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(linear_tiled_kernel<BN, PAIRED, TRACED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_done = true;
-    }
+    static DeviceOnce once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once, linear_tiled_kernel<BN, PAIRED, TRACED>, (int)smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * std::min(P.tiles, sm_count() / 2));
     cfg.blockDim = dim3(LT_THREADS);

@@ -288,11 +288,8 @@ __global__ void __launch_bounds__(AR_ROWS * 32) attn_paged_rows_kernel(const T* 
 template <typename T, int VR>
 static jsm_status rows_go(const AttnDims& d, const AttnWeights& w, const AttnCache& cache, const StepTokens& tk, const AttnTiles& tl, const void* q,
                           const float* gates, void* out, cudaStream_t st) {
-    static bool attr_done = false;
-    if (!attr_done) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(attn_paged_rows_kernel<T, VR>, cudaFuncAttributeMaxDynamicSharedMemorySize, AR_MAX_SMEM));
-        attr_done = true;
-    }
+    static DeviceOnce once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once, attn_paged_rows_kernel<T, VR>, AR_MAX_SMEM));
     JSM_CUDA_CHECK(launch_spread(attn_paged_rows_kernel<T, VR>, dim3(tl.n_tiles, d.G, (tl.rows + AR_ROWS - 1) / AR_ROWS), dim3(AR_ROWS * 32), ar_smem(d), st,
                                   (const T*)q, d, w.sink, (const T*)cache.pool, cache.block_table, cache.max_pages, tk, tl.tile_seg, tl.tile_r0, tl.rows, gates, (T*)out));
     JSM_LAUNCH_CHECK();
@@ -625,11 +622,8 @@ int attn_counters() { return 2 * sm_count(); }
 
 template <int NB, int VT>
 static jsm_status launch_attn_mma(const AttnArgs& a, const AttnDims& d, int n_tiles, cudaStream_t st) {
-    static bool attr_done = false;
-    if (!attr_done) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(attn_paged_mma_kernel<NB, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
-        attr_done = true;
-    }
+    static DeviceOnce once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once, attn_paged_mma_kernel<NB, VT>, 224 * 1024));
     JSM_CUDA_CHECK(launch_chained(attn_paged_mma_kernel<NB, VT>, dim3(n_tiles, d.G, a.splits), dim3(AM_THREADS), am_smem(d, NB), st, a, d));
     JSM_LAUNCH_CHECK();
     return JSM_OK;

@@ -583,11 +583,8 @@ static ScanArgs scan_args(const ScanDims& d, const ScanWeights& w, const ScanSta
 
 template <typename T, int NS>
 static jsm_status scan_go(const ScanArgs& a, cudaStream_t st) {
-    static bool attr_done = false;
-    if (!attr_done) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(scan_kernel<T, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-        attr_done = true;
-    }
+    static DeviceOnce once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once, scan_kernel<T, NS>, 220 * 1024));
     JSM_CUDA_CHECK(launch_spread(scan_kernel<T, NS>, dim3((a.ip + SC_CH - 1) / SC_CH, a.n_segs), dim3(SC_THREADS), scan_smem<T>(a.np, NS), st, a));
     JSM_LAUNCH_CHECK();
     return JSM_OK;
@@ -595,11 +592,8 @@ static jsm_status scan_go(const ScanArgs& a, cudaStream_t st) {
 template <typename T, int NP>
 static jsm_status step_go(const ScanArgs& a, cudaStream_t st) {
     const size_t smem = (size_t)ST_BB * (2 * a.np + (sizeof(T) == 2 ? 0 : a.rp)) * sizeof(float);
-    static bool attr_done = false;
-    if (!attr_done) {
-        JSM_CUDA_CHECK(cudaFuncSetAttribute(scan_step_kernel<T, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        attr_done = true;
-    }
+    static DeviceOnce once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once, scan_step_kernel<T, NP>, 200 * 1024));
     JSM_CUDA_CHECK(launch_chained(scan_step_kernel<T, NP>, dim3((a.ip + ST_CH - 1) / ST_CH, (a.n_segs + ST_BB - 1) / ST_BB), dim3(ST_THREADS), smem, st, a));
     JSM_LAUNCH_CHECK();
     return JSM_OK;
