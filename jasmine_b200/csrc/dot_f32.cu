@@ -27,45 +27,67 @@ constexpr int dot_stages(int tnn) { return tnn == 1 ? 8 : 4; }
 constexpr int dot_smem(int tmm, int tnn) { return dot_stages(tnn) * (8 * tmm + 16 * tnn) * DOT_PITCH * 4; }
 
 // One thread's part in staging 32 products' worth of ROWS rows of an operand (row stride rs, stride ks along the products), zeros where
-// there is nothing.  vec: contiguous products, 16-byte aligned rows; a thread has the same four products of every 16th row, so
-// its addresses and bounds are worked out once.
+// there is nothing.  Its first address and its bounds are worked out once; a warp walks
+//   VEC  contiguous products in 16-byte aligned rows: four products of every 16th row per thread
+//   ROW  contiguous rows (a transposed operand): eight rows by four products at a time, whole sectors of memory and all banks
+//   ANY  other strides, or contiguous products off alignment: 32 products of every fourth row
+// (With addresses worked out per element of four bytes a transposed operand cost as many instructions as a sixth of the products.  In the
+// reference's order, us, both operands transposed / the second / none: 1024 x 4096 x 128 87 / 83 / 73, here 79 / 75 / 73; 512 x 512 x 512
+// 46 / 35 / 26, here 33 / 30 / 26.)
+enum DotWalk { DOT_VEC, DOT_ROW, DOT_ANY };
 template <int ROWS>
 struct DotLoader {
-    static constexpr int STEP = DOT_THREADS / (DOT_KB / 4), N = ROWS / STEP;  // rows per pass, passes
-    static_assert(ROWS % STEP == 0, "whole passes");
-    const float *base, *p;  // the operand; vec: first piece of the thread
+    static constexpr int WARPS = DOT_THREADS / 32, STEP = DOT_THREADS / (DOT_KB / 4), OCTETS = ROWS / 8;
+    static_assert(ROWS % STEP == 0 && (OCTETS == 2 || OCTETS == 2 * WARPS), "whole passes");
+    const float *base, *p;  // the operand; first element of the thread
     long long rs, ks;
-    int row0, rows, K, c;
-    bool vec;
-    uint32_t dst;     // offset of the thread's first piece in a stage
-    __device__ __forceinline__ DotLoader(const float* base, int row0, int rows, long long rs, long long ks, int K, bool vec)
-        : base(base), p(base), rs(rs), ks(ks), row0(row0), rows(rows), K(K), vec(vec) {
-        const int r = threadIdx.x / (DOT_KB / 4);
-        c = threadIdx.x % (DOT_KB / 4) * 4;
-        dst = (r * DOT_PITCH + c) * 4;
-        if (vec) {
-            p = base + (long long)(row0 + r) * rs + c;
-            this->rows = rows - row0 - r;  // pass i has a row if i STEP < rows
-        }
+    int rows, left, walk;   // rows from the thread's first on, products of the operand from its first on
+    uint32_t dst;           // offset of the thread's first element in a stage
+    __device__ __forceinline__ DotLoader(const float* base, int row0, int rows, long long rs, long long ks, int K, int walk)
+        : base(base), rs(rs), ks(ks), walk(walk) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        int r, x;
+        if (walk == DOT_VEC) { r = threadIdx.x / (DOT_KB / 4); x = threadIdx.x % (DOT_KB / 4) * 4; }
+        else if (walk == DOT_ROW) { r = warp % OCTETS * 8 + lane % 8; x = warp / OCTETS * 4 + lane / 8; }
+        else { r = warp; x = lane; }
+        p = base + (row0 + r) * rs + x * ks;
+        this->rows = rows - row0 - r;
+        left = K - x;
+        dst = (r * DOT_PITCH + x) * 4;
     }
     __device__ __forceinline__ void operator()(uint32_t stage, int k0) const {
-        if (vec) {
-            const int left = min(max(K - k0 - c, 0), 4) * 4;
+        const int n = left - k0;  // products left
+        const uint32_t to = stage + dst;
+        if (walk == DOT_VEC) {
+            const int bytes_row = min(max(n, 0), 4) * 4;
             const float* src = p + k0;
 #pragma unroll
-            for (int i = 0; i < N; ++i) {
-                const int bytes = i * STEP < rows ? left : 0;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(stage + dst + i * STEP * DOT_PITCH * 4),
+            for (int i = 0; i < ROWS / STEP; ++i) {
+                const int bytes = i * STEP < rows ? bytes_row : 0;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + i * STEP * DOT_PITCH * 4),
                              "l"(reinterpret_cast<uint64_t>(bytes ? src : base)), "r"(bytes)
                              : "memory");
                 src += STEP * rs;
             }
+        } else if (walk == DOT_ROW) {
+            const float* src = p + k0 * ks;
+            constexpr int RUN = OCTETS > WARPS ? OCTETS / WARPS : 1, KSTEP = OCTETS > WARPS ? 4 : WARPS / OCTETS * 4;  // octets of rows per step of KSTEP products
+#pragma unroll
+            for (int x = 0; x < DOT_KB; x += KSTEP) {
+#pragma unroll
+                for (int i = 0; i < RUN; ++i) {
+                    const bool on = x < n && i * WARPS * 8 < rows;
+                    cp_async4(to + (i * WARPS * 8 * DOT_PITCH + x) * 4, on ? src + i * WARPS * 8 : base, on);
+                }
+                src += KSTEP * ks;
+            }
         } else {
-            const bool along_k = rs != 1;  // the threads walk the contiguous direction
-            for (int e = threadIdx.x; e < ROWS * DOT_KB; e += DOT_THREADS) {
-                const int r = along_k ? e / DOT_KB : e % ROWS, x = along_k ? e % DOT_KB : e / ROWS;
-                const bool on = row0 + r < rows && k0 + x < K;
-                cp_async4(stage + (r * DOT_PITCH + x) * 4, on ? base + (row0 + r) * rs + (k0 + x) * ks : base, on);
+            const float* src = p + k0 * ks;
+#pragma unroll 4
+            for (int i = 0; i < ROWS / WARPS; ++i) {
+                const bool on = n > 0 && i * WARPS < rows;
+                cp_async4(to + i * WARPS * DOT_PITCH * 4, on ? src : base, on);
+                src += WARPS * rs;
             }
         }
     }
@@ -80,7 +102,7 @@ struct DotLoader {
 // once per block; a cluster of CTAs shares the products of a tile (whole blocks each) and adds its totals in rank order.
 template <bool ORDERED, int TMM, int TNN>
 __global__ void __launch_bounds__(DOT_THREADS, TMM == 8 ? 3 : 4) dot_f32_kernel(MatD A, MatD B, MatD bias, int has_bias, int epilogue, MatD R,
-                                                              float* Cp, long long crs, long long ccs, int M, int N, int K, int vec_a, int vec_b) {
+                                                              float* Cp, long long crs, long long ccs, int M, int N, int K, int walk_a, int walk_b) {
     constexpr int BM = 8 * TMM, BN = 16 * TNN, STAGES = dot_stages(TNN), STAGE = (BM + BN) * DOT_PITCH;
     static_assert(STAGES * STAGE >= BM * BN, "the totals of a tile are exchanged through the ring");
     extern __shared__ __align__(16) float dot_ring[];
@@ -90,8 +112,8 @@ __global__ void __launch_bounds__(DOT_THREADS, TMM == 8 ? 3 : 4) dot_f32_kernel(
     const int splits = ORDERED ? 1 : gridDim.z, rank = ORDERED ? 0 : blockIdx.z;
     const int blocks = (K + DOT_KB - 1) / DOT_KB, b0 = (int)((long long)blocks * rank / splits), mine = (int)((long long)blocks * (rank + 1) / splits) - b0;
     const uint32_t ring = smem_u32(dot_ring);
-    const DotLoader<BM> load_a(A.p, m0, M, A.rs, A.cs, K, vec_a);
-    const DotLoader<BN> load_b(B.p, n0, N, B.cs, B.rs, K, vec_b);
+    const DotLoader<BM> load_a(A.p, m0, M, A.rs, A.cs, K, walk_a);
+    const DotLoader<BN> load_b(B.p, n0, N, B.cs, B.rs, K, walk_b);
     auto stage_a = [&](int i) { load_a(ring + (i % STAGES) * STAGE * 4, (b0 + i) * DOT_KB); };
     auto stage_b = [&](int i) { load_b(ring + ((i % STAGES) * STAGE + BM * DOT_PITCH) * 4, (b0 + i) * DOT_KB); };
     if (!ORDERED) chain_trigger();
@@ -216,8 +238,9 @@ static MatD to_d(const jsm_mat& m) {
     return d;
 }
 
-// contiguous products in 16-byte aligned rows
-static int dot_vec(const float* p, long long rs, long long ks) { return ks == 1 && rs % 4 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+static int dot_walk(const float* p, long long rs, long long ks) {
+    return ks == 1 && rs % 4 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0 ? DOT_VEC : rs == 1 ? DOT_ROW : DOT_ANY;
+}
 
 template <bool ORDERED, int TMM, int TNN>
 static jsm_status dot_launch(const MatD& A, const MatD& B, const MatD* bias, int epilogue, const MatD* R, float* C, long long crs, long long ccs, int splits,
@@ -238,7 +261,7 @@ static jsm_status dot_launch(const MatD& A, const MatD& B, const MatD* bias, int
     cfg.attrs = attr;
     cfg.numAttrs = splits > 1 ? 1 : 0;
     JSM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, dot_f32_kernel<ORDERED, TMM, TNN>, A, B, bias ? *bias : none, bias ? 1 : 0, epilogue, R ? *R : none, C, crs, ccs, A.rows,
-                                      B.cols, A.cols, dot_vec(A.p, A.rs, A.cs), dot_vec(B.p, B.cs, B.rs)));
+                                      B.cols, A.cols, dot_walk(A.p, A.rs, A.cs), dot_walk(B.p, B.cs, B.rs)));
     g_launches.fetch_add(1);
     return JSM_OK;
 }
