@@ -282,6 +282,19 @@ jsm_status dot_f32_launch(const jsm_mat& A, const jsm_mat& B, const jsm_mat& Cm,
                : dot_launch<false, 8, 4>(to_d(A), to_d(B), nullptr, 0, nullptr, C, Cm.row_stride, Cm.col_stride, splits, st);
 }
 
+// whether the spans of memory of two matrices meet
+static bool dot_overlap(const jsm_mat& a, const jsm_mat& b) {
+    auto span = [](const jsm_mat& m, uintptr_t& lo, uintptr_t& hi) {
+        const long long r = (m.rows - 1) * (long long)m.row_stride * 4, c = (m.cols - 1) * (long long)m.col_stride * 4;
+        lo = reinterpret_cast<uintptr_t>(m.data) + (r < 0 ? r : 0) + (c < 0 ? c : 0);
+        hi = reinterpret_cast<uintptr_t>(m.data) + (r > 0 ? r : 0) + (c > 0 ? c : 0) + 4;
+    };
+    uintptr_t a0, a1, b0, b1;
+    span(a, a0, a1);
+    span(b, b0, b1);
+    return a0 < b1 && b0 < a1;
+}
+
 }  // namespace jsm
 
 using namespace jsm;
@@ -305,8 +318,10 @@ extern "C" jsm_status jsm_dot_f32(jsm_mat A, jsm_mat B, const jsm_mat* bias, int
     if (R) rd = to_d(*R);
     const MatD *pb = bias ? &bd : nullptr, *pr = R ? &rd : nullptr;
     float* C = reinterpret_cast<float*>(Cm.data);
-    // 64 x 64 tiles once they occupy half of the multiprocessors, 16 x 16 tiles (one output pair per thread) below
-    if ((long long)((Cm.cols + 63) / 64) * ((Cm.rows + 63) / 64) * 2 > sm_count())
+    // 64 x 64 tiles once they occupy half of the multiprocessors, 16 x 16 tiles (one output pair per thread) below.  A product of one 64 x 64
+    // tile may lie in an operand's memory (x <- x W): its one CTA has read everything before it writes, several would not.
+    const long long tiles = (long long)((Cm.cols + 63) / 64) * ((Cm.rows + 63) / 64);
+    if (tiles * 2 > sm_count() || (tiles == 1 && (dot_overlap(Cm, A) || dot_overlap(Cm, B))))
         return dot_launch<true, 8, 4>(to_d(A), to_d(B), pb, epilogue, pr, C, Cm.row_stride, Cm.col_stride, 1, as_stream(stream));
     return dot_launch<true, 2, 1>(to_d(A), to_d(B), pb, epilogue, pr, C, Cm.row_stride, Cm.col_stride, 1, as_stream(stream));
 }

@@ -33,3 +33,16 @@ def test_same_bits_in_every_layout(M, N, K):
             out = torch.full((M + 1, N), 7.0, device="cuda")
             jb.dot_f32(laid_out(A, la), laid_out(B, lb), out[:M])
             assert torch.equal(out[:M], want) and bool((out[M] == 7.0).all()), (la, lb)
+
+
+@pytest.mark.parametrize("n,K", [(64, 64), (50, 50), (17, 17), (16, 16)])
+@pytest.mark.parametrize("into", ["left", "right", "transposed"])
+def test_products_of_one_tile_in_place_of_an_operand(n, K, into):
+    """x <- x W of up to 64 x 64: everything is read before the first write."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    for _ in range(5):
+        A, B = torch.randn(n, K, generator=g, device="cuda"), torch.randn(K, n, generator=g, device="cuda")
+        want = jb.dot_f32(A, B, torch.empty(n, n, device="cuda"))
+        out = {"left": A, "right": B, "transposed": B.t()}[into]
+        jb.dot_f32(A, B, out)
+        assert torch.equal(out, want)
