@@ -163,9 +163,12 @@ __global__ void __launch_bounds__(256) embed_residual_kernel(const T* __restrict
 // One CTA per token; the sublayer's output y stays in registers between the statistics and the update (MAXV > 0: wp <=
 // 2048 * MAXV), or is read twice (MAXV 0).  Padding columns of y and of the gain are zero.
 // SUM false: x <- x + norm(y); true: x <- norm(alpha x + y)
-template <int MAXV, bool SUM>
+// EARLY: the gain arrives while the predecessor ends, not in a round trip of its own behind the sum.  Only where no kernel of the stream
+// writes it, and only up to a token per SM: with more tokens than that other CTAs hide the trip, and the registers that keep the gain cost more
+// (back to back, us, late / early: 512 x 4096 5.3 / 5.8, sums 2048 x 4096 15.1 / 16.5).
+template <int MAXV, bool SUM, bool EARLY>
 __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restrict__ y, float* __restrict__ x, const float* __restrict__ gain,
-                                                            float eps, float alpha, __nv_bfloat16* __restrict__ xa, int d, int wp, int fixed_gain) {
+                                                            float eps, float alpha, __nv_bfloat16* __restrict__ xa, int d, int wp) {
     __shared__ float smem[8];
     chain_trigger();
     const long long base = (long long)blockIdx.x * wp;
@@ -173,10 +176,8 @@ __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restr
         const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     };
-    // a gain that no kernel of the stream writes arrives while the predecessor ends, not in a round trip of its own behind the sum
-    if (!fixed_gain) chain_wait();
-    float gv[MAXV ? MAXV : 1][8];
-    if constexpr (MAXV > 0)
+    float gv[EARLY ? MAXV : 1][8];
+    if constexpr (EARLY)
 #pragma unroll
         for (int i = 0; i < MAXV; ++i)
             if ((i * 256 + (int)threadIdx.x) * 8 < wp) load8(gain + (i * 256 + threadIdx.x) * 8, gv[i]);
@@ -212,7 +213,8 @@ __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restr
     }
     q = block_sum(q, smem) / (float)d;
     const float rms = sqrtf(q + eps);
-    auto update = [&](int c, const float (&v)[8], float (&r)[8], const float (&g)[8]) {
+    auto update = [&](int c, const float (&v)[8], float (&r)[8], float (&g)[8]) {
+        if constexpr (!EARLY) load8(gain + c, g);
 #pragma unroll
         for (int e = 0; e < 8; ++e) r[e] = SUM ? v[e] / rms * g[e] : r[e] + v[e] / rms * g[e];
         reinterpret_cast<float4*>(x + base + c)[0] = make_float4(r[0], r[1], r[2], r[3]);
@@ -223,7 +225,7 @@ __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restr
 #pragma unroll
         for (int i = 0; i < MAXV; ++i) {
             const int c = (i * 256 + threadIdx.x) * 8;
-            if (c < wp) update(c, keep[i], res[i], gv[i]);
+            if (c < wp) update(c, keep[i], res[i], gv[EARLY ? i : 0]);
         }
     } else {
         for (int c = threadIdx.x * 8; c < wp; c += 2048) {
@@ -233,7 +235,6 @@ __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restr
             if (SUM)
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[e] = fmaf(alpha, r[e], v[e]);
-            load8(gain + c, gv[0]);
             update(c, v, r, gv[0]);
         }
     }
@@ -332,8 +333,11 @@ jsm_status embed_residual_launch(bool f32, const void* table, const int32_t* ids
 template <bool SUM>
 static jsm_status norm_residual(const float* y, float* x, const float* gain, float eps, float alpha, void* xa, int T, int d, int wp, cudaStream_t st,
                                 bool fixed_gain) {
-    auto go = [&](auto kernel) { return launch_chained(kernel, dim3(T), dim3(256), 0, st, y, x, gain, eps, alpha, (__nv_bfloat16*)xa, d, wp, fixed_gain ? 1 : 0); };
-    JSM_CUDA_CHECK(wp <= 2048 ? go(post_norm_add_kernel<1, SUM>) : wp <= 4096 ? go(post_norm_add_kernel<2, SUM>) : go(post_norm_add_kernel<0, SUM>));
+    auto go = [&](auto kernel) { return launch_chained(kernel, dim3(T), dim3(256), 0, st, y, x, gain, eps, alpha, (__nv_bfloat16*)xa, d, wp); };
+    const bool early = fixed_gain && T <= sm_count();
+    JSM_CUDA_CHECK(wp > 4096 ? go(post_norm_add_kernel<0, SUM, false>)
+                   : early   ? wp <= 2048 ? go(post_norm_add_kernel<1, SUM, true>) : go(post_norm_add_kernel<2, SUM, true>)
+                   : wp <= 2048 ? go(post_norm_add_kernel<1, SUM, false>) : go(post_norm_add_kernel<2, SUM, false>));
     JSM_LAUNCH_CHECK();
     return JSM_OK;
 }
