@@ -255,6 +255,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1)
         const int c4 = (lane & 7) * 4, r4 = lane >> 3;  // the place a lane reads back: 4 columns of every fourth row
         chain_wait();
         int it = 0;
+        bool ok = true;  // a warp that gave up a wait walks on without work: it still meets the others at the barriers of the row statistics
         for (int tile = cluster; tile < P.tiles; tile += n_clusters, ++it) {
             const int ft = tile / P.tok_blocks, tb = tile - ft * P.tok_blocks;
             const int t0 = tb * LT_BM + (int)rank * 128 + quad * 32;  // first token of this warp
@@ -266,11 +267,11 @@ __global__ void __launch_bounds__(LT_THREADS, 1)
                     for (int j = 0; j < P.ssq_in_tiles; ++j) q += __ldcg(P.ssq_in + (size_t)j * P.ssq_stride + t0 + lane);
                 scale = rsqrtf(q * P.inv_d + P.eps);
             }
-            if (!mbar_wait(&acc_full[buf], (it >> 1) & 1, &abort_flag, P.err, TC_TIMEOUT_ACC)) break;
+            ok = ok && mbar_wait(&acc_full[buf], (it >> 1) & 1, &abort_flag, P.err, TC_TIMEOUT_ACC);
             tc_fence_after();
             const uint32_t acc = lane_addr + (uint32_t)(buf * BN);
             constexpr int CHUNKS = PAIRED ? BN / 64 : BN / 32, MINE = CHUNKS > 1 ? CHUNKS / 2 : 1;
-            const int c_end = CHUNKS > 1 || half == 0 ? (half + 1) * MINE : 0;
+            const int c_end = ok && (CHUNKS > 1 || half == 0) ? (half + 1) * MINE : 0;
             float ssq[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) ssq[k] = 0.0f;
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1)
                 }
                 __syncwarp();  // the staging tile is free again
             }
-            if (CHUNKS == 1 && half == 1) {  // (nothing of this tile to read)
+            if (ok && CHUNKS == 1 && half == 1) {  // (nothing of this tile to read)
                 __syncwarp();
                 if (lane == 0) lt_arrive_leader(empty_leader[buf]);
             }
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1)
                     asm volatile("bar.sync 1, %0;" ::"n"(32 * LT_EPI) : "memory");  // (the next tile writes it again)
                 }
                 const int tile128 = BN == 256 ? 2 * ft + half : ft;
-                if ((BN == 256 || half == 0) && (lane & 7) == 0 && tile128 * 128 < P.N)
+                if (ok && (BN == 256 || half == 0) && (lane & 7) == 0 && tile128 * 128 < P.N)
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
                         if (t0 + 4 * k + r4 < P.T) P.ssq_out[(size_t)tile128 * P.ssq_stride + t0 + 4 * k + r4] = ssq[k];
