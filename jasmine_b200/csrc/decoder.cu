@@ -1050,9 +1050,6 @@ jsm_status jsm_decoder_finalize(jsm_decoder* m) {
     DEC_TRY(dalloc(m, &m->keys, 8 * (size_t)m->cap_rows));
     DEC_TRY(dalloc(m, &m->key_ctrs, 4 * (size_t)m->cap_rows));
     DEC_TRY(dalloc(m, &m->next_dev, 4 * (size_t)m->cap_rows));
-    // (partials of a split row-major projection: at most one 128 x 128 tile per SM)
-    m->ws_floats = std::max(m->ws_floats, (size_t)sm_count() * 128 * 128);
-    m->n_counters = std::max(m->n_counters, sm_count());
     DEC_TRY(dalloc(m, &m->ws, 4 * m->ws_floats));
     DEC_TRY(dalloc(m, &m->counters, 4 * (size_t)m->n_counters));
     std::map<std::pair<int, int>, int> tilings;
