@@ -1154,7 +1154,10 @@ static int packed_paired(const PackedArgs& a) {
 // 4096 x 4096 9.1 / 8.2, 4096 x 11008 17.4 / 16.3) and where most SMs have a tile of their own, so that nothing is folded (9600 x 4096 15.5 / 15.0,
 // 12288 x 4096 18.5 / 17.5, at 4 tokens 16384 x 4096 22.3 / 21.6); in between the even split (8192 x 2048 9.0 / 9.1).
 // Up to 64, clusters up to a tile per SM; beyond, at 17 and 64 tokens: gate/up 11008 x 4096 33 / 41 and 39 / 46, 24000 x 2048 20 / 29 and 24 / 34,
-// 32000 x 4096 43 / 44 and 48 / 50.  Three or four blocks of depth and 16 tiles or more have nothing to split: 8192 x 256 at 17 3.4 / 4.1,
+// 32000 x 4096 43 / 44 and 48 / 50.  Deep matrices whose tiles cover the SMs in either kernel (qkv, wo and down of the 7B shape) take the same time
+// alone (4096 x 4096 at 64 10.8 / 9.9, 12288 x 4096 22.7 / 22.3), but a CTA of the clusters leaves 18 KB of an SM's shared memory to its neighbours in
+// the stream, and the attention between them lost more: eight layers of that shape at context 560, 64, 32 and 17 sequences, us a
+// step, 1560 / 1685, 1134 / 1207, 969 / 986; attention 92 / 119 a layer.  Three or four blocks of depth and 16 tiles or more have nothing to split: 8192 x 256 at 17 3.4 / 4.1,
 // gate/up 2048 x 256 at 8 3.1 / 4.2 (at 32 6.2 / 4.6).
 // Up to 128, of matrices less than 4096 deep: clusters up to a tile per SM (1024 x 2752 at 65 - / 9.2 / 11.2; gate/up pairs keep the tiled kernel:
 // 3072 x 1024 at 128 - / 9.0 / 8.2), else tiled (22016 x 2048 at 65 34 / 33 / 26).  Deeper: the tokens' bytes pass through every CTA of a
@@ -1170,7 +1173,10 @@ static PackedRoute packed_route(const PackedArgs& a) {
     pk_dims(a.N, K, paired, &nt, &kbt);
     if (K > 128 && K <= 256 && nt >= 16 && nt <= sms && T <= (paired ? 16 : 24)) return ROUTE_STREAM;
     if (T <= 16) return nt * 4 <= sms || (nt * 10 >= sms * 6 && nt <= sms) ? ROUTE_CLUSTERS : ROUTE_STREAM;
-    if (T <= 64) return nt > sms && (K >= 512 || !paired) ? ROUTE_STREAM : ROUTE_CLUSTERS;
+    if (T <= 64) {
+        const bool covers = (nt * 4 <= sms && nt * 5 >= sms) || nt * 10 >= sms * 6;  // clusters of four, or a tile each, on most SMs
+        return (nt > sms && (K >= 512 || !paired)) || (K >= 4096 && nt <= sms && covers) ? ROUTE_STREAM : ROUTE_CLUSTERS;
+    }
     if (T <= 128) {
         if (K < 4096) return nt <= sms && !paired && K >= 512 ? ROUTE_CLUSTERS : ROUTE_TILED;
         if ((K >= 8192 && (nt * 10 >= sms * 6 || (T <= 80 && nt * 10 >= sms * 3))) || nt >= 2 * sms) return ROUTE_STREAM;
@@ -1260,9 +1266,9 @@ jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st) {
     // A launch pays for the size of the image it runs.  The common launches of up to 64 tokens have lean images of their own, chosen
     // below; what remains runs the general images.
     const bool with_cl = cluster > 1 || a.T >= 32;
-    if (P.tp_mode == 0) {  // (no cluster forms up to 64 tokens: more tiles than SMs, or fewer than 32 tokens)
-#define PK_IMAGE(BN_, PRM_) return launch_packed<BN_, false, 0, PRM_>(mx, mx2, P, grid, cluster, a.chained, st)
-#define PK_IMAGES(BN_, QKV_, RES_)                                                                                                         \
+    if (P.tp_mode == 0) {
+#define PK_IMAGE(BN_, PRM_) return launch_packed<BN_, PK_CL, 0, PRM_>(mx, mx2, P, grid, cluster, a.chained, st)
+#define PK_IMAGES(BN_)                                                                                                                     \
     do {                                                                                                                                  \
         if (a.epilogue == LIN_GELU_GLU) PK_IMAGE(BN_, 9);                                                                                 \
         if (a.epilogue == LIN_CLAMPED_GLU) PK_IMAGE(BN_, 6);                                                                              \
@@ -1272,15 +1278,20 @@ jsm_status linear_packed_launch(const PackedArgs& a, cudaStream_t st) {
         }                                                                                                                                 \
         const bool lean = !a.bias && !a.out_f32; /* the projections of a LLaMA-style decoder step */                                      \
         if (lean && paired && a.ssq_in) PK_IMAGE(BN_, 4);                                                                                 \
-        if (lean && !paired && a.epilogue == LIN_NONE && a.ssq_in && !a.ssq_out) PK_IMAGE(BN_, QKV_);                                     \
-        if (lean && !paired && a.epilogue == LIN_RESIDUAL && !a.ssq_in && a.ssq_out) PK_IMAGE(BN_, RES_);                                 \
+        if (lean && !paired && a.epilogue == LIN_NONE && a.ssq_in && !a.ssq_out) PK_IMAGE(BN_, 2);                                        \
+        if (lean && !paired && a.epilogue == LIN_RESIDUAL && !a.ssq_in && a.ssq_out) PK_IMAGE(BN_, 3);                                    \
         if (paired) PK_IMAGE(BN_, 1);                                                                                                     \
         PK_IMAGE(BN_, 0);                                                                                                                 \
     } while (0)
-        if (cluster > 1 && bn <= 64) JSM_FAIL(JSM_UNSUPPORTED, "linear_packed: %d tokens over %d tiles have a kernel of their own", a.T, P.n_tiles);
-        if (bn == 16) PK_IMAGES(16, 2, 3);
-        if (bn == 32) PK_IMAGES(32, 0, 0);  // (more outputs than a model's qkv or width has: no image of their own)
-        if (bn == 64) PK_IMAGES(64, 0, 0);
+#define PK_CL false
+        if (bn == 16) PK_IMAGES(16);
+        if (bn == 32 && cluster <= 1) PK_IMAGES(32);
+        if (bn == 64 && cluster <= 1) PK_IMAGES(64);
+#undef PK_CL
+#define PK_CL true
+        if (bn == 32) PK_IMAGES(32);
+        if (bn == 64) PK_IMAGES(64);
+#undef PK_CL
 #undef PK_IMAGES
 #undef PK_IMAGE
 #define PK_IMAGE(BN_, PRM_) return launch_packed<BN_, true, 0, PRM_>(mx, mx2, P, grid, cluster, a.chained, st)

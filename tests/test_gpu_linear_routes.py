@@ -1,5 +1,5 @@
 """Projections that stay with the streaming kernel beyond 16 tokens: more packed tiles of 128 rows than the chip has multiprocessors (17 to 64
-tokens), deep or wide matrices up to 128 tokens, very deep ones of a few tiles up to 256, and shallow ones of few blocks of depth."""
+tokens), deep ones whose tiles cover them, deep or wide matrices up to 128 tokens, very deep ones of a few tiles up to 256, and shallow ones of few blocks of depth."""
 import pytest
 import torch
 
@@ -12,9 +12,9 @@ from test_gpu_trace import traced
 pytestmark = pytest.mark.gpu
 
 # both edges of the token blocks of 32 / 64 / 128 / 256, ragged last tiles and blocks of depth
-SHAPES = [(17, 19204, 520), (32, 19076, 1032), (33, 20000, 520), (64, 18948, 1096), (24, 8192, 256), (16, 4100, 200), (65, 9604, 4104), (96, 9600, 4096),
+SHAPES = [(17, 4096, 4096), (32, 4100, 4104), (33, 4096, 4352), (64, 4700, 4104), (31, 11400, 4096), (64, 12288, 4104), (17, 19204, 520), (32, 19076, 1032), (33, 20000, 520), (64, 18948, 1096), (24, 8192, 256), (16, 4100, 200), (65, 9604, 4104), (96, 9600, 4096),
           (80, 19204, 4104), (128, 37892, 4104), (128, 11400, 8200), (80, 5892, 8200), (129, 292, 8200), (256, 1000, 8264)]
-PAIRS = [(17, 9604, 520), (32, 9540, 1032), (33, 10000, 520), (64, 9476, 1096), (16, 1028, 200), (65, 4804, 4104), (80, 9604, 4104), (128, 18948, 4104),
+PAIRS = [(17, 2048, 4096), (32, 2052, 4104), (64, 2300, 4160), (48, 6000, 4096), (17, 9604, 520), (32, 9540, 1032), (33, 10000, 520), (64, 9476, 1096), (16, 1028, 200), (65, 4804, 4104), (80, 9604, 4104), (128, 18948, 4104),
          (160, 292, 8200)]
 
 
@@ -43,10 +43,10 @@ def test_more_tiles_than_multiprocessors_are_split_evenly(T):
     assert int((rec[:, 6] > 0).sum()) > sms // 2  # most CTAs end a second piece of the stream
 
 
-@pytest.mark.parametrize("d,kv,ffn,batch", [(1024, 8, 9600, 17), (1024, 2, 9608, 64), (512, 4, 9608, 32), (2048, 4, 11008, 33)])
+@pytest.mark.parametrize("d,kv,ffn,batch", [(1024, 8, 9600, 17), (1024, 2, 9608, 64), (512, 4, 9608, 32), (2048, 4, 11008, 33), (4096, 32, 1024, 17), (4096, 32, 1024, 40), (4096, 4, 4608, 64)])
 def test_batched_steps_of_wide_projections(d, kv, ffn, batch):
-    """A step with the fused norm in front of a gate/up projection and a vocabulary of more tiles than SMs."""
-    vocab = 19100
+    """A step with the fused norm in front of a gate/up projection and a vocabulary of more tiles than SMs, or with the projections of the 7B width."""
+    vocab = 19100 if d < 4096 else 1000
     m = Llama(1, d, d // 128, kv, ffn, vocab, max_batch=batch, max_context=64, seed=11)
     ref = Reference(m, 1, d, d // 128, kv, ffn, vocab)
     g = torch.Generator(device="cuda").manual_seed(batch)
