@@ -1,8 +1,8 @@
 // fp32 contraction with the summation order of the reference's mat_dot_t
 // (mat_express_t.hpp:730-736): each output element is s = 0; s += a(i,k) * b(k,j)
 // for k ascending, multiply and add rounded separately.  Used for the
-// reference-exact fp32 paths (small models, parity tests); the bf16 projections of
-// the large model go through the tcgen05 kernel instead.
+// reference-exact fp32 paths (small models, parity tests) and, in another order, for few
+// tokens of f32 models; their other products run on the tensor cores (dot_split.cu).
 #include "common.cuh"
 #include "mma_utils.cuh"
 #include "tc_utils.cuh"
@@ -266,20 +266,29 @@ static jsm_status dot_launch(const MatD& A, const MatD& B, const MatD* bias, int
     return JSM_OK;
 }
 
-// C = A . B in fp32 without the reference's order (operands as in jsm_dot_f32, checked by the caller).  Few rows take 16 x 64 tiles.  The products of a tile are shared by as many CTAs as even out the
-// multiprocessors' loads: rounds of CTAs times blocks of products each, and about four blocks' time for a CTA's start and end.
+bool dot_split_usable(const void* X, long long ldx, const void* W, long long ldw, const void* C, long long ldc, int N, int K);
+jsm_status dot_split_launch(const float* X, long long ldx, const float* W, long long ldw, float* C, long long ldc, int T, int N, int K, cudaStream_t st);
+
+// C = A . B in fp32 without the reference's order (operands as in jsm_dot_f32, checked by the caller).  Rows of aligned fours go to the tensor cores
+// (dot_split.cu) from 33 rows of A on, and below that from a million weights on: with fewer their start and end cost more than the products
+// (8 rows, here / there, us: 512 x 512 4.0 / 4.5, 256 x 1024 5.1 / 5.5, 1024 x 1024 7.0 / 6.7, 4096 x 512 9.0 / 7.6, 2752 x 1024 13.5 / 8.9; 32 rows:
+// 512 x 512 4.9 / 5.0, 2752 x 1024 21.5 / 9.5; 33 rows, in the 64 x 64 tiles that this kernel had for them: 64 x 64 7.7 / 3.6, 512 x 512 6.5 / 5.1).
+// The others take 16 x 64 tiles, whose products are shared by as many CTAs as even out the multiprocessors' loads: rounds of
+// CTAs times blocks of products each, and about four blocks' time for a CTA's start and end.
 jsm_status dot_f32_launch(const jsm_mat& A, const jsm_mat& B, const jsm_mat& Cm, cudaStream_t st) {
-    const bool few = A.rows <= 32;
-    const int tiles = (B.cols + 63) / 64 * (few ? (A.rows + 15) / 16 : (A.rows + 63) / 64), blocks = (A.cols + DOT_KB - 1) / DOT_KB;
+    float* C = reinterpret_cast<float*>(Cm.data);
+    if ((A.rows > 32 || (long long)B.cols * A.cols >= 1 << 20) && A.col_stride == 1 && B.row_stride == 1 && Cm.col_stride == 1 &&
+        dot_split_usable(A.data, A.row_stride, B.data, B.col_stride, C, Cm.row_stride, B.cols, A.cols))
+        return dot_split_launch(static_cast<const float*>(A.data), A.row_stride, static_cast<const float*>(B.data), B.col_stride, C, Cm.row_stride, A.rows,
+                                B.cols, A.cols, st);
+    const int tiles = (B.cols + 63) / 64 * ((A.rows + 15) / 16), blocks = (A.cols + DOT_KB - 1) / DOT_KB;
     int splits = 1;
     long long best = -1;
     for (int s = 1; s <= 8 && s <= blocks; s *= 2) {
         const long long cost = (long long)((tiles * s + sm_count() - 1) / sm_count()) * ((blocks + s - 1) / s + 4);
         if (best < 0 || cost < best) { best = cost; splits = s; }
     }
-    float* C = reinterpret_cast<float*>(Cm.data);
-    return few ? dot_launch<false, 2, 4>(to_d(A), to_d(B), nullptr, 0, nullptr, C, Cm.row_stride, Cm.col_stride, splits, st)
-               : dot_launch<false, 8, 4>(to_d(A), to_d(B), nullptr, 0, nullptr, C, Cm.row_stride, Cm.col_stride, splits, st);
+    return dot_launch<false, 2, 4>(to_d(A), to_d(B), nullptr, 0, nullptr, C, Cm.row_stride, Cm.col_stride, splits, st);
 }
 
 // whether the spans of memory of two matrices meet

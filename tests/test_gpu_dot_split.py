@@ -1,0 +1,79 @@
+"""fp32 products on the tensor cores (dot_split.cu) against float64: the vocabulary projection of an f32 model whose layers pass the token through, so that the
+operands are known: on both sides of the lines of its dispatch (33 tokens, a million weights), at both edges of the token tiles of 32 / 64 / 96 / 128, of the feature tile of 128 and of the blocks of 64 products,
+with clusters of one to eight CTAs; weights of 24 bits and weights that fit bf16; infinities, NaN and numbers beyond bf16's range."""
+import numpy as np
+import pytest
+
+import vagonex_util as vu
+
+pytestmark = pytest.mark.gpu
+
+
+def head_model(width, embed, T):
+    """A model whose sublayers add nothing: the operand of the vocabulary projection is the normed embedding."""
+    vocab = embed.shape[0]
+    cfg = vu.config([vu.lightning(heads=1, dim=8, vdim=8)], width=width, vocab=vocab, alpha=1.0, scale=1.0, eps=1e-6)
+    w = {"embed": embed, "final.norm": np.ones(width, np.float32), "l0.norm1": np.ones(width, np.float32), "l0.mix.norm": np.ones(8, np.float32)}
+    for s in "qkvg":
+        w["l0.mix." + s] = np.zeros((8, width), np.float32)
+    w["l0.mix.o"] = np.zeros((width, 8), np.float32)
+    return vu.build(cfg, w, "float32", max_batch=1, max_context=512, max_step_tokens=512)
+
+
+def operand(embed, toks):
+    x = embed[toks].astype(np.float64)
+    for _ in range(2):
+        x = x / np.sqrt((x * x).mean(-1, keepdims=True) + 1e-6)
+    return x
+
+
+def logits(m, toks):
+    row = m.open()
+    _, lg = m.step([(row, toks)], range(len(toks)))
+    m.retire(row)
+    return lg
+
+
+def check(got, x, w):
+    """Every addition of a block truncates (24 per block at most), the others round: 2^-19 of the sum of magnitudes covers them and the two norms."""
+    want, size = x @ w.T, np.abs(x) @ np.abs(w).T
+    assert np.all(np.abs(got - want) <= 2.0 ** -19 * size)
+    # and on the whole no further off than fp32 additions in any order
+    assert np.sqrt(((got - want) ** 2).mean() / (want ** 2).mean()) < 5e-7
+
+
+@pytest.mark.parametrize("kind", ["full", "bf16", "mixed"])
+@pytest.mark.parametrize("T,vocab,width", [(1, 1024, 1024), (17, 7712, 136), (32, 4097, 264), (32, 1016, 1032), (33, 40, 8), (64, 128, 64), (65, 136, 72), (96, 300, 1032), (97, 1000, 136), (128, 260, 520), (129, 2049, 200), (250, 1003, 2056)])
+def test_against_float64(T, vocab, width, kind):
+    rng = np.random.default_rng(T * vocab)
+    embed = rng.standard_normal((vocab, width)).astype(np.float32)
+    short = (embed.view(np.uint32) & np.uint32(0xFFFF0000)).view(np.float32)
+    if kind == "bf16":
+        embed = short
+    elif kind == "mixed":  # blocks with and without further parts, next to each other
+        pick = rng.random((vocab // 32 + 1, width // 64 + 1)) < 0.5
+        embed = np.where(np.repeat(np.repeat(pick, 32, 0), 64, 1)[:vocab, :width], embed, short)
+    toks = rng.integers(0, vocab, T)
+    m = head_model(width, embed, T)
+    check(logits(m, toks), operand(embed, toks), embed.astype(np.float64))
+    m.close()
+
+
+def test_numbers_that_do_not_split():
+    rng = np.random.default_rng(3)
+    embed = rng.standard_normal((200, 136)).astype(np.float32)
+    toks = rng.integers(0, 150, 70)  # (the rows behind are only features)
+    embed[150, 7], embed[151, 9], embed[152, 100] = np.inf, np.nan, -np.inf
+    embed[153, [1, 2]] = np.inf, -np.inf
+    embed[154:160] = 0.0
+    embed[154, 135], embed[155, 0], embed[156, 64] = 3.4e38, -3.39e38, 1e-38
+    m = head_model(136, embed, 70)
+    got, x = logits(m, toks), operand(embed, toks)
+    with np.errstate(all="ignore"):
+        want = (x @ embed.astype(np.float64).T).astype(np.float32)
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+    fine = np.isfinite(want)
+    assert fine[:, 154].any() and np.isinf(want[:, 154]).any()
+    assert np.allclose(got[fine], want[fine], rtol=2e-5, atol=2e-5)
+    assert np.allclose(got[:, 156], want[:, 156], rtol=1e-5, atol=2.0 ** -133)
+    m.close()
