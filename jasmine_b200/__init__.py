@@ -213,6 +213,31 @@ def _torch():
     return _torch_module
 
 
+# csrc/py_calls.cpp: the frequent calls without ctypes (None: not looked for yet, False: not built).  Its functions return a status, or None for
+# arguments that they leave to the code here.
+_calls_module = None
+
+
+def _calls():
+    global _calls_module
+    if _calls_module is None:
+        _torch()
+        try:
+            from . import _native as m
+            m.bind(lib()._handle)
+        except ImportError:
+            m = False
+        _calls_module = m
+    return _calls_module
+
+
+def _done(status) -> bool:
+    """Whether a call of the extension module was made (an error raises)."""
+    if status:
+        check(status)
+    return status is not None
+
+
 def stream_ptr() -> int:
     """Address of torch's current stream (the raw query: no Stream object is made for it)."""
     torch = _torch()
@@ -263,6 +288,9 @@ def _leaves(ts):
 
 
 def eval_elementwise(instrs, leaves, out):
+    m = _calls_module or _calls()
+    if m and _done(m.eval_elementwise(instrs, leaves, out)):
+        return out
     p, n = program(instrs)
     l, nl = _leaves(leaves)
     check(lib().jsm_eval_elementwise(p, n, l, nl, mat(out), stream_ptr()))
@@ -270,6 +298,9 @@ def eval_elementwise(instrs, leaves, out):
 
 
 def eval_rows(kind, axis, instrs, leaves, out, gain=None, bias=None, eps=0.0):
+    m = _calls_module or _calls()
+    if m and _done(m.eval_rows(kind, axis, instrs, leaves, out, gain, bias, eps)):
+        return out
     p, n = program(instrs)
     l, nl = _leaves(leaves)
     check(lib().jsm_eval_rows(kind, axis, p, n, l, nl, gain.data_ptr() if gain is not None else None,
@@ -285,6 +316,9 @@ def eval_full(kind, instrs, leaves, out):
 
 
 def dot_f32(A, B, out, bias=None, epilogue=0, residual=None):
+    m = _calls_module or _calls()
+    if m and _done(m.dot_f32(A, B, out, bias, epilogue, residual)):
+        return out
     b = mat(bias) if bias is not None else None
     r = mat(residual) if residual is not None else None
     check(lib().jsm_dot_f32(mat(A), mat(B), C.byref(b) if b is not None else None, epilogue,
@@ -386,8 +420,11 @@ def rope_apply_qk(q, k, table, d, Hq, Hkv, positions=None, q_out=None, k_out=Non
 def attn_prefill(q, k, v, batch, Hq, Hkv, D, causal=True, scale=None, rope=None, impl=0, out=None):
     torch = _torch()
     out = torch.empty_like(q) if out is None else out
-    Tq, Tk = q.shape[0] // batch, k.shape[0] // batch
     scale = float(D) ** -0.5 if scale is None else scale
+    m = _calls_module or _calls()
+    if m and _done(m.attn_prefill(q, k, v, batch, Hq, Hkv, D, causal, scale, rope, impl, out)):
+        return out
+    Tq, Tk = q.shape[0] // batch, k.shape[0] // batch
     check(lib().jsm_attn_prefill(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dtype_of(q), batch, Tq, Tk,
                                  Hq, Hkv, D, int(causal), scale, rope.data_ptr() if rope is not None else None, impl,
                                  stream_ptr()))
@@ -410,6 +447,9 @@ def attn_decode(q, pool, block_table, context_lens, Hq, Hkv, D, max_context, sca
         nbytes = lib().jsm_attn_decode_scratch_bytes(n, Hq, D, max_context)
         scratch = torch.empty(nbytes // 4, dtype=torch.float32, device=q.device)
     scale = float(D) ** -0.5 if scale is None else scale
+    m = _calls_module or _calls()
+    if m and _done(m.attn_decode(q, pool, block_table, context_lens, Hq, Hkv, D, max_context, scale, rope, scratch, out)):
+        return out
     check(lib().jsm_attn_decode(q.data_ptr(), q.stride(0), pool.data_ptr(), block_table.data_ptr(),
                                 block_table.shape[1], context_lens.data_ptr(), n, Hq, Hkv, D, scale,
                                 rope.data_ptr() if rope is not None else None, max_context, scratch.data_ptr(),
@@ -458,6 +498,9 @@ def embedding(table, ids, pos_table=None, positions=None, out=None):
     torch = _torch()
     T, d = ids.shape[0], table.shape[1]
     out = torch.empty(T, d, dtype=table.dtype, device=table.device) if out is None else out
+    m = _calls_module or _calls()
+    if m and _done(m.embedding(table, ids, pos_table, positions, out)):
+        return out
     check(lib().jsm_embedding(table.data_ptr(), pos_table.data_ptr() if pos_table is not None else None, ids.data_ptr(),
                               positions.data_ptr() if positions is not None else None, out.data_ptr(), dtype_of(table),
                               T, d, stream_ptr()))

@@ -6,21 +6,28 @@ is linked statically and the driver API is reached through
 cudaGetDriverEntryPoint, so the library loads on a machine without a GPU
 driver (compute calls then return JSM_CUDA).
 
+The frequent calls of the Python plumbing are a small extension module beside it (csrc/py_calls.cpp -> jasmine_b200/_native.so, g++
+against the headers of the installed torch); where torch is not installed it is left out, and the plumbing goes through ctypes.
+
 Run as `python -m jasmine_b200.build [--force] [--verbose]`.
 """
 from __future__ import annotations
 
 import concurrent.futures as cf
 import hashlib
+import importlib.metadata
+import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "build"
 LIB = PKG / "libjasmine_b200.so"
+CALLS = PKG / "_native.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -64,11 +71,33 @@ def _compile(src: Path, force: bool, verbose: bool) -> Path:
     return obj
 
 
+def _build_calls(force: bool) -> None:
+    spec = importlib.util.find_spec("torch")
+    if spec is None or not spec.submodule_search_locations:
+        return
+    torch = Path(spec.submodule_search_locations[0])
+    src = CSRC / "py_calls.cpp"
+    cmd = [os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", "-I" + sysconfig.get_paths()["include"],
+           f"-I{torch}/include", f"-I{torch}/include/torch/csrc/api/include", "-I/usr/local/cuda/include", str(src), "-o", str(CALLS), f"-L{torch}/lib",
+           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    stamp = hashlib.sha256(" ".join([*cmd, importlib.metadata.version("torch"), sys.version]).encode() + src.read_bytes() +
+                           (PKG.parent / "include" / "jasmine_b200.h").read_bytes()).hexdigest()
+    stamp_file = OBJ / "py_calls.stamp"
+    if not force and CALLS.exists() and stamp_file.exists() and stamp_file.read_text() == stamp:
+        return
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for {src.name}:\n{res.stderr[-6000:]}")
+    stamp_file.write_text(stamp)
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     OBJ.mkdir(exist_ok=True)
     sources = sorted(CSRC.glob("*.cu"))
     with cf.ThreadPoolExecutor(max_workers=min(8, len(sources))) as ex:
+        calls = ex.submit(_build_calls, force)
         objs = list(ex.map(lambda s: _compile(s, force, verbose), sources))
+        calls.result()
     newest = max(o.stat().st_mtime for o in objs)
     if force or not LIB.exists() or LIB.stat().st_mtime < newest:
         cmd = [_nvcc(), "-shared", "-o", str(LIB), *map(str, objs), "-cudart", "static",
