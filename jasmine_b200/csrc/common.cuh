@@ -177,6 +177,11 @@ __host__ __device__ inline float bf16_bits_to_f32(uint16_t b) {
 #ifdef __CUDACC__
 __device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// What earlier passes or the host left (positions, block tables, a layer's own state) may be read before chain_wait, past L1, whose lines may be
+// older than the pass.  A kernel that works before chain_wait must not declare what its predecessors write `const __restrict__`: the
+// compiler then takes it for constant and may move the loads to the other side of the wait (a convolution of three taps lost tokens).
+template <typename T>
+__device__ __forceinline__ T load_early(const T* p) { return __ldcg(p); }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ float bf16lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }

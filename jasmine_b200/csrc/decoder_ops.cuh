@@ -220,9 +220,10 @@ jsm_status sum_norm_launch(const float* y, float* x, const float* gain, float ep
 // out[i] = x[rows[i]] / rms * gain, act [n][wp]
 jsm_status final_norm_launch(bool f32, const float* x, const int32_t* rows, const float* gain, float eps, void* out, int n, int d, int wp,
                              cudaStream_t st);
-// logits <- cap * tanh(logits / cap) in place (cap <= 0: unchanged) and the arg-max of every row (first maximum)
+// logits <- cap * tanh(logits / cap) in place (cap <= 0: unchanged) and the arg-max of every row (first maximum).
+// err_out (or null): [rows], each the value of *err after the earlier kernels of the stream
 jsm_status logits_finish_launch(float* logits, int pitch, int vocab, float cap, int rows, unsigned long long* keys, int32_t* ctrs,
-                                int32_t* next, cudaStream_t st);
+                                int32_t* next, cudaStream_t st, const int* err = nullptr, int32_t* err_out = nullptr);
 // act = min(g, limit) * sigmoid(alpha * min(g, limit)) * (clamp(u, -limit, limit) + 1), all f32 [T][n]
 jsm_status clamped_glu_f32_launch(const float* gate, const float* up, float* act, float alpha, float limit, long long n, cudaStream_t st);
 // act = gelu_tanh(gate) * up, all f32

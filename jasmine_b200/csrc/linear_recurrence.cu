@@ -714,8 +714,8 @@ __global__ void __launch_bounds__(RT_THREADS, 3) rec_step_kernel(RecArgs a, RecD
     const int h = blockIdx.x, g = h / (d.H / d.G), seg = blockIdx.y;
     const int rg = tid / lpr, c = (tid % lpr) * 4;
     const bool on = c < vp;
-    const bool fresh = a.seg_pos0[seg] == 0;
-    float* state = a.S + ((long long)a.seg_slot[seg] * d.H + h) * kp * vp;
+    const bool fresh = load_early(a.seg_pos0 + seg) == 0;
+    float* state = a.S + ((long long)load_early(a.seg_slot + seg) * d.H + h) * kp * vp;
     if (IN_SMEM) {
         if (fresh) {
             for (int i = tid; i < kp * vp / 4; i += RT_THREADS) reinterpret_cast<float4*>(rt_sm)[i] = make_float4(0.f, 0.f, 0.f, 0.f);

@@ -38,18 +38,18 @@ __device__ __forceinline__ T* cache_at(T* pool, const AttnDims& d, int page, int
 // A warp takes one unit of TOK consecutive tokens: the query heads, then the key heads, the value heads (own_kv), and one unit
 // for the gates.  wide row of a token: [q | gates | k | v].  NP: pairs of components per lane (0: any number, read twice).
 template <typename T, int NP, int TOK>
-__global__ void __launch_bounds__(256) attn_prep_kernel(const float* __restrict__ wide, AttnDims d, AttnWeights w, float eps, T* __restrict__ pool,
+__global__ void __launch_bounds__(256) attn_prep_kernel(const float* wide, AttnDims d, AttnWeights w, float eps, T* pool,
                                                         const int32_t* __restrict__ block_table, int max_pages, const float2* __restrict__ rope,
                                                         const int32_t* __restrict__ tok_row, const int32_t* __restrict__ tok_pos, int own_kv, int n_tok,
-                                                        T* __restrict__ q, float* __restrict__ gate) {
+                                                        T* q, float* gate) {
     static_assert(NP > 0 || TOK == 1, "heads of any width take one token");
     const int t0 = blockIdx.x * TOK, unit = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int kv_units = own_kv ? 2 * d.G : 0;
     const int off = d.q_cols() + pad8(d.H), pitch = d.wide_cols(own_kv != 0);
     chain_trigger();
-    chain_wait();
     if (unit >= d.H + kv_units + d.gated) return;
     if (unit == d.H + kv_units) {
+        chain_wait();
         for (int t = t0; t < min(n_tok, t0 + TOK); ++t)
             for (int h = lane; h < d.H; h += 32) gate[(long long)t * d.H + h] = 1.0f / (1.0f + expf(-wide[(long long)t * pitch + d.q_cols() + h]));
         return;
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) attn_prep_kernel(const float* __restrict_
     };
     // where pair pr of a token goes
     auto entry = [&](int t, int pos) {  // keys and values: first element of the token's row in the first slab
-        return cache_at(pool, d, block_table[(long long)tok_row[t] * max_pages + pos / PAGE], hd, value ? 1 : 0, pos % PAGE, 0) - slab_index<T>(pos % PAGE, 0) + pos % PAGE * 64;
+        return cache_at(pool, d, load_early(block_table + (long long)load_early(tok_row + t) * max_pages + pos / PAGE), hd, value ? 1 : 0, pos % PAGE, 0) - slab_index<T>(pos % PAGE, 0) + pos % PAGE * 64;
     };
     auto store = [&](T* row, int pos, int pr, const float2& v) {
         put(key || value ? row + (pr >> 5) * SLAB + ((((pr >> 2) & 7) ^ (pos & 7)) << 3) + (pr & 3) * 2 : row + 2 * pr, v);
@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(256) attn_prep_kernel(const float* __restrict_
     };
     auto length = [&](float ss) { return gain ? 1.0f / sqrtf(warp_sum(ss) / (float)n + eps) : 1.0f; };
     if (value) {
+        chain_wait();
         for (int i = 0; i < TOK; ++i) {
             const int t = t0 + i;
             if (t >= n_tok) break;
@@ -105,10 +106,13 @@ __global__ void __launch_bounds__(256) attn_prep_kernel(const float* __restrict_
         }
     } else if constexpr (NP > 0) {
         float2 v[TOK][NP], g[NP];
+        const int first_pos = load_early(tok_pos + min(t0, n_tok - 1));
+        T* first_row = key ? entry(min(t0, n_tok - 1), first_pos) : nullptr;
         {
             float2 b[NP];
 #pragma unroll
             for (int k = 0; k < NP; ++k) { b[k] = vec(bias, k * 32 + lane, 0.0f); g[k] = vec(gain, k * 32 + lane, 1.0f); }
+            chain_wait();  // (what describes the pass and the constants are older)
 #pragma unroll
             for (int i = 0; i < TOK; ++i)
 #pragma unroll
@@ -122,13 +126,14 @@ __global__ void __launch_bounds__(256) attn_prep_kernel(const float* __restrict_
 #pragma unroll
             for (int k = 0; k < NP; ++k) ss = fmaf(v[i][k].x, v[i][k].x, fmaf(v[i][k].y, v[i][k].y, ss));
             const float inv = length(ss);
-            const int pos = tok_pos[t];
-            T* row = key ? entry(t, pos) : q + (long long)t * d.q_cols() + hd * d.qh();
+            const int pos = i == 0 ? first_pos : tok_pos[t];
+            T* row = !key ? q + (long long)t * d.q_cols() + hd * d.qh() : i == 0 ? first_row : entry(t, pos);
 #pragma unroll
             for (int k = 0; k < NP; ++k)
                 if (k * 32 + lane < end) store(row, pos, k * 32 + lane, turn(pos, k * 32 + lane, v[i][k], inv, g[k]));
         }
     } else {
+        chain_wait();
         float ss = 0.0f;
         for (int pr = lane; 2 * pr < n; pr += 32) {
             const float2 v = pair(t0, pr, vec(bias, pr, 0.0f));
@@ -359,17 +364,26 @@ __global__ void __launch_bounds__(AM_THREADS, 1) attn_paged_mma_kernel(AttnArgs 
         tc::mbar_fence_init();
     }
     __syncthreads();
-    chain_wait();
     const int tile = blockIdx.x, g = blockIdx.y, sp = blockIdx.z;
-    const int seg = a.tile_seg[tile], r0 = a.tile_r0[tile];
-    const int start = a.seg_start[seg], pos0 = a.seg_pos0[seg];
-    const int n_rows = min(R, a.seg_len[seg] * gs - r0);
+    const int seg = load_early(a.tile_seg + tile), r0 = load_early(a.tile_r0 + tile);
+    const int start = load_early(a.seg_start + seg), pos0 = load_early(a.seg_pos0 + seg);
+    const int n_rows = min(R, load_early(a.seg_len + seg) * gs - r0);
     const int key_lo = d.mask.first(pos0 + r0 / gs), key_hi = pos0 + (r0 + n_rows - 1) / gs + 1;
     const int pg_lo = key_lo / PAGE, n_pg = (key_hi - 1) / PAGE - pg_lo + 1;
     const int live = min(a.splits, n_pg);  // the grid is made for the longest context
     if (sp >= live) return;
     const int pb = pg_lo + n_pg * sp / live, n_it = pg_lo + n_pg * (sp + 1) / live - pb;
-    const int32_t* bt = a.block_table + (long long)a.seg_row[seg] * a.max_pages + pb;
+    const int32_t* bt = a.block_table + (long long)load_early(a.seg_row + seg) * a.max_pages + pb;
+    auto load_page = [&](int it) {
+        const int s = it % AM_STAGES;
+        tc::mbar_expect_tx(&full_bar[s], stage_bytes);
+        tc::bulk_load(ring + s * stage_bytes, a.pool + (long long)(load_early(bt + it) * d.G + g) * (stage_bytes / 2), stage_bytes, &full_bar[s]);
+    };
+    // Pages that end before the segment hold nothing of this pass: the ring is filled with them while the predecessors still run.
+    const int early = min(min(n_it, AM_STAGES), pos0 / PAGE - pb);
+    if (threadIdx.x == AM_WARPS * 32)
+        for (int it = 0; it < early; ++it) load_page(it);
+    chain_wait();
 
     // queries (columns behind the head's are zero)
     for (int i = threadIdx.x; i < R * ks * 8; i += AM_THREADS) {
@@ -391,12 +405,10 @@ __global__ void __launch_bounds__(AM_THREADS, 1) attn_paged_mma_kernel(AttnArgs 
     }
     if (warp == AM_WARPS) {
         if (lane == 0) {
-            int issued = 0;
-            for (int it = 0; it < n_it; ++it) {
-                const int s = it % AM_STAGES;
-                if (it >= AM_STAGES && !tc::mbar_wait(&empty_bar[s], ((it / AM_STAGES) - 1) & 1, &abort_flag, a.err, AM_ERR_EMPTY)) break;
-                tc::mbar_expect_tx(&full_bar[s], stage_bytes);
-                tc::bulk_load(ring + s * stage_bytes, a.pool + (long long)(bt[it] * d.G + g) * (stage_bytes / 2), stage_bytes, &full_bar[s]);
+            int issued = max(early, 0);
+            for (int it = issued; it < n_it; ++it) {
+                if (it >= AM_STAGES && !tc::mbar_wait(&empty_bar[it % AM_STAGES], ((it / AM_STAGES) - 1) & 1, &abort_flag, a.err, AM_ERR_EMPTY)) break;
+                load_page(it);
                 issued = it + 1;
             }
             if (abort_flag) {  // let the copies in flight land (bounded)

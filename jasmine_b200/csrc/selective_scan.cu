@@ -20,6 +20,7 @@
 #include "tc_utils.cuh"
 #include <math.h>
 #include <algorithm>
+#include <type_traits>
 
 namespace jsm {
 
@@ -72,6 +73,9 @@ struct Vec8<float> {
         const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     }
+    __device__ static void load_old(const float* p, float (&v)[8]) {
+        widen(Raw{load_early(reinterpret_cast<const float4*>(p)), load_early(reinterpret_cast<const float4*>(p) + 1)}, v);
+    }
     __device__ static void store(float* p, const float (&v)[8]) {
         reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
         reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
@@ -82,6 +86,7 @@ struct Vec8<__nv_bfloat16> {
     using Raw = uint4;
     __device__ static Raw fetch(const __nv_bfloat16* p) { return *reinterpret_cast<const uint4*>(p); }
     __device__ static void load(const __nv_bfloat16* p, float (&v)[8]) { widen(fetch(p), v); }
+    __device__ static void load_old(const __nv_bfloat16* p, float (&v)[8]) { widen(load_early(reinterpret_cast<const uint4*>(p)), v); }
     __device__ static void widen(const uint4& w, float (&v)[8]) {
         v[0] = bf16lo(w.x); v[1] = bf16hi(w.x); v[2] = bf16lo(w.y); v[3] = bf16hi(w.y);
         v[4] = bf16lo(w.z); v[5] = bf16hi(w.z); v[6] = bf16lo(w.w); v[7] = bf16hi(w.w);
@@ -107,50 +112,59 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&v)[4]) {
 }
 
 // ---- convolution --------------------------------------------------------------------------------------------------
-// A thread owns 8 channels of CONV_TOK consecutive tokens; TAPS 0: taps is only known at run time.  carry: every segment is
-// one token, and the state moves on by it here (otherwise the scan does that, once every CTA has read the old state)
-constexpr int CONV_TOK = 8;
-template <typename T, int TAPS>
-__global__ void __launch_bounds__(256, 2) scan_conv_kernel(const T* __restrict__ xz, long long pitch, T* __restrict__ xc, T* state,
+// A thread owns 8 channels of TOK consecutive tokens (8 share the loads of a window; a pass that would leave multiprocessors without
+// threads takes 2, a decode step 1); TAPS 0: taps is only known at run time.  carry: every segment is one token, and the state
+// moves on by it here (otherwise the scan does that, once every CTA has read the old state)
+template <typename T, int TAPS, int TOK>
+__global__ void __launch_bounds__(256, 2) scan_conv_kernel(const T* xz, long long pitch, T* xc, T* state,
                                                         const float* __restrict__ w, const float* __restrict__ b,
                                                         const int32_t* __restrict__ seg_start, const int32_t* __restrict__ seg_len,
                                                         const int32_t* __restrict__ seg_pos0, const int32_t* __restrict__ seg_slot, int ip,
                                                         int taps_rt, int carry) {
+    // What describes the pass, the constants and the inputs before the segment, kept from earlier passes, are there before the predecessor ends;
+    // only the segment's own inputs are waited for (3.9 us a launch in a step of eight sequences, most of it four round trips).
     chain_trigger();
-    chain_wait();
     const int taps = TAPS ? TAPS : taps_rt;
     const int seg = blockIdx.y, vec = ip / 8;
-    const int start = seg_start[seg], len = seg_len[seg], pos0 = seg_pos0[seg];
+    const int start = load_early(seg_start + seg), len = load_early(seg_len + seg), pos0 = load_early(seg_pos0 + seg);
     const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
-    const int c = (int)(i % vec) * 8, j0 = (int)(i / vec) * CONV_TOK;
+    const int c = (int)(i % vec) * 8, j0 = (int)(i / vec) * TOK;
     if (j0 >= len) return;
-    T* st = state + (long long)seg_slot[seg] * (taps - 1) * ip + c;
+    T* st = state + (long long)load_early(seg_slot + seg) * (taps - 1) * ip + c;
     // input of the segment's token j (negative: before the segment)
-    auto input = [&](int j, float (&v)[8]) {
-        if (j >= 0) Vec8<T>::load(xz + (start + j) * pitch + c, v);
-        else if (pos0 + j >= 0) Vec8<T>::load(st + (long long)(taps - 1 + j) * ip, v);
+    auto before = [&](int j, float (&v)[8]) {
+        if (pos0 + j >= 0) Vec8<T>::load_old(st + (long long)(taps - 1 + j) * ip, v);
         else
             for (int e = 0; e < 8; ++e) v[e] = 0.0f;
+    };
+    auto input = [&](int j, float (&v)[8]) {
+        if (j >= 0) Vec8<T>::load(xz + (start + j) * pitch + c, v);
+        else before(j, v);
     };
     float bias[8];
     if (b) Vec8<float>::load(b + c, bias);
     else
 #pragma unroll
         for (int e = 0; e < 8; ++e) bias[e] = 0.0f;
-    const int j1 = min(len, j0 + CONV_TOK);
+    const int j1 = min(len, j0 + TOK);
     if constexpr (TAPS > 0) {
-        // all the thread's inputs are requested before the first is used
-        typename Vec8<T>::Raw raw[CONV_TOK];
-#pragma unroll
-        for (int u = 0; u < CONV_TOK; ++u)
-            if (j0 + u < j1) raw[u] = Vec8<T>::fetch(xz + (start + j0 + u) * pitch + c);
         float win[TAPS][8], wt[TAPS][8];
 #pragma unroll
         for (int k = 0; k < TAPS; ++k) Vec8<float>::load(w + (long long)k * ip + c, wt[k]);
 #pragma unroll
-        for (int k = 0; k + 1 < TAPS; ++k) input(j0 - TAPS + 1 + k, win[k + 1]);
+        for (int k = 0; k + 1 < TAPS; ++k)
+            if (j0 - TAPS + 1 + k < 0) before(j0 - TAPS + 1 + k, win[k + 1]);
+        chain_wait();
+        // all the thread's inputs are requested before the first is used
+        typename Vec8<T>::Raw raw[TOK];
 #pragma unroll
-        for (int u = 0; u < CONV_TOK; ++u) {
+        for (int u = 0; u < TOK; ++u)
+            if (j0 + u < j1) raw[u] = Vec8<T>::fetch(xz + (start + j0 + u) * pitch + c);
+#pragma unroll
+        for (int k = 0; k + 1 < TAPS; ++k)
+            if (j0 - TAPS + 1 + k >= 0) input(j0 - TAPS + 1 + k, win[k + 1]);
+#pragma unroll
+        for (int u = 0; u < TOK; ++u) {
             const int j = j0 + u;
             if (j >= j1) break;
 #pragma unroll
@@ -172,6 +186,7 @@ __global__ void __launch_bounds__(256, 2) scan_conv_kernel(const T* __restrict__
 #pragma unroll
             for (int k = 0; k + 1 < TAPS; ++k) Vec8<T>::store(st + (long long)k * ip, win[k + 1]);
     } else {
+        chain_wait();
         for (int j = j0; j < j1; ++j) {
             float o[8];
             for (int e = 0; e < 8; ++e) o[e] = bias[e];
@@ -422,27 +437,31 @@ __global__ void __launch_bounds__(ST_THREADS) scan_step_kernel(ScanArgs a) {
 #pragma unroll
         for (int i = 0; i < NP; ++i) A[i] = i < planes ? Ap[(long long)i * a.ip] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float bias = a.dt_b[cl], dv = a.D[cl];
+    // only this kernel writes the states, and passes are separated by the host: they are requested before the predecessor ends
+    float4 S[R][NP ? NP : 1];
+    float4* Sp[R];
+    bool fresh[R];
+    int tok[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        const int sg = s0 + min(q * ST_WARPS + warp, nb - 1);
+        tok[q] = load_early(a.seg_start + sg);
+        fresh[q] = load_early(a.seg_pos0 + sg) == 0;
+        Sp[q] = reinterpret_cast<float4*>(a.S + (long long)load_early(a.seg_slot + sg) * a.ip * a.np) + cl;
+        if (NP > 0)
+#pragma unroll
+            for (int i = 0; i < NP; ++i)
+                S[q][i] = (i < planes && !fresh[q]) ? load_early(Sp[q] + (long long)i * a.ip) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     chain_wait();
     for (int i = tid; i < nb * (sc / 4); i += ST_THREADS) {
         const int b = i / (sc / 4), v = i % (sc / 4);
         cp_async16(smem_u32(st_dyn + i * 4), a.proj + (long long)a.seg_start[s0 + b] * pc + off + v * 4, true);
     }
     cp_async_commit();
-    float4 S[R][NP ? NP : 1];
-    float4* Sp[R];
-    bool fresh[R];
-    int tok[R];
     T xv[R], zv[R];
 #pragma unroll
     for (int q = 0; q < R; ++q) {
-        const int sg = s0 + min(q * ST_WARPS + warp, nb - 1);
-        tok[q] = a.seg_start[sg];
-        fresh[q] = a.seg_pos0[sg] == 0;
-        Sp[q] = reinterpret_cast<float4*>(a.S + (long long)a.seg_slot[sg] * a.ip * a.np) + cl;
-        if (NP > 0)
-#pragma unroll
-            for (int i = 0; i < NP; ++i)
-                S[q][i] = (i < planes && !fresh[q]) ? Sp[q][(long long)i * a.ip] : make_float4(0.f, 0.f, 0.f, 0.f);
         xv[q] = static_cast<const T*>(a.xc)[(long long)tok[q] * a.ip + cl];
         zv[q] = static_cast<const T*>(a.xz)[(long long)tok[q] * 2 * a.ip + a.ip + cl];
     }
@@ -528,16 +547,23 @@ __global__ void __launch_bounds__(256) scan_dt_operand_kernel(const float* __res
 template <typename T>
 static jsm_status conv_typed(const void* x, long long pitch, int cp, int taps, const float* w, const float* b, void* state, const StepTokens& tk, void* out,
                              bool carry, cudaStream_t st) {
-    const long long n = (long long)((tk.max_len + CONV_TOK - 1) / CONV_TOK) * (cp / 8);
-    const dim3 grid((unsigned)((n + 255) / 256), tk.n_segs);
-    auto go = [&](auto kernel) {
-        return launch_chained(kernel, grid, dim3(256), 0, st, (const T*)x, pitch, (T*)out, (T*)state, w, b, tk.seg_start, tk.seg_len, tk.seg_pos0,
-                              tk.seg_slot, cp, taps, carry ? 1 : 0);
+    auto run = [&](auto tok) -> jsm_status {
+        constexpr int TOK = decltype(tok)::value;
+        const long long n = (long long)((tk.max_len + TOK - 1) / TOK) * (cp / 8);
+        const dim3 grid((unsigned)((n + 255) / 256), tk.n_segs);
+        auto go = [&](auto kernel) {
+            return launch_chained(kernel, grid, dim3(256), 0, st, (const T*)x, pitch, (T*)out, (T*)state, w, b, tk.seg_start, tk.seg_len, tk.seg_pos0,
+                                  tk.seg_slot, cp, taps, carry ? 1 : 0);
+        };
+        JSM_CUDA_CHECK(taps == 1 ? go(scan_conv_kernel<T, 1, TOK>) : taps == 2 ? go(scan_conv_kernel<T, 2, TOK>) : taps == 3 ? go(scan_conv_kernel<T, 3, TOK>)
+                       : taps == 4 ? go(scan_conv_kernel<T, 4, TOK>) : go(scan_conv_kernel<T, 0, TOK>));
+        JSM_LAUNCH_CHECK();
+        return JSM_OK;
     };
-    JSM_CUDA_CHECK(taps == 1 ? go(scan_conv_kernel<T, 1>) : taps == 2 ? go(scan_conv_kernel<T, 2>) : taps == 3 ? go(scan_conv_kernel<T, 3>)
-                   : taps == 4 ? go(scan_conv_kernel<T, 4>) : go(scan_conv_kernel<T, 0>));
-    JSM_LAUNCH_CHECK();
-    return JSM_OK;
+    if (tk.max_len == 1) return run(std::integral_constant<int, 1>());
+    // two CTAs per multiprocessor with eight tokens a thread, else two tokens
+    const long long ctas = (long long)((tk.max_len + 7) / 8) * (cp / 8) * tk.n_segs / 256;
+    return ctas < 2 * sm_count() ? run(std::integral_constant<int, 2>()) : run(std::integral_constant<int, 8>());
 }
 
 jsm_status short_conv_launch(bool f32, const void* x, long long x_pitch, int cp, int taps, const float* w, const float* bias, void* state,

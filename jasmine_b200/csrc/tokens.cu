@@ -4,6 +4,7 @@
 // with eps under the square root, RMSNorm drops the mean.
 #include "common.cuh"
 #include "decoder_ops.cuh"
+#include "mma_utils.cuh"
 #include <math.h>
 #include <algorithm>
 
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(256) embed_residual_kernel(const T* __restrict
 // writes it, and only up to a token per SM: with more tokens than that other CTAs hide the trip, and the registers that keep the gain cost more
 // (back to back, us, late / early: 512 x 4096 5.3 / 5.8, sums 2048 x 4096 15.1 / 16.5).
 template <int MAXV, bool SUM, bool EARLY>
-__global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restrict__ y, float* __restrict__ x, const float* __restrict__ gain,
+__global__ void __launch_bounds__(256) post_norm_add_kernel(const float* y, float* x, const float* __restrict__ gain,
                                                             float eps, float alpha, __nv_bfloat16* __restrict__ xa, int d, int wp) {
     __shared__ float smem[8];
     chain_trigger();
@@ -241,14 +242,44 @@ __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restr
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) final_norm_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, const float* __restrict__ gain,
+__global__ void __launch_bounds__(256) final_norm_kernel(const float* x, const int32_t* __restrict__ rows, const float* __restrict__ gain,
                                                          float eps, T* __restrict__ out, int d, int wp) {
     __shared__ float smem[8];
-    constexpr int N = VecIO<T>::N;
+    constexpr int N = VecIO<T>::N, MAXV = 2;
     chain_trigger();
+    float q = 0.0f;
+    if (wp <= 2048 * MAXV) {  // the row stays in registers; padding columns of x and of the gain are zero
+        float v[MAXV][8], g[MAXV][8];
+        const float* src = x + (long long)load_early(rows + blockIdx.x) * wp;
+#pragma unroll
+        for (int i = 0; i < MAXV; ++i) {
+            const int c = (i * 256 + threadIdx.x) * 8;
+            if (c < wp) load_f32x8(gain + c, g[i]);
+        }
+        chain_wait();
+#pragma unroll
+        for (int i = 0; i < MAXV; ++i) {
+            const int c = (i * 256 + threadIdx.x) * 8;
+            if (c < wp) {
+                load_f32x8(src + c, v[i]);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) q = fmaf(v[i][e], v[i][e], q);
+            }
+        }
+        const float rms = sqrtf(block_sum(q, smem) / (float)d + eps);
+#pragma unroll
+        for (int i = 0; i < MAXV; ++i) {
+            const int c = (i * 256 + threadIdx.x) * 8;
+            if (c < wp) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[i][e] = v[i][e] / rms * g[i][e];
+                store_f32x8(out + (long long)blockIdx.x * wp + c, v[i]);
+            }
+        }
+        return;
+    }
     chain_wait();
     const float* src = x + (long long)rows[blockIdx.x] * wp;
-    float q = 0.0f;
     for (int c = threadIdx.x; c < d; c += 256) q = fmaf(src[c], src[c], q);
     q = block_sum(q, smem) / (float)d;
     const float rms = sqrtf(q + eps);
@@ -263,26 +294,54 @@ __global__ void __launch_bounds__(256) final_norm_kernel(const float* __restrict
 // Logits of one row per blockIdx.y, split over gridDim.x CTAs: the cap in place and the arg-max over the capped values.  A
 // slice's best (value, index) becomes one monotone 64-bit key that goes into the row's key with atomicMax (larger value
 // first, then the lower index); the CTA that arrives last writes the token and resets both words for the next launch.
+//
+// VEC: rows of 16-byte aligned fours.  A thread requests all its logits before it caps the first: read one after the other, with a store between
+// two loads, a step's 32000-wide rows took 6.4 us.
+template <bool VEC>
 __global__ void __launch_bounds__(256) logits_finish_kernel(float* __restrict__ logits, int pitch, int vocab, float cap,
                                                             unsigned long long* __restrict__ keys, int32_t* __restrict__ ctrs,
-                                                            int32_t* __restrict__ next) {
+                                                            int32_t* __restrict__ next, const int* __restrict__ err, int32_t* __restrict__ err_out) {
     __shared__ unsigned long long best[8];
     chain_trigger();
     chain_wait();
+    constexpr int W = VEC ? 4 : 1, DEEP = 4;
     const int r = blockIdx.y;
     float* row = logits + (long long)r * pitch;
-    const int lo = (int)((long long)blockIdx.x * vocab / gridDim.x), hi = (int)((long long)(blockIdx.x + 1) * vocab / gridDim.x);
+    const int groups = (vocab + W - 1) / W;  // (a last group may reach into the row's padding)
+    const int lo = (int)((long long)blockIdx.x * groups / gridDim.x), hi = (int)((long long)(blockIdx.x + 1) * groups / gridDim.x);
     unsigned long long key = 0;  // below every value's key
-    for (int i = lo + threadIdx.x; i < hi; i += 256) {
-        float v = row[i];
-        if (cap > 0.0f) {
-            v = cap * tanhf(v / cap);
-            row[i] = v;
+    for (int i0 = lo + threadIdx.x; i0 < hi; i0 += 256 * DEEP) {
+        float v[DEEP][W];
+#pragma unroll
+        for (int u = 0; u < DEEP; ++u) {
+            const int i = i0 + u * 256;
+            if (i >= hi) continue;
+            if constexpr (VEC) {
+                const float4 f = *reinterpret_cast<const float4*>(row + i * 4);
+                v[u][0] = f.x; v[u][1] = f.y; v[u][2] = f.z; v[u][3] = f.w;
+            } else {
+                v[u][0] = row[i];
+            }
         }
-        const uint32_t bits = __float_as_uint(v);
-        const uint32_t mono = (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
-        const unsigned long long k = ((unsigned long long)mono << 32) | (0xffffffffu - (uint32_t)i);
-        if (v == v && k > key) key = k;
+#pragma unroll
+        for (int u = 0; u < DEEP; ++u) {
+            const int i = i0 + u * 256;
+            if (i >= hi) continue;
+#pragma unroll
+            for (int e = 0; e < W; ++e) {
+                if (cap > 0.0f) v[u][e] = cap * tanhf(v[u][e] / cap);
+                const uint32_t bits = __float_as_uint(v[u][e]), at = (uint32_t)(i * W + e);
+                const uint32_t mono = (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
+                const unsigned long long k = ((unsigned long long)mono << 32) | (0xffffffffu - at);
+                if (v[u][e] == v[u][e] && (!VEC || (int)at < vocab) && k > key) key = k;
+            }
+            if (cap > 0.0f) {
+                if (VEC && i * 4 + 4 <= vocab) *reinterpret_cast<float4*>(row + i * 4) = make_float4(v[u][0], v[u][1 % W], v[u][2 % W], v[u][3 % W]);
+                else
+                    for (int e = 0; e < W; ++e)
+                        if (i * W + e < vocab) row[i * W + e] = v[u][e];
+            }
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -302,6 +361,7 @@ __global__ void __launch_bounds__(256) logits_finish_kernel(float* __restrict__ 
             const unsigned long long top = atomicExch(keys + r, 0ull);
             next[r] = top ? (int32_t)(0xffffffffu - (uint32_t)(top & 0xffffffffull)) : 0;
             ctrs[r] = 0;
+            if (err_out) err_out[r] = __ldcg(err);  // (the step's earlier kernels have ended)
         }
     }
 }
@@ -360,10 +420,11 @@ jsm_status final_norm_launch(bool f32, const float* x, const int32_t* rows, cons
 }
 
 jsm_status logits_finish_launch(float* logits, int pitch, int vocab, float cap, int rows, unsigned long long* keys, int32_t* ctrs, int32_t* next,
-                                cudaStream_t st) {
+                                cudaStream_t st, const int* err, int32_t* err_out) {
     if (rows <= 0) return JSM_OK;
     const int slices = std::max(1, std::min(16, vocab / 1024));
-    JSM_CUDA_CHECK(launch_chained(logits_finish_kernel, dim3(slices, rows), dim3(256), 0, st, logits, pitch, vocab, cap, keys, ctrs, next));
+    const bool vec = pitch % 4 == 0 && reinterpret_cast<uintptr_t>(logits) % 16 == 0;  // (then pitch >= vocab rounded up to fours)
+    JSM_CUDA_CHECK(launch_chained(vec ? logits_finish_kernel<true> : logits_finish_kernel<false>, dim3(slices, rows), dim3(256), 0, st, logits, pitch, vocab, cap, keys, ctrs, next, err, err_out));
     JSM_LAUNCH_CHECK();
     return JSM_OK;
 }
