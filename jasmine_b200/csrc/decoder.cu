@@ -106,6 +106,8 @@ struct jsm_decoder {
     int* attn_ctrs = nullptr;
     unsigned long long* keys = nullptr;
     int32_t *key_ctrs = nullptr, *next_dev = nullptr, *meta = nullptr, *h_meta = nullptr;
+    // results of a step: next tokens [rows], then the device's error word as every row's last kernel found it [rows]; next_dev and, pinned, h_out
+    int32_t* h_out = nullptr;
     size_t meta_cap = 0;
     std::map<int, cudaGraphExec_t> graphs;
     float* tap = nullptr;
@@ -662,11 +664,11 @@ static jsm_status run_layers(jsm_decoder* m, const Pass& P, cudaStream_t st) {
     return JSM_OK;
 }
 
-// logits and arg-max of wanted rows [w0, w0 + n) of the pass into the logits buffer
+// logits and arg-max of wanted rows [w0, w0 + n) of the pass into the logits buffer, tokens and error words into next_dev
 static jsm_status run_head(jsm_decoder* m, const Pass& P, int w0, int n, cudaStream_t st) {
     DEC_TRY(final_norm_launch(m->f32, m->x, P.want + w0, m->final_norm, m->c.norm_eps, m->head_in, n, m->c.d_model, m->wp, st));
     DEC_TRY(linear(m, m->head, m->head_in, m->wp, m->logits, true, n, st));
-    return logits_finish_launch(m->logits, m->vp, m->c.vocab, m->c.logit_softcap, n, m->keys, m->key_ctrs, m->next_dev, st);
+    return logits_finish_launch(m->logits, m->vp, m->c.vocab, m->c.logit_softcap, n, m->keys, m->key_ctrs, m->next_dev, st, tc_error_word(), m->next_dev + n);
 }
 
 // first position that a token at `pos` or later can see in any layer
@@ -756,6 +758,7 @@ static jsm_status run_pass(jsm_decoder* m, std::vector<PassSeg> segs, const int3
 
     const int n_head = std::min(P.n_want, m->cap_rows);
     const bool graph = P.decode && !m->tap && (P.n_want == 0 || (P.n_want == E && E <= m->cap_rows));
+    const bool one_copy = P.n_want > 0 && P.n_want <= m->cap_rows;  // one launch finishes all logits: tokens and errors come back together
     if (graph) {
         const int key = 2 * E + (P.n_want ? 1 : 0);
         auto it = m->graphs.find(key);
@@ -784,15 +787,28 @@ static jsm_status run_pass(jsm_decoder* m, std::vector<PassSeg> segs, const int3
             int j = i + 1;
             while (j < n && want[w0 + j].second == want[w0 + j - 1].second + 1) ++j;
             const int out = want[w0 + i].second;
-            if (h_next) JSM_CUDA_CHECK(cudaMemcpyAsync(h_next + out, m->next_dev + i, sizeof(int32_t) * (j - i), cudaMemcpyDeviceToHost, st));
+            if (h_next && !one_copy) JSM_CUDA_CHECK(cudaMemcpyAsync(h_next + out, m->next_dev + i, sizeof(int32_t) * (j - i), cudaMemcpyDeviceToHost, st));
             if (h_logits)
                 JSM_CUDA_CHECK(cudaMemcpy2DAsync(h_logits + (size_t)out * m->c.vocab, sizeof(float) * m->c.vocab, m->logits + (size_t)i * m->vp,
                                                  sizeof(float) * m->vp, sizeof(float) * m->c.vocab, j - i, cudaMemcpyDeviceToHost, st));
             i = j;
         }
     }
-    DEC_TRY(tc_check_error(st, "jsm_decoder_step"));  // synchronises: the metadata buffer is free, the outputs are valid
-    JSM_CUDA_CHECK(cudaStreamSynchronize(st));
+    // the stream is waited for: the metadata buffer is free, the outputs are valid
+    if (one_copy) {
+        // (two copies to pageable memory and a wait for each held a step up by 20 us)
+        JSM_CUDA_CHECK(cudaMemcpyAsync(m->h_out, m->next_dev, 2 * sizeof(int32_t) * P.n_want, cudaMemcpyDeviceToHost, st));
+        JSM_CUDA_CHECK(cudaStreamSynchronize(st));
+        bool failed = false;
+        for (int i = 0; i < P.n_want; ++i) {
+            if (h_next) h_next[want[i].second] = m->h_out[i];
+            failed |= m->h_out[P.n_want + i] != 0;
+        }
+        if (failed) DEC_TRY(tc_check_error(st, "jsm_decoder_step"));
+    } else {
+        DEC_TRY(tc_check_error(st, "jsm_decoder_step"));
+        JSM_CUDA_CHECK(cudaStreamSynchronize(st));
+    }
     for (const PassSeg& s : segs) {
         m->rows.h_ctx[s.row] = s.pos0 + s.len;
         if (m->has_attention) m->rows.release_before(s.row, first_needed(m, s.pos0 + s.len));
@@ -885,6 +901,7 @@ jsm_status jsm_decoder_destroy(jsm_decoder* m) {
     for (auto& g : m->graphs) cudaGraphExecDestroy(g.second);
     for (void* p : m->allocs) cudaFree(p);
     if (m->h_meta) cudaFreeHost(m->h_meta);
+    if (m->h_out) cudaFreeHost(m->h_out);
     if (m->own_stream) cudaStreamDestroy(m->own_stream);
     delete m;
     return JSM_OK;
@@ -1049,7 +1066,7 @@ jsm_status jsm_decoder_finalize(jsm_decoder* m) {
     DEC_TRY(dalloc(m, &m->logits, 4 * (size_t)m->cap_rows * m->vp));
     DEC_TRY(dalloc(m, &m->keys, 8 * (size_t)m->cap_rows));
     DEC_TRY(dalloc(m, &m->key_ctrs, 4 * (size_t)m->cap_rows));
-    DEC_TRY(dalloc(m, &m->next_dev, 4 * (size_t)m->cap_rows));
+    DEC_TRY(dalloc(m, &m->next_dev, 2 * 4 * (size_t)m->cap_rows));
     DEC_TRY(dalloc(m, &m->ws, 4 * m->ws_floats));
     DEC_TRY(dalloc(m, &m->counters, 4 * (size_t)m->n_counters));
     std::map<std::pair<int, int>, int> tilings;
@@ -1064,6 +1081,7 @@ jsm_status jsm_decoder_finalize(jsm_decoder* m) {
     for (auto& t : tilings) m->meta_cap += 2 * (T * t.first.first / t.first.second + T + 1);
     DEC_TRY(dalloc(m, &m->meta, 4 * m->meta_cap));
     JSM_CUDA_CHECK(cudaMallocHost(reinterpret_cast<void**>(&m->h_meta), 4 * m->meta_cap));
+    JSM_CUDA_CHECK(cudaMallocHost(reinterpret_cast<void**>(&m->h_out), 2 * 4 * (size_t)m->cap_rows));
     tc_error_word();  // first use allocates the device's error word: here, not inside a captured step
     // bytes of weights one decode step streams (a shared layer streams them again)
     auto pb = [&](const Proj& p) { return (uint64_t)(p.paired ? 2 : 1) * p.N * p.K * es; };
