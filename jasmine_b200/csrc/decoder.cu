@@ -538,13 +538,15 @@ static jsm_status latent_mixer(jsm_decoder* m, DecLayer& L, const Pass& P, cudaS
     DEC_TRY(linear(m, L.qd, xin, m->wp, m->wide, true, T, st));
     const bool flash = L.expand.packed != nullptr && P.n_flash > 0;
     const TileList& tl = (flash ? P.tiles_short : P.tiles_all).at(L.tiling(P.decode));
-    DEC_TRY(latent_prep_launch(m->f32, m->wide, d, L.lw, m->c.norm_eps, L.cache, P.tk, m->q, tl.n > 0 ? m->q_lat : nullptr, st));
+    const bool latent_only = !m->f32 && !flash && latent_query_usable(d);
+    if (latent_only) DEC_TRY(latent_query_launch(m->wide, d, L.lw, m->c.norm_eps, L.cache, P.tk, m->q_lat, st));
+    else DEC_TRY(latent_prep_launch(m->f32, m->wide, d, L.lw, m->c.norm_eps, L.cache, P.tk, m->q, tl.n > 0 ? m->q_lat : nullptr, st));
     if (tl.n > 0) {
         LatentTiles t;
         t.tile_seg = P.meta + tl.seg_off; t.tile_r0 = P.meta + tl.r0_off; t.n_tiles = tl.n; t.t_first = 0; t.t_count = tl.tokens;
         t.max_keys = std::min(d.window, m->c.max_context);
         LatentScratch sc{m->q_lat, m->o_lat, m->part, m->part_floats};
-        DEC_TRY(latent_attn_launch(m->f32, d, L.lw, L.cache, P.tk, t, m->q, sc, m->att, st));
+        DEC_TRY(latent_attn_launch(m->f32, d, L.lw, L.cache, P.tk, t, latent_only ? nullptr : m->q, sc, m->att, st));
     }
     if (flash) {
         for (size_t i = P.segs.size() - P.n_flash; i < P.segs.size(); ++i) {

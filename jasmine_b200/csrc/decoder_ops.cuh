@@ -55,7 +55,11 @@ struct LatentCache {
 // (act [T][H][cr], behind their rank columns; may be null).
 jsm_status latent_prep_launch(bool f32, const float* qd, const LatentDims& d, const LatentWeights& w, float eps, const LatentCache& cache,
                               const StepTokens& tk, void* q, void* q_lat, cudaStream_t st);
-// Attention in the latent space for the tokens listed in tiles: queries are taken into the latent space (the rank columns of q_lat), scored
+// The same for passes whose queries are only needed in the latent space (bf16): cache entries, and whole latent queries
+bool latent_query_usable(const LatentDims& d);
+jsm_status latent_query_launch(const float* qd, const LatentDims& d, const LatentWeights& w, float eps, const LatentCache& cache, const StepTokens& tk,
+                               void* q_lat, cudaStream_t st);
+// Attention in the latent space for the tokens listed in tiles: queries (null: q_lat is complete) are taken into the latent space (the rank columns of q_lat), scored
 // against the cache, and the weighted latents (o_lat) expanded to values: out act [T][out_cols].
 struct LatentScratch {
     void* q_lat;             // act [T][H][cr]

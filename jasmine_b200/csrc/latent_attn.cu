@@ -43,6 +43,37 @@ __device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
+// The cache entry of one token, by 256 threads: the latent's RMS norm and the rotated key part.
+__device__ __forceinline__ long long cache_offset(const int32_t* block_table, int max_pages, int row, int pos, int cr) {
+    return ((long long)load_early(block_table + (long long)row * max_pages + pos / PAGE) * PAGE + pos % PAGE) * cr;
+}
+template <typename T>
+__device__ __forceinline__ void latent_entry(const float* down, const LatentDims& d, const float* __restrict__ gain, float eps, T* dst,
+                                             const float2* __restrict__ cs, float* red) {
+    const int cr = pad8(d.rank + d.rot), half = d.rot / 2;
+    float ss = 0.0f;
+    for (int i = threadIdx.x; i < d.rank; i += 256) ss += down[i] * down[i];
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    ss = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) ss += red[w];
+    const float rms = sqrtf(ss / (float)d.rank + eps);
+    for (int i = threadIdx.x; i < cr; i += 256) {
+        float v = 0.0f;
+        if (i < d.rank) {
+            v = down[i] / rms * gain[i];
+        } else if (i < d.rank + d.rot) {
+            const int r = i - d.rank, p = r < half ? r : r - half;
+            const float2 e = cs[p];
+            const float a = down[d.rank + p], b = down[d.rank + p + half];
+            v = r < half ? a * e.x - b * e.y : b * e.x + a * e.y;
+        }
+        dst[i] = from_f32<T>(v);
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) latent_prep_kernel(const float* __restrict__ qd, LatentDims d, const float* __restrict__ gain, float eps,
                                                           T* __restrict__ pool, const int32_t* __restrict__ block_table, int max_pages,
@@ -105,31 +136,7 @@ __global__ void __launch_bounds__(256) latent_prep_kernel(const float* __restric
         }
         return;
     }
-    // latent: RMS norm, then the cache entry
-    const float* down = src + q_cols;
-    float ss = 0.0f;
-    for (int i = threadIdx.x; i < d.rank; i += 256) ss += down[i] * down[i];
-    ss = warp_sum(ss);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
-    __syncthreads();
-    ss = 0.0f;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) ss += red[w];
-    const float rms = sqrtf(ss / (float)d.rank + eps);
-    const int page = block_table[(long long)tok_row[t] * max_pages + pos / PAGE];
-    T* dst = pool + ((long long)page * PAGE + pos % PAGE) * cr;
-    for (int i = threadIdx.x; i < cr; i += 256) {
-        float v = 0.0f;
-        if (i < d.rank) {
-            v = down[i] / rms * gain[i];
-        } else if (i < d.rank + d.rot) {
-            const int r = i - d.rank, p = r < half ? r : r - half;
-            const float2 e = cs[p];
-            const float a = down[d.rank + p], b = down[d.rank + p + half];
-            v = r < half ? a * e.x - b * e.y : b * e.x + a * e.y;
-        }
-        dst[i] = from_f32<T>(v);
-    }
+    latent_entry(src + q_cols, d, gain, eps, pool + cache_offset(block_table, max_pages, tok_row[t], pos, cr), cs, red);
 }
 
 // ---- per-head projections -----------------------------------------------------------------------------------------
@@ -162,34 +169,30 @@ __global__ void __launch_bounds__(256) latent_project_simt_kernel(ProjectArgs a)
 // rows.  A lane's eight consecutive k of a 32-wide block feed two k16 products - both operands in the same order, so every
 // fragment is one 16-byte load straight from global memory.  Four warps per CTA: 16 output rows each, or (KSPLIT) the same
 // 16 rows and a quarter of k each, added in warp order; up to 32 tokens.
-template <bool KSPLIT>
-__global__ void __launch_bounds__(128) latent_project_mma_kernel(ProjectArgs a) {
-    __shared__ float fold[KSPLIT ? 3 * 16 * 32 : 1];
-    chain_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y;
-    const int n0 = KSPLIT ? blockIdx.x * 16 : blockIdx.x * 64 + warp * 16;
-    const int g = lane >> 2, kq = (lane & 3) * 8;
-    const int t_begin = a.t0 + blockIdx.z * 32, t_end = min(a.t0 + a.T, t_begin + 32);
-    const int n_blk = a.kw / 32;
-    const int b0 = KSPLIT ? n_blk * warp / 4 : 0, b1 = KSPLIT ? n_blk * (warp + 1) / 4 : n_blk;
-    const bool on = n0 < a.N;
-    const __nv_bfloat16* w0 = static_cast<const __nv_bfloat16*>(a.W) + ((long long)h * a.nw + (on ? n0 : 0) + g) * a.kw + kq;
-    const __nv_bfloat16* w1 = w0 + 8 * a.kw;
-    // the weights are constant: the first blocks are requested before the predecessor kernel has finished
-    constexpr int PRE = 4;
+//
+// One warp's part: rows n0 .. n0 + 15 of head h over the blocks [b0, b1) of 32 k.  fetch(t, k): components k .. k + 7 of token t as bf16.
+struct ProjectWarp {
+    static constexpr int PRE = 4;
+    const __nv_bfloat16 *w0, *w1;
     uint4 px[PRE], py[PRE];
+    int b0, b1;
+    // the weights are constant: the first blocks are requested before the predecessor kernel has finished
+    __device__ __forceinline__ ProjectWarp(const ProjectArgs& a, int h, int n0, int b0, int b1, bool on) : b0(b0), b1(on ? b1 : b0) {
+        const int lane = threadIdx.x & 31;
+        w0 = static_cast<const __nv_bfloat16*>(a.W) + ((long long)h * a.nw + (on ? n0 : 0) + (lane >> 2)) * a.kw + (lane & 3) * 8;
+        w1 = w0 + 8 * a.kw;
 #pragma unroll
-    for (int i = 0; i < PRE; ++i)
-        if (on && b0 + i < b1) {
-            px[i] = __ldg(reinterpret_cast<const uint4*>(w0 + (b0 + i) * 32));
-            py[i] = __ldg(reinterpret_cast<const uint4*>(w1 + (b0 + i) * 32));
-        }
-    chain_wait();
-    float acc[4][4];
+        for (int i = 0; i < PRE; ++i)
+            if (b0 + i < this->b1) {
+                px[i] = __ldg(reinterpret_cast<const uint4*>(w0 + (b0 + i) * 32));
+                py[i] = __ldg(reinterpret_cast<const uint4*>(w1 + (b0 + i) * 32));
+            }
+    }
+    template <typename Fetch>
+    __device__ __forceinline__ void run(const ProjectArgs& a, int t_begin, int t_end, float (&acc)[4][4], Fetch fetch) const {
+        const int lane = threadIdx.x & 31, g = lane >> 2, kq = (lane & 3) * 8;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
-    if (on) {
-        const __nv_bfloat16* in = static_cast<const __nv_bfloat16*>(a.in) + h * a.in_hs + kq;
+        for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
         auto block = [&](int k, const uint4& x, const uint4& y) {
             const uint32_t a0[4] = {x.x, y.x, x.y, y.y}, a1[4] = {x.z, y.z, x.w, y.w};
             const bool k_in = k + kq < a.K;  // the operand's pitch covers K rounded up to 8; weights beyond K are zero
@@ -198,7 +201,7 @@ __global__ void __launch_bounds__(128) latent_project_mma_kernel(ProjectArgs a) 
                 if (t_begin + j * 8 >= t_end) break;
                 const int t = t_begin + j * 8 + g;
                 uint4 b = make_uint4(0, 0, 0, 0);
-                if (k_in && t < t_end) b = *reinterpret_cast<const uint4*>(in + t * a.in_ts + k);
+                if (k_in && t < t_end) b = fetch(t, k + kq);
                 mma_16816(acc[j], a0, b.x, b.y);
                 mma_16816(acc[j], a1, b.z, b.w);
             }
@@ -210,22 +213,8 @@ __global__ void __launch_bounds__(128) latent_project_mma_kernel(ProjectArgs a) 
         for (int i = b0 + PRE; i < b1; ++i)
             block(i * 32, __ldg(reinterpret_cast<const uint4*>(w0 + i * 32)), __ldg(reinterpret_cast<const uint4*>(w1 + i * 32)));
     }
-    if constexpr (KSPLIT) {
-        if (warp > 0)
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) fold[((warp - 1) * 16 + j * 4 + e) * 32 + lane] = acc[j][e];
-        __syncthreads();
-        if (warp == 0)
-#pragma unroll
-            for (int w = 0; w < 3; ++w)
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[j][e] += fold[(w * 16 + j * 4 + e) * 32 + lane];
-    }
-    if (on && (!KSPLIT || warp == 0)) {
+    __device__ __forceinline__ static void store(const ProjectArgs& a, int h, int n0, int t_begin, int t_end, const float (&acc)[4][4]) {
+        const int lane = threadIdx.x & 31, g = lane >> 2;
         __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out) + h * a.out_hs;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
@@ -235,6 +224,95 @@ __global__ void __launch_bounds__(128) latent_project_mma_kernel(ProjectArgs a) 
                 if (t < t_end && n < a.N) out[t * a.out_ts + n] = __float2bfloat16_rn(acc[j][e]);
             }
     }
+};
+// sums of the four warps of a CTA in warp order, left with warp 0
+__device__ __forceinline__ void fold_warps(float (&acc)[4][4], float* fold) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp > 0)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) fold[((warp - 1) * 16 + j * 4 + e) * 32 + lane] = acc[j][e];
+    __syncthreads();
+    if (warp == 0)
+#pragma unroll
+        for (int w = 0; w < 3; ++w)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[j][e] += fold[(w * 16 + j * 4 + e) * 32 + lane];
+}
+
+template <bool KSPLIT>
+__global__ void __launch_bounds__(128) latent_project_mma_kernel(ProjectArgs a) {
+    __shared__ float fold[KSPLIT ? 3 * 16 * 32 : 1];
+    chain_trigger();
+    const int warp = threadIdx.x >> 5, h = blockIdx.y;
+    const int n0 = KSPLIT ? blockIdx.x * 16 : blockIdx.x * 64 + warp * 16;
+    const int t_begin = a.t0 + blockIdx.z * 32, t_end = min(a.t0 + a.T, t_begin + 32);
+    const int n_blk = a.kw / 32;
+    const bool on = n0 < a.N;
+    const ProjectWarp w(a, h, n0, KSPLIT ? n_blk * warp / 4 : 0, KSPLIT ? n_blk * (warp + 1) / 4 : n_blk, on);
+    chain_wait();
+    float acc[4][4];
+    const __nv_bfloat16* in = static_cast<const __nv_bfloat16*>(a.in) + h * a.in_hs;
+    w.run(a, t_begin, t_end, acc, [&](int t, int k) { return *reinterpret_cast<const uint4*>(in + t * a.in_ts + k); });
+    if constexpr (KSPLIT) fold_warps(acc, fold);
+    if (on && (!KSPLIT || warp == 0)) ProjectWarp::store(a, h, n0, t_begin, t_end, acc);
+}
+
+// What stands between the fused projection and the attention, for queries that are only needed in the latent space (no long portion in the
+// pass): the first CTAs take the unrotated query components, straight from the fp32 projection (rounded to bf16 as the stored
+// queries were), into the latent space; the others append the cache entries and rotate the rest of the queries.  Apart, the projection
+// waited for the rotation although it reads none of it: two launches of 4.3 and 3.9 us in a step of eight sequences.
+__global__ void __launch_bounds__(256) latent_query_kernel(const float* qd, LatentDims d, const float* __restrict__ gain, float eps,
+                                                           __nv_bfloat16* pool, const int32_t* __restrict__ block_table, int max_pages,
+                                                           const float2* __restrict__ rope, const int32_t* __restrict__ tok_row,
+                                                           const int32_t* __restrict__ tok_pos, __nv_bfloat16* q_lat, ProjectArgs a,
+                                                           int row_blocks, int n_project, int parts) {
+    __shared__ float red[8];
+    chain_trigger();
+    const int qh = pad8(d.dim + d.rot), cr = pad8(d.rank + d.rot), q_cols = d.H * qh, half = d.rot / 2;
+    const long long pitch = q_cols + cr;
+    if ((int)blockIdx.x < n_project) {
+        const int nb = blockIdx.x % row_blocks, h = blockIdx.x / row_blocks % d.H, z = blockIdx.x / (row_blocks * d.H);
+        const int n0 = nb * 128 + (threadIdx.x >> 5) * 16, t_begin = a.t0 + z * 32, t_end = min(a.t0 + a.T, t_begin + 32);
+        const bool on = n0 < a.N;
+        const ProjectWarp w(a, h, n0, 0, a.kw / 32, on);
+        chain_wait();
+        float acc[4][4];
+        const float* in = qd + h * qh;
+        w.run(a, t_begin, t_end, acc, [&](int t, int k) {
+            float v[8];
+            load8(in + t * pitch + k, v);
+            return make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+        });
+        if (on) ProjectWarp::store(a, h, n0, t_begin, t_end, acc);
+        return;
+    }
+    const int t = (blockIdx.x - n_project) / parts, part = (blockIdx.x - n_project) % parts;
+    const int pos = load_early(tok_pos + t);
+    const float2* cs = rope + (long long)pos * half;
+    const float* src = qd + t * pitch;
+    if (part + 1 == parts) {
+        __nv_bfloat16* dst = pool + cache_offset(block_table, max_pages, load_early(tok_row + t), pos, cr);
+        chain_wait();
+        latent_entry(src + q_cols, d, gain, eps, dst, cs, red);
+        return;
+    }
+    const int i = part * 256 + threadIdx.x, per_head = d.rot / 8;
+    if (i >= d.H * per_head) return;
+    const int h = i / per_head, r = i % per_head * 8, p = r < half ? r : r - half;
+    float v[8], o[8], c[16];
+    load8(reinterpret_cast<const float*>(cs + p), reinterpret_cast<float(&)[8]>(c[0]));
+    load8(reinterpret_cast<const float*>(cs + p + 4), reinterpret_cast<float(&)[8]>(c[8]));
+    chain_wait();
+    const float* q = src + h * qh + d.dim + r;
+    load8(q, v);
+    load8(r < half ? q + half : q - half, o);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = r < half ? v[e] * c[2 * e] - o[e] * c[2 * e + 1] : v[e] * c[2 * e] + o[e] * c[2 * e + 1];
+    store8(q_lat + ((long long)t * d.H + h) * cr + d.rank + r, v);
 }
 
 static jsm_status project(bool f32, const ProjectArgs& a, int H, cudaStream_t st) {
@@ -359,10 +437,9 @@ __global__ void __launch_bounds__(256, 1) latent_attn_mma_kernel(const __nv_bflo
         for (int i = threadIdx.x; i < 2 * PAGE * (cr16 - cr); i += 256) kv[(i / (cr16 - cr)) * pitch + cr + i % (cr16 - cr)] = __float2bfloat16_rn(0.0f);
     if (threadIdx.x < LA_ROWS) { row_m[threadIdx.x] = -INFINITY; row_l[threadIdx.x] = 0.0f; }
     __syncthreads();
-    chain_wait();
     const int tile = blockIdx.x, sp = blockIdx.y;
-    const int seg = tile_seg[tile], r0 = tile_r0[tile];
-    const int start = seg_start[seg], len = seg_len[seg], pos0 = seg_pos0[seg];
+    const int seg = load_early(tile_seg + tile), r0 = load_early(tile_r0 + tile);
+    const int start = load_early(seg_start + seg), len = load_early(seg_len + seg), pos0 = load_early(seg_pos0 + seg);
     const int n_rows = min(LA_ROWS, len * d.H - r0);
     const int p_first = pos0 + r0 / d.H, p_last = pos0 + (r0 + n_rows - 1) / d.H;
     const int key_lo = max(0, p_first - d.window + 1), key_hi = p_last + 1;
@@ -370,22 +447,26 @@ __global__ void __launch_bounds__(256, 1) latent_attn_mma_kernel(const __nv_bflo
     const int live = min(splits, n_pg);  // the grid is made for the longest context: the splits behind the pages of this one rest
     if (sp >= live) return;
     const int pb = pg_lo + n_pg * sp / live, pe = pg_lo + n_pg * (sp + 1) / live;
-    const int32_t* bt = block_table + (long long)seg_row[seg] * max_pages;
+    const int32_t* bt = block_table + (long long)load_early(seg_row + seg) * max_pages;
     const int vec = cr / 8;  // 16-byte vectors per entry
     // A row per copy, issued by the first eight lanes of every warp (a thread's copies go out one after the other, and one
     // warp would hold up the others).  A copy that lands before the expected bytes are announced cannot complete the phase:
     // the announcement is also its only arrival.
-    auto load_page = [&](int pg, int stage) {
-        const int lo = max(key_lo - pg * PAGE, 0), hi = min(key_hi - pg * PAGE, PAGE);
-        if (threadIdx.x == 0) tc::mbar_expect_tx(&full[stage], (uint32_t)(hi - lo) * cr * 2);
+    // part 1: the entries that earlier passes appended, 2: this pass's, 3: all
+    auto load_page = [&](int pg, int stage, int part) {
+        const int lo = max(key_lo - pg * PAGE, 0), hi = min(key_hi - pg * PAGE, PAGE), old = pos0 - pg * PAGE;
+        if (threadIdx.x == 0 && (part & 1)) tc::mbar_expect_tx(&full[stage], (uint32_t)(hi - lo) * cr * 2);
         const int r = warp * 8 + lane;
-        if (lane < 8 && r >= lo && r < hi)
+        if (lane < 8 && r >= lo && r < hi && (part & (r < old ? 1 : 2)))
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                              smem_u32(kv + (stage * PAGE + r) * pitch)),
-                         "l"(reinterpret_cast<uint64_t>(pool + ((long long)bt[pg] * PAGE + r) * cr)), "r"(cr * 2), "r"(smem_u32(&full[stage]))
+                         "l"(reinterpret_cast<uint64_t>(pool + ((long long)load_early(bt + pg) * PAGE + r) * cr)), "r"(cr * 2), "r"(smem_u32(&full[stage]))
                          : "memory");
     };
-    load_page(pb, 0);
+    // The tile's place and the older entries of its first page were there before the pass began: both round trips lie behind the predecessors.
+    load_page(pb, 0, 1);
+    chain_wait();
+    load_page(pb, 0, 2);
     // the queries pass through the second stage into registers
     for (int i = threadIdx.x; i < LA_ROWS * vec; i += 256) {
         const int r = i / vec, c = i - r * vec, g = r0 + r;
@@ -415,7 +496,7 @@ __global__ void __launch_bounds__(256, 1) latent_attn_mma_kernel(const __nv_bflo
     bool ok = true;
     for (int pg = pb; pg < pe; ++pg) {
         const int i = pg - pb, stage = i & 1;
-        if (pg + 1 < pe) load_page(pg + 1, stage ^ 1);
+        if (pg + 1 < pe) load_page(pg + 1, stage ^ 1, 3);
         __nv_bfloat16* kvs = kv + stage * PAGE * pitch;
         {   // entries outside the tile's key range are not fetched: their rows are zero (a weight of 0 must meet a number)
             const int lo = max(key_lo - pg * PAGE, 0), hi = min(key_hi - pg * PAGE, PAGE);
@@ -621,6 +702,92 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(const float* __rest
     }
 }
 
+// Decode steps of few tokens: the merge inside the projection to values.  A CTA has 16 rows of one head; its four warps share the rank.  A
+// lane weighs the splits of its token and adds its own components of them while the operand forms (the same sums as in
+// latent_combine_kernel, rounded to bf16 as the stored latents were); four splits of all its components are requested at once, so that
+// a short context costs one round trip.  Eight CTAs read a head's partial sums: with many tokens a merge of its own is cheaper.
+constexpr int LV_MAX_TOKENS = 16, LV_BLOCKS = 4;
+__global__ void __launch_bounds__(128) latent_value_kernel(ProjectArgs a, const float* part, LatentDims d, const int32_t* __restrict__ tok_pos,
+                                                           int max_splits) {
+    __shared__ float fold[3 * 16 * 32];
+    chain_trigger();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y, n0 = blockIdx.x * 16, n_blk = a.kw / 32;
+    const int g = lane >> 2, kq = (lane & 3) * 8, b0 = n_blk * warp / 4, b1 = n_blk * (warp + 1) / 4;
+    const bool on = n0 < a.N;
+    const __nv_bfloat16* w = static_cast<const __nv_bfloat16*>(a.W) + ((long long)h * a.nw + (on ? n0 : 0) + g) * a.kw + kq;
+    uint4 wx[LV_BLOCKS], wy[LV_BLOCKS];
+#pragma unroll
+    for (int i = 0; i < LV_BLOCKS; ++i)
+        if (b0 + i < b1) {
+            wx[i] = __ldg(reinterpret_cast<const uint4*>(w + (b0 + i) * 32));
+            wy[i] = __ldg(reinterpret_cast<const uint4*>(w + 8 * a.kw + (b0 + i) * 32));
+        }
+    const int rp = pad8(d.rank), tiles = (d.H + LA_ROWS - 1) / LA_ROWS;  // (per token)
+    const long long stride = (long long)LA_ROWS * (rp + LA_ML);
+    int live[LV_MAX_TOKENS / 8];
+#pragma unroll
+    for (int j = 0; j < LV_MAX_TOKENS / 8; ++j) {
+        const int t = j * 8 + g, pos = t < a.T ? load_early(tok_pos + t) : 0;
+        live[j] = t < a.T ? min(max_splits, pos / PAGE - max(0, pos - d.window + 1) / PAGE + 1) : 0;
+    }
+    chain_wait();
+    float acc[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+#pragma unroll
+    for (int j = 0; j < LV_MAX_TOKENS / 8; ++j) {
+        if (j * 8 >= a.T) break;
+        const int t = min(j * 8 + g, a.T - 1), n = live[j];
+        const float* p = part + ((long long)(t * tiles + h / LA_ROWS) * max_splits * LA_ROWS + h % LA_ROWS) * (rp + LA_ML);
+        float v[LV_BLOCKS][8], m = -INFINITY, l = 0.0f;
+#pragma unroll
+        for (int i = 0; i < LV_BLOCKS; ++i)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[i][e] = 0.0f;
+        for (int s = 4; s < n; ++s) m = fmaxf(m, p[s * stride + rp]);
+        for (int s0 = 0; s0 < n; s0 += 4) {
+            float2 ml[4];
+            float u[4][LV_BLOCKS][8];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float* ps = p + (s0 + q) * stride;
+                ml[q] = s0 + q < n ? *reinterpret_cast<const float2*>(ps + rp) : make_float2(-INFINITY, 0.0f);
+#pragma unroll
+                for (int i = 0; i < LV_BLOCKS; ++i) {
+                    const int k = (b0 + i) * 32 + kq;
+                    if (s0 + q < n && b0 + i < b1 && k < a.K) load8(ps + k, u[q][i]);
+                    else
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) u[q][i][e] = 0.0f;
+                }
+            }
+            if (s0 == 0) m = fmaxf(m, fmaxf(fmaxf(ml[0].x, ml[1].x), fmaxf(ml[2].x, ml[3].x)));
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float f = __expf(ml[q].x - m);
+                l = fmaf(f, ml[q].y, l);
+#pragma unroll
+                for (int i = 0; i < LV_BLOCKS; ++i)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[i][e] = fmaf(f, u[q][i][e], v[i][e]);
+            }
+        }
+        const float inv = 1.0f / l;
+#pragma unroll
+        for (int i = 0; i < LV_BLOCKS; ++i)
+            if (b0 + i < b1) {
+                uint4 b = make_uint4(pack_bf16x2(v[i][0] * inv, v[i][1] * inv), pack_bf16x2(v[i][2] * inv, v[i][3] * inv),
+                                     pack_bf16x2(v[i][4] * inv, v[i][5] * inv), pack_bf16x2(v[i][6] * inv, v[i][7] * inv));
+                if (n == 0) b = make_uint4(0, 0, 0, 0);  // (a column without a token)
+                const uint32_t a0[4] = {wx[i].x, wy[i].x, wx[i].y, wy[i].y}, a1[4] = {wx[i].z, wy[i].z, wx[i].w, wy[i].w};
+                mma_16816(acc[j], a0, b.x, b.y);
+                mma_16816(acc[j], a1, b.z, b.w);
+            }
+    }
+    fold_warps(acc, fold);
+    if (on && warp == 0) ProjectWarp::store(a, h, n0, 0, a.T, acc);
+}
+
 __global__ void __launch_bounds__(256) latent_gather_kernel(const __nv_bfloat16* __restrict__ pool, const int32_t* __restrict__ bt, int p0, int n,
                                                             int vec, uint4* __restrict__ out) {
     chain_trigger();
@@ -656,8 +823,9 @@ bool latent_mma_usable(const LatentDims& d) {
 
 int latent_splits(int n_tiles, int max_keys) {
     if (n_tiles <= 0) return 1;
+    // a split of its own for every page of a short context, two pages each beyond
     const int pages = max_keys / PAGE + 2;
-    return std::max(1, std::min({sm_count() / n_tiles, pages / 2, LA_MAX_SPLITS}));
+    return std::max(1, std::min({sm_count() / n_tiles, std::max(std::min(pages, 4), pages / 2), LA_MAX_SPLITS}));
 }
 size_t latent_part_floats(const LatentDims& d) { return (size_t)sm_count() * LA_ROWS * (pad8(d.rank) + LA_ML); }
 
@@ -673,17 +841,40 @@ static jsm_status launch_mma(const LatentDims& d, const LatentCache& cache, cons
     return JSM_OK;
 }
 
+// queries into the latent space: the rank columns of q_lat
+static ProjectArgs query_project(const LatentDims& d, const LatentWeights& w, const void* q, void* q_lat, int t_first, int t_count) {
+    ProjectArgs a;
+    a.in = q; a.in_ts = d.q_cols(); a.in_hs = d.qh();
+    a.W = w.uk; a.N = d.rank; a.K = d.dim; a.nw = pad_to(d.rank, 16); a.kw = pad_to(d.dim, 32);
+    a.out = q_lat; a.out_ts = (long long)d.H * d.cr(); a.out_hs = d.cr();
+    a.t0 = t_first; a.T = t_count;
+    return a;
+}
+
+bool latent_query_usable(const LatentDims& d) { return latent_mma_usable(d) && d.dim % 8 == 0 && d.rot % 16 == 0 && d.rot > 0 && d.rank % 8 == 0; }
+jsm_status latent_query_launch(const float* qd, const LatentDims& d, const LatentWeights& w, float eps, const LatentCache& cache, const StepTokens& tk,
+                               void* q_lat, cudaStream_t st) {
+    const ProjectArgs a = query_project(d, w, nullptr, q_lat, 0, tk.T);
+    const int row_blocks = (d.rank + 127) / 128, n_project = row_blocks * d.H * ((tk.T + 31) / 32), parts = (d.H * (d.rot / 8) + 255) / 256 + 1;
+    JSM_CUDA_CHECK(launch_chained(latent_query_kernel, dim3(n_project + tk.T * parts), dim3(256), 0, st, qd, d, w.down_norm, eps, (__nv_bfloat16*)cache.pool,
+                                  cache.block_table, cache.max_pages, cache.rope, tk.tok_row, tk.tok_pos, (__nv_bfloat16*)q_lat, a, row_blocks, n_project,
+                                  parts));
+    JSM_LAUNCH_CHECK();
+    return JSM_OK;
+}
+
 jsm_status latent_attn_launch(bool f32, const LatentDims& d, const LatentWeights& w, const LatentCache& cache, const StepTokens& tk,
                               const LatentTiles& tl, const void* q, const LatentScratch& sc, void* out, cudaStream_t st) {
     if (tl.n_tiles <= 0 || tl.t_count <= 0) return JSM_OK;
     const int cr = d.cr(), rp = pad8(d.rank);
-    ProjectArgs a;
-    a.in = q; a.in_ts = d.q_cols(); a.in_hs = d.qh();
-    a.W = w.uk; a.N = d.rank; a.K = d.dim; a.nw = pad_to(d.rank, 16); a.kw = pad_to(d.dim, 32);
-    a.out = sc.q_lat; a.out_ts = (long long)d.H * cr; a.out_hs = cr;
-    a.t0 = tl.t_first; a.T = tl.t_count;
-    jsm_status s = project(f32, a, d.H, st);
+    jsm_status s = q ? project(f32, query_project(d, w, q, sc.q_lat, tl.t_first, tl.t_count), d.H, st) : JSM_OK;
     if (s != JSM_OK) return s;
+    // values: out[t][h * vdim + j] = Wuv[h][j] . o_lat[t][h]
+    ProjectArgs a;
+    a.in = sc.o_lat; a.in_ts = (long long)d.H * rp; a.in_hs = rp;
+    a.W = w.uv; a.N = d.vdim; a.K = d.rank; a.nw = pad_to(d.vdim, 16); a.kw = pad_to(d.rank, 32);
+    a.out = out; a.out_ts = d.out_cols(); a.out_hs = d.vdim;
+    a.t0 = tl.t_first; a.T = tl.t_count;
     if (f32 || !latent_mma_usable(d)) {
         const size_t smem = sizeof(float) * (cr + d.rank + 128 + 8);
         if (smem > 48 * 1024) JSM_FAIL(JSM_UNSUPPORTED, "latent attention: latent of %d + %d components", d.rank, d.rot);
@@ -707,16 +898,17 @@ jsm_status latent_attn_launch(bool f32, const LatentDims& d, const LatentWeights
             default: s = launch_mma<8>(d, cache, tk, tl, sc, splits, st); break;
         }
         if (s != JSM_OK) return s;
+        if (splits > 1 && tk.max_len == 1 && tl.t_first == 0 && tl.t_count <= LV_MAX_TOKENS && d.rank % 8 == 0 && a.kw <= 4 * LV_BLOCKS * 32) {
+            JSM_CUDA_CHECK(launch_chained(latent_value_kernel, dim3((d.vdim + 15) / 16, d.H), dim3(128), 0, st, a, (const float*)sc.part, d, tk.tok_pos, splits));
+            JSM_LAUNCH_CHECK();
+            return JSM_OK;
+        }
         if (splits > 1) {
             JSM_CUDA_CHECK(launch_chained(latent_combine_kernel, dim3(tl.n_tiles, LA_ROWS), dim3(128), 0, st, (const float*)sc.part, d, tk.seg_start,
                                           tk.seg_len, tl.tile_seg, tk.seg_pos0, tl.tile_r0, splits, (__nv_bfloat16*)sc.o_lat));
             JSM_LAUNCH_CHECK();
         }
     }
-    // values: out[t][h * vdim + j] = Wuv[h][j] . o_lat[t][h]
-    a.in = sc.o_lat; a.in_ts = (long long)d.H * rp; a.in_hs = rp;
-    a.W = w.uv; a.N = d.vdim; a.K = d.rank; a.nw = pad_to(d.vdim, 16); a.kw = pad_to(d.rank, 32);
-    a.out = out; a.out_ts = d.out_cols(); a.out_hs = d.vdim;
     return project(f32, a, d.H, st);
 }
 
