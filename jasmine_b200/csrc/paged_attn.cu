@@ -202,108 +202,221 @@ __global__ void __launch_bounds__(128) attn_paged_simt_kernel(const T* __restric
     for (int i = threadIdx.x; i < d.vdim; i += 128) out[(long long)t * d.out_cols() + h * d.vdim + i] = from_f32<T>(o[i] * f);
 }
 
-// The same for portions of prompts: a warp per (token, head of the group) row, eight rows of one kv head per CTA, which share
-// tiles of 32 keys and values in shared memory - the kernel above reads every key once per token and head and waits for it, 32
-// lanes a key.  Here a lane owns a key of the tile (vector loads, an odd number of 16-byte pieces per row: no bank conflicts)
-// and then columns lane, lane + 32, ... of the output.  The next tile is on its way while one is used.
-constexpr int AR_ROWS = 8, AR_KEYS = 32, AR_MAX_SMEM = 160 * 1024;
+// The same for portions of prompts: rows of one kv head share tiles of 32 keys and values in shared memory - the kernel above reads every key
+// once per token and head and waits for it, 32 lanes a key.  Here a lane owns a key of the tile (vector loads, an odd number of 16-byte
+// pieces per row: no bank conflicts) and then four columns of the output (eight where values are wider than 128).  What bounds it
+// is shared memory: a warp takes two rows, so that a key and a value are read once for both (four rows and four warps: too few to hide
+// anything behind, 64 us; 300 tokens, 8 heads of 128, 2 kv heads: 49 -> 35 us).  The next tile is on its way while one is used.
+constexpr int AR_WARPS = 8, AR_EACH = 2, AR_ROWS = AR_WARPS * AR_EACH, AR_KEYS = 32, AR_MAX_SMEM = 224 * 1024;
 __host__ __device__ constexpr int ar_pitch(int n) { return ((n + 3) / 4 | 1) * 4; }
-static size_t ar_smem(const AttnDims& d) { return sizeof(float) * ((size_t)(2 * AR_KEYS + AR_ROWS) * ar_pitch(d.dim) + 2 * AR_KEYS * ar_pitch(d.vdim)); }
-
-template <typename T, int VR>  // VR: output columns per lane
-__global__ void __launch_bounds__(AR_ROWS * 32) attn_paged_rows_kernel(const T* __restrict__ q, AttnDims d, const float* __restrict__ sink, const T* __restrict__ pool,
-                                                                       const int32_t* __restrict__ block_table, int max_pages, StepTokens tk,
-                                                                       const int32_t* __restrict__ tile_seg, const int32_t* __restrict__ tile_r0, int rows,
-                                                                       const float* __restrict__ gate, T* __restrict__ out) {
-    extern __shared__ __align__(16) float ar_sm[];
-    const int kpitch = ar_pitch(d.dim), vpitch = ar_pitch(d.vdim), dim4 = (d.dim + 3) / 4, vdim4 = (d.vdim + 3) / 4;
-    float *K2 = ar_sm, *V2 = K2 + 2 * AR_KEYS * kpitch, *Qs = V2 + 2 * AR_KEYS * vpitch;  // two tiles of keys and values
-    chain_trigger();
-    chain_wait();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = blockIdx.y, gs = d.H / d.G;
-    const int seg = tile_seg[blockIdx.x], rb = tile_r0[blockIdx.x] + blockIdx.z * AR_ROWS;
-    const int n_rows = min(min(AR_ROWS, rows - (int)blockIdx.z * AR_ROWS), tk.seg_len[seg] * gs - rb);
-    if (n_rows <= 0) return;
-    const int pos0 = tk.seg_pos0[seg], r = rb + min(warp, n_rows - 1), h = g * gs + r % gs, pos = pos0 + r / gs;  // (a warp without a row repeats the last one)
-    const long long t = tk.seg_start[seg] + r / gs;
-    const int32_t* bt = block_table + (long long)tk.seg_row[seg] * max_pages;
-    float* qrow = Qs + warp * kpitch;
-    for (int i = lane; i < dim4 * 4; i += 32) qrow[i] = i < d.dim ? to_f32(q[t * d.q_cols() + h * d.qh() + i]) : 0.0f;
-    const int first = d.mask.first(pos), lo = d.mask.first(pos0 + rb / gs), hi = pos0 + (rb + n_rows - 1) / gs;
-    float m = sink ? sink[h] : -INFINITY, l = sink ? 1.0f : 0.0f, o[VR];
-#pragma unroll
-    for (int i = 0; i < VR; ++i) o[i] = 0.0f;
-    auto stage = [&](int c0, int buf) {
-        for (int e = threadIdx.x; e < AR_KEYS * (dim4 + vdim4); e += AR_ROWS * 32) {
-            const int j = e / (dim4 + vdim4), x = e % (dim4 + vdim4), key = c0 + j;
-            const bool value = x >= dim4, on = key <= hi;
-            const int c = (value ? x - dim4 : x) * 4;
-            const T* src = on ? cache_at(const_cast<T*>(pool), d, bt[key / PAGE], g, value ? 1 : 0, key % PAGE, c) : pool;
-            float* dst = (value ? V2 + (buf * AR_KEYS + j) * vpitch : K2 + (buf * AR_KEYS + j) * kpitch) + c;
-            if constexpr (sizeof(T) == 4) {
-                cp_async16(smem_u32(dst), src, on);
-            } else {
-                const uint2 w = on ? *reinterpret_cast<const uint2*>(src) : make_uint2(0u, 0u);
-                *reinterpret_cast<float4*>(dst) = make_float4(bf16lo(w.x), bf16hi(w.x), bf16lo(w.y), bf16hi(w.y));
-            }
-        }
-    };
-    stage(lo, 0);
-    cp_async_commit();
-    for (int c0 = lo, buf = 0; c0 <= hi; c0 += AR_KEYS, buf ^= 1) {
-        if (c0 + AR_KEYS <= hi) stage(c0 + AR_KEYS, buf ^ 1);
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        const float *Ks = K2 + buf * AR_KEYS * kpitch, *Vs = V2 + buf * AR_KEYS * vpitch;
-        float a0 = 0.0f, a1 = 0.0f;
-        for (int i = 0; i < dim4; ++i) {
-            const float4 x = *reinterpret_cast<const float4*>(qrow + 4 * i), y = *reinterpret_cast<const float4*>(Ks + lane * kpitch + 4 * i);
-            a0 = fmaf(x.x, y.x, a0); a1 = fmaf(x.y, y.y, a1);
-            a0 = fmaf(x.z, y.z, a0); a1 = fmaf(x.w, y.w, a1);
-        }
-        const int key = c0 + lane;
-        const float s = key >= first && key <= pos ? (a0 + a1) * d.scale : -INFINITY;
-        const float m_new = fmaxf(m, warp_max(s));
-        // (else no key of this row has weight yet: the whole warp agrees; the maximum passes over NaN, which has to reach the sums)
-        if (!(m_new == -INFINITY) || __any_sync(0xffffffffu, s != s)) {
-            const float p = expf(s - m_new), alpha = expf(m - m_new);
-            l = l * alpha + warp_sum(p);
-            m = m_new;
-#pragma unroll
-            for (int i = 0; i < VR; ++i) o[i] *= alpha;
-            const int j_end = min(AR_KEYS, pos + 1 - c0);  // (a value that the row does not see may be anything)
-#pragma unroll 4
-            for (int j = max(0, first - c0); j < j_end; ++j) {
-                const float pj = __shfl_sync(0xffffffffu, p, j);
-#pragma unroll
-                for (int i = 0; i < VR; ++i)
-                    if (lane + 32 * i < d.vdim) o[i] = fmaf(pj, Vs[j * vpitch + lane + 32 * i], o[i]);
-            }
-        }
-        __syncthreads();  // the tile is used up
-    }
-    if (warp >= n_rows) return;
-    const float f = (gate ? gate[t * d.H + h] : 1.0f) / l;
-#pragma unroll
-    for (int i = 0; i < VR; ++i)
-        if (lane + 32 * i < d.vdim) out[t * d.out_cols() + h * d.vdim + lane + 32 * i] = from_f32<T>(o[i] * f);
+static size_t ar_smem(const AttnDims& d, int parts) {
+    return sizeof(float) * (parts * 2 * AR_KEYS * ((size_t)ar_pitch(d.dim) + ar_pitch(d.vdim)) + AR_ROWS * (size_t)ar_pitch(d.dim) +
+                            parts * AR_WARPS * AR_KEYS * AR_EACH);
 }
 
-template <typename T, int VR>
+template <typename T, int VR, int PARTS>  // VR: output columns per lane; PARTS: groups of warps, each with every PARTS-th tile of keys
+__global__ void __launch_bounds__(AR_WARPS * PARTS * 32, 1) attn_paged_rows_kernel(const T* __restrict__ q, AttnDims d, const float* __restrict__ sink, const T* __restrict__ pool,
+                                                                        const int32_t* __restrict__ block_table, int max_pages, StepTokens tk,
+                                                                        const int32_t* __restrict__ tile_seg, const int32_t* __restrict__ tile_r0, int rows,
+                                                                        const float* __restrict__ gate, T* __restrict__ out) {
+    constexpr int R = AR_EACH;
+    extern __shared__ __align__(16) float ar_sm[];
+    const int kpitch = ar_pitch(d.dim), vpitch = ar_pitch(d.vdim), dim4 = (d.dim + 3) / 4, vdim4 = (d.vdim + 3) / 4;
+    constexpr int VL = VR * 32 + 4;                                                     // a row's sums on the way between the parts
+    const int part = threadIdx.x / (AR_WARPS * 32), tid = threadIdx.x % (AR_WARPS * 32);
+    float* tiles = ar_sm + part * 2 * AR_KEYS * (kpitch + vpitch);
+    float *K2 = tiles, *V2 = K2 + 2 * AR_KEYS * kpitch, *Qs = ar_sm + PARTS * 2 * AR_KEYS * (kpitch + vpitch);  // two tiles of keys and values
+    chain_trigger();
+    chain_wait();
+    const int warp = tid >> 5, lane = threadIdx.x & 31, g = blockIdx.y, gs = d.H / d.G;
+    float2* weights = reinterpret_cast<float2*>(Qs + AR_ROWS * kpitch) + (part * AR_WARPS + warp) * AR_KEYS;  // of the warp's rows, per key of the tile
+    const int tile = gridDim.x - 1 - blockIdx.x;  // (the rows with the most keys start first: a second wave then has the short ones)
+    const int seg = tile_seg[tile], rb = tile_r0[tile] + blockIdx.z * AR_ROWS;
+    const int n_rows = min(min(AR_ROWS, rows - (int)blockIdx.z * AR_ROWS), tk.seg_len[seg] * gs - rb);
+    if (n_rows <= 0) return;
+    const int pos0 = tk.seg_pos0[seg], start = tk.seg_start[seg];
+    const int32_t* bt = block_table + (long long)tk.seg_row[seg] * max_pages;
+    const int lo = d.mask.first(pos0 + rb / gs) & ~(AR_KEYS - 1), hi = pos0 + (rb + n_rows - 1) / gs;
+    const float* qrows = Qs + warp * R * kpitch;
+    int pos[R], first[R], head[R];
+    float m[R], l[R], o[R][VR];
+#pragma unroll
+    for (int x = 0; x < R; ++x) {
+        const int r = rb + min(warp * R + x, n_rows - 1);  // (places without a row repeat the last one)
+        head[x] = g * gs + r % gs;
+        pos[x] = pos0 + r / gs;
+        first[x] = d.mask.first(pos[x]);
+        const T* src = q + (long long)(start + r / gs) * d.q_cols() + head[x] * d.qh();
+        if (part == 0)
+            for (int i = lane; i < dim4 * 4; i += 32) Qs[(warp * R + x) * kpitch + i] = i < d.dim ? to_f32(src[i]) : 0.0f;
+        m[x] = sink && part == 0 ? sink[head[x]] : -INFINITY;
+        l[x] = sink && part == 0 ? 1.0f : 0.0f;
+#pragma unroll
+        for (int i = 0; i < VR; ++i) o[x][i] = 0.0f;
+    }
+    // Tiles begin at multiples of 32: a tile lies in one page, and a thread's places in it are the same for every tile (a key per eight threads).
+    static_assert(AR_WARPS * 32 == AR_KEYS * 8 && PAGE % AR_KEYS == 0, "eight threads per key");
+    const int kj = tid >> 3, kx = tid & 7;
+    auto stage = [&](int c0, int buf) {
+        const bool on = c0 + kj <= hi;
+        const T* src = pool + (long long)(bt[c0 / PAGE] * d.G + g) * (d.ks() + d.vs()) * SLAB + (c0 % PAGE + kj) * 64;
+        float *kd = K2 + (buf * AR_KEYS + kj) * kpitch, *vd = V2 + (buf * AR_KEYS + kj) * vpitch;
+        auto copy = [&](float* dst, const T* from, int n4) {
+#pragma unroll 4
+            for (int x = kx; x < n4; x += 8) {
+                const int c = x * 4;
+                const T* e = from + (c >> 6) * SLAB + ((((c >> 3) & 7) ^ (kj & 7)) << 3) + (c & 7);
+                if constexpr (sizeof(T) == 4) {
+                    cp_async16(smem_u32(dst + c), on ? e : pool, on);
+                } else {
+                    const uint2 w = on ? *reinterpret_cast<const uint2*>(e) : make_uint2(0u, 0u);
+                    *reinterpret_cast<float4*>(dst + c) = make_float4(bf16lo(w.x), bf16hi(w.x), bf16lo(w.y), bf16hi(w.y));
+                }
+            }
+        };
+        copy(kd, src, dim4);
+        copy(vd, src + d.ks() * SLAB, vdim4);
+    };
+    auto meet = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + part), "n"(AR_WARPS * 32) : "memory"); };
+    constexpr int STEP = PARTS * AR_KEYS;
+    if (lo + part * AR_KEYS <= hi) stage(lo + part * AR_KEYS, 0);
+    cp_async_commit();
+    __syncthreads();  // the queries
+    for (int c0 = lo + part * AR_KEYS, buf = 0; c0 <= hi; c0 += STEP, buf ^= 1) {
+        if (c0 + STEP <= hi) stage(c0 + STEP, buf ^ 1);
+        cp_async_commit();
+        cp_async_wait<1>();
+        meet();
+        const float *Ks = K2 + buf * AR_KEYS * kpitch + lane * kpitch, *Vs = V2 + buf * AR_KEYS * vpitch;
+        float a0[R], a1[R];
+#pragma unroll
+        for (int x = 0; x < R; ++x) a0[x] = a1[x] = 0.0f;
+#pragma unroll 4
+        for (int i = 0; i < dim4; ++i) {
+            const float4 y = *reinterpret_cast<const float4*>(Ks + 4 * i);
+#pragma unroll
+            for (int x = 0; x < R; ++x) {
+                const float4 w = *reinterpret_cast<const float4*>(qrows + x * kpitch + 4 * i);
+                a0[x] = fmaf(w.x, y.x, a0[x]); a1[x] = fmaf(w.y, y.y, a1[x]);
+                a0[x] = fmaf(w.z, y.z, a0[x]); a1[x] = fmaf(w.w, y.w, a1[x]);
+            }
+        }
+        const int key = c0 + lane;
+        float p[R], sc[R], m_new[R], sum[R];
+        int j0[R], j1[R], any0 = AR_KEYS, any1 = 0, all0 = 0, all1 = AR_KEYS;  // keys of the tile that a row, any row, every row sees
+#pragma unroll
+        for (int x = 0; x < R; ++x) m_new[x] = sc[x] = key >= first[x] && key <= pos[x] ? (a0[x] + a1[x]) * d.scale : -INFINITY;
+#pragma unroll
+        for (int i = 16; i > 0; i >>= 1)
+#pragma unroll
+            for (int x = 0; x < R; ++x) m_new[x] = fmaxf(m_new[x], __shfl_xor_sync(0xffffffffu, m_new[x], i));
+        bool weighs[R];
+#pragma unroll
+        for (int x = 0; x < R; ++x) {
+            m_new[x] = fmaxf(m[x], m_new[x]);
+            // (else no key of this row has weight yet: the whole warp agrees; the maximum passes over NaN, which has to reach the sums)
+            weighs[x] = !(m_new[x] == -INFINITY) || __any_sync(0xffffffffu, sc[x] != sc[x]);
+            sum[x] = p[x] = weighs[x] ? expf(sc[x] - m_new[x]) : 0.0f;
+        }
+#pragma unroll
+        for (int i = 16; i > 0; i >>= 1)
+#pragma unroll
+            for (int x = 0; x < R; ++x) sum[x] += __shfl_xor_sync(0xffffffffu, sum[x], i);
+#pragma unroll
+        for (int x = 0; x < R; ++x) {
+            const float alpha = weighs[x] ? expf(m[x] - m_new[x]) : 1.0f;
+            l[x] = l[x] * alpha + sum[x];
+            if (weighs[x]) m[x] = m_new[x];
+#pragma unroll
+            for (int i = 0; i < VR; ++i) o[x][i] *= alpha;
+            // (a value that the row does not see may be anything)
+            j0[x] = max(0, first[x] - c0);
+            j1[x] = weighs[x] ? min(AR_KEYS, pos[x] + 1 - c0) : 0;
+            any0 = min(any0, j0[x]); any1 = max(any1, j1[x]);
+            all0 = max(all0, j0[x]); all1 = min(all1, j1[x]);
+        }
+        weights[lane] = make_float2(p[0], p[1]);
+        __syncwarp();
+        auto add = [&](int j, bool every) {
+            const float2 w = weights[j];
+            const float wx[R] = {w.x, w.y};
+#pragma unroll
+            for (int i = 0; i < VR; i += 4) {
+                const int c = i * 32 + lane * 4;
+                if (c >= vdim4 * 4) continue;
+                const float4 v = *reinterpret_cast<const float4*>(Vs + j * vpitch + c);
+#pragma unroll
+                for (int x = 0; x < R; ++x)
+                    if (every || (j >= j0[x] && j < j1[x])) {
+                        o[x][i] = fmaf(wx[x], v.x, o[x][i]); o[x][i + 1] = fmaf(wx[x], v.y, o[x][i + 1]);
+                        o[x][i + 2] = fmaf(wx[x], v.z, o[x][i + 2]); o[x][i + 3] = fmaf(wx[x], v.w, o[x][i + 3]);
+                    }
+            }
+        };
+        if (all0 >= all1) all0 = all1 = any1;
+#pragma unroll 1
+        for (int j = any0; j < all0; ++j) add(j, false);
+#pragma unroll 4
+        for (int j = all0; j < all1; ++j) add(j, true);
+#pragma unroll 1
+        for (int j = all1; j < any1; ++j) add(j, false);
+        meet();  // the tile is used up
+    }
+    // the second group's sums join the first's
+    if (PARTS > 1) __syncthreads();
+    float* shared = ar_sm + warp * R * VL;
+    if (part == 1) {
+#pragma unroll
+        for (int x = 0; x < R; ++x) {
+#pragma unroll
+            for (int i = 0; i < VR; i += 4) *reinterpret_cast<float4*>(shared + x * VL + i * 32 + lane * 4) = make_float4(o[x][i], o[x][i + 1], o[x][i + 2], o[x][i + 3]);
+            if (lane == 0) { shared[x * VL + VR * 32] = m[x]; shared[x * VL + VR * 32 + 1] = l[x]; }
+        }
+    }
+    if (PARTS > 1) __syncthreads();
+    if (part == 1) return;
+#pragma unroll
+    for (int x = 0; x < R; ++x) {
+        if (warp * R + x >= n_rows) break;
+        if constexpr (PARTS > 1) {
+            const float m1 = shared[x * VL + VR * 32], l1 = shared[x * VL + VR * 32 + 1], top = fmaxf(m[x], m1);
+            // (a half without a weight has sums of zero, or NaN, and no maximum)
+            const float f0 = m[x] == -INFINITY ? 1.0f : expf(m[x] - top), f1 = m1 == -INFINITY ? 1.0f : expf(m1 - top);
+            l[x] = fmaf(l[x], f0, l1 * f1);
+#pragma unroll
+            for (int i = 0; i < VR; i += 4) {
+                const float4 w = *reinterpret_cast<const float4*>(shared + x * VL + i * 32 + lane * 4);
+                o[x][i] = fmaf(o[x][i], f0, w.x * f1); o[x][i + 1] = fmaf(o[x][i + 1], f0, w.y * f1);
+                o[x][i + 2] = fmaf(o[x][i + 2], f0, w.z * f1); o[x][i + 3] = fmaf(o[x][i + 3], f0, w.w * f1);
+            }
+        }
+        const long long t = start + pos[x] - pos0;
+        const float f = (gate ? gate[t * d.H + head[x]] : 1.0f) / l[x];
+#pragma unroll
+        for (int i = 0; i < VR; ++i) {
+            const int c = (i & ~3) * 32 + lane * 4 + (i & 3);
+            if (c < d.vdim) out[t * d.out_cols() + head[x] * d.vdim + c] = from_f32<T>(o[x][i] * f);
+        }
+    }
+}
+
+template <typename T, int VR, int PARTS>
 static jsm_status rows_go(const AttnDims& d, const AttnWeights& w, const AttnCache& cache, const StepTokens& tk, const AttnTiles& tl, const void* q,
                           const float* gates, void* out, cudaStream_t st) {
     static DeviceOnce once;  // per instantiation
-    JSM_CUDA_CHECK(allow_shared(once, attn_paged_rows_kernel<T, VR>, AR_MAX_SMEM));
-    JSM_CUDA_CHECK(launch_spread(attn_paged_rows_kernel<T, VR>, dim3(tl.n_tiles, d.G, (tl.rows + AR_ROWS - 1) / AR_ROWS), dim3(AR_ROWS * 32), ar_smem(d), st,
-                                  (const T*)q, d, w.sink, (const T*)cache.pool, cache.block_table, cache.max_pages, tk, tl.tile_seg, tl.tile_r0, tl.rows, gates, (T*)out));
+    JSM_CUDA_CHECK(allow_shared(once, attn_paged_rows_kernel<T, VR, PARTS>, AR_MAX_SMEM));
+    JSM_CUDA_CHECK(launch_spread(attn_paged_rows_kernel<T, VR, PARTS>, dim3(tl.n_tiles, d.G, (tl.rows + AR_ROWS - 1) / AR_ROWS), dim3(AR_WARPS * PARTS * 32),
+                                 ar_smem(d, PARTS), st, (const T*)q, d, w.sink, (const T*)cache.pool, cache.block_table, cache.max_pages, tk, tl.tile_seg,
+                                 tl.tile_r0, tl.rows, gates, (T*)out));
     JSM_LAUNCH_CHECK();
     return JSM_OK;
 }
 template <typename T>
 static jsm_status rows_sized(const AttnDims& d, const AttnWeights& w, const AttnCache& cache, const StepTokens& tk, const AttnTiles& tl, const void* q,
                              const float* gates, void* out, cudaStream_t st) {
-    return d.vdim <= 128 ? rows_go<T, 4>(d, w, cache, tk, tl, q, gates, out, st) : rows_go<T, 8>(d, w, cache, tk, tl, q, gates, out, st);
+    if (ar_smem(d, 2) > AR_MAX_SMEM)
+        return d.vdim <= 128 ? rows_go<T, 4, 1>(d, w, cache, tk, tl, q, gates, out, st) : rows_go<T, 8, 1>(d, w, cache, tk, tl, q, gates, out, st);
+    return d.vdim <= 128 ? rows_go<T, 4, 2>(d, w, cache, tk, tl, q, gates, out, st) : rows_go<T, 8, 2>(d, w, cache, tk, tl, q, gates, out, st);
 }
 
 // ---- bf16 on the tensor cores -------------------------------------------------------------------------------------
@@ -646,8 +759,8 @@ jsm_status attn_paged_launch(bool f32, const AttnDims& d, const AttnWeights& w, 
     if (tl.n_tiles <= 0 || tl.t_count <= 0) return JSM_OK;
     const float* gates = d.gated ? gate : nullptr;
     if (f32 || !attn_mma_usable(d)) {
-        // rows in groups of eight once they make a CTA for every multiprocessor; a few rows keep a CTA each
-        if (tk.max_len > 1 && d.vdim <= 256 && ar_smem(d) <= AR_MAX_SMEM && (long long)tl.t_count * d.H >= (long long)AR_ROWS * sm_count())
+        // rows in groups once they would make a CTA of eight for every multiprocessor; a few rows keep a CTA each
+        if (tk.max_len > 1 && d.vdim <= 256 && ar_smem(d, 1) <= AR_MAX_SMEM && (long long)tl.t_count * d.H >= 8ll * sm_count())
             return f32 ? rows_sized<float>(d, w, cache, tk, tl, q, gates, out, st) : rows_sized<__nv_bfloat16>(d, w, cache, tk, tl, q, gates, out, st);
         const size_t smem = sizeof(float) * (pad8(d.dim) + pad8(d.vdim) + 128 + 8);
         if (smem > 48 * 1024) JSM_FAIL(JSM_UNSUPPORTED, "attention: heads of %d / %d components", d.dim, d.vdim);
