@@ -29,6 +29,9 @@ namespace jsm {
 
 int* tc_error_word();
 jsm_status dot_f32_launch(const jsm_mat& A, const jsm_mat& B, const jsm_mat& C, cudaStream_t st);
+bool dot_f32_splits(const void* X, long long ldx, const void* W, long long ldw, const void* C, long long ldc, int T, int N, int K);
+jsm_status dot_split_glu_launch(const float* X, long long ldx, const float* gate, const float* up, long long ldw, float* act, long long ldc, int T, int N, int K,
+                                bool gelu, float alpha, float limit, cudaStream_t st);
 
 struct Proj {  // one projection: N outputs, K inputs, both rounded up to multiples of 8 (zero rows / columns)
     int N = 0, K = 0, paired = 0;
@@ -647,7 +650,10 @@ static jsm_status run_layers(jsm_decoder* m, const Pass& P, cudaStream_t st) {
         DEC_TRY(join_residual(m, L.norm1, T, st));
         if (L.c.ff > 0) {
             const void* xin = m->f32 ? m->x : m->xa;
-            if (m->f32) {
+            if (m->f32 && dot_f32_splits(xin, wp, L.gate.w32, L.gate.K, m->act, L.ffp(), T, 2 * L.gate.N, L.gate.K)) {
+                DEC_TRY(dot_split_glu_launch(static_cast<const float*>(xin), wp, L.gate.w32, L.up.w32, L.gate.K, static_cast<float*>(m->act), L.ffp(), T, L.gate.N,
+                                             L.gate.K, L.c.ff_kind == JSM_FF_GELU_GLU, GLU_ALPHA, L.c.ff_limit, st));
+            } else if (m->f32) {
                 float* up = m->gate32 + (size_t)m->c.max_step_tokens * L.ffp();
                 DEC_TRY(linear(m, L.gate, xin, wp, m->gate32, true, T, st));
                 DEC_TRY(linear(m, L.up, xin, wp, up, true, T, st));

@@ -269,6 +269,11 @@ static jsm_status dot_launch(const MatD& A, const MatD& B, const MatD* bias, int
 bool dot_split_usable(const void* X, long long ldx, const void* W, long long ldw, const void* C, long long ldc, int N, int K);
 jsm_status dot_split_launch(const float* X, long long ldx, const float* W, long long ldw, float* C, long long ldc, int T, int N, int K, cudaStream_t st);
 
+// whether the tensor cores take X . W^T (below): rows of aligned fours
+bool dot_f32_splits(const void* X, long long ldx, const void* W, long long ldw, const void* C, long long ldc, int T, int N, int K) {
+    return (T > 32 || (long long)N * K >= 1 << 20) && dot_split_usable(X, ldx, W, ldw, C, ldc, N, K);
+}
+
 // C = A . B in fp32 without the reference's order (operands as in jsm_dot_f32, checked by the caller).  Rows of aligned fours go to the tensor cores
 // (dot_split.cu) from 33 rows of A on, and below that from a million weights on: with fewer their start and end cost more than the products
 // (8 rows, here / there, us: 512 x 512 4.0 / 4.5, 256 x 1024 5.1 / 5.5, 1024 x 1024 7.0 / 6.7, 4096 x 512 9.0 / 7.6, 2752 x 1024 13.5 / 8.9; 32 rows:
@@ -277,8 +282,8 @@ jsm_status dot_split_launch(const float* X, long long ldx, const float* W, long 
 // CTAs times blocks of products each, and about four blocks' time for a CTA's start and end.
 jsm_status dot_f32_launch(const jsm_mat& A, const jsm_mat& B, const jsm_mat& Cm, cudaStream_t st) {
     float* C = reinterpret_cast<float*>(Cm.data);
-    if ((A.rows > 32 || (long long)B.cols * A.cols >= 1 << 20) && A.col_stride == 1 && B.row_stride == 1 && Cm.col_stride == 1 &&
-        dot_split_usable(A.data, A.row_stride, B.data, B.col_stride, C, Cm.row_stride, B.cols, A.cols))
+    if (A.col_stride == 1 && B.row_stride == 1 && Cm.col_stride == 1 &&
+        dot_f32_splits(A.data, A.row_stride, B.data, B.col_stride, C, Cm.row_stride, A.rows, B.cols, A.cols))
         return dot_split_launch(static_cast<const float*>(A.data), A.row_stride, static_cast<const float*>(B.data), B.col_stride, C, Cm.row_stride, A.rows,
                                 B.cols, A.cols, st);
     const int tiles = (B.cols + 63) / 64 * ((A.rows + 15) / 16), blocks = (A.cols + DOT_KB - 1) / DOT_KB;

@@ -18,9 +18,13 @@
 // three planes of a block into shared memory (128-byte swizzle, two stages); warps 8-15 add the blocks' sums (two per quadrant of TMEM
 // lanes, half of the tokens each); warp 8 also issues the MMAs (features are the rows, tokens the columns).
 //
+// Gate and up projections of a feed-forward run as pairs: 64 features' gate and up rows make one tile, and the activation follows where the sums meet (the
+// two products and a launch for the activation, 300 x 2752 x 1024: 43 us, here 32).
+//
 // Numbers beyond bf16's range (infinities, NaN, the last 2^-9 below fp32's largest) do not survive the split; every result that is not
 // finite is formed again by plain fp32 additions.  Parts below 2^-133 are lost.
 #include "tc_utils.cuh"
+#include "linear_epilogue.cuh"
 #include <algorithm>
 #include <mutex>
 
@@ -34,11 +38,13 @@ constexpr int ds_plane(int bn) { return (DS_ROWS + bn) * 128; }
 constexpr int ds_smem(int bn) { return 2 * 3 * ds_plane(bn) + 1024; }
 
 struct DotSplitParams {
-    const float *X, *W;
+    const float *X, *W, *W2;  // W2: the up rows of gate / up pairs
     float* C;
     long long ldx, ldw, ldc;
     int T, N, K, tok_blocks;
     int* err;
+    int gelu;                 // pairs: the activation, and what the clamped one needs
+    float alpha, limit;
 };
 
 __device__ __forceinline__ uint32_t ds_cluster_size() {
@@ -62,9 +68,30 @@ __device__ __forceinline__ uint32_t ds_part(float& a, float& b) {
     return p;
 }
 
-// BN: tokens of a tile
-template <int BN>
+// Products of one row of X with four rows of W by plain fp32 additions: blocks of 32 in two chains, as dot_f32_kernel adds them (what overflows on the
+// way is the same)
+static __device__ __noinline__ float4 ds_again(const float* w, long long ldw, const float* x, int K) {
+    float v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        float sum = 0.0f;
+        for (int k0 = 0; k0 < K && sum == sum; k0 += 32) {
+            float even = 0.0f, odd = 0.0f;
+            for (int k = k0; k < min(K, k0 + 32); k += 2) {
+                even = fmaf(x[k], w[j * ldw + k], even);
+                odd = fmaf(x[k + 1], w[j * ldw + k + 1], odd);
+            }
+            sum += even + odd;
+        }
+        v[j] = sum;
+    }
+    return make_float4(v[0], v[1], v[2], v[3]);
+}
+
+// BN: tokens of a tile.  PAIRED: a tile has the gate rows of 64 features, then their up rows; C = activation(gate, up)
+template <int BN, bool PAIRED>
 __global__ void __launch_bounds__(DS_THREADS, 1) dot_split_kernel(DotSplitParams P) {
+    constexpr int FEATURES = PAIRED ? DS_ROWS / 2 : DS_ROWS;
     constexpr int PLANE = ds_plane(BN), STAGE = 3 * PLANE, X_OFF = DS_ROWS * 128;
     constexpr int ROWS_PASS = DS_SPLIT_WARPS * 4, W_ITEMS = DS_ROWS / ROWS_PASS, X_ITEMS = BN / ROWS_PASS, ITEMS = W_ITEMS + X_ITEMS;
     constexpr uint32_t BUF = BN <= 32 ? 32 : BN <= 64 ? 64 : 128;  // tensor-memory columns between the two accumulators
@@ -79,7 +106,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dot_split_kernel(DotSplitParams
     chain_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int S = (int)ds_cluster_size(), rank = (int)ds_cluster_rank(), tile = (int)blockIdx.x / S;
-    const int n0 = tile / P.tok_blocks * DS_ROWS, t0 = tile % P.tok_blocks * BN;
+    const int n0 = tile / P.tok_blocks * FEATURES, t0 = tile % P.tok_blocks * BN;
     const int blocks = (P.K + DS_KB - 1) / DS_KB, b0 = blocks * rank / S, b1 = blocks * (rank + 1) / S;
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -105,14 +132,15 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dot_split_kernel(DotSplitParams
         // eight lanes take a row's 64 numbers; a pass of the eight warps covers 32 rows
         const int r0 = warp * 4 + (lane >> 3), chunk = lane & 7;
         const float* wp = P.W + (long long)(n0 + r0) * P.ldw + chunk * 8;
+        const float* wp2 = PAIRED ? P.W2 + (long long)(n0 + r0) * P.ldw + chunk * 8 : nullptr;
         const float* xp = P.X + (long long)(t0 + r0) * P.ldx + chunk * 8;
         uint8_t* const dst = ring + r0 * 128 + ((chunk ^ (r0 & 7)) << 4);  // (rows of a thread differ by 32: the same swizzle)
         float4 v[ITEMS][2];
         auto load = [&](int i, int b) {
-            const bool w = i < W_ITEMS;
-            const int r = (w ? i : i - W_ITEMS) * ROWS_PASS;
+            const bool w = i < W_ITEMS, up = PAIRED && w && i >= W_ITEMS / 2;
+            const int r = (up ? i - W_ITEMS / 2 : w ? i : i - W_ITEMS) * ROWS_PASS;
             const bool on = b < b1 && b * DS_KB + chunk * 8 < P.K && (w ? n0 + r0 + r < P.N : t0 + r0 + r < P.T);
-            const float4* p = reinterpret_cast<const float4*>((w ? wp + r * P.ldw : xp + r * P.ldx) + b * DS_KB);
+            const float4* p = reinterpret_cast<const float4*>((up ? wp2 + r * P.ldw : w ? wp + r * P.ldw : xp + r * P.ldx) + b * DS_KB);
             v[i][0] = on ? p[0] : make_float4(0.f, 0.f, 0.f, 0.f);
             v[i][1] = on ? p[1] : make_float4(0.f, 0.f, 0.f, 0.f);
         };
@@ -237,45 +265,39 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dot_split_kernel(DotSplitParams
     if (!abort_flag) {
         // this CTA's share of the tokens, four features per thread, the ranks' sums in order
         const int lo = BN * rank / S, hi = BN * (rank + 1) / S;
-        for (int e = threadIdx.x; e < (hi - lo) * (DS_ROWS / 4); e += DS_THREADS) {
-            const int t = lo + e / (DS_ROWS / 4), n = e % (DS_ROWS / 4) * 4;
+        for (int e = threadIdx.x; e < (hi - lo) * (FEATURES / 4); e += DS_THREADS) {
+            const int t = lo + e / (FEATURES / 4), n = e % (FEATURES / 4) * 4;
             if (t0 + t >= P.T || n0 + n >= P.N) continue;
-            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            const uint32_t at = smem_u32(ring) + (t * DS_ROWS + n) * 4;
+            // sums of four rows of the tile, formed again where they are not finite
+            auto sums = [&](int row, const float* W) {
+                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                const uint32_t at = smem_u32(ring) + (t * DS_ROWS + row) * 4;
 #pragma unroll 4
-            for (int z = 0; z < S; ++z) {
-                uint32_t addr;
-                float4 q;
-                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(at), "r"(z));
-                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w) : "r"(addr) : "memory");
-                v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
-            }
-            float* c = P.C + (long long)(t0 + t) * P.ldc + n0 + n;
-            if (fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))) < INFINITY && v.x + v.y + v.z + v.w == v.x + v.y + v.z + v.w) {
-                *reinterpret_cast<float4*>(c) = v;
-            } else {
-                const float *w = P.W + (long long)(n0 + n) * P.ldw, *x = P.X + (long long)(t0 + t) * P.ldx;
-#pragma unroll 1
-                for (int j = 0; j < 4; ++j) {
-                    float sum = 0.0f;  // blocks of 32 in two chains, as dot_f32_kernel adds them: what overflows on the way is the same
-                    for (int k0 = 0; k0 < P.K && sum == sum; k0 += 32) {
-                        float even = 0.0f, odd = 0.0f;
-                        for (int k = k0; k < min(P.K, k0 + 32); k += 2) {
-                            even = fmaf(x[k], w[j * P.ldw + k], even);
-                            odd = fmaf(x[k + 1], w[j * P.ldw + k + 1], odd);
-                        }
-                        sum += even + odd;
-                    }
-                    c[j] = sum;
+                for (int z = 0; z < S; ++z) {
+                    uint32_t addr;
+                    float4 q;
+                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(at), "r"(z));
+                    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w) : "r"(addr) : "memory");
+                    v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
                 }
+                if (!(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))) < INFINITY && v.x + v.y + v.z + v.w == v.x + v.y + v.z + v.w))
+                    v = ds_again(W + (long long)(n0 + n) * P.ldw, P.ldw, P.X + (long long)(t0 + t) * P.ldx, P.K);
+                return v;
+            };
+            float4 v = sums(n, P.W);
+            if constexpr (PAIRED) {
+                const float4 u = sums(n + FEATURES, P.W2);
+                auto act = [&](float g, float x) { return P.gelu ? gelu_glu_f32(g, x) : clamped_glu_f32(g, x, P.alpha, P.limit); };
+                v = make_float4(act(v.x, u.x), act(v.y, u.y), act(v.z, u.z), act(v.w, u.w));
             }
+            *reinterpret_cast<float4*>(P.C + (long long)(t0 + t) * P.ldc + n0 + n) = v;
         }
     }
     if (S > 1) ds_cluster_sync();  // nobody leaves while a peer reads its sums
 }
 
 // clusters of S CTAs that the chip holds at once
-template <int BN>
+template <int BN, bool PAIRED>
 static int ds_capacity(int S) {
     static std::mutex mu;
     static int known[64][9];  // per device
@@ -295,7 +317,7 @@ static int ds_capacity(int S) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, dot_split_kernel<BN>, &cfg) != cudaSuccess || n <= 0) {
+        if (cudaOccupancyMaxActiveClusters(&n, dot_split_kernel<BN, PAIRED>, &cfg) != cudaSuccess || n <= 0) {
             cudaGetLastError();
             n = guess;
         }
@@ -304,10 +326,10 @@ static int ds_capacity(int S) {
     return known[dev][S];
 }
 
-template <int BN>
+template <int BN, bool PAIRED>
 static jsm_status ds_allow() {
-    static DeviceOnce once;
-    JSM_CUDA_CHECK(allow_shared(once, dot_split_kernel<BN>, ds_smem(BN)));
+    static DeviceOnce once;  // per instantiation
+    JSM_CUDA_CHECK(allow_shared(once, dot_split_kernel<BN, PAIRED>, ds_smem(BN)));
     return JSM_OK;
 }
 
@@ -315,25 +337,25 @@ static jsm_status ds_allow() {
 // seven around its blocks; clusters that do not fit the chip at once wait for the first ones.  300 tokens, tokens of a tile / CTAs of a
 // cluster: 1024 x 2752 96/4 19.9 us, 128/5 20.0, 64/3 22.7, 96/3 24.7, 64/4 (40 clusters, the chip holds 33) 34.8; 4096 x 512 96/1 14.9,
 // 128/1 16.7, 64/1 (160 CTAs) 25.9; 33 tokens: 1024 x 1024 64/8 7.2, 96/8 7.6, 32/6 8.2, 32/8 (16 clusters, the chip holds 15) 11.2.
-template <int BN>
+template <int BN, bool PAIRED>
 static jsm_status ds_shape(int T, int N, int K, float* best, int* bn, int* splits) {
     constexpr float block_us = BN == 32 ? 1.04f : BN == 64 ? 1.13f : BN == 96 ? 1.2f : 1.4f, around_us = BN <= 64 ? 5.2f : BN == 96 ? 5.5f : 6.6f;
-    jsm_status st = ds_allow<BN>();
+    jsm_status st = ds_allow<BN, PAIRED>();
     if (st != JSM_OK) return st;
-    const int blocks = (K + DS_KB - 1) / DS_KB, tiles = (N + DS_ROWS - 1) / DS_ROWS * ((T + BN - 1) / BN);
+    const int blocks = (K + DS_KB - 1) / DS_KB, tiles = ((PAIRED ? 2 : 1) * N + DS_ROWS - 1) / DS_ROWS * ((T + BN - 1) / BN);
     for (int S = 1; S <= 8 && S <= blocks; ++S) {
-        const int cap = ds_capacity<BN>(S);
+        const int cap = ds_capacity<BN, PAIRED>(S);
         const float cost = (float)((tiles + cap - 1) / cap) * (around_us + (S > 1 ? 0.5f : 0.0f) + (float)((blocks + S - 1) / S) * block_us);
         if (*bn == 0 || cost < *best) { *best = cost; *bn = BN; *splits = S; }
     }
     return JSM_OK;
 }
 
-template <int BN>
+template <int BN, bool PAIRED>
 static jsm_status ds_launch(DotSplitParams& P, int S, cudaStream_t st) {
     P.tok_blocks = (P.T + BN - 1) / BN;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((P.N + DS_ROWS - 1) / DS_ROWS * P.tok_blocks * S));
+    cfg.gridDim = dim3((unsigned)(((PAIRED ? 2 : 1) * P.N + DS_ROWS - 1) / DS_ROWS * P.tok_blocks * S));
     cfg.blockDim = dim3(DS_THREADS);
     cfg.dynamicSmemBytes = ds_smem(BN);
     cfg.stream = st;
@@ -345,7 +367,7 @@ static jsm_status ds_launch(DotSplitParams& P, int S, cudaStream_t st) {
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = chained_launch_enabled() ? 2 : 1;
-    JSM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, dot_split_kernel<BN>, P));
+    JSM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, dot_split_kernel<BN, PAIRED>, P));
     g_launches.fetch_add(1);
     return JSM_OK;
 }
@@ -356,14 +378,25 @@ bool dot_split_usable(const void* X, long long ldx, const void* W, long long ldw
     return fours(X, ldx) && fours(W, ldw) && fours(C, ldc) && N % 4 == 0 && K % 8 == 0;
 }
 
-jsm_status dot_split_launch(const float* X, long long ldx, const float* W, long long ldw, float* C, long long ldc, int T, int N, int K, cudaStream_t st) {
-    DotSplitParams P{X, W, C, ldx, ldw, ldc, T, N, K, 0, tc_error_word()};
+template <bool PAIRED>
+static jsm_status ds_go(DotSplitParams& P, cudaStream_t st) {
     float best = 0.0f;
     int bn = 0, S = 1;
-    for (jsm_status s : {ds_shape<128>(T, N, K, &best, &bn, &S), ds_shape<96>(T, N, K, &best, &bn, &S), ds_shape<64>(T, N, K, &best, &bn, &S),
-                         ds_shape<32>(T, N, K, &best, &bn, &S)})
+    for (auto shape : {ds_shape<128, PAIRED>, ds_shape<96, PAIRED>, ds_shape<64, PAIRED>, ds_shape<32, PAIRED>}) {
+        const jsm_status s = shape(P.T, P.N, P.K, &best, &bn, &S);
         if (s != JSM_OK) return s;
-    return bn == 128 ? ds_launch<128>(P, S, st) : bn == 96 ? ds_launch<96>(P, S, st) : bn == 64 ? ds_launch<64>(P, S, st) : ds_launch<32>(P, S, st);
+    }
+    return bn == 128 ? ds_launch<128, PAIRED>(P, S, st) : bn == 96 ? ds_launch<96, PAIRED>(P, S, st)
+         : bn == 64 ? ds_launch<64, PAIRED>(P, S, st) : ds_launch<32, PAIRED>(P, S, st);
+}
+jsm_status dot_split_launch(const float* X, long long ldx, const float* W, long long ldw, float* C, long long ldc, int T, int N, int K, cudaStream_t st) {
+    DotSplitParams P{X, W, nullptr, C, ldx, ldw, ldc, T, N, K, 0, tc_error_word(), 0, 0.0f, 0.0f};
+    return ds_go<false>(P, st);
+}
+jsm_status dot_split_glu_launch(const float* X, long long ldx, const float* gate, const float* up, long long ldw, float* act, long long ldc, int T, int N, int K,
+                                bool gelu, float alpha, float limit, cudaStream_t st) {
+    DotSplitParams P{X, gate, up, act, ldx, ldw, ldc, T, N, K, 0, tc_error_word(), gelu ? 1 : 0, alpha, limit};
+    return ds_go<true>(P, st);
 }
 
 }  // namespace jsm

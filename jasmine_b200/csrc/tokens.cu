@@ -4,6 +4,7 @@
 // with eps under the square root, RMSNorm drops the mean.
 #include "common.cuh"
 #include "decoder_ops.cuh"
+#include "linear_epilogue.cuh"
 #include "mma_utils.cuh"
 #include <math.h>
 #include <algorithm>
@@ -366,17 +367,12 @@ __global__ void __launch_bounds__(256) logits_finish_kernel(float* __restrict__ 
     }
 }
 
-__device__ __forceinline__ float clamped_glu(float g, float u, float alpha, float limit) {
-    g = fminf(g, limit);
-    u = fminf(fmaxf(u, -limit), limit);
-    return g / (1.0f + expf(-alpha * g)) * (u + 1.0f);
-}
 __global__ void __launch_bounds__(256) clamped_glu_f32_kernel(const float* __restrict__ gate, const float* __restrict__ up, float* __restrict__ act,
                                                               float alpha, float limit, long long n) {
     chain_trigger();
     chain_wait();
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256)
-        act[i] = clamped_glu(gate[i], up[i], alpha, limit);
+        act[i] = clamped_glu_f32(gate[i], up[i], alpha, limit);
 }
 
 jsm_status embed_residual_launch(bool f32, const void* table, const int32_t* ids, float scale, float* x, void* xa, int T, int wp, cudaStream_t st) {
@@ -433,8 +429,7 @@ __global__ void __launch_bounds__(256) gelu_glu_f32_kernel(const float* __restri
     chain_trigger();
     chain_wait();
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
-        const float z = gate[i];
-        act[i] = 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z))) * up[i];
+        act[i] = gelu_glu_f32(gate[i], up[i]);
     }
 }
 jsm_status gelu_glu_f32_launch(const float* gate, const float* up, float* act, long long n, cudaStream_t st) {

@@ -4,7 +4,10 @@ with clusters of one to eight CTAs; weights of 24 bits and weights that fit bf16
 import numpy as np
 import pytest
 
+import vagonex_oracle as vo
 import vagonex_util as vu
+import zugolorn_oracle as zo
+import zugolorn_util as zu
 
 pytestmark = pytest.mark.gpu
 
@@ -76,4 +79,25 @@ def test_numbers_that_do_not_split():
     assert fine[:, 154].any() and np.isinf(want[:, 154]).any()
     assert np.allclose(got[fine], want[fine], rtol=2e-5, atol=2e-5)
     assert np.allclose(got[:, 156], want[:, 156], rtol=1e-5, atol=2.0 ** -133)
+    m.close()
+
+
+@pytest.mark.parametrize("T,width,ff", [(33, 40, 20), (64, 64, 64), (70, 72, 72), (129, 136, 200), (40, 200, 1000), (5, 520, 1016), (300, 64, 129)])
+@pytest.mark.parametrize("design", ["vagonex", "zugolorn"])
+def test_gate_up_pairs(design, T, width, ff):
+    """A feed-forward in one launch of pairs: tiles of 64 features and their remainders, both activations, weights of 24 bits, against the whole model in float64."""
+    if design == "vagonex":
+        util, forward = vu, vo.forward
+        cfg = vu.config([vu.lightning(heads=2, dim=12, vdim=12, ff=ff)], width=width)
+    else:
+        util, forward = zu, zo.forward
+        cfg = zu.config([zu.mamba(inner=48, ff=ff, limit=0.8)], width=width)
+    rng = np.random.default_rng(ff)
+    w = {k: vu.widen(v).astype(np.float32) for k, v in util.random_weights(cfg, T).items()}
+    for k in w:  # (numbers that bf16 does not hold; the zeros of a design stay)
+        w[k] = np.where(w[k] == 0, w[k], w[k] * (1 + 2.0 ** -9 * rng.standard_normal(w[k].shape))).astype(np.float32)
+    toks = vu.tokens(T, cfg["vocab"], T)
+    m = util.build(cfg, w, "float32")
+    got = logits(m, toks)
+    assert util.error(got, forward(cfg, {k: v.astype(np.float64) for k, v in w.items()}, toks)) < 4e-5  # (the bar of the other fp32 models)
     m.close()
