@@ -10,7 +10,8 @@
 //
 // Prompts: a CTA owns 16 channels of one segment and walks its tokens in tiles of 32 that cp.async brings into a two-stage
 // ring; eight threads share a channel's states, so that the chain of dependent steps is one FMA per state and the partial
-// sums of eight tokens are exchanged with seven shuffles.  Decode: one thread per channel and sequence, eight sequences per
+// sums of eight tokens are exchanged with seven shuffles; where that fills the chip more than twice, fewer threads walk
+// (scan_wide_kernel).  Decode: one thread per channel and sequence, eight sequences per
 // CTA; the states are requested first and arrive while the step sizes (a small projection) are computed.
 //
 // Layout of S and A: planes of four states, [plane][channel][4], so that neighbouring threads - channels - read neighbouring
@@ -30,7 +31,6 @@ constexpr int SC_CH = 16;       // channels per CTA
 constexpr int SC_SUB = 8;       // threads per channel (prompts)
 constexpr int SC_THREADS = SC_CH * SC_SUB;
 constexpr int SC_TT = 32;       // tokens per tile
-constexpr int SC_YP = SC_CH + 4;  // pitch of the output tile (floats)
 constexpr int ST_WARPS = 4;     // decode step: a warp per sequence
 constexpr int ST_CH = 32;       // channels per CTA: a lane each
 constexpr int ST_THREADS = ST_CH * ST_WARPS;
@@ -244,12 +244,35 @@ __device__ __forceinline__ void lds_vec(const float* p, float (&v)[NS]) {
     }
 }
 
+template <int NS>
+__device__ __forceinline__ void lds_pairs(const float* p, uint64_t (&v)[NS / 2]) {
+    if constexpr (NS % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < NS / 2; i += 2) {
+            const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(p + 2 * i);
+            v[i] = w.x; v[i + 1] = w.y;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < NS / 2; ++i) v[i] = *reinterpret_cast<const uint64_t*>(p + 2 * i);
+    }
+}
+
+// eight tokens' partial sums on each of SUB lanes -> the sums of tokens 8 / SUB * sub .. in y[0 ..]
+template <int SUB>
+__device__ __forceinline__ void column_sums(float (&y)[8], int sub) {
+#pragma unroll
+    for (int w = SUB / 2, m = 4; w >= 1; w >>= 1, m >>= 1) {
+        const bool high = sub & w;
+#pragma unroll
+        for (int u = 0; u < m; ++u) y[u] = (high ? y[m + u] : y[u]) + __shfl_xor_sync(0xffffffffu, high ? y[u] : y[m + u], w);
+    }
+}
+
 // ---- scan of prompts ----------------------------------------------------------------------------------------------
-__host__ __device__ inline int scan_nb(int np, int ns) { return np > SC_SUB * ns ? np : SC_SUB * ns; }  // B / C columns per tile row
-template <typename T>
-static size_t scan_smem(int np, int ns) {
-    return 2 * (size_t)SC_TT * SC_CH * (2 * sizeof(T) + 4) + 2 * (size_t)SC_TT * 2 * scan_nb(np, ns) * 4 + (size_t)SC_TT * SC_YP * 4 +
-           (size_t)SC_TT * SC_CH * 16;
+template <typename T, int NS>
+constexpr int scan_smem() {
+    return 2 * SC_TT * SC_CH * (2 * (int)sizeof(T) + 4) + 2 * SC_TT * 2 * SC_SUB * NS * 4 + SC_TT * (SC_CH + 4) * 4 + SC_TT * SC_CH * 16;
 }
 
 struct ScanArgs {
@@ -261,29 +284,32 @@ struct ScanArgs {
     int ip, np, rp, state, taps, n_segs;
 };
 
+// NS states per thread
 template <typename T, int NS>
 __global__ void __launch_bounds__(SC_THREADS) scan_kernel(ScanArgs a) {
     extern __shared__ __align__(16) uint8_t sc_dyn[];
-    const int nb = scan_nb(a.np, NS);
+    constexpr int CH = SC_CH, SUB = SC_SUB, YP = CH + 4, NB = SUB * NS;     // YP: pitch of the output tile; NB: B / C columns per tile row
+    constexpr int EL = SC_TT * CH / SC_THREADS;                             // elements of a tile per thread
     T* xs = reinterpret_cast<T*>(sc_dyn);                                   // 2 x [TT][CH]
-    T* zs = xs + 2 * SC_TT * SC_CH;                                         // 2 x [TT][CH]
-    float* dts = reinterpret_cast<float*>(zs + 2 * SC_TT * SC_CH);          // 2 x [TT][CH]
-    float* bc = dts + 2 * SC_TT * SC_CH;                                    // 2 x [TT][B: nb | C: nb]
-    float* ys = bc + 2 * SC_TT * 2 * nb;                                    // [TT][YP]
-    float4* dd = reinterpret_cast<float4*>(ys + SC_TT * SC_YP);             // [TT][CH]: dt, dt, dt x, dt x
+    T* zs = xs + 2 * SC_TT * CH;                                         // 2 x [TT][CH]
+    float* dts = reinterpret_cast<float*>(zs + 2 * SC_TT * CH);          // 2 x [TT][CH]
+    float* bc = dts + 2 * SC_TT * CH;                                    // 2 x [TT][B: NB | C: NB]
+    float* ys = bc + 2 * SC_TT * 2 * NB;                                    // [TT][YP]
+    float4* dd = reinterpret_cast<float4*>(ys + SC_TT * YP);             // [TT][CH]: dt, dt, dt x, dt x
     constexpr bool PAIRS = sizeof(T) == 2 && NS % 2 == 0;                   // bf16 models: states in pairs, base-2 exponentials
     chain_trigger();
-    const int tid = threadIdx.x, ch = tid / SC_SUB, sub = tid % SC_SUB;
-    const int c0 = blockIdx.x * SC_CH, c = c0 + ch;
+    const int tid = threadIdx.x, ch = tid / SUB, sub = tid % SUB;
+    const int c0 = blockIdx.x * CH, c = c0 + ch;
     const bool live = c < a.ip;
     float A[NS], S[NS];
+    uint64_t A2[PAIRS ? NS / 2 : 1], S2[PAIRS ? NS / 2 : 1];
 #pragma unroll
     for (int i = 0; i < NS; ++i) {
         const int n = sub * NS + i;
         A[i] = (live && n < a.state) ? a.A[plane_index(n, c, a.ip)] : 0.0f;
         if (PAIRS) A[i] *= LOG2E;
     }
-    for (int i = tid; i < 2 * SC_TT * 2 * nb; i += SC_THREADS) bc[i] = 0.0f;  // columns behind np stay zero
+    for (int i = tid; i < 2 * SC_TT * 2 * NB; i += SC_THREADS) bc[i] = 0.0f;  // columns behind np stay zero
     __syncthreads();
     chain_wait();
     const int seg = blockIdx.y;
@@ -294,38 +320,41 @@ __global__ void __launch_bounds__(SC_THREADS) scan_kernel(ScanArgs a) {
         const int n = sub * NS + i;
         S[i] = (live && n < a.state && pos0 > 0) ? state[plane_index(n, c, a.ip)] : 0.0f;
     }
+    if constexpr (PAIRS)
+#pragma unroll
+        for (int i = 0; i < NS / 2; ++i) { A2[i] = f2_pack(A[2 * i], A[2 * i + 1]); S2[i] = f2_pack(S[2 * i], S[2 * i + 1]); }
     const int pc = a.rp + 2 * a.np;
     const T* xz = static_cast<const T*>(a.xz);
     const T* xc = static_cast<const T*>(a.xc);
     auto load_tile = [&](int t0, int stage) {
-        constexpr int EV = 16 / sizeof(T), XV = SC_CH / EV;  // elements per vector, vectors per row
+        constexpr int EV = 16 / sizeof(T), XV = CH / EV;  // elements per vector, vectors per row
         for (int i = tid; i < SC_TT * XV; i += SC_THREADS) {
             const int r = i / XV, v = (i % XV) * EV;
             const bool ok = t0 + r < len && c0 + v < a.ip;
             const long long t = start + (ok ? t0 + r : 0);
             const int cc = ok ? c0 + v : 0;
-            cp_async16(smem_u32(xs + (stage * SC_TT + r) * SC_CH + v), xc + t * a.ip + cc, ok);
-            cp_async16(smem_u32(zs + (stage * SC_TT + r) * SC_CH + v), xz + t * 2 * a.ip + a.ip + cc, ok);
+            cp_async16(smem_u32(xs + (stage * SC_TT + r) * CH + v), xc + t * a.ip + cc, ok);
+            cp_async16(smem_u32(zs + (stage * SC_TT + r) * CH + v), xz + t * 2 * a.ip + a.ip + cc, ok);
         }
-        for (int i = tid; i < SC_TT * (SC_CH / 4); i += SC_THREADS) {
-            const int r = i / (SC_CH / 4), v = (i % (SC_CH / 4)) * 4;
+        for (int i = tid; i < SC_TT * (CH / 4); i += SC_THREADS) {
+            const int r = i / (CH / 4), v = (i % (CH / 4)) * 4;
             const bool ok = t0 + r < len && c0 + v < a.ip;
-            cp_async16(smem_u32(dts + (stage * SC_TT + r) * SC_CH + v), a.dt_raw + (long long)(start + (ok ? t0 + r : 0)) * a.ip + (ok ? c0 + v : 0), ok);
+            cp_async16(smem_u32(dts + (stage * SC_TT + r) * CH + v), a.dt_raw + (long long)(start + (ok ? t0 + r : 0)) * a.ip + (ok ? c0 + v : 0), ok);
         }
-        const int bv = a.np / 4;
-        for (int i = tid; i < SC_TT * 2 * bv; i += SC_THREADS) {
-            const int r = i / (2 * bv), v = i % (2 * bv);
+        for (int i = tid; i < SC_TT * 2 * (NB / 4); i += SC_THREADS) {
+            const int r = i / (2 * (NB / 4)), part = i / (NB / 4) & 1, v = i % (NB / 4) * 4;
+            if (v >= a.np) continue;
             const bool ok = t0 + r < len;
-            const float* src = a.proj + (long long)(start + (ok ? t0 + r : 0)) * pc + a.rp + v * 4;
-            cp_async16(smem_u32(bc + ((stage * SC_TT + r) * 2 + (v >= bv)) * nb + (v % bv) * 4), src, ok);
+            const float* src = a.proj + (long long)(start + (ok ? t0 + r : 0)) * pc + a.rp + part * a.np + v;
+            cp_async16(smem_u32(bc + ((stage * SC_TT + r) * 2 + part) * NB + v), src, ok);
         }
     };
     load_tile(0, 0);
     cp_async_commit();
     // every pass over a tile gives a thread the same channels: their constants stay in registers
-    static_assert(SC_THREADS % SC_CH == 0 && SC_TT * SC_CH == SC_THREADS * 4, "four elements of a tile per thread");
-    const float bias = c0 + (tid & (SC_CH - 1)) < a.ip ? a.dt_b[c0 + (tid & (SC_CH - 1))] : 0.0f;
-    const int ov = (tid & (SC_CH / 4 - 1)) * 4, orow = tid / (SC_CH / 4);  // output pass: four channels of one token
+    static_assert(SC_THREADS % CH == 0 && EL == 4, "four elements of a tile per thread");
+    const float bias = c0 + (tid & (CH - 1)) < a.ip ? a.dt_b[c0 + (tid & (CH - 1))] : 0.0f;
+    const int ov = (tid & (CH / 4 - 1)) * 4, orow = tid / (CH / 4);  // output pass: four channels of one token
     const bool olive = c0 + ov < a.ip;
     const float4 Dv = olive ? *reinterpret_cast<const float4*>(a.D + c0 + ov) : make_float4(0.f, 0.f, 0.f, 0.f);
     const int nt = (len + SC_TT - 1) / SC_TT;
@@ -335,17 +364,17 @@ __global__ void __launch_bounds__(SC_THREADS) scan_kernel(ScanArgs a) {
         cp_async_commit();
         cp_async_wait<1>();
         __syncthreads();
-        const float* dt = dts + stage * SC_TT * SC_CH;
-        const T* x = xs + stage * SC_TT * SC_CH;
+        const float* dt = dts + stage * SC_TT * CH;
+        const T* x = xs + stage * SC_TT * CH;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < EL; ++u) {
             const int i = u * SC_THREADS + tid;
             // a step size of zero leaves the state as it is: the rows behind the segment (and channels behind the last)
-            const float d = i / SC_CH < n ? softplus_t<T>(dt[i] + bias) : 0.0f, dx = d * to_f32(x[i]);
+            const float d = i / CH < n ? softplus_t<T>(dt[i] + bias) : 0.0f, dx = d * to_f32(x[i]);
             dd[i] = make_float4(d, d, dx, dx);
         }
         __syncthreads();
-        const float* bt = bc + stage * SC_TT * 2 * nb + sub * NS;
+        const float* bt = bc + stage * SC_TT * 2 * NB + sub * NS;
 #pragma unroll 1
         for (int t8 = 0; t8 < n; t8 += 8) {
             float y[8];
@@ -353,26 +382,26 @@ __global__ void __launch_bounds__(SC_THREADS) scan_kernel(ScanArgs a) {
             for (int u = 0; u < 8; ++u) {
                 const int t = t8 + u;
                 if constexpr (PAIRS) {
-                    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(dd + t * SC_CH + ch);  // (dt, dt), (dt x, dt x)
-                    const uint64_t* B = reinterpret_cast<const uint64_t*>(bt + t * 2 * nb);
-                    const uint64_t* C = reinterpret_cast<const uint64_t*>(bt + t * 2 * nb + nb);
+                    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(dd + t * CH + ch);  // (dt, dt), (dt x, dt x)
+                    uint64_t B[NS / 2], C[NS / 2];
+                    lds_pairs<NS>(bt + t * 2 * NB, B);
+                    lds_pairs<NS>(bt + t * 2 * NB + NB, C);
                     uint64_t acc = 0;
 #pragma unroll
                     for (int i = 0; i < NS / 2; ++i) {
                         float e0, e1;
-                        f2_unpack(f2_mul(w.x, f2_pack(A[2 * i], A[2 * i + 1])), e0, e1);
-                        const uint64_t s2 = f2_fma(f2_pack(fast_ex2(e0), fast_ex2(e1)), f2_pack(S[2 * i], S[2 * i + 1]), f2_mul(w.y, B[i]));
-                        f2_unpack(s2, S[2 * i], S[2 * i + 1]);
-                        acc = i == 0 ? f2_mul(s2, C[i]) : f2_fma(s2, C[i], acc);
+                        f2_unpack(f2_mul(w.x, A2[i]), e0, e1);
+                        S2[i] = f2_fma(f2_pack(fast_ex2(e0), fast_ex2(e1)), S2[i], f2_mul(w.y, B[i]));
+                        acc = i == 0 ? f2_mul(S2[i], C[i]) : f2_fma(S2[i], C[i], acc);
                     }
                     float lo, hi;
                     f2_unpack(acc, lo, hi);
                     y[u] = lo + hi;
                 } else {
-                    const float4 w = dd[t * SC_CH + ch];
+                    const float4 w = dd[t * CH + ch];
                     float B[NS], C[NS];
-                    lds_vec<NS>(bt + t * 2 * nb, B);
-                    lds_vec<NS>(bt + t * 2 * nb + nb, C);
+                    lds_vec<NS>(bt + t * 2 * NB, B);
+                    lds_vec<NS>(bt + t * 2 * NB + NB, C);
                     float acc = 0.0f;
 #pragma unroll
                     for (int i = 0; i < NS; ++i) {
@@ -382,35 +411,224 @@ __global__ void __launch_bounds__(SC_THREADS) scan_kernel(ScanArgs a) {
                     y[u] = acc;
                 }
             }
-            // eight partial sums on each of eight lanes -> lane `sub` holds the sum of token t8 + sub
-            float k4[4], k2[2];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) k4[u] = ((sub & 4) ? y[4 + u] : y[u]) + __shfl_xor_sync(0xffffffffu, (sub & 4) ? y[u] : y[4 + u], 4);
-#pragma unroll
-            for (int u = 0; u < 2; ++u) k2[u] = ((sub & 2) ? k4[2 + u] : k4[u]) + __shfl_xor_sync(0xffffffffu, (sub & 2) ? k4[u] : k4[2 + u], 2);
-            const float k = ((sub & 1) ? k2[1] : k2[0]) + __shfl_xor_sync(0xffffffffu, (sub & 1) ? k2[0] : k2[1], 1);
-            ys[(t8 + sub) * SC_YP + ch] = k;
+            column_sums<SUB>(y, sub);
+            ys[(t8 + sub) * YP + ch] = y[0];
         }
         __syncthreads();
-        const T* z = zs + stage * SC_TT * SC_CH;
+        const T* z = zs + stage * SC_TT * CH;
         if (orow < n && olive) {
             float xv[4], zv[4], o[4];
-            load4(x + orow * SC_CH + ov, xv);
-            load4(z + orow * SC_CH + ov, zv);
-            const float4 yv = *reinterpret_cast<const float4*>(ys + orow * SC_YP + ov);
+            load4(x + orow * CH + ov, xv);
+            load4(z + orow * CH + ov, zv);
+            const float4 yv = *reinterpret_cast<const float4*>(ys + orow * YP + ov);
             o[0] = fmaf(Dv.x, xv[0], yv.x) * silu_t<T>(zv[0]); o[1] = fmaf(Dv.y, xv[1], yv.y) * silu_t<T>(zv[1]);
             o[2] = fmaf(Dv.z, xv[2], yv.z) * silu_t<T>(zv[2]); o[3] = fmaf(Dv.w, xv[3], yv.w) * silu_t<T>(zv[3]);
             store4(static_cast<T*>(a.y) + (long long)(start + t0 + orow) * a.ip + c0 + ov, o);
         }
         __syncthreads();
     }
+    if constexpr (PAIRS)
+#pragma unroll
+        for (int i = 0; i < NS / 2; ++i) f2_unpack(S2[i], S[2 * i], S[2 * i + 1]);
     if (live)
 #pragma unroll
         for (int i = 0; i < NS; ++i)
             if (sub * NS + i < a.state) state[plane_index(sub * NS + i, c, a.ip)] = S[i];
-    if (tid < SC_CH && c0 + tid < a.ip)
+    if (tid < CH && c0 + tid < a.ip)
         carry_conv_state(static_cast<T*>(a.conv) + (long long)slot * (a.taps - 1) * a.ip, xz, 2 * a.ip, c0 + tid, a.ip, a.taps, start, len,
                             pos0);
+}
+
+// ---- scan of prompts, bf16 models with 9 to 16 states, chip filled --------------------------------------------------
+// What bounds it: instructions, then exponentials.  In scan_kernel above the exchange of partial sums, the broadcast of step
+// sizes as pairs and the passes over a tile cost as much as the states themselves (33 instructions per warp and token, the
+// issue slots of the fullest SMs 72 % in use).  Here two threads share a channel, eight states each, so that a token costs half the
+// instructions per state and one exchange per eight tokens and channel; and four warps that do nothing else walk the tokens,
+// one per scheduler, the decays of a token computed while the one before it moves the state.  Four more warps bring the
+// tiles, make the step sizes of the next one and write the outputs of the last one meanwhile.  A CTA owns 64 channels.
+// 2048 tokens, 16 states, 8192 channels: 219 -> 131 us (scan_kernel 186, where addresses with constant strides and states kept as pairs save a
+// seventh); the exponential units are then about 2/3 in use on the SMs that have a CTA.  Eight walking warps of four states
+// 148 us, eight warps beside the walking ones 156; 2 CTAs per SM are named because the compiler then takes 126 registers, without that 66 (165 us).
+constexpr int SW_CH = 64, SW_SUB = 2, SW_NS = 8, SW_HELP = 128, SW_MAIN = SW_CH * SW_SUB, SW_THREADS = SW_MAIN + SW_HELP, SW_YP = SW_CH + 4;
+struct ScanWideTile {  // a tile as it arrives
+    __nv_bfloat16 x[SC_TT][SW_CH], z[SC_TT][SW_CH];
+};
+struct ScanWideShared {
+    ScanWideTile in[3];
+    float bc[3][SC_TT + 2][2][SW_SUB * SW_NS];  // (two rows more: what is fetched ahead behind a tile's end is not used)
+    float raw[2][SC_TT][SW_CH];   // step sizes before the softplus
+    float2 dd[2][SC_TT + 2][SW_CH];  // dt, dt x
+    float y[2][SC_TT][SW_YP];
+};
+
+__global__ void __launch_bounds__(SW_THREADS, 2) scan_wide_kernel(ScanArgs a) {
+    extern __shared__ __align__(16) uint8_t sc_dyn[];
+    ScanWideShared& sh = *reinterpret_cast<ScanWideShared*>(sc_dyn);
+    constexpr int NS = SW_NS, NB = SW_SUB * NS;
+    chain_trigger();
+    const int tid = threadIdx.x, c0 = blockIdx.x * SW_CH, seg = blockIdx.y;
+    chain_wait();
+    const int start = a.seg_start[seg], len = a.seg_len[seg], pos0 = a.seg_pos0[seg], slot = a.seg_slot[seg];
+    const int nt = (len + SC_TT - 1) / SC_TT;
+    if (tid >= SW_MAIN) {
+        const int h = tid - SW_MAIN, pc = a.rp + 2 * NB;  // (9 to 16 states are kept as 16)
+        const __nv_bfloat16 *xz = static_cast<const __nv_bfloat16*>(a.xz), *xc = static_cast<const __nv_bfloat16*>(a.xc);
+        auto load = [&](int it) {
+            const int t0 = it * SC_TT, b3 = it % 3;
+            ScanWideTile& in = sh.in[b3];
+#pragma unroll
+            for (int u = 0; u < SC_TT * (SW_CH / 8) / SW_HELP; ++u) {
+                const int r = (h + u * SW_HELP) / (SW_CH / 8), v = (h + u * SW_HELP) % (SW_CH / 8) * 8;
+                const bool ok = t0 + r < len && c0 + v < a.ip;
+                const long long t = start + (ok ? t0 + r : 0);
+                const int cc = ok ? c0 + v : 0;
+                cp_async16(smem_u32(&in.x[r][v]), xc + t * a.ip + cc, ok);
+                cp_async16(smem_u32(&in.z[r][v]), xz + t * 2 * a.ip + a.ip + cc, ok);
+            }
+#pragma unroll
+            for (int u = 0; u < SC_TT * (SW_CH / 4) / SW_HELP; ++u) {
+                const int r = (h + u * SW_HELP) / (SW_CH / 4), v = (h + u * SW_HELP) % (SW_CH / 4) * 4;
+                const bool ok = t0 + r < len && c0 + v < a.ip;
+                cp_async16(smem_u32(&sh.raw[it & 1][r][v]), a.dt_raw + (long long)(start + (ok ? t0 + r : 0)) * a.ip + (ok ? c0 + v : 0), ok);
+            }
+#pragma unroll
+            for (int u = 0; u < SC_TT * 2 * (NB / 4) / SW_HELP; ++u) {
+                const int i = h + u * SW_HELP, r = i / (2 * (NB / 4)), part = i / (NB / 4) & 1, v = i % (NB / 4) * 4;
+                const bool ok = t0 + r < len;
+                cp_async16(smem_u32(&sh.bc[b3][r][part][v]), a.proj + (long long)(start + (ok ? t0 + r : 0)) * pc + a.rp + part * NB + v, ok);
+            }
+            cp_async_commit();
+        };
+        const int ov = h % (SW_CH / 4) * 4, row0 = h / (SW_CH / 4);  // four channels of every eighth token
+        const bool olive = c0 + ov < a.ip;
+        const float4 bias = olive ? *reinterpret_cast<const float4*>(a.dt_b + c0 + ov) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 D = olive ? *reinterpret_cast<const float4*>(a.D + c0 + ov) : make_float4(0.f, 0.f, 0.f, 0.f);
+        auto step_sizes = [&](int it) {
+            const int n = len - it * SC_TT;
+#pragma unroll
+            for (int r = row0; r < SC_TT; r += SW_HELP / (SW_CH / 4)) {
+                // a step size of zero leaves the state as it is: the rows behind the segment
+                const float4 w = *reinterpret_cast<const float4*>(&sh.raw[it & 1][r][ov]);
+                float x[4], d[4] = {softplus_t<__nv_bfloat16>(w.x + bias.x), softplus_t<__nv_bfloat16>(w.y + bias.y),
+                                    softplus_t<__nv_bfloat16>(w.z + bias.z), softplus_t<__nv_bfloat16>(w.w + bias.w)};
+                load4(&sh.in[it % 3].x[r][ov], x);
+                if (r >= n) d[0] = d[1] = d[2] = d[3] = 0.0f;
+                float4* o = reinterpret_cast<float4*>(&sh.dd[it & 1][r][ov]);
+                o[0] = make_float4(d[0], d[0] * x[0], d[1], d[1] * x[1]);
+                o[1] = make_float4(d[2], d[2] * x[2], d[3], d[3] * x[3]);
+            }
+        };
+        auto outputs = [&](int it) {
+            const int t0 = it * SC_TT, n = min(SC_TT, len - t0);
+            if (!olive) return;
+#pragma unroll
+            for (int r = row0; r < SC_TT; r += SW_HELP / (SW_CH / 4)) {
+                if (r >= n) break;
+                float xv[4], zv[4], o[4];
+                load4(&sh.in[it % 3].x[r][ov], xv);
+                load4(&sh.in[it % 3].z[r][ov], zv);
+                const float4 y = *reinterpret_cast<const float4*>(&sh.y[it & 1][r][ov]);
+                o[0] = fmaf(D.x, xv[0], y.x) * silu_t<__nv_bfloat16>(zv[0]); o[1] = fmaf(D.y, xv[1], y.y) * silu_t<__nv_bfloat16>(zv[1]);
+                o[2] = fmaf(D.z, xv[2], y.z) * silu_t<__nv_bfloat16>(zv[2]); o[3] = fmaf(D.w, xv[3], y.w) * silu_t<__nv_bfloat16>(zv[3]);
+                store4(static_cast<__nv_bfloat16*>(a.y) + (long long)(start + t0 + r) * a.ip + c0 + ov, o);
+            }
+        };
+        auto helpers_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(SW_HELP) : "memory"); };
+        load(0);
+        if (nt > 1) load(1);
+        if (nt > 1) cp_async_wait<1>();
+        else cp_async_wait<0>();
+        helpers_sync();
+        step_sizes(0);
+        __syncthreads();
+        for (int it = 0; it < nt; ++it) {
+            if (it > 0) outputs(it - 1);
+            if (it + 1 < nt) {
+                cp_async_wait<0>();
+                helpers_sync();  // tile it + 1 is there; nobody reads tile it - 1 any more
+                if (it + 2 < nt) load(it + 2);
+                step_sizes(it + 1);
+            }
+            __syncthreads();
+        }
+        if (nt > 0) outputs(nt - 1);
+        if (h < SW_CH && c0 + h < a.ip)
+            carry_conv_state(static_cast<__nv_bfloat16*>(a.conv) + (long long)slot * (a.taps - 1) * a.ip, xz, 2 * a.ip, c0 + h, a.ip, a.taps, start, len, pos0);
+        return;
+    }
+    const int ch = tid / SW_SUB, sub = tid % SW_SUB, c = c0 + ch;
+    const bool live = c < a.ip;
+    float* state = a.S + (long long)slot * a.ip * NB;
+    uint64_t A[NS / 2], S[NS / 2];
+#pragma unroll
+    for (int i = 0; i < NS / 2; ++i) {
+        float p[2], q[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int n = sub * NS + 2 * i + e;
+            p[e] = live && n < a.state ? a.A[plane_index(n, c, a.ip)] * LOG2E : 0.0f;
+            q[e] = live && n < a.state && pos0 > 0 ? state[plane_index(n, c, a.ip)] : 0.0f;
+        }
+        A[i] = f2_pack(p[0], p[1]);
+        S[i] = f2_pack(q[0], q[1]);
+    }
+    __syncthreads();
+    for (int it = 0; it < nt; ++it) {
+        const int n = min(SC_TT, len - it * SC_TT), b3 = it % 3, b2 = it & 1;
+        float2 w[4];
+        uint64_t B[2][NS / 2], C[2][NS / 2], decay[2][NS / 2];
+        auto fetch = [&](int t, int x) {
+            lds_pairs<NS>(&sh.bc[b3][t][0][sub * NS], B[x & 1]);
+            lds_pairs<NS>(&sh.bc[b3][t][1][sub * NS], C[x & 1]);
+        };
+        auto decays = [&](int x) {
+            const uint64_t dt = f2_pack(w[x & 3].x, w[x & 3].x);
+#pragma unroll
+            for (int i = 0; i < NS / 2; ++i) {
+                float e0, e1;
+                f2_unpack(f2_mul(dt, A[i]), e0, e1);
+                decay[x & 1][i] = f2_pack(fast_ex2(e0), fast_ex2(e1));
+            }
+        };
+        w[0] = sh.dd[b2][0][ch];
+        w[1] = sh.dd[b2][1][ch];
+        fetch(0, 0);
+        decays(0);
+#pragma unroll 1
+        for (int t8 = 0; t8 < n; t8 += 8) {
+            float y[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                fetch(t8 + u + 1, u + 1);
+                w[(u + 2) & 3] = sh.dd[b2][t8 + u + 2][ch];
+                decays(u + 1);
+                const uint64_t dx = f2_pack(w[u & 3].y, w[u & 3].y);
+                uint64_t acc[2] = {0, 0};
+#pragma unroll
+                for (int i = 0; i < NS / 2; ++i) {
+                    S[i] = f2_fma(decay[u & 1][i], S[i], f2_mul(dx, B[u & 1][i]));
+                    acc[i & 1] = i < 2 ? f2_mul(S[i], C[u & 1][i]) : f2_fma(S[i], C[u & 1][i], acc[i & 1]);
+                }
+                float lo[2], hi[2];
+                f2_unpack(acc[0], lo[0], hi[0]);
+                f2_unpack(acc[1], lo[1], hi[1]);
+                y[u] = (lo[0] + lo[1]) + (hi[0] + hi[1]);
+            }
+            column_sums<SW_SUB>(y, sub);
+#pragma unroll
+            for (int u = 0; u < 8 / SW_SUB; ++u) sh.y[b2][t8 + 8 / SW_SUB * sub + u][ch] = y[u];
+        }
+        __syncthreads();
+    }
+    if (live)
+#pragma unroll
+        for (int i = 0; i < NS / 2; ++i) {
+            float p[2];
+            f2_unpack(S[i], p[0], p[1]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                if (sub * NS + 2 * i + e < a.state) state[plane_index(sub * NS + 2 * i + e, c, a.ip)] = p[e];
+        }
 }
 
 // ---- decode step --------------------------------------------------------------------------------------------------
@@ -609,9 +827,10 @@ static ScanArgs scan_args(const ScanDims& d, const ScanWeights& w, const ScanSta
 
 template <typename T, int NS>
 static jsm_status scan_go(const ScanArgs& a, cudaStream_t st) {
+    constexpr int smem = scan_smem<T, NS>();
     static DeviceOnce once;  // per instantiation
-    JSM_CUDA_CHECK(allow_shared(once, scan_kernel<T, NS>, 220 * 1024));
-    JSM_CUDA_CHECK(launch_spread(scan_kernel<T, NS>, dim3((a.ip + SC_CH - 1) / SC_CH, a.n_segs), dim3(SC_THREADS), scan_smem<T>(a.np, NS), st, a));
+    JSM_CUDA_CHECK(allow_shared(once, scan_kernel<T, NS>, smem));
+    JSM_CUDA_CHECK(launch_spread(scan_kernel<T, NS>, dim3((a.ip + SC_CH - 1) / SC_CH, a.n_segs), dim3(SC_THREADS), smem, st, a));
     JSM_LAUNCH_CHECK();
     return JSM_OK;
 }
@@ -624,9 +843,20 @@ static jsm_status step_go(const ScanArgs& a, cudaStream_t st) {
     JSM_LAUNCH_CHECK();
     return JSM_OK;
 }
+static jsm_status scan_wide_go(const ScanArgs& a, cudaStream_t st) {
+    static DeviceOnce once;
+    JSM_CUDA_CHECK(allow_shared(once, scan_wide_kernel, (int)sizeof(ScanWideShared)));
+    JSM_CUDA_CHECK(launch_spread(scan_wide_kernel, dim3((a.ip + SW_CH - 1) / SW_CH, a.n_segs), dim3(SW_THREADS), sizeof(ScanWideShared), st, a));
+    JSM_LAUNCH_CHECK();
+    return JSM_OK;
+}
 // the smallest instance whose threads hold a channel's states
 template <typename T>
 static jsm_status scan_dispatch(const ScanArgs& a, cudaStream_t st) {
+    // Two blocks of scan_kernel fit beside one another on an SM without slowing each other down much (2048 tokens, scan_kernel / scan_wide_kernel, us:
+    // 128 blocks 118 / 129, 256 blocks 134 / 130, 384 blocks 156 / 131, 512 blocks 186 / 131; 64 tokens, 256 blocks 8.1 / 8.1, 512 blocks 10.4 / 8.9).
+    if constexpr (sizeof(T) == 2)
+        if (a.state > 8 && a.state <= 16 && (long long)((a.ip + SC_CH - 1) / SC_CH) * a.n_segs > 2ll * sm_count()) return scan_wide_go(a, st);
     return a.state <= 8 ? scan_go<T, 1>(a, st) : a.state <= 16 ? scan_go<T, 2>(a, st) : a.state <= 24 ? scan_go<T, 3>(a, st)
          : a.state <= 32 ? scan_go<T, 4>(a, st) : a.state <= 64 ? scan_go<T, 8>(a, st) : scan_go<T, 16>(a, st);
 }
