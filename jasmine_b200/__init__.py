@@ -3,7 +3,8 @@
 The product is the CUDA library and the C++20 headers under include/jasmine/.
 This package only loads the library with ctypes and wraps torch tensors (used
 for device memory, streams and torch.distributed) into the C structs, for the
-tests and bench.py.  There is no CPU or eager fallback: when the shared library
+tests and bench.py; the short calls go through _native.so (csrc/py_calls.cpp),
+which does the same without the interpreter.  There is no CPU or eager fallback: when the shared library
 is missing, `lib()` raises.
 """
 from __future__ import annotations

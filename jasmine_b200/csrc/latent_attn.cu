@@ -8,9 +8,10 @@
 // expanded to values once per query.  That form serves decode steps and short portions of a prompt: the cache entry is
 // read once for all heads.  Long portions expand keys and values instead (decoder.cu) and run the flash kernel.
 //
-// Kernels: latent_prep (norm of the latent, rotations, append), latent_project_* (queries into the latent space, latents to
-// values: one small matrix per head), latent_attn_* (scores, softmax, weighted sum; split over the keys when there are few
-// queries), latent_combine (merges the splits), latent_gather (contiguous copy of cached entries).
+// Kernels: latent_query (append, and queries into the latent space), latent_attn_* (scores, softmax, weighted sum; split over the
+// keys when there are few queries), latent_value (merges the splits and takes the latents to values); where those do not
+// apply latent_prep (norm of the latent, rotations, append), latent_project_* (one small matrix per head) before and after,
+// latent_combine (merges the splits); latent_gather (contiguous copy of cached entries).
 #include "decoder_ops.cuh"
 #include "mma_utils.cuh"
 #include "tc_utils.cuh"
