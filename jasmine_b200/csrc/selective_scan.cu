@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(SC_THREADS) scan_kernel(ScanArgs a) {
 // one per scheduler, the decays of a token computed while the one before it moves the state.  Four more warps bring the
 // tiles, make the step sizes of the next one and write the outputs of the last one meanwhile.  A CTA owns 64 channels.
 // 2048 tokens, 16 states, 8192 channels: 219 -> 131 us (scan_kernel 186, where addresses with constant strides and states kept as pairs save a
-// seventh); the exponential units are then about 2/3 in use on the SMs that have a CTA.  Eight walking warps of four states
+// seventh); the exponential units are then 77 % in use on the 128 SMs that have a CTA.  Eight walking warps of four states
 // 148 us, eight warps beside the walking ones 156; 2 CTAs per SM are named because the compiler then takes 126 registers, without that 66 (165 us).
 constexpr int SW_CH = 64, SW_SUB = 2, SW_NS = 8, SW_HELP = 128, SW_MAIN = SW_CH * SW_SUB, SW_THREADS = SW_MAIN + SW_HELP, SW_YP = SW_CH + 4;
 struct ScanWideTile {  // a tile as it arrives
