@@ -284,9 +284,10 @@ struct ScanArgs {
     int ip, np, rp, state, taps, n_segs;
 };
 
-// NS states per thread
+// NS states per thread.  The bf16 instance of 9 to 16 states only runs with up to two CTAs per SM (scan_dispatch): a minimum of four gives it 120
+// registers instead of 54, and the loads of a group of tokens move ahead (2048 tokens, 2048 channels 118 -> 107 us, 4096 channels 135 -> 127).
 template <typename T, int NS>
-__global__ void __launch_bounds__(SC_THREADS) scan_kernel(ScanArgs a) {
+__global__ void __launch_bounds__(SC_THREADS, sizeof(T) == 2 && NS == 2 ? 4 : 0) scan_kernel(ScanArgs a) {
     extern __shared__ __align__(16) uint8_t sc_dyn[];
     constexpr int CH = SC_CH, SUB = SC_SUB, YP = CH + 4, NB = SUB * NS;     // YP: pitch of the output tile; NB: B / C columns per tile row
     constexpr int EL = SC_TT * CH / SC_THREADS;                             // elements of a tile per thread
@@ -854,7 +855,8 @@ static jsm_status scan_wide_go(const ScanArgs& a, cudaStream_t st) {
 template <typename T>
 static jsm_status scan_dispatch(const ScanArgs& a, cudaStream_t st) {
     // Two blocks of scan_kernel fit beside one another on an SM without slowing each other down much (2048 tokens, scan_kernel / scan_wide_kernel, us:
-    // 128 blocks 118 / 129, 256 blocks 134 / 130, 384 blocks 156 / 131, 512 blocks 186 / 131; 64 tokens, 256 blocks 8.1 / 8.1, 512 blocks 10.4 / 8.9).
+    // 128 blocks 107 / 129, 256 blocks 127 / 130, 384 blocks 156 / 131, 512 blocks 186 / 131; 64 tokens, 256 blocks 8.1 / 8.1, 512 blocks 10.4 / 8.9;
+    // the figures of 384 and 512 blocks before the register target above).
     if constexpr (sizeof(T) == 2)
         if (a.state > 8 && a.state <= 16 && (long long)((a.ip + SC_CH - 1) / SC_CH) * a.n_segs > 2ll * sm_count()) return scan_wide_go(a, st);
     return a.state <= 8 ? scan_go<T, 1>(a, st) : a.state <= 16 ? scan_go<T, 2>(a, st) : a.state <= 24 ? scan_go<T, 3>(a, st)
