@@ -704,7 +704,7 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(const float* __rest
 }
 
 // Decode steps of few tokens: the merge inside the projection to values.  A CTA has 16 rows of one head; its four warps share the rank.  A
-// lane weighs the splits of its token and adds its own components of them while the operand forms (the same sums as in
+// lane weighs the splits of its token and adds its own components of them while the operand forms (the same sums in the same order as in
 // latent_combine_kernel, rounded to bf16 as the stored latents were); four splits of all its components are requested at once, so that
 // a short context costs one round trip.  Eight CTAs read a head's partial sums: with many tokens a merge of its own is cheaper.
 constexpr int LV_MAX_TOKENS = 16, LV_BLOCKS = 4;
@@ -731,6 +731,29 @@ __global__ void __launch_bounds__(128) latent_value_kernel(ProjectArgs a, const 
         const int t = j * 8 + g, pos = t < a.T ? load_early(tok_pos + t) : 0;
         live[j] = t < a.T ? min(max_splits, pos / PAGE - max(0, pos - d.window + 1) / PAGE + 1) : 0;
     }
+    // Maximum and sum of a row over its n splits, by the four lanes of a token: lane x takes the splits x, x + 4, ..., and the sums meet in the order of
+    // latent_combine_kernel (lane s % 32 there holds split s, five exchanges from 16 down).
+    const uint32_t quad = 0xFu << (lane & 28);
+    auto weigh = [&](const float* p, int n, float& m, float& l) {
+        float2 ml[8];
+        const float* mine = p + (lane & 3) * stride + rp;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) ml[k] = 4 * k + (lane & 3) < n ? *reinterpret_cast<const float2*>(mine + 4 * k * stride) : make_float2(-INFINITY, 0.0f);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) m = fmaxf(m, ml[k].x);
+        for (int s = 32 + (lane & 3); s < n; s += 4) m = fmaxf(m, p[s * stride + rp]);
+        m = fmaxf(m, __shfl_xor_sync(quad, m, 2));
+        m = fmaxf(m, __shfl_xor_sync(quad, m, 1));
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            float sum = __expf(ml[k].x - m) * ml[k].y;
+            for (int s = 32 + 4 * k + (lane & 3); s < n; s += 32) sum = fmaf(__expf(p[s * stride + rp] - m), p[s * stride + rp + 1], sum);
+            ml[k].y = sum;
+        }
+        l = ((ml[0].y + ml[4].y) + (ml[2].y + ml[6].y)) + ((ml[1].y + ml[5].y) + (ml[3].y + ml[7].y));
+        l += __shfl_xor_sync(quad, l, 2);
+        l += __shfl_xor_sync(quad, l, 1);
+    };
     chain_wait();
     float acc[4][4];
 #pragma unroll
@@ -745,14 +768,12 @@ __global__ void __launch_bounds__(128) latent_value_kernel(ProjectArgs a, const 
         for (int i = 0; i < LV_BLOCKS; ++i)
 #pragma unroll
             for (int e = 0; e < 8; ++e) v[i][e] = 0.0f;
-        for (int s = 4; s < n; ++s) m = fmaxf(m, p[s * stride + rp]);
         for (int s0 = 0; s0 < n; s0 += 4) {
-            float2 ml[4];
-            float u[4][LV_BLOCKS][8];
+            float ms[4], u[4][LV_BLOCKS][8];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const float* ps = p + (s0 + q) * stride;
-                ml[q] = s0 + q < n ? *reinterpret_cast<const float2*>(ps + rp) : make_float2(-INFINITY, 0.0f);
+                ms[q] = s0 + q < n ? ps[rp] : -INFINITY;
 #pragma unroll
                 for (int i = 0; i < LV_BLOCKS; ++i) {
                     const int k = (b0 + i) * 32 + kq;
@@ -762,17 +783,17 @@ __global__ void __launch_bounds__(128) latent_value_kernel(ProjectArgs a, const 
                         for (int e = 0; e < 8; ++e) u[q][i][e] = 0.0f;
                 }
             }
-            if (s0 == 0) m = fmaxf(m, fmaxf(fmaxf(ml[0].x, ml[1].x), fmaxf(ml[2].x, ml[3].x)));
+            if (s0 == 0) weigh(p, n, m, l);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const float f = __expf(ml[q].x - m);
-                l = fmaf(f, ml[q].y, l);
+                const float f = __expf(ms[q] - m);
 #pragma unroll
                 for (int i = 0; i < LV_BLOCKS; ++i)
 #pragma unroll
                     for (int e = 0; e < 8; ++e) v[i][e] = fmaf(f, u[q][i][e], v[i][e]);
             }
         }
+        __syncwarp();
         const float inv = 1.0f / l;
 #pragma unroll
         for (int i = 0; i < LV_BLOCKS; ++i)
@@ -824,9 +845,9 @@ bool latent_mma_usable(const LatentDims& d) {
 
 int latent_splits(int n_tiles, int max_keys) {
     if (n_tiles <= 0) return 1;
-    // a split of its own for every page of a short context, two pages each beyond
+    // Two pages and more each.  A split rounds its weights to bf16 under its own maximum: the number of splits is part of the result.
     const int pages = max_keys / PAGE + 2;
-    return std::max(1, std::min({sm_count() / n_tiles, std::max(std::min(pages, 4), pages / 2), LA_MAX_SPLITS}));
+    return std::max(1, std::min({sm_count() / n_tiles, pages / 2, LA_MAX_SPLITS}));
 }
 size_t latent_part_floats(const LatentDims& d) { return (size_t)sm_count() * LA_ROWS * (pad8(d.rank) + LA_ML); }
 
