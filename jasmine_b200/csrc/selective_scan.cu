@@ -461,6 +461,11 @@ struct ScanWideShared {
     float2 dd[2][SC_TT + 2][SW_CH];  // dt, dt x
     float y[2][SC_TT][SW_YP];
 };
+// A token's sum over the states is formed in the order of scan_kernel, so that a prompt's outputs do not depend on which of the two runs: there thread k
+// adds states 2 k and 2 k + 1, and eight such pairs meet in exchanges of distance 4, 2 and 1.  So a thread here has the pairs sub, sub + 2, sub + 4
+// and sub + 6, the even and the odd states of two pairs packed: element e of register i is state sw_state(sub, i, e), which lies at sw_place.
+__device__ __forceinline__ int sw_state(int sub, int i, int e) { return 2 * (sub + 2 * e + 4 * (i >> 1)) + (i & 1); }
+__device__ __forceinline__ int sw_place(int n) { return (n >> 1 & 1) * SW_NS + (n >> 3) * 4 + (n & 1) * 2 + (n >> 2 & 1); }
 
 __global__ void __launch_bounds__(SW_THREADS, 2) scan_wide_kernel(ScanArgs a) {
     extern __shared__ __align__(16) uint8_t sc_dyn[];
@@ -493,10 +498,10 @@ __global__ void __launch_bounds__(SW_THREADS, 2) scan_wide_kernel(ScanArgs a) {
                 cp_async16(smem_u32(&sh.raw[it & 1][r][v]), a.dt_raw + (long long)(start + (ok ? t0 + r : 0)) * a.ip + (ok ? c0 + v : 0), ok);
             }
 #pragma unroll
-            for (int u = 0; u < SC_TT * 2 * (NB / 4) / SW_HELP; ++u) {
-                const int i = h + u * SW_HELP, r = i / (2 * (NB / 4)), part = i / (NB / 4) & 1, v = i % (NB / 4) * 4;
+            for (int u = 0; u < SC_TT * 2 * NB / SW_HELP; ++u) {
+                const int r = h / (2 * NB) + u * (SW_HELP / (2 * NB)), part = h / NB & 1, n = h % NB;
                 const bool ok = t0 + r < len;
-                cp_async16(smem_u32(&sh.bc[b3][r][part][v]), a.proj + (long long)(start + (ok ? t0 + r : 0)) * pc + a.rp + part * NB + v, ok);
+                cp_async4(smem_u32(&sh.bc[b3][r][part][sw_place(n)]), a.proj + (long long)(start + (ok ? t0 + r : 0)) * pc + a.rp + part * NB + n, ok);
             }
             cp_async_commit();
         };
@@ -566,7 +571,7 @@ __global__ void __launch_bounds__(SW_THREADS, 2) scan_wide_kernel(ScanArgs a) {
         float p[2], q[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-            const int n = sub * NS + 2 * i + e;
+            const int n = sw_state(sub, i, e);
             p[e] = live && n < a.state ? a.A[plane_index(n, c, a.ip)] * LOG2E : 0.0f;
             q[e] = live && n < a.state && pos0 > 0 ? state[plane_index(n, c, a.ip)] : 0.0f;
         }
@@ -604,16 +609,17 @@ __global__ void __launch_bounds__(SW_THREADS, 2) scan_wide_kernel(ScanArgs a) {
                 w[(u + 2) & 3] = sh.dd[b2][t8 + u + 2][ch];
                 decays(u + 1);
                 const uint64_t dx = f2_pack(w[u & 3].y, w[u & 3].y);
-                uint64_t acc[2] = {0, 0};
+                uint64_t part[NS / 2];
 #pragma unroll
                 for (int i = 0; i < NS / 2; ++i) {
                     S[i] = f2_fma(decay[u & 1][i], S[i], f2_mul(dx, B[u & 1][i]));
-                    acc[i & 1] = i < 2 ? f2_mul(S[i], C[u & 1][i]) : f2_fma(S[i], C[u & 1][i], acc[i & 1]);
+                    part[i] = f2_mul(S[i], C[u & 1][i]);
                 }
-                float lo[2], hi[2];
-                f2_unpack(acc[0], lo[0], hi[0]);
-                f2_unpack(acc[1], lo[1], hi[1]);
-                y[u] = (lo[0] + lo[1]) + (hi[0] + hi[1]);
+                // (apart: a packed product whose only use is a packed sum becomes an FMA, which does not round the product)
+                float p[NS / 2][2];
+#pragma unroll
+                for (int i = 0; i < NS / 2; ++i) f2_unpack(part[i], p[i][0], p[i][1]);
+                y[u] = ((p[0][0] + p[1][0]) + (p[2][0] + p[3][0])) + ((p[0][1] + p[1][1]) + (p[2][1] + p[3][1]));
             }
             column_sums<SW_SUB>(y, sub);
 #pragma unroll
@@ -628,7 +634,7 @@ __global__ void __launch_bounds__(SW_THREADS, 2) scan_wide_kernel(ScanArgs a) {
             f2_unpack(S[i], p[0], p[1]);
 #pragma unroll
             for (int e = 0; e < 2; ++e)
-                if (sub * NS + 2 * i + e < a.state) state[plane_index(sub * NS + 2 * i + e, c, a.ip)] = p[e];
+                if (sw_state(sub, i, e) < a.state) state[plane_index(sw_state(sub, i, e), c, a.ip)] = p[e];
         }
 }
 

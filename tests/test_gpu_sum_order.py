@@ -1,4 +1,5 @@
-"""Sums whose order is part of a result.  A latent attention step against logits recorded with two pages and more per split."""
+"""Sums whose order is part of a result.  A latent attention step against logits recorded with two pages and more per split; a selective scan of prompts
+that has to give the same bits whichever of its kernels runs."""
 from pathlib import Path
 
 import numpy as np
@@ -33,3 +34,22 @@ def test_latent_steps_round_as_recorded(name):
     pages either way: not at all).  Sums in another order only turn a rounding here and there, 2^-8 of one of thousands of numbers: under 1e-4."""
     got, want = latent_steps(*CASES[name]).astype(np.float64), np.load(RECORDED)[name].astype(np.float64)
     assert np.sqrt(((got - want) ** 2).mean() / (want ** 2).mean()) < 2e-4
+
+
+def test_scan_does_not_depend_on_the_batch():
+    """27 blocks of 16 channels: with 12 segments more than twice the 148 SMs (two threads per channel), with 7 fewer (eight threads).  The first six
+    segments lie at the same places of equally many tokens, so that only the scan differs."""
+    cfg = zu.config([zu.mamba(inner=424, state=16, conv=4)], width=48)
+    w = zu.random_weights(cfg, 5)
+    lens = [130, 97, 64, 33, 150, 126]
+    seqs = [zu.tokens(n, cfg["vocab"], n) for n in lens]
+    rest = zu.tokens(120, cfg["vocab"], 1)
+    got = []
+    for parts in ([20] * 6, [120]):
+        m = zu.build(cfg, w, "bfloat16", max_batch=12, max_step_tokens=1024)
+        ends = np.concatenate([[0], np.cumsum(parts)])
+        entries = seqs + [rest[a:b] for a, b in zip(ends[:-1], ends[1:])]
+        _, lg = m.step([(m.open(), s) for s in entries], range(sum(lens)))
+        got.append(lg.copy())
+        m.close()
+    assert np.array_equal(got[0], got[1])
