@@ -258,15 +258,19 @@ __global__ void __launch_bounds__(256) final_norm_kernel(const float* x, const i
             if (c < wp) load_f32x8(gain + c, g[i]);
         }
         chain_wait();
+        float s[8 * MAXV];  // (the sum runs over every 256th component, as below: both ways give the same number)
+#pragma unroll
+        for (int i = 0; i < 8 * MAXV; ++i) {
+            const int c = i * 256 + threadIdx.x;
+            s[i] = c < d ? src[c] : 0.0f;
+        }
 #pragma unroll
         for (int i = 0; i < MAXV; ++i) {
             const int c = (i * 256 + threadIdx.x) * 8;
-            if (c < wp) {
-                load_f32x8(src + c, v[i]);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) q = fmaf(v[i][e], v[i][e], q);
-            }
+            if (c < wp) load_f32x8(src + c, v[i]);
         }
+#pragma unroll
+        for (int i = 0; i < 8 * MAXV; ++i) q = fmaf(s[i], s[i], q);
         const float rms = sqrtf(block_sum(q, smem) / (float)d + eps);
 #pragma unroll
         for (int i = 0; i < MAXV; ++i) {

@@ -1,10 +1,11 @@
 """Sums whose order is part of a result.  A latent attention step against logits recorded with two pages and more per split; a selective scan of prompts
-that has to give the same bits whichever of its kernels runs."""
+that has to give the same bits whichever of its kernels runs; the sum of squares of the final norm."""
 from pathlib import Path
 
 import numpy as np
 import pytest
 
+import vagonex_util as vu
 import zugolorn_util as zu
 
 pytestmark = pytest.mark.gpu
@@ -53,3 +54,36 @@ def test_scan_does_not_depend_on_the_batch():
         got.append(lg.copy())
         m.close()
     assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("width", [40, 520, 1032, 4096, 4104])
+def test_sum_of_squares_of_the_final_norm(width):
+    """Component c belongs to thread c % 256, a warp's sums meet in exchanges from 16 down, the warps' sums in order: with an embedding whose first rows are
+    those of the identity the logits are the normed row, bit for bit."""
+    import torch
+    rng = np.random.default_rng(width)
+    n = 40
+    embed = np.concatenate([np.eye(width), rng.standard_normal((n, width))]).astype(np.float32)
+    cfg = vu.config([vu.lightning(heads=1, dim=8, vdim=8)], width=width, vocab=width + n, alpha=1.0, scale=1.0, eps=1e-6)
+    gain = rng.standard_normal(width).astype(np.float32)
+    w = {"embed": embed, "final.norm": gain, "l0.norm1": np.ones(width, np.float32), "l0.mix.norm": np.ones(8, np.float32)}
+    w.update({"l0.mix." + s: np.zeros((8, width), np.float32) for s in "qkvg"}, **{"l0.mix.o": np.zeros((width, 8), np.float32)})
+    m = vu.build(cfg, w, "float32", max_batch=1, max_context=64, max_step_tokens=64)
+    tap = torch.zeros(1, n, width, device="cuda")
+    m.set_tap(tap)
+    _, lg = m.step([(m.open(), list(range(width, width + n)))], range(n))
+    m.close()
+    x = tap[0].cpu().numpy()
+    f32 = np.float32
+    part = np.zeros((n, 256), f32)
+    for c0 in range(0, width, 256):
+        v = x[:, c0:c0 + 256].astype(np.float64)
+        part[:, :v.shape[1]] = (v * v + part[:, :v.shape[1]]).astype(f32)
+    lanes = part.reshape(n, 8, 32)
+    for o in (16, 8, 4, 2, 1):
+        lanes = lanes + lanes[..., np.arange(32) ^ o]
+    total = np.zeros(n, f32)
+    for k in range(8):
+        total = total + lanes[:, k, 0]
+    rms = np.sqrt(total / f32(width) + f32(1e-6))
+    assert np.array_equal(lg[:, :width], x / rms[:, None] * gain)
