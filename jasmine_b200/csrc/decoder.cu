@@ -18,6 +18,7 @@
 #include "linear_bf16.cuh"
 #include "attn.cuh"
 #include "paged_rows.cuh"
+#include "pass_errors.h"
 #include <math.h>
 #include <string.h>
 #include <algorithm>
@@ -807,12 +808,9 @@ static jsm_status run_pass(jsm_decoder* m, std::vector<PassSeg> segs, const int3
         // (two copies to pageable memory and a wait for each held a step up by 20 us)
         JSM_CUDA_CHECK(cudaMemcpyAsync(m->h_out, m->next_dev, 2 * sizeof(int32_t) * P.n_want, cudaMemcpyDeviceToHost, st));
         JSM_CUDA_CHECK(cudaStreamSynchronize(st));
-        bool failed = false;
-        for (int i = 0; i < P.n_want; ++i) {
-            if (h_next) h_next[want[i].second] = m->h_out[i];
-            failed |= m->h_out[P.n_want + i] != 0;
-        }
-        if (failed) DEC_TRY(tc_check_error(st, "jsm_decoder_step"));
+        for (int i = 0; h_next && i < P.n_want; ++i) h_next[want[i].second] = m->h_out[i];
+        DEC_TRY(pass_status(
+            m->h_out + P.n_want, P.n_want, [&] { return tc_check_error(st, "jsm_decoder_step"); }, [](int code) { return tc_error_status(code, "jsm_decoder_step"); }));
     } else {
         DEC_TRY(tc_check_error(st, "jsm_decoder_step"));
         JSM_CUDA_CHECK(cudaStreamSynchronize(st));

@@ -393,6 +393,10 @@ jsm_status linear_bf16_launch(const LinearArgs& a, cudaStream_t st) {
     }
 }
 
+jsm_status tc_error_status(int code, const char* who) {
+    if (code == 32) JSM_FAIL(JSM_SHAPE, "%s: context overflow: a decode step met a sequence that already holds max_context tokens", who);
+    JSM_FAIL(JSM_TIMEOUT, "%s: a bounded device-side wait ran out (code %d)", who, code);
+}
 jsm_status tc_check_error(cudaStream_t st, const char* who) {
     int* w = tc_error_word();
     if (!w) return JSM_OK;
@@ -401,8 +405,7 @@ jsm_status tc_check_error(cudaStream_t st, const char* who) {
     JSM_CUDA_CHECK(cudaStreamSynchronize(st));
     if (h != 0) {
         cudaMemsetAsync(w, 0, sizeof(int), st);
-        if (h == 32) JSM_FAIL(JSM_SHAPE, "%s: context overflow: a decode step met a sequence that already holds max_context tokens", who);
-        JSM_FAIL(JSM_TIMEOUT, "%s: a bounded device-side wait ran out (code %d)", who, h);
+        return tc_error_status(h, who);
     }
     return JSM_OK;
 }

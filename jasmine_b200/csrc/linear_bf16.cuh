@@ -128,6 +128,7 @@ long long tp_wait_limit_cycles();
 bool linear_packed_can_push(int N, int K, int T);
 // dimensions of the packed image
 void pk_dims(int N, int K, int paired, int* n_tiles, int* kbt);
+jsm_status tc_error_status(int code, const char* who);  // the failure that a code of the error word stands for
 // reads (and clears) the device error word of the tensor-core kernels; synchronises the stream
 jsm_status tc_check_error(cudaStream_t st, const char* who);
 
