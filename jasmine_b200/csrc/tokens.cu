@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(256) logits_finish_kernel(float* __restrict__ 
             const unsigned long long top = atomicExch(keys + r, 0ull);
             next[r] = top ? (int32_t)(0xffffffffu - (uint32_t)(top & 0xffffffffull)) : 0;
             ctrs[r] = 0;
-            if (err_out) err_out[r] = __ldcg(err);  // (the step's earlier kernels have ended)
+            if (err_out) err_out[r] = err ? __ldcg(err) : 0;  // (the step's earlier kernels have ended)
         }
     }
 }
