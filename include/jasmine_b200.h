@@ -340,6 +340,7 @@ jsm_status jsm_post_norm_add(const float* d_y, float* d_x, const float* d_gain, 
 jsm_status jsm_sum_norm(const float* d_y, float* d_x, const float* d_gain, float eps, float alpha, void* d_x_bf16, int T, int d,
                         void* stream);
 /* logits <- cap * tanh(logits / cap) in place (cap 0: unchanged) and the arg-max of every row (the first maximum).
+ * Nothing behind a row's vocab logits is read or written: the last row needs no padding.
  * d_keys U64 [rows], d_counters I32 [rows]: zero before the first call; the kernel leaves them zero. */
 jsm_status jsm_logits_finish(float* d_logits, int pitch, int rows, int vocab, float cap, uint64_t* d_keys, int32_t* d_counters,
                              int32_t* d_next, void* stream);

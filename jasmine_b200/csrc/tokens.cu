@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(256) logits_finish_kernel(float* __restrict__ 
     constexpr int W = VEC ? 4 : 1, DEEP = 4;
     const int r = blockIdx.y;
     float* row = logits + (long long)r * pitch;
-    const int groups = (vocab + W - 1) / W;  // (a last group may reach into the row's padding)
+    const int groups = (vocab + W - 1) / W;  // (a last group may be a part of one)
     const int lo = (int)((long long)blockIdx.x * groups / gridDim.x), hi = (int)((long long)(blockIdx.x + 1) * groups / gridDim.x);
     unsigned long long key = 0;  // below every value's key
     for (int i0 = lo + threadIdx.x; i0 < hi; i0 += 256 * DEEP) {
@@ -321,9 +321,12 @@ __global__ void __launch_bounds__(256) logits_finish_kernel(float* __restrict__ 
         for (int u = 0; u < DEEP; ++u) {
             const int i = i0 + u * 256;
             if (i >= hi) continue;
-            if constexpr (VEC) {
+            if (VEC && i * 4 + 4 <= vocab) {
                 const float4 f = *reinterpret_cast<const float4*>(row + i * 4);
-                v[u][0] = f.x; v[u][1] = f.y; v[u][2] = f.z; v[u][3] = f.w;
+                v[u][0] = f.x; v[u][1 % W] = f.y; v[u][2 % W] = f.z; v[u][3 % W] = f.w;
+            } else if (VEC) {  // (the last row may end with the vocabulary)
+#pragma unroll
+                for (int e = 0; e < W; ++e) v[u][e] = i * W + e < vocab ? row[i * W + e] : 0.0f;
             } else {
                 v[u][0] = row[i];
             }
@@ -423,7 +426,7 @@ jsm_status logits_finish_launch(float* logits, int pitch, int vocab, float cap, 
                                 cudaStream_t st, const int* err, int32_t* err_out) {
     if (rows <= 0) return JSM_OK;
     const int slices = std::max(1, std::min(16, vocab / 1024));
-    const bool vec = pitch % 4 == 0 && reinterpret_cast<uintptr_t>(logits) % 16 == 0;  // (then pitch >= vocab rounded up to fours)
+    const bool vec = pitch % 4 == 0 && reinterpret_cast<uintptr_t>(logits) % 16 == 0;
     JSM_CUDA_CHECK(launch_chained(vec ? logits_finish_kernel<true> : logits_finish_kernel<false>, dim3(slices, rows), dim3(256), 0, st, logits, pitch, vocab, cap, keys, ctrs, next, err, err_out));
     JSM_LAUNCH_CHECK();
     return JSM_OK;

@@ -63,3 +63,22 @@ def test_logits_and_their_maximum(rows, pitch, vocab, cap):
     nxt = jb.logits_finish(x, vocab, cap)
     assert torch.allclose(x.double(), want, rtol=1e-6, atol=1e-6)
     assert nxt.tolist() == x[:, :vocab].cpu().numpy().argmax(1).tolist() and nxt[0] == vocab // 2
+
+
+@pytest.mark.parametrize("rows,pitch,vocab,cap", [(1, 4, 1, 2.0), (3, 72, 70, 5.0), (2, 8196, 8193, 0.0), (2, 8196, 8195, 3.0)])
+def test_logits_whose_last_row_has_no_padding(rows, pitch, vocab, cap):
+    """Rows of aligned fours in an allocation that ends with the last row's vocabulary (what lies behind it is not the caller's: nothing there is read)."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(vocab)
+    x = 4 * torch.randn((rows - 1) * pitch + vocab, generator=g, device="cuda")
+    valid = torch.cat([torch.arange(vocab) + r * pitch for r in range(rows)]).cuda()
+    before = x.clone()
+    want = before[valid].reshape(rows, vocab).double()
+    want = cap * torch.tanh(want / cap) if cap else want
+    keys, ctrs, nxt = torch.zeros(rows, dtype=torch.int64, device="cuda"), torch.zeros(rows, dtype=torch.int32, device="cuda"), torch.empty(rows, dtype=torch.int32, device="cuda")
+    jb.check(jb.lib().jsm_logits_finish(x.data_ptr(), pitch, rows, vocab, cap, keys.data_ptr(), ctrs.data_ptr(), nxt.data_ptr(), jb.stream_ptr()))
+    got = x[valid].reshape(rows, vocab)
+    assert torch.allclose(got.double(), want, rtol=1e-6, atol=1e-6)
+    assert nxt.tolist() == got.argmax(1).tolist()
+    padding = torch.ones_like(x, dtype=torch.bool).index_fill(0, valid, False)
+    assert torch.equal(x[padding], before[padding])
