@@ -380,8 +380,10 @@ __global__ void __launch_bounds__(AR_WARPS * PARTS * 32, 1) attn_paged_rows_kern
         if (warp * R + x >= n_rows) break;
         if constexpr (PARTS > 1) {
             const float m1 = shared[x * VL + VR * 32], l1 = shared[x * VL + VR * 32 + 1], top = fmaxf(m[x], m1);
-            // (a half without a weight has sums of zero, or NaN, and no maximum)
-            const float f0 = m[x] == -INFINITY ? 1.0f : expf(m[x] - top), f1 = m1 == -INFINITY ? 1.0f : expf(m1 - top);
+            // (a half without a weight has no maximum: its sums, zero or NaN or those of a sink of -inf, go in with a factor of 0; without
+            // any weight both stay as they are)
+            const bool none = top == -INFINITY;
+            const float f0 = none ? 1.0f : expf(m[x] - top), f1 = none ? 1.0f : expf(m1 - top);
             l[x] = fmaf(l[x], f0, l1 * f1);
 #pragma unroll
             for (int i = 0; i < VR; i += 4) {

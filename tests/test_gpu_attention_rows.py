@@ -21,3 +21,16 @@ def test_rows_that_share_keys(kw, sizes):
     m = vu.build(cfg, w)
     assert_close(vu.run_portions(m, toks, sizes), vo.forward(cfg, vu.oracle_weights(w), toks), 4e-5)  # (the bar of the other fp32 models)
     m.close()
+
+
+@pytest.mark.parametrize("size", [None, 33, 40, 70])
+@pytest.mark.parametrize("heads,kv_heads", [(16, 16), (16, 4), (16, 1)])
+def test_a_sink_that_is_switched_off(heads, kv_heads, size):
+    """A sink of -inf has no weight, also in a row whose keys all lie in the second group's tiles (a later chunk than that of the rows beside it)."""
+    import numpy as np
+    cfg = vu.config([vu.attention(heads=heads, kv_heads=kv_heads, dim=24, vdim=20, rot_dims=8, size=size)], alpha=0.6)
+    w, toks = vu.random_weights(cfg, 53), vu.tokens(100, 72, 54)
+    w["l0.mix.sink"] = vu.bf16_bits(np.where(np.arange(heads) % 3 == 2, 0.5, -np.inf))
+    m = vu.build(cfg, w)
+    assert_close(vu.run_portions(m, toks, [100]), vo.forward(cfg, vu.oracle_weights(w), toks), 4e-5)  # (the bar of the other fp32 models)
+    m.close()
