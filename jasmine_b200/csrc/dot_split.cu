@@ -21,10 +21,12 @@
 // Gate and up projections of a feed-forward run as pairs: 64 features' gate and up rows make one tile, and the activation follows where the sums meet (the
 // two products and a launch for the activation, 300 x 2752 x 1024: 43 us, here 32).
 //
-// Numbers beyond bf16's range (infinities, NaN, the last 2^-9 below fp32's largest) do not survive the split; every result that is not
-// finite is formed again by plain fp32 additions.  Parts below 2^-133 are lost.
+// Range.  Both operands are scaled by 2^39 on the way in, so that every fp32 number, the subnormal ones too, keeps all its parts, and the sums by 2^-78 on the
+// way out.  What leaves the range then (infinities, NaN, operands above 2^88, sums above 2^49) comes out as no finite number, and every such result is
+// formed again by plain fp32 additions.
 #include "tc_utils.cuh"
 #include "linear_epilogue.cuh"
+#include "mma_utils.cuh"
 #include <algorithm>
 #include <mutex>
 
@@ -68,22 +70,39 @@ __device__ __forceinline__ uint32_t ds_part(float& a, float& b) {
     return p;
 }
 
+// Operands are scaled on the way in: the smallest number that fp32 holds, 2^-149, keeps its parts above 2^-133, where bf16 ends
+constexpr float DS_SCALE = 0x1p39f, DS_BACK = 1.0f / (DS_SCALE * DS_SCALE);
+
+// sum += q; what the rounding leaves out goes to lost
+__device__ __forceinline__ void ds_add(float& sum, float& lost, float q) {
+    const float t = sum + q, p = t - sum;
+    lost += (sum - (t - p)) + (q - p);
+    sum = t;
+}
 // Products of one row of X with four rows of W by plain fp32 additions: blocks of 32 in two chains, as dot_f32_kernel adds them (what overflows on the
-// way is the same)
-static __device__ __noinline__ float4 ds_again(const float* w, long long ldw, const float* x, int K) {
-    float v[4];
-#pragma unroll
+// way is the same).  rows: bit j, whether number j is formed again.
+static __device__ __noinline__ float4 ds_again(float4 old, uint32_t rows, const float* w, long long ldw, const float* x, int K) {
+    float v[4] = {old.x, old.y, old.z, old.w};
+#pragma unroll 1
     for (int j = 0; j < 4; ++j) {
-        float sum = 0.0f;
+        if (!(rows >> j & 1)) continue;
+        float sum = 0.0f, lost = 0.0f;
         for (int k0 = 0; k0 < K && sum == sum; k0 += 32) {
             float even = 0.0f, odd = 0.0f;
-            for (int k = k0; k < min(K, k0 + 32); k += 2) {
-                even = fmaf(x[k], w[j * ldw + k], even);
-                odd = fmaf(x[k + 1], w[j * ldw + k + 1], odd);
+#pragma unroll
+            for (int k = k0; k < k0 + 32; k += 4) {
+                if (k >= K) break;
+                const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + j * ldw + k);
+                even = fmaf(a.x, b.x, even); odd = fmaf(a.y, b.y, odd);
+                even = fmaf(a.z, b.z, even); odd = fmaf(a.w, b.w, odd);
             }
-            sum += even + odd;
+            ds_add(sum, lost, even + odd);
         }
-        v[j] = sum;
+        if (fabsf(sum + lost) < INFINITY) sum += lost;
+        if (j == 0) v[0] = sum;
+        else if (j == 1) v[1] = sum;
+        else if (j == 2) v[2] = sum;
+        else v[3] = sum;
     }
     return make_float4(v[0], v[1], v[2], v[3]);
 }
@@ -160,6 +179,8 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dot_split_kernel(DotSplitParams
             for (int i = 0; i < ITEMS; ++i) {
                 float f[8] = {v[i][0].x, v[i][0].y, v[i][0].z, v[i][0].w, v[i][1].x, v[i][1].y, v[i][1].z, v[i][1].w};
                 load(i, b + 1);
+#pragma unroll
+                for (int e = 0; e < 8; e += 2) f2_unpack(f2_mul(f2_pack(f[e], f[e + 1]), f2_pack(DS_SCALE, DS_SCALE)), f[e], f[e + 1]);
                 uint4* at = reinterpret_cast<uint4*>(to + (i < W_ITEMS ? i * ROWS_PASS * 128 : X_OFF + (i - W_ITEMS) * ROWS_PASS * 128));
                 auto part = [&]() {
                     uint4 h;
@@ -280,8 +301,10 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dot_split_kernel(DotSplitParams
                     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w) : "r"(addr) : "memory");
                     v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
                 }
-                if (!(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))) < INFINITY && v.x + v.y + v.z + v.w == v.x + v.y + v.z + v.w))
-                    v = ds_again(W + (long long)(n0 + n) * P.ldw, P.ldw, P.X + (long long)(t0 + t) * P.ldx, P.K);
+                auto bad = [](float x) { return !(fabsf(x) < INFINITY); };
+                uint32_t again = (bad(v.x) ? 1u : 0u) | (bad(v.y) ? 2u : 0u) | (bad(v.z) ? 4u : 0u) | (bad(v.w) ? 8u : 0u);
+                v.x *= DS_BACK; v.y *= DS_BACK; v.z *= DS_BACK; v.w *= DS_BACK;
+                if (again) v = ds_again(v, again, W + (long long)(n0 + n) * P.ldw, P.ldw, P.X + (long long)(t0 + t) * P.ldx, P.K);
                 return v;
             };
             float4 v = sums(n, P.W);

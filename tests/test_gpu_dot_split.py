@@ -101,3 +101,45 @@ def test_gate_up_pairs(design, T, width, ff):
     got = logits(m, toks)
     assert util.error(got, forward(cfg, {k: v.astype(np.float64) for k, v in w.items()}, toks)) < 4e-5  # (the bar of the other fp32 models)
     m.close()
+
+
+def products(x, w, scale_x=1.0, scale_w=1.0):
+    """x . w^T scaled by powers of two, as a model's logits, and what float64 makes of the very operands: a second model, whose vocabulary has the rows of
+    the identity, shows the normed x bit for bit."""
+    (T, K), eye = x.shape, np.eye(x.shape[1], dtype=np.float32)
+    out = []
+    for embed, gain, toks in ((np.concatenate([eye, x]), 1.0, K + np.arange(T)), (np.concatenate([x, w * np.float32(scale_w)]), scale_x, np.arange(T))):
+        cfg = vu.config([vu.lightning(heads=1, dim=8, vdim=8)], width=K, vocab=len(embed), alpha=1.0, scale=1.0, eps=1e-6)
+        ws = {"embed": embed, "final.norm": np.full(K, gain, np.float32), "l0.norm1": np.ones(K, np.float32), "l0.mix.norm": np.ones(8, np.float32), "l0.mix.o": np.zeros((K, 8), np.float32)}
+        ws.update({"l0.mix." + n: np.zeros((8, K), np.float32) for n in "qkvg"})
+        m = vu.build(cfg, ws, "float32", max_batch=1, max_context=512, max_step_tokens=512)
+        out.append(logits(m, toks).astype(np.float64))
+        m.close()
+    normed = out[0][:, :K] * scale_x
+    return out[1][:, T:], normed @ (w.astype(np.float64) * scale_w).T
+
+
+def rms(got, want):
+    return float(np.sqrt(((got - want) ** 2).mean() / (want ** 2).mean()))
+
+
+@pytest.mark.parametrize("scale_x,scale_w", [(1.0, 2.0 ** -118), (2.0 ** -118, 2.0 ** 20), (2.0 ** -60, 2.0 ** -60), (2.0 ** -20, 2.0 ** 100), (1.0, 2.0 ** 110)])
+@pytest.mark.parametrize("T,K", [(9, 1032), (64, 136)])
+def test_operands_far_from_one(T, K, scale_x, scale_w):
+    """Powers of two change nothing: no part of a small number is lost, and what leaves bf16's range is formed again in fp32.  The bar is that of operands around
+    one, fp32 additions of random signs (1.1e-7 for chains of this length)."""
+    rng = np.random.default_rng(K)
+    x, w = rng.standard_normal((T, K)).astype(np.float32), rng.standard_normal((1024 if T < 33 else 72, K)).astype(np.float32)
+    assert rms(*products(x, w, scale_x, scale_w)) < 1.1e-7
+
+
+def test_a_few_small_numbers_among_others():
+    """A product's rows with numbers of all magnitudes: each result against the sum of its own magnitudes."""
+    rng = np.random.default_rng(8)
+    x, w = rng.standard_normal((40, 136)).astype(np.float32), rng.standard_normal((96, 136)) * 2.0 ** rng.integers(-125, 3, (96, 136))
+    w[:48] *= 2.0 ** -20  # subnormal ones among them
+    w = w.astype(np.float32)
+    got, want = products(x, w)
+    size = np.abs(want).max(axis=0)  # (of a feature)
+    assert np.all(np.abs(got - want).max(axis=0) <= 2.0 ** -21 * size + 2.0 ** -148)
+
