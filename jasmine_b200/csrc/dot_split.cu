@@ -2,24 +2,32 @@
 // weight_net_t::forward (mat_net_t.hpp:38-49) in f32 models.
 //
 // Method.  An fp32 number is the sum of three bf16 numbers, x = h + m + l, each the rest of the one before rounded to 8 bits: 24 bits,
-// nothing is lost.  Of the nine products of two such sums the six largest are taken (the others are below 2^-26 of the product, half an
-// fp32 rounding of it), the smallest first.  The tensor core's running sum is only kept for a block of 64 products; blocks are added in registers,
-// rounded to nearest.  A block of weights whose m or l parts are all zero (weights that came as bf16) leaves those products out: the
-// sums are the same to the bit.
+// nothing is lost (splitting fp32 into bf16 numbers for matrix units: Henry, Tang, Heinecke, "Leveraging the bfloat16 artificial intelligence
+// datatype for higher-precision computations", 2019).  Of the nine products of two such sums the six largest are taken, the smallest first; of the others m l
+// and l m are 2^-25 of the product each at most, l l 2^-34.  The tensor core truncates: an addition to a running sum drops what lies below its
+// last place, always toward zero.  So no large product is ever added to another one there except within one MMA of 16: a block of
+// 64 products has four accumulators, one per step, the first of which also takes all the small products before its large ones; they are added in
+// registers, rounded to nearest, and the ranks of a cluster with what each rounding leaves out.  A block of weights whose m or l parts are all zero
+// (weights that came as bf16) leaves those products out: the sums are the same to the bit.
 //
-// What bounds it.  The fp32 pipe ran at half of its rate at best; 300 tokens, there -> here, us: 1024 x 1024 41 -> 12, 1024 x 2752 59 -> 22, 2752 x 1024
-// 53 -> 20, 8000 x 1024 151 -> 54 (weights that fit bf16: 11, 20, 18, 49); 33 tokens: 1024 x 2752 26 -> 13; 1 token: 8000 x 1024 22 -> 15.
+// Error against 64 bits, rms, fp32 chains -> here: operands of random sign 0.83e-7 -> 0.49e-7 (64 products), 1.05e-7 -> 0.61e-7 (1024), 1.17e-7 ->
+// 0.72e-7 (2752); of one sign 0.48e-7 -> 0.45e-7, 0.52e-7 -> 0.39e-7, 0.49e-7 -> 0.34e-7 (one accumulator per block: 0.95e-7, two: 0.65e-7),
+// and where a CTA adds all blocks of 1024 products by itself 0.64e-7 -> 0.67e-7 (random signs: 1.16e-7 -> 0.89e-7).
+//
+// What bounds it.  The fp32 pipe ran at half of its rate at best; 300 tokens, there -> here, us: 1024 x 1024 41 -> 13, 1024 x 2752 59 -> 24, 2752 x 1024
+// 53 -> 22, 8000 x 1024 151 -> 63 (weights that fit bf16: 12, 22, 20, 56); 33 tokens: 1024 x 2752 26 -> 14; 1 token: 8000 x 1024 22 -> 15.
 // A block of products takes 12 to 24 MMAs, and taking the operands apart is the longer part: about 70 instructions per eight numbers,
-// half of the issue slots, and the latency of the next block's loads behind them (1.0 to 1.4 us a block; twice the warps, or the
+// half of the issue slots, and the latency of the next block's loads behind them (1.0 to 1.6 us a block; twice the warps, or the
 // weights' lines asked into L2 four blocks ahead: 5 to 30 % slower).  So few CTAs share an operand's rows as possible: 128 features and up to
-// 128 tokens per CTA, and a cluster of CTAs shares the products of a tile.
+// 128 tokens per CTA, and a cluster of CTAs shares the products of a tile.  The four accumulators cost 3 to 11 % (300 x 2752 x 1024 in pairs
+// 29.7 -> 32.8): they fill the tensor memory, so a block's MMAs wait until the block before it has been added, which the splitting hides.
 //
 // Roles (512 threads, a whole number of warps per scheduler: 128 registers each): warps 0-7 read fp32 rows, take them apart and write the
 // three planes of a block into shared memory (128-byte swizzle, two stages); warps 8-15 add the blocks' sums (two per quadrant of TMEM
 // lanes, half of the tokens each); warp 8 also issues the MMAs (features are the rows, tokens the columns).
 //
 // Gate and up projections of a feed-forward run as pairs: 64 features' gate and up rows make one tile, and the activation follows where the sums meet (the
-// two products and a launch for the activation, 300 x 2752 x 1024: 43 us, here 32).
+// two products and a launch for the activation, 300 x 2752 x 1024: 43 us, here 33; 38 with weights of 24 bits).
 //
 // Range.  Both operands are scaled by 2^39 on the way in, so that every fp32 number, the subnormal ones too, keeps all its parts, and the sums by 2^-78 on the
 // way out.  What leaves the range then (infinities, NaN, operands above 2^88, sums above 2^49) comes out as no finite number, and every such result is
@@ -113,11 +121,11 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dot_split_kernel(DotSplitParams
     constexpr int FEATURES = PAIRED ? DS_ROWS / 2 : DS_ROWS;
     constexpr int PLANE = ds_plane(BN), STAGE = 3 * PLANE, X_OFF = DS_ROWS * 128;
     constexpr int ROWS_PASS = DS_SPLIT_WARPS * 4, W_ITEMS = DS_ROWS / ROWS_PASS, X_ITEMS = BN / ROWS_PASS, ITEMS = W_ITEMS + X_ITEMS;
-    constexpr uint32_t BUF = BN <= 32 ? 32 : BN <= 64 ? 64 : 128;  // tensor-memory columns between the two accumulators
+    constexpr uint32_t BUF = BN <= 32 ? 32 : BN <= 64 ? 64 : 128;  // tensor-memory columns between the four accumulators
     constexpr int COLS = BN / 2;                                   // columns of an adding warp
     extern __shared__ uint8_t smem_raw[];
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    __shared__ __align__(8) uint64_t full_bar[2], empty_bar[2], acc_full[2], acc_empty[2];
+    __shared__ __align__(8) uint64_t full_bar[2], empty_bar[2], acc_full, acc_empty;
     __shared__ uint32_t w_parts[2][DS_SPLIT_WARPS];  // which of a block's weights have an m part (1), an l part (2)
     __shared__ uint32_t tmem_base_smem;
     __shared__ int abort_flag;
@@ -132,13 +140,13 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dot_split_kernel(DotSplitParams
         for (int s = 0; s < 2; ++s) {
             mbar_init(&full_bar[s], DS_SPLIT_WARPS);
             mbar_init(&empty_bar[s], 1);
-            mbar_init(&acc_full[s], 1);
-            mbar_init(&acc_empty[s], DS_ADD_WARPS);
         }
+        mbar_init(&acc_full, 1);
+        mbar_init(&acc_empty, DS_ADD_WARPS);
         mbar_fence_init();
     }
     if (warp == DS_SPLIT_WARPS) {
-        tmem_alloc(&tmem_base_smem, 2 * BUF);
+        tmem_alloc(&tmem_base_smem, 4 * BUF);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -181,13 +189,13 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dot_split_kernel(DotSplitParams
                 load(i, b + 1);
 #pragma unroll
                 for (int e = 0; e < 8; e += 2) f2_unpack(f2_mul(f2_pack(f[e], f[e + 1]), f2_pack(DS_SCALE, DS_SCALE)), f[e], f[e + 1]);
-                uint4* at = reinterpret_cast<uint4*>(to + (i < W_ITEMS ? i * ROWS_PASS * 128 : X_OFF + (i - W_ITEMS) * ROWS_PASS * 128));
+                uint4* out = reinterpret_cast<uint4*>(to + (i < W_ITEMS ? i * ROWS_PASS * 128 : X_OFF + (i - W_ITEMS) * ROWS_PASS * 128));
                 auto part = [&]() {
                     uint4 h;
                     h.x = ds_part(f[0], f[1]); h.y = ds_part(f[2], f[3]); h.z = ds_part(f[4], f[5]); h.w = ds_part(f[6], f[7]);
                     return h;
                 };
-                at[0] = part();
+                out[0] = part();
                 if (i < W_ITEMS) {
                     // (weights that fit bf16: the parts stay as they are, zero, once they have been cleared)
                     uint32_t rest = 0;
@@ -199,8 +207,8 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dot_split_kernel(DotSplitParams
                     filled = some ? filled | bit : filled & ~bit;
                 }
                 const uint4 m = part(), l = part();
-                at[PLANE / 16] = m;
-                at[2 * (PLANE / 16)] = l;
+                out[PLANE / 16] = m;
+                out[2 * (PLANE / 16)] = l;
                 if (i < W_ITEMS) {
                     any_m |= m.x | m.y | m.z | m.w;
                     any_l |= l.x | l.y | l.z | l.w;
@@ -221,58 +229,60 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dot_split_kernel(DotSplitParams
 #pragma unroll
         for (int j = 0; j < COLS; ++j) acc[j] = 0.0f;
 #pragma unroll 1
-        for (int i0 = 0; i0 <= n; ++i0) {
-            if (warp == DS_SPLIT_WARPS && i0 < n) {  // block i0's products, while the one before it is added
-                const int s = i0 & 1;
-                bool ok = mbar_wait_warp(&full_bar[s], (i0 >> 1) & 1, &abort_flag, P.err, TC_TIMEOUT_FULL);
-                if (ok && i0 >= 2) ok = mbar_wait_warp(&acc_empty[s], ((i0 >> 1) - 1) & 1, &abort_flag, P.err, TC_TIMEOUT_MISC);
+        for (int i = 0; i < n; ++i) {
+            if (warp == DS_SPLIT_WARPS) {
+                const int s = i & 1;
+                bool ok = mbar_wait_warp(&full_bar[s], (i >> 1) & 1, &abort_flag, P.err, TC_TIMEOUT_FULL);
+                if (ok && i > 0) ok = mbar_wait_warp(&acc_empty, (i - 1) & 1, &abort_flag, P.err, TC_TIMEOUT_MISC);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t parts = __reduce_or_sync(0xffffffffu, lane < DS_SPLIT_WARPS ? w_parts[s][lane] : 0u);
                 const uint64_t w = smem_desc_sw128(smem_u32(ring) + s * STAGE), x = smem_desc_sw128(smem_u32(ring) + s * STAGE + X_OFF);
                 if (elect_one()) {
-                    uint32_t add = 0;
-                    auto product = [&](int pw, int px) {
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            mma_ss(tmem + s * BUF, w + (uint64_t)(pw * (PLANE >> 4) + k * 2), x + (uint64_t)(px * (PLANE >> 4) + k * 2), idesc, add);
-                            add = 1;
-                        }
+                    auto mma = [&](int to, int pw, int px, int k, uint32_t add) {
+                        mma_ss(tmem + to * BUF, w + (uint64_t)(pw * (PLANE >> 4) + k * 2), x + (uint64_t)(px * (PLANE >> 4) + k * 2), idesc, add);
                     };
-                    product(0, 2);
-                    if (parts & 2) product(2, 0);
-                    if (parts & 1) product(1, 1);
-                    if (parts & 1) product(1, 0);
-                    product(0, 1);
-                    product(0, 0);
+                    auto product = [&](int pw, int px, uint32_t add) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) mma(0, pw, px, k, k > 0 ? 1u : add);
+                    };
+                    // the first accumulator also takes the small products, before its large ones
+                    product(0, 2, 0);
+                    if (parts & 2) product(2, 0, 1);
+                    if (parts & 1) product(1, 1, 1);
+                    if (parts & 1) product(1, 0, 1);
+                    product(0, 1, 1);
+                    mma(0, 0, 0, 0, 1);
+                    mma(1, 0, 0, 1, 0);
+                    mma(2, 0, 0, 2, 0);
+                    mma(3, 0, 0, 3, 0);
                     mma_commit(&empty_bar[s]);
-                    mma_commit(&acc_full[s]);
+                    mma_commit(&acc_full);
                 }
                 __syncwarp();
             }
-            if (i0 > 0) {
-                const int i = i0 - 1, s = i & 1;
-                if (!mbar_wait_warp(&acc_full[s], (i >> 1) & 1, &abort_flag, P.err, TC_TIMEOUT_ACC)) break;
-                tc_fence_after();
+            if (!mbar_wait_warp(&acc_full, i & 1, &abort_flag, P.err, TC_TIMEOUT_ACC)) break;
+            tc_fence_after();
 #pragma unroll
-                for (int c = 0; c < COLS; c += 16) {
-                    uint32_t r[16];
-                    tmem_ld16(from + s * BUF + c, r);
-                    tmem_ld_wait();
+            for (int c = 0; c < COLS; c += 8) {
+                uint32_t r[4][8];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(r[j]);
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty[s]);
+                for (int q = 0; q < 4; ++q) tmem_ld8(from + q * BUF + c, r[q]);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    acc[c + j] += (__uint_as_float(r[0][j]) + __uint_as_float(r[1][j])) + (__uint_as_float(r[2][j]) + __uint_as_float(r[3][j]));
             }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty);
         }
     }
     tc_fence_before();
     __syncthreads();  // every MMA of this CTA has read its operands (the adding warps waited for the last): the ring is free
     if (warp == DS_SPLIT_WARPS) {
         tc_fence_after();
-        tmem_dealloc(tmem, 2 * BUF);
+        tmem_dealloc(tmem, 4 * BUF);
     }
     if (warp >= DS_SPLIT_WARPS) {
         const int quad = warp & 3, half = (warp - DS_SPLIT_WARPS) >> 2;
@@ -291,16 +301,17 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dot_split_kernel(DotSplitParams
             if (t0 + t >= P.T || n0 + n >= P.N) continue;
             // sums of four rows of the tile, formed again where they are not finite
             auto sums = [&](int row, const float* W) {
-                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 const uint32_t at = smem_u32(ring) + (t * DS_ROWS + row) * 4;
+                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f), lost = v;
 #pragma unroll 4
                 for (int z = 0; z < S; ++z) {
                     uint32_t addr;
                     float4 q;
                     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(at), "r"(z));
                     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w) : "r"(addr) : "memory");
-                    v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
+                    ds_add(v.x, lost.x, q.x); ds_add(v.y, lost.y, q.y); ds_add(v.z, lost.z, q.z); ds_add(v.w, lost.w, q.w);
                 }
+                v.x += lost.x; v.y += lost.y; v.z += lost.z; v.w += lost.w;
                 auto bad = [](float x) { return !(fabsf(x) < INFINITY); };
                 uint32_t again = (bad(v.x) ? 1u : 0u) | (bad(v.y) ? 2u : 0u) | (bad(v.z) ? 4u : 0u) | (bad(v.w) ? 8u : 0u);
                 v.x *= DS_BACK; v.y *= DS_BACK; v.z *= DS_BACK; v.w *= DS_BACK;
@@ -358,8 +369,8 @@ static jsm_status ds_allow() {
 
 // Tokens of a tile and CTAs of a cluster.  A CTA takes a bit more than a microsecond per block, most of it for the 128 rows of weights, and five to
 // seven around its blocks; clusters that do not fit the chip at once wait for the first ones.  300 tokens, tokens of a tile / CTAs of a
-// cluster: 1024 x 2752 96/4 19.9 us, 128/5 20.0, 64/3 22.7, 96/3 24.7, 64/4 (40 clusters, the chip holds 33) 34.8; 4096 x 512 96/1 14.9,
-// 128/1 16.7, 64/1 (160 CTAs) 25.9; 33 tokens: 1024 x 1024 64/8 7.2, 96/8 7.6, 32/6 8.2, 32/8 (16 clusters, the chip holds 15) 11.2.
+// cluster: 1024 x 2752 96/4 24.5 us, 128/5 24.1, 64/3 26.4, 96/3 30.9, 64/4 (40 clusters, the chip holds 33) 40.7; 4096 x 512 96/1 18.6,
+// 128/1 21.4, 64/1 (160 CTAs) 30.5; 33 tokens: 1024 x 1024 64/8 8.3, 96/8 8.8, 32/6 9.1, 32/8 (16 clusters, the chip holds 15) 12.8.
 template <int BN, bool PAIRED>
 static jsm_status ds_shape(int T, int N, int K, float* best, int* bn, int* splits) {
     constexpr float block_us = BN == 32 ? 1.04f : BN == 64 ? 1.13f : BN == 96 ? 1.2f : 1.4f, around_us = BN <= 64 ? 5.2f : BN == 96 ? 5.5f : 6.6f;

@@ -123,6 +123,21 @@ def rms(got, want):
     return float(np.sqrt(((got - want) ** 2).mean() / (want ** 2).mean()))
 
 
+@pytest.mark.parametrize("T,K", [(40, 64), (40, 200), (128, 520), (40, 1024), (128, 2752)])
+@pytest.mark.parametrize("kind", ["positive", "bf16 weights", "mantissas"])
+def test_operands_of_one_sign(kind, T, K):
+    """Nothing cancels: the truncated additions of the tensor core all err to the same side, a quarter to a half of 2^-24 each time an accumulator is
+    finished, and the left-out products m l and l m are 2^-24 of the product together at worst (mantissas just below a bf16 midpoint).  With a rounding
+    or two of 2^-25 on the whole sum that is under 2^-24; the additions of fp32 chains stay between 4.5e-8 and 8e-8 here."""
+    rng = np.random.default_rng(T * K)
+    x, w = np.abs(rng.standard_normal((T, K))).astype(np.float32), np.abs(rng.standard_normal((256, K))).astype(np.float32)
+    if kind == "bf16 weights":
+        w = (w.view(np.uint32) & np.uint32(0xFFFF0000)).view(np.float32)
+    elif kind == "mantissas":
+        x, w = (np.float32(1.00390625 - 2.0 ** -17) * 2.0 ** rng.integers(-1, 2, a.shape) for a in (x, w))
+    assert rms(*products(x.astype(np.float32), w.astype(np.float32))) < 2.0 ** -24
+
+
 @pytest.mark.parametrize("scale_x,scale_w", [(1.0, 2.0 ** -118), (2.0 ** -118, 2.0 ** 20), (2.0 ** -60, 2.0 ** -60), (2.0 ** -20, 2.0 ** 100), (1.0, 2.0 ** 110)])
 @pytest.mark.parametrize("T,K", [(9, 1032), (64, 136)])
 def test_operands_far_from_one(T, K, scale_x, scale_w):
