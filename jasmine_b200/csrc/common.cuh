@@ -68,7 +68,10 @@ int sm_count();
 // predecessor's results.  Rules every kernel launched through launch_chained keeps:
 //   * chain_trigger() first, so that its own successor can be made resident early;
 //   * chain_wait() before the first access (read or write) to anything another kernel of the stream
-//     produces or consumes; it returns once the predecessor grid has completed and its writes are visible.
+//     produces or consumes; it returns once the predecessor grid has completed and its writes are visible;
+//   * the one exception is load_early (below): what no kernel of the running pass writes.  It rests on two things that the host sees to: every
+//     pass ends in a wait for its stream, so that nothing of an earlier pass still runs, and a pass has every sequence once, so that
+//     what lies before a segment's first position was written by earlier passes.
 // Both are no-ops for a kernel launched without the attribute.
 bool chained_launch_enabled();  // JSM_PDL=0 in the environment turns the attribute off (plain stream order)
 

@@ -407,8 +407,8 @@ static size_t la_smem(const LatentDims& d) {
 }
 
 template <int NT>  // KS: 16-wide steps of half the components, at most
-__global__ void __launch_bounds__(256, 1) latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ q_lat, LatentDims d,
-                                                              const __nv_bfloat16* __restrict__ pool, const int32_t* __restrict__ block_table,
+__global__ void __launch_bounds__(256, 1) latent_attn_mma_kernel(const __nv_bfloat16* q_lat, LatentDims d,
+                                                              const __nv_bfloat16* pool, const int32_t* __restrict__ block_table,
                                                               int max_pages, const int32_t* __restrict__ seg_start,
                                                               const int32_t* __restrict__ seg_len, const int32_t* __restrict__ seg_pos0,
                                                               const int32_t* __restrict__ seg_row, const int32_t* __restrict__ tile_seg,
