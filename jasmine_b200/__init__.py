@@ -11,7 +11,9 @@ from __future__ import annotations
 
 import ctypes as C
 import functools
+import importlib
 import os
+import warnings
 from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
@@ -222,12 +224,18 @@ _calls_module = None
 def _calls():
     global _calls_module
     if _calls_module is None:
-        _torch()
-        try:
-            from . import _native as m
-            m.bind(lib()._handle)
-        except ImportError:
-            m = False
+        torch, m = _torch(), False
+        if (PKG_DIR / "_native.so").exists():
+            try:
+                native = importlib.import_module("._native", __name__)
+                built_for = getattr(native, "torch", "of another time")
+                if built_for == f"{torch.__version__} {torch.version.git_version}":
+                    native.bind(lib()._handle)
+                    m = native
+                else:
+                    warnings.warn(f"jasmine_b200: _native.so was built for torch {built_for}: calls go through ctypes until `python -m jasmine_b200.build`")
+            except ImportError as e:
+                warnings.warn(f"jasmine_b200: _native.so does not load, calls go through ctypes: {e}")
         _calls_module = m
     return _calls_module
 

@@ -16,9 +16,9 @@ from __future__ import annotations
 
 import concurrent.futures as cf
 import hashlib
-import importlib.metadata
 import importlib.util
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -73,6 +73,12 @@ def _compile(src: Path, force: bool, verbose: bool) -> Path:
     return obj
 
 
+def _torch_id(torch: Path) -> str:
+    """What a torch says it is, `<version> <revision>`, without importing it."""
+    text = (torch / "version.py").read_text()
+    return " ".join(re.search(rf"^{name}\b[^=\n]*=\s*['\"]([^'\"]*)['\"]", text, re.M)[1] for name in ("__version__", "git_version"))
+
+
 def _build_calls(force: bool) -> None:
     spec = importlib.util.find_spec("torch")
     if spec is None or not spec.submodule_search_locations:
@@ -80,10 +86,11 @@ def _build_calls(force: bool) -> None:
     torch = Path(spec.submodule_search_locations[0])
     nvcc = shutil.which(_nvcc())
     cuda = Path(nvcc).resolve().parents[1] if nvcc else Path("/usr/local/cuda")
-    src = CSRC / "py_calls.cpp"
-    cmd = [os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", "-I" + sysconfig.get_paths()["include"], f"-I{torch}/include", f"-I{torch}/include/torch/csrc/api/include", f"-I{cuda}/include", str(src), "-o", str(CALLS),
+    src, built_for = CSRC / "py_calls.cpp", _torch_id(torch)
+    cmd = [os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", f'-DJSM_TORCH="{built_for}"',
+           "-I" + sysconfig.get_paths()["include"], f"-I{torch}/include", f"-I{torch}/include/torch/csrc/api/include", f"-I{cuda}/include", str(src), "-o", str(CALLS),
            f"-L{torch}/lib", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
-    stamp = hashlib.sha256(" ".join([*cmd, importlib.metadata.version("torch"), sys.version]).encode() + src.read_bytes() + (PKG.parent / "include" / "jasmine_b200.h").read_bytes()).hexdigest()
+    stamp = hashlib.sha256(" ".join([*cmd, sys.version]).encode() + src.read_bytes() + (PKG.parent / "include" / "jasmine_b200.h").read_bytes()).hexdigest()
     stamp_file = OBJ / "py_calls.stamp"
     if not force and CALLS.exists() and stamp_file.exists() and stamp_file.read_text() == stamp:
         return

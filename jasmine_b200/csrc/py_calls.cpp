@@ -208,4 +208,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nu
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__native() { return PyModule_Create(&module); }
+// torch: the torch whose headers this module has been built with, `<version> <revision>`.  The fields of a tensor are read at their places in that one.
+PyMODINIT_FUNC PyInit__native() {
+    PyObject* m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "torch", JSM_TORCH) != 0) Py_CLEAR(m);
+    return m;
+}

@@ -1,5 +1,7 @@
 """The extension module behind the frequent calls of the Python plumbing (csrc/py_calls.cpp): the same results, refusals and exceptions as through ctypes
 for every form of operand, and nothing taken that is not a plain dense CUDA tensor."""
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -19,6 +21,29 @@ def test_what_it_leaves_to_the_python_code():
     assert m.embedding(t, t, None, None, None) is None
     with pytest.raises(TypeError):
         m.bind()
+
+
+def test_a_module_of_another_torch_is_not_used(monkeypatch):
+    m = jb._calls()
+    assert m.torch == f"{torch.__version__} {torch.version.git_version}"
+    monkeypatch.setattr(jb, "_calls_module", None)
+    monkeypatch.setattr(m, "torch", "1.0 0000")
+    with pytest.warns(UserWarning, match="built for torch 1.0"):
+        assert jb._calls() is False
+    assert jb._calls() is False  # (asked once)
+
+
+def test_a_module_that_does_not_load_is_said(monkeypatch):
+    monkeypatch.setattr(jb, "_calls_module", None)
+    monkeypatch.setitem(sys.modules, "jasmine_b200._native", None)
+    with pytest.warns(UserWarning, match="does not load"):
+        assert jb._calls() is False
+
+
+def test_a_module_that_is_not_there_is_no_matter(monkeypatch, tmp_path, recwarn):
+    monkeypatch.setattr(jb, "_calls_module", None)
+    monkeypatch.setattr(jb, "PKG_DIR", tmp_path)
+    assert jb._calls() is False and not recwarn.list
 
 
 def both(monkeypatch, call):
