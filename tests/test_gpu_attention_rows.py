@@ -1,5 +1,6 @@
-"""Attention of prompts in f32 with enough (token, head) rows for the kernel that shares keys between eight of them: edges of its
-tiles of 32 keys and of its eight rows, every mask, against the plain float64 implementation."""
+"""Attention of prompts with enough (token, head) rows for the kernel that shares keys between sixteen of them: edges of its tiles of 32 keys and of its
+sixteen rows (two per warp), every mask, one and two groups of warps, against the plain float64 implementation."""
+import numpy as np
 import pytest
 
 import vagonex_oracle as vo
@@ -27,10 +28,22 @@ def test_rows_that_share_keys(kw, sizes):
 @pytest.mark.parametrize("heads,kv_heads", [(16, 16), (16, 4), (16, 1)])
 def test_a_sink_that_is_switched_off(heads, kv_heads, size):
     """A sink of -inf has no weight, also in a row whose keys all lie in the second group's tiles (a later chunk than that of the rows beside it)."""
-    import numpy as np
     cfg = vu.config([vu.attention(heads=heads, kv_heads=kv_heads, dim=24, vdim=20, rot_dims=8, size=size)], alpha=0.6)
     w, toks = vu.random_weights(cfg, 53), vu.tokens(100, 72, 54)
     w["l0.mix.sink"] = vu.bf16_bits(np.where(np.arange(heads) % 3 == 2, 0.5, -np.inf))
     m = vu.build(cfg, w)
     assert_close(vu.run_portions(m, toks, [100]), vo.forward(cfg, vu.oracle_weights(w), toks), 4e-5)  # (the bar of the other fp32 models)
+    m.close()
+
+
+@pytest.mark.parametrize("dtype,tol", [("float32", 4e-5), ("bfloat16", 0.08)])  # (the bars of the other models of these types)
+@pytest.mark.parametrize("dim,vdim", [(256, 256), (320, 128), (300, 120), (320, 250)])
+@pytest.mark.parametrize("sizes,size", [([75, 76], None), ([100], 33)], ids=str)
+def test_heads_too_wide_for_two_groups(dim, vdim, sizes, size, dtype, tol):
+    """Two tiles of keys and values for each of two groups of warps would not fit in shared memory: one group (bf16 heads up to 256 wide run on the tensor cores)."""
+    cfg = vu.config([vu.attention(heads=16, kv_heads=4, dim=dim, vdim=vdim, rot_dims=32, size=size)], alpha=0.6)
+    w, toks = vu.random_weights(cfg, 55), vu.tokens(sum(sizes), 72, 56)
+    m = vu.build(cfg, w, dtype)
+    got, want = vu.run_portions(m, toks, sizes), vo.forward(cfg, vu.oracle_weights(w), toks)
+    assert vu.error(got, want) < tol
     m.close()

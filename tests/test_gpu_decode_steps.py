@@ -1,6 +1,6 @@
 """Decode steps of the layer-list decoder against float64 at the sizes where their kernels change form: batches around 8 and 16 (the merge of the
-attention's splits inside the projection to values), 16 and 40 heads (one and two tiles of rows), contexts of one to more than four splits,
-sequences whose newest entry opens a page, and prompts for the forms of the convolution."""
+attention's splits inside the projection to values), 16 and 40 heads (one and two tiles of rows), contexts of one to nine splits, with
+fewer and more than four beside one another, sequences whose newest entry opens a page, and prompts for the forms of the convolution."""
 import numpy as np
 import pytest
 
@@ -29,6 +29,30 @@ def test_latent_attention_steps(heads, batch):
         for b in range(batch):
             assert zu.error(lg[b:b + 1], want[b][k:k + 1]) < TOL, (b, lens[b], k)
         assert np.array_equal(nxt, lg.argmax(1))
+    jb.check_device_errors()
+    m.close()
+
+
+@pytest.mark.parametrize("heads,batch,context", [(16, 3, 1100), (16, 9, 1100), (16, 16, 1100), (40, 5, 1100), (16, 1, 4160), (3, 2, 4160)])
+def test_latent_attention_steps_of_many_splits(heads, batch, context):
+    """Up to nine splits of two pages and more for tokens of both groups of eight, next to tokens of one to four; 33 splits and more of a long context (the merge's
+    weights are formed in groups of 32).  The oracle's logits of the last tokens, whose keys are the whole window."""
+    window = context - 60
+    cfg = zu.config([zu.attention(heads=heads, dim=40, rot_dim=16, vdim=24, kv_rank=72, window=window)], width=64)
+    w = zu.random_weights(cfg, heads * batch)
+    longest = context - 8
+    lens = [(longest, 70, 130, longest // 2, 257, 63, longest - 65, 520)[b % 8] - b // 8 for b in range(batch)]
+    seqs = [zu.tokens(n + 3, cfg["vocab"], 11 * n + b) for b, n in enumerate(lens)]
+    want = [zo.forward(cfg, zu.oracle_weights(w), s)[-3:] for s in seqs]
+    m = zu.build(cfg, w, "bfloat16", max_batch=batch, max_context=context, max_step_tokens=2048)
+    rows = [m.open() for _ in seqs]
+    for r, s, n in zip(rows, seqs, lens):
+        m.step([(r, s[:n])], [n - 1])
+    nxt, lg = np.empty(batch, np.int32), np.empty((batch, cfg["vocab"]), np.float32)
+    for k in range(3):
+        m.step_active(np.array([s[n + k] for s, n in zip(seqs, lens)], np.int32), nxt, lg)
+        for b in range(batch):
+            assert zu.error(lg[b:b + 1], want[b][k:k + 1]) < TOL, (b, lens[b], k)
     jb.check_device_errors()
     m.close()
 
