@@ -201,7 +201,17 @@ JSM_FAST(attn_decode) {  // q, pool, block_table, context_lens, Hq, Hkv, D, max_
     });
 }
 
-#define JSM_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
+// torch throws for tensors that keep their memory to themselves (sizes or addresses that are not to be read): the Python code meets the same and raises
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyObject* guarded(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+    try {
+        return F(self, a, n);
+    } catch (...) {
+        Py_RETURN_NONE;
+    }
+}
+
+#define JSM_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&guarded<name>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {JSM_METHOD(bind), JSM_METHOD(eval_elementwise), JSM_METHOD(eval_rows), JSM_METHOD(dot_f32), JSM_METHOD(embedding),
                          JSM_METHOD(attn_prefill), JSM_METHOD(attn_decode), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -129,3 +129,16 @@ def test_the_current_stream_is_taken():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.allclose(out, a @ b, atol=1e-3)
+
+
+@pytest.mark.gpu
+def test_a_tensor_that_keeps_its_address_raises():
+    """An exception of torch inside the module is the Python code's to raise, not the end of the process."""
+    closed = torch.randn(8, 8, device="cuda")
+    torch._C._set_throw_on_mutable_data_ptr(closed)
+    a, out, ids = torch.randn(8, 8, device="cuda"), torch.empty(8, 8, device="cuda"), torch.zeros(8, dtype=torch.int32, device="cuda")
+    for call in (lambda: jb.dot_f32(a, closed, out), lambda: jb.dot_f32(closed, a, out), lambda: jb.eval_elementwise(LEAF, [closed], out),
+                 lambda: jb.eval_rows(jb.ROWS_SOFTMAX, 1, LEAF, [a], closed), lambda: jb.embedding(closed, ids), lambda: jb.attn_prefill(closed, a, a, 1, 1, 1, 8)):
+        with pytest.raises(RuntimeError, match="data pointer"):
+            call()
+    assert torch.allclose(jb.dot_f32(a, a, out), a @ a, atol=1e-4)
