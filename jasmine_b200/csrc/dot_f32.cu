@@ -275,9 +275,11 @@ bool dot_f32_splits(const void* X, long long ldx, const void* W, long long ldw, 
 }
 
 // C = A . B in fp32 without the reference's order (operands as in jsm_dot_f32, checked by the caller).  Rows of aligned fours go to the tensor cores
-// (dot_split.cu) from 33 rows of A on, and below that from a million weights on: with fewer their start and end cost more than the products
-// (8 rows, here / there, us: 512 x 512 4.0 / 4.5, 256 x 1024 5.1 / 5.5, 1024 x 1024 7.0 / 6.7, 4096 x 512 9.0 / 7.6, 2752 x 1024 13.5 / 8.9; 32 rows:
-// 512 x 512 4.9 / 5.0, 2752 x 1024 21.5 / 9.5; 33 rows, in the 64 x 64 tiles that this kernel had for them: 64 x 64 7.7 / 3.6, 512 x 512 6.5 / 5.1).
+// (dot_split.cu) from 33 rows of A on, and below that from a million weights on.  The line lies between what a launch takes by itself and what it takes
+// in a chain, where its start lies behind its predecessor (us, here / there; by itself, then back to back: 8 rows, 512 x 512 5.0 / 7.5, 6.2 / 5.4; 1024 x
+// 1024 7.4 / 8.5, 8.2 / 7.2; 4096 x 512 9.3 / 8.5, 10.3 / 7.7; 2752 x 1024 13.9 / 9.8, 15.5 / 9.4; 32 rows, 512 x 512 5.8 / 7.7, 6.2 / 5.8; 1024 x 1024
+// 8.8 / 8.9, 10.3 / 7.7; 2752 x 1024 21.6 / 10.4, 22.6 / 9.8; weights of 24 bits).  33 rows, in the 64 x 64 tiles that this kernel had for them, back to
+// back: 64 x 64 7.7 / 4.1, 512 x 512 6.5 / 5.9.
 // The others take 16 x 64 tiles, whose products are shared by as many CTAs as even out the multiprocessors' loads: rounds of
 // CTAs times blocks of products each, and about four blocks' time for a CTA's start and end.
 jsm_status dot_f32_launch(const jsm_mat& A, const jsm_mat& B, const jsm_mat& Cm, cudaStream_t st) {

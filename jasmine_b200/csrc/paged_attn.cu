@@ -761,7 +761,9 @@ jsm_status attn_paged_launch(bool f32, const AttnDims& d, const AttnWeights& w, 
     if (tl.n_tiles <= 0 || tl.t_count <= 0) return JSM_OK;
     const float* gates = d.gated ? gate : nullptr;
     if (f32 || !attn_mma_usable(d)) {
-        // rows in groups once they would make a CTA of eight for every multiprocessor; a few rows keep a CTA each
+        // Rows in groups of sixteen from eight per multiprocessor on; fewer keep a CTA each.  At the line the groups are far ahead, although only half of the
+        // multiprocessors get one (us, groups / a CTA per row: 149 tokens of 8 heads of 128 21 / 56, 75 of 16 heads of 64 13 / 26, 297 of 4 heads of 32
+        // 26 / 72; 297 tokens of 8 heads of 128 36 / 134).
         if (tk.max_len > 1 && d.vdim <= 256 && ar_smem(d, 1) <= AR_MAX_SMEM && (long long)tl.t_count * d.H >= 8ll * sm_count())
             return f32 ? rows_sized<float>(d, w, cache, tk, tl, q, gates, out, st) : rows_sized<__nv_bfloat16>(d, w, cache, tk, tl, q, gates, out, st);
         const size_t smem = sizeof(float) * (pad8(d.dim) + pad8(d.vdim) + 128 + 8);

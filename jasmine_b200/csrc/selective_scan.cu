@@ -447,9 +447,9 @@ __global__ void __launch_bounds__(SC_THREADS, sizeof(T) == 2 && NS == 2 ? 4 : 0)
 // instructions per state and one exchange per eight tokens and channel; and four warps that do nothing else walk the tokens,
 // one per scheduler, the decays of a token computed while the one before it moves the state.  Four more warps bring the
 // tiles, make the step sizes of the next one and write the outputs of the last one meanwhile.  A CTA owns 64 channels.
-// 2048 tokens, 16 states, 8192 channels: 219 -> 131 us (scan_kernel 186, where addresses with constant strides and states kept as pairs save a
-// seventh); the exponential units are then 77 % in use on the 128 SMs that have a CTA.  Eight walking warps of four states
-// 148 us, eight warps beside the walking ones 156; 2 CTAs per SM are named because the compiler then takes 126 registers, without that 66 (165 us).
+// 2048 tokens, 16 states, 8192 channels: 224 -> 139 us with cold caches (scan_kernel 194, where addresses with constant strides and states kept as pairs save a
+// seventh); the exponential units are then three quarters in use on the 128 SMs that have a CTA.  With sums in an order of their own, warm 131 us: eight walking warps of
+// four states 148 us, eight warps beside the walking ones 156; 2 CTAs per SM are named because the compiler then takes 126 registers, without that 66 (165 us).
 constexpr int SW_CH = 64, SW_SUB = 2, SW_NS = 8, SW_HELP = 128, SW_MAIN = SW_CH * SW_SUB, SW_THREADS = SW_MAIN + SW_HELP, SW_YP = SW_CH + 4;
 struct ScanWideTile {  // a tile as it arrives
     __nv_bfloat16 x[SC_TT][SW_CH], z[SC_TT][SW_CH];
@@ -860,9 +860,9 @@ static jsm_status scan_wide_go(const ScanArgs& a, cudaStream_t st) {
 // the smallest instance whose threads hold a channel's states
 template <typename T>
 static jsm_status scan_dispatch(const ScanArgs& a, cudaStream_t st) {
-    // Two blocks of scan_kernel fit beside one another on an SM without slowing each other down much (2048 tokens, scan_kernel / scan_wide_kernel, us:
-    // 128 blocks 107 / 129, 256 blocks 127 / 130, 384 blocks 156 / 131, 512 blocks 186 / 131; 64 tokens, 256 blocks 8.1 / 8.1, 512 blocks 10.4 / 8.9;
-    // the figures of 384 and 512 blocks before the register target above).
+    // Two blocks of scan_kernel fit beside one another on an SM without slowing each other down much (2048 tokens, scan_kernel / scan_wide_kernel, us with
+    // cold caches: 128 blocks 109 / 132, 256 blocks 131 / 134, 296 blocks 132 / 134, 300 blocks 158 / 135, 384 blocks 160 / 137, 512 blocks 194 / 139; 300
+    // tokens: 296 blocks 24.5 / 25.3, 304 blocks 28.2 / 25.1; 64 tokens: 296 blocks 9.3 / 9.8, 304 blocks 10.3 / 10.2, 512 blocks 11.9 / 10.4).
     if constexpr (sizeof(T) == 2)
         if (a.state > 8 && a.state <= 16 && (long long)((a.ip + SC_CH - 1) / SC_CH) * a.n_segs > 2ll * sm_count()) return scan_wide_go(a, st);
     return a.state <= 8 ? scan_go<T, 1>(a, st) : a.state <= 16 ? scan_go<T, 2>(a, st) : a.state <= 24 ? scan_go<T, 3>(a, st)
